@@ -18,9 +18,15 @@
 
 #include <algorithm>
 #include <cfloat>
+#include <cmath>
 #include <cstdlib>
+#include <cstring>
+
+#include <map>
+#include <string>
 
 #include "gb_common.cuh"
+#include "gb_dfr.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -508,6 +514,295 @@ __global__ void __launch_bounds__(128) k_constrain_cl(ConArgs A, const ClusterTa
   }
 }
 
+// ------------------------------------ clusters of at most 3 constraints, in scalars
+// The Jacobi sweeps of a small cluster only ever move its atoms along the cluster's own
+// (fixed) bond vectors b_i, so the state of a cluster is one scalar per constraint, t_i
+// = M_i/2 * sum(gamma_i) (SHAKE) or sum(b_i . dv) (RATTLE), M_i = amt_i + amt_j:
+//   bond     d_c = u_c + sum_i K_ci b_i t_i,    K_ci = (s_ai amt_a - s_bi amt_b) / M_i, (a, b) the ends of c
+//   atom     x_a = x_a(0) + sum_i W_ai b_i t_i,  W_ai = s_ai amt_a / M_i, s_ai = -1 / +1 / 0 (i end, j end, neither)
+//   SHAKE    t_c += q_c / (2 p_c), q_c = |d_c|^2 - d0_c^2 a quadratic in t, p_c = b_c . d_c linear in t
+//   RATTLE   t_c += g_c, g_c = b_c . (v_a - v_b) linear in t
+// (constraints.F90:898-969 and 687-742 written in these variables; the sweeps, their tests
+// and their number are the same).  The polynomials' constants are formed once per cluster
+// and a sweep is double-float arithmetic on the FP32 pipes: |q| is a difference from
+// |u|^2 - d0^2 (FP64) by terms of the size of the correction, so it is as exact as the FP64
+// form's, whose coordinates carry the rounding of the box's size (7e-15 A at 50 A).
+// An FP64 instruction takes 16 issue slots of an SM sub-partition here: the FP64 form of
+// the sweep (~110 FP64 instructions with 3 divisions, k_constrain_cl) took 0.83 ms a call
+// for 32,768 waters (~67 sweeps) and 0.52 ms for 2,197; the scalar form takes 0.133 (SHAKE)
+// and 0.055 ms (RATTLE), and 0.090 and 0.043 ms, bound by FP32 issue at two warps per
+// scheduler and by the dependent operations of a sweep.
+// Sweeps run in chunks of CS_CHUNK between grid barriers; a cluster keeps the scalars of
+// the chunk's start and repeats the chunk's committed sweeps once the last one is known.
+constexpr int CS_THREADS = 64, CS_CHUNK = 16, CS_MAXC = 3;
+
+struct ClKind {        // clusters with equal masses, lengths and topology share one
+  int na, nc;
+  int li[CS_MAXC], lj[CS_MAXC];         // local ends of the constraints
+  float2 K[CS_MAXC][CS_MAXC];           // double-float
+  float2 tol_s[CS_MAXC], tol_r;         // bounds on |q| (2 tol d0) and |g| (2 tol / tstep)
+  double W[CL_MAXA][CS_MAXC];
+  double d0sq[CS_MAXC];
+  double two_m[CS_MAXC];                // gamma sum = two_m * t (SHAKE)
+  double wh[CL_MAXA];                   // weight / hstep, 0: frozen
+};
+
+// double to double-float by integer operations (an FP64 conversion would take the FP64
+// unit): the top 24 bits, then the other 29; 0 below 2^-60, infinite above 2^100
+__device__ __forceinline__ df dbl_split(double v) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  const unsigned h = (unsigned)(b >> 32), l = (unsigned)b, s = h & 0x80000000u;
+  const int e = (int)((h >> 20) & 0x7FFu) - 1023;
+  if (e < -60) return df_make(0.f, 0.f);
+  if (e > 100) return df_make(__uint_as_float(s | 0x7F800000u), 0.f);
+  const float hi = __uint_as_float(s | ((unsigned)(e + 127) << 23) | ((h & 0xFFFFFu) << 3) | (l >> 29));
+  const float lo = __uint2float_rn(l & 0x1FFFFFFFu) * __uint_as_float((unsigned)(e - 52 + 127) << 23);
+  return quick_two_sum(hi, __uint_as_float(__float_as_uint(lo) ^ s));
+}
+
+__device__ __forceinline__ df df_of(float2 a) { return df_make(a.x, a.y); }
+
+__device__ __forceinline__ df df_dot(const df (&a)[3], const df (&b)[3]) {
+  dacc s = {0.f, 0.f};
+  dacc_add_prod(s, a[0], b[0]);
+  dacc_add_prod(s, a[1], b[1]);
+  dacc_add_prod(s, a[2], b[2]);
+  return quick_two_sum(s.s, s.c);
+}
+
+// |a| < b; false for NaN
+__device__ __forceinline__ bool df_abs_less(df a, float2 b) {
+  const bool neg = a.hi < 0.f;
+  const float h = neg ? -a.hi : a.hi, l = neg ? -a.lo : a.lo;
+  return h < b.x || (h == b.x && l < b.y);
+}
+
+struct ClPoly {
+  df c0[CS_MAXC], l[CS_MAXC][CS_MAXC], q[CS_MAXC][6];  // q_c or g_c (l only)
+  df p0[CS_MAXC], p[CS_MAXC][CS_MAXC];                 // p_c
+};
+
+template <bool RATTLE>
+__device__ __forceinline__ void cs_setup(const ConArgs& A, const ClusterTab& T, const ClKind& D, long long quarter,
+                                         ClPoly& P) {
+  df b[CS_MAXC][3], u[CS_MAXC][3], B[CS_MAXC][CS_MAXC], K[CS_MAXC][CS_MAXC];
+#pragma unroll
+  for (int c = 0; c < CS_MAXC; ++c) {
+#pragma unroll
+    for (int k = 0; k < 3; ++k) b[c][k] = u[c][k] = df_make(0.f, 0.f);
+    P.c0[c] = df_make(0.f, 0.f);
+    if (c < D.nc) {
+      const int k = T.con[c], i = T.atom[D.li[c]], j = T.atom[D.lj[c]];
+      double bx = A.dxx[k], by = A.dyy[k], bz = A.dzz[k];
+      if (RATTLE) {
+        const double b2 = bx * bx + by * by + bz * bz;
+        double r = rsqrt_seeded(b2);
+        r = r * fma(-0.5 * b2 * r, r, 1.5);
+        bx *= r; by *= r; bz *= r;
+      }
+      b[c][0] = dbl_split(bx); b[c][1] = dbl_split(by); b[c][2] = dbl_split(bz);
+      if (RATTLE) {
+        const double dx = A.vx[i] - A.vx[j], dy = A.vy[i] - A.vy[j], dz = A.vz[i] - A.vz[j];
+        P.c0[c] = dbl_split(bx * dx + by * dy + bz * dz);
+      } else {
+        const double dx = image_short(A.x[i] - A.x[j], quarter, A.c0, A.a0);
+        const double dy = image_short(A.y[i] - A.y[j], quarter, A.c0, A.a0);
+        const double dz = image_short(A.z[i] - A.z[j], quarter, A.c0, A.a0);
+        u[c][0] = dbl_split(dx); u[c][1] = dbl_split(dy); u[c][2] = dbl_split(dz);
+        P.c0[c] = dbl_split(dx * dx + dy * dy + dz * dz - D.d0sq[c]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < CS_MAXC; ++k) K[c][k] = df_of(D.K[c][k]);
+  }
+#pragma unroll
+  for (int c = 0; c < CS_MAXC; ++c)
+#pragma unroll
+    for (int k = c; k < CS_MAXC; ++k) B[c][k] = B[k][c] = df_dot(b[c], b[k]);
+#pragma unroll
+  for (int c = 0; c < CS_MAXC; ++c) {
+    int m = 0;
+#pragma unroll
+    for (int k = 0; k < CS_MAXC; ++k) {
+      P.p[c][k] = df_mul(K[c][k], B[c][k]);
+      if (RATTLE) {
+        P.l[c][k] = P.p[c][k];
+        continue;
+      }
+      const df w = df_mul(K[c][k], df_dot(u[c], b[k]));
+      P.l[c][k] = df_make(2.f * w.hi, 2.f * w.lo);
+#pragma unroll
+      for (int n = k; n < CS_MAXC; ++n, ++m) {
+        const df e = df_mul(df_mul(K[c][k], K[c][n]), B[k][n]);
+        const float f = n == k ? 1.f : 2.f;
+        P.q[c][m] = df_make(f * e.hi, f * e.lo);
+      }
+    }
+    if (!RATTLE) {
+      P.p0[c] = df_dot(u[c], b[c]);
+      if (c >= D.nc) P.p0[c] = df_make(1.f, 0.f);
+    }
+  }
+}
+
+// one sweep from the scalars t: true when a constraint fails its test; t updated
+template <bool RATTLE>
+__device__ __forceinline__ bool cs_sweep(const ClKind& D, const ClPoly& P, df (&t)[CS_MAXC]) {
+  bool fail = false;
+  df m[6];
+  if (!RATTLE) {
+    int k = 0;
+#pragma unroll
+    for (int i = 0; i < CS_MAXC; ++i)
+#pragma unroll
+      for (int j = i; j < CS_MAXC; ++j, ++k) m[k] = df_mul(t[i], t[j]);
+  }
+  df step[CS_MAXC];
+#pragma unroll
+  for (int c = 0; c < CS_MAXC; ++c) {
+    dacc a = {P.c0[c].hi, P.c0[c].lo};
+#pragma unroll
+    for (int i = 0; i < CS_MAXC; ++i) dacc_add_prod(a, P.l[c][i], t[i]);
+    if constexpr (RATTLE) {
+      step[c] = quick_two_sum(a.s, a.c);
+      if (c < D.nc && !df_abs_less(step[c], D.tol_r)) fail = true;
+    } else {
+#pragma unroll
+      for (int i = 0; i < 6; ++i) dacc_add_prod(a, P.q[c][i], m[i]);
+      const df q = quick_two_sum(a.s, a.c);
+      if (c < D.nc && !df_abs_less(q, D.tol_s[c])) fail = true;
+      dacc e = {P.p0[c].hi, P.p0[c].lo};
+#pragma unroll
+      for (int i = 0; i < CS_MAXC; ++i) dacc_add_prod(e, P.p[c][i], t[i]);
+      const df p = quick_two_sum(e.s, e.c);
+      // 1/p: FP32 reciprocal and the first-order remainder (relative error about 2^-46)
+      const float r = __frcp_rn(p.hi);
+      const float h = __fmaf_rn(-p.lo, r, __fmaf_rn(-p.hi, r, 1.f));
+      const df s = df_mul(q, df_make(r, r * h));
+      step[c] = df_make(0.5f * s.hi, 0.5f * s.lo);
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < CS_MAXC; ++c) t[c] = df_add(t[c], step[c]);
+  return fail;
+}
+
+// SHAKE with its epilogue (apply_shake: v += dr/dt, f += dr/dt m/(dt/2)) or RATTLE.  tbuf: the
+// scalars between chunks when a thread has several clusters (ncl > threads), 2 x 3 per cluster.
+template <bool RATTLE>
+__global__ void __launch_bounds__(CS_THREADS) k_constrain_small(ConArgs A, const ClusterTab* __restrict__ tabs,
+                                                               const int* __restrict__ kind_of,
+                                                               const ClKind* __restrict__ kinds, int ncl,
+                                                               float2* __restrict__ tbuf, double rstep, double* fx,
+                                                               double* fy, double* fz) {
+  cg::grid_group grid = cg::this_grid();
+  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
+  const int nth = gridDim.x * blockDim.x;
+  const long long quarter = __double_as_longlong(0.25 * A.c0);
+  const bool multi = ncl > nth;
+  ClPoly P;
+  df t[CS_MAXC], tb[CS_MAXC];
+#pragma unroll
+  for (int c = 0; c < CS_MAXC; ++c) t[c] = tb[c] = df_make(0.f, 0.f);
+  int it0 = 0, nfinal = -1, last = 0;
+  for (int ch = 0;; ++ch) {
+    unsigned bad = 0;
+    const int n = min(CS_CHUNK, A.maxit - it0);
+    for (int cl = tid; cl < ncl; cl += nth) {
+      const ClKind& D = kinds[kind_of[cl]];
+      if (multi || it0 == 0) cs_setup<RATTLE>(A, tabs[cl], D, quarter, P);
+#pragma unroll
+      for (int c = 0; c < CS_MAXC; ++c) {
+        if (multi) t[c] = it0 ? df_of(tbuf[(size_t)(2 * c) * ncl + cl]) : df_make(0.f, 0.f);
+        tb[c] = t[c];
+        if (multi) tbuf[(size_t)(2 * c + 1) * ncl + cl] = make_float2(t[c].hi, t[c].lo);
+      }
+      for (int s = 0; s < n; ++s)
+        if (cs_sweep<RATTLE>(D, P, t)) bad |= 1u << s;
+      if (multi) {
+#pragma unroll
+        for (int c = 0; c < CS_MAXC; ++c) tbuf[(size_t)(2 * c) * ncl + cl] = make_float2(t[c].hi, t[c].lo);
+      }
+    }
+    bad = __reduce_or_sync(0xffffffffu, bad);
+    if (bad && (threadIdx.x & 31) == 0) atomicOr(&A.flags[ch], (int)bad);
+    grid.sync();
+    const unsigned f = ~(unsigned)__ldcg(&A.flags[ch]) & ((n == 32) ? 0xffffffffu : (1u << n) - 1u);
+    last = n;  // committed sweeps of this chunk: all, or those before the first that nobody failed
+    if (f) {
+      last = __ffs((int)f) - 1;
+      nfinal = it0 + last + 1;
+      break;
+    }
+    if (it0 + n >= A.maxit) break;
+    it0 += n;
+  }
+  if (tid == 0) {
+    (RATTLE ? A.sc->rattle_iters : A.sc->shake_iters) = nfinal > 0 ? nfinal : A.maxit;
+    if (nfinal < 0) A.sc->status |= RATTLE ? ST_RATTLE_FAIL : ST_SHAKE_FAIL;
+  }
+  double st[6] = {0, 0, 0, 0, 0, 0};
+  for (int cl = tid; cl < ncl; cl += nth) {
+    const ClusterTab& T = tabs[cl];
+    const ClKind& D = kinds[kind_of[cl]];
+    if (multi) {
+      cs_setup<RATTLE>(A, T, D, quarter, P);
+#pragma unroll
+      for (int c = 0; c < CS_MAXC; ++c) tb[c] = df_of(tbuf[(size_t)(2 * c + 1) * ncl + cl]);
+    }
+    for (int s = 0; s < last; ++s) cs_sweep<RATTLE>(D, P, tb);
+    double tt[CS_MAXC], b[CS_MAXC][3];
+#pragma unroll
+    for (int c = 0; c < CS_MAXC; ++c) {
+      tt[c] = b[c][0] = b[c][1] = b[c][2] = 0.0;
+      if (c >= D.nc) continue;
+      const int k = T.con[c];
+      tt[c] = df_to_double(tb[c]);
+      b[c][0] = A.dxx[k]; b[c][1] = A.dyy[k]; b[c][2] = A.dzz[k];
+      if (RATTLE) {
+        const double b2 = b[c][0] * b[c][0] + b[c][1] * b[c][1] + b[c][2] * b[c][2];
+        double r = rsqrt_seeded(b2);
+        r = r * fma(-0.5 * b2 * r, r, 1.5);
+        tt[c] *= r;  // unit bond vectors
+      } else {
+        const double g = D.two_m[c] * tt[c];
+        const double gx = g * b[c][0], gy = g * b[c][1], gz = g * b[c][2];
+        st[0] -= gx * b[c][0]; st[1] -= gx * b[c][1]; st[2] -= gx * b[c][2];
+        st[3] -= gy * b[c][1]; st[4] -= gy * b[c][2]; st[5] -= gz * b[c][2];
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < CL_MAXA; ++a) {
+      if (a >= D.na || __double_as_longlong(D.wh[a]) == 0) continue;
+      double dx = 0.0, dy = 0.0, dz = 0.0;
+#pragma unroll
+      for (int c = 0; c < CS_MAXC; ++c) {
+        const double w = D.W[a][c];
+        if (__double_as_longlong(w) == 0) continue;
+        const double f = w * tt[c];
+        dx = fma(f, b[c][0], dx); dy = fma(f, b[c][1], dy); dz = fma(f, b[c][2], dz);
+      }
+      const int i = T.atom[a];
+      if (RATTLE) {
+        A.vx[i] += dx; A.vy[i] += dy; A.vz[i] += dz;
+      } else {
+        const double x0 = A.x[i], y0 = A.y[i], z0 = A.z[i];
+        const double x1 = x0 + dx, y1 = y0 + dy, z1 = z0 + dz;
+        A.x[i] = x1; A.y[i] = y1; A.z[i] = z1;
+        const double ux = (x1 - x0) * rstep, uy = (y1 - y0) * rstep, uz = (z1 - z0) * rstep;
+        A.vx[i] += ux; A.vy[i] += uy; A.vz[i] += uz;
+        fx[i] += ux * D.wh[a]; fy[i] += uy * D.wh[a]; fz[i] += uz * D.wh[a];
+      }
+    }
+  }
+  if (!RATTLE) {
+    dfr sd[6];
+#pragma unroll
+    for (int k = 0; k < 6; ++k) sd[k] = to_dfr(dbl_split(st[k]));
+    block_reduce_store<6>(sd, A.blk);
+  }
+}
+
 // apply_shake epilogue: v += dr/dt, f += dr/dt * m/(dt/2) for constrained atoms
 __global__ void k_shake_post(int n, const int* astart, const int* lfrzn, double rstep, double hstep, const double* w,
                              const double* x, const double* y, const double* z, const double* ox, const double* oy,
@@ -535,7 +830,12 @@ double* d_clring = nullptr;  // per-cluster state ring (CL_RING slots of CL_SLOT
 double* d_clgsum = nullptr;  // per-cluster committed SHAKE gamma sums
 int n_clusters = 0, coop_blocks_cl = 0;
 constexpr int CL_THREADS = 128;  // small blocks spread the clusters over every SM
-const void* cl_kernel = nullptr;  // k_constrain_cl instantiation for the largest cluster
+// clusters of at most 3 constraints (k_constrain_small)
+int* d_clkind = nullptr;     // kind of each cluster
+ClKind* d_kinds = nullptr;
+float2* d_clt = nullptr;     // scalars between chunks, when there are more clusters than resident threads
+bool cl_small = false;
+int coop_blocks_small = 0;
 
 // connected constraint clusters; false when one exceeds CL_MAXA atoms or CL_MAXC constraints
 bool build_clusters(const std::vector<int>& ci, const std::vector<int>& cj, std::vector<ClusterTab>& out) {
@@ -594,6 +894,64 @@ bool build_clusters(const std::vector<int>& ci, const std::vector<int>& cj, std:
   return true;
 }
 
+// Kinds of the clusters for k_constrain_small; false when a cluster has more than 3
+// constraints, a constraint has no movable end (its gamma divides by zero) or a length
+// that reaches the range where the minimum image of a moving bond can change.
+bool build_kinds(const std::vector<ClusterTab>& tabs, const std::vector<double>& d0, std::vector<int>& kind_of,
+                 std::vector<ClKind>& kinds) {
+  std::vector<double> w(g.natms);
+  std::vector<int> frz(g.natms);
+  GB_CUDA(cudaMemcpy(w.data(), g.weight, sizeof(double) * g.natms, cudaMemcpyDeviceToHost));
+  GB_CUDA(cudaMemcpy(frz.data(), g.lfrzn, sizeof(int) * g.natms, cudaMemcpyDeviceToHost));
+  const double dt = g.p.tstep, tol = g.p.shake_tol;
+  auto split = [](double v) {
+    float2 r;
+    df_split(v, &r.x, &r.y);
+    return r;
+  };
+  std::map<std::string, int> seen;
+  kind_of.resize(tabs.size());
+  kinds.clear();
+  for (size_t q = 0; q < tabs.size(); ++q) {
+    const ClusterTab& T = tabs[q];
+    ClKind D;
+    std::memset((void*)&D, 0, sizeof(D));
+    D.na = T.meta & 15;
+    D.nc = (T.meta >> 4) & 15;
+    if (D.nc > CS_MAXC || D.na > CL_MAXA) return false;
+    double iw[CL_MAXA] = {0, 0, 0, 0};  // amt without its power of tstep
+    for (int a = 0; a < D.na; ++a) {
+      const int i = T.atom[a];
+      iw[a] = frz[i] ? 0.0 : 1.0 / w[i];
+      D.wh[a] = frz[i] ? 0.0 : w[i] / (0.5 * dt);
+    }
+    double W[CL_MAXA][CS_MAXC] = {};
+    for (int c = 0; c < D.nc; ++c) {
+      D.li[c] = T.pair[c] & 15;
+      D.lj[c] = T.pair[c] >> 4;
+      const double m = iw[D.li[c]] + iw[D.lj[c]], len = d0[T.con[c]];
+      if (!(m > 0.0) || !std::isfinite(m) || !(len > 0.0 && len < 0.125 * g.cell[0]) || D.li[c] == D.lj[c]) return false;
+      W[D.li[c]][c] -= iw[D.li[c]] / m;
+      W[D.lj[c]][c] += iw[D.lj[c]] / m;
+      D.d0sq[c] = len * len;
+      D.two_m[c] = 2.0 / (m * dt * dt);
+      D.tol_s[c] = split(2.0 * (tol * len));
+    }
+    D.tol_r = split(tol / (0.5 * dt));
+    std::memcpy(D.W, W, sizeof(W));
+    for (int c = 0; c < D.nc; ++c)
+      for (int k = 0; k < D.nc; ++k) D.K[c][k] = split(W[D.li[c]][k] - W[D.lj[c]][k]);
+    const std::string key((const char*)&D, sizeof(D));
+    auto it = seen.find(key);
+    if (it == seen.end()) {
+      it = seen.emplace(key, (int)kinds.size()).first;
+      kinds.push_back(D);
+    }
+    kind_of[q] = it->second;
+  }
+  return true;
+}
+
 }  // namespace
 
 // ===================================================================== host
@@ -643,6 +1001,10 @@ void integ_setup_constraints(const int32_t* listcon, const double* prmcon) {
   if (d_cltab) { cudaFree(d_cltab); d_cltab = nullptr; }
   if (d_clring) { cudaFree(d_clring); d_clring = nullptr; }
   if (d_clgsum) { cudaFree(d_clgsum); d_clgsum = nullptr; }
+  if (d_clkind) { cudaFree(d_clkind); d_clkind = nullptr; }
+  if (d_kinds) { cudaFree(d_kinds); d_kinds = nullptr; }
+  if (d_clt) { cudaFree(d_clt); d_clt = nullptr; }
+  cl_small = false;
   n_clusters = 0;
   const char* env = std::getenv("GB_SHAKE_GLOBAL");
   std::vector<ClusterTab> tabs;
@@ -650,15 +1012,27 @@ void integ_setup_constraints(const int32_t* listcon, const double* prmcon) {
     n_clusters = (int)tabs.size();
     GB_CUDA(cudaMalloc(&d_cltab, sizeof(ClusterTab) * tabs.size()));
     GB_CUDA(cudaMemcpy(d_cltab, tabs.data(), sizeof(ClusterTab) * tabs.size(), cudaMemcpyHostToDevice));
-    GB_CUDA(cudaMalloc(&d_clring, sizeof(double) * CL_RING * CL_SLOT * tabs.size()));
-    GB_CUDA(cudaMalloc(&d_clgsum, sizeof(double) * CL_MAXC * tabs.size()));
-    // rigid 3-site molecules get register arrays sized 3 x 3 (more resident warps)
-    bool small = true;
-    for (const ClusterTab& T : tabs)
-      if ((T.meta & 15) > 3 || ((T.meta >> 4) & 15) > 3) small = false;
-    cl_kernel = small ? (const void*)k_constrain_cl<3, 3> : (const void*)k_constrain_cl<CL_MAXA, CL_MAXC>;
-    GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, cl_kernel, CL_THREADS, 0));
-    coop_blocks_cl = std::max(1, std::min(bps * g.nsm, nblocks(n_clusters, CL_THREADS)));
+    std::vector<int> kind_of;
+    std::vector<ClKind> kinds;
+    // k_constrain_small where it applies (water: 0.83 ms a call in k_constrain_cl)
+    cl_small = build_kinds(tabs, d0, kind_of, kinds);
+    if (cl_small) {
+      GB_CUDA(cudaMalloc(&d_clkind, sizeof(int) * kind_of.size()));
+      GB_CUDA(cudaMemcpy(d_clkind, kind_of.data(), sizeof(int) * kind_of.size(), cudaMemcpyHostToDevice));
+      GB_CUDA(cudaMalloc(&d_kinds, sizeof(ClKind) * kinds.size()));
+      GB_CUDA(cudaMemcpy(d_kinds, kinds.data(), sizeof(ClKind) * kinds.size(), cudaMemcpyHostToDevice));
+      int b0 = 0, b1 = 0;
+      GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b0, k_constrain_small<false>, CS_THREADS, 0));
+      GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_constrain_small<true>, CS_THREADS, 0));
+      coop_blocks_small = std::max(1, std::min(std::min(b0, b1) * g.nsm, nblocks(n_clusters, CS_THREADS)));
+      if ((long long)coop_blocks_small * CS_THREADS < n_clusters)
+        GB_CUDA(cudaMalloc(&d_clt, sizeof(float2) * 2 * CS_MAXC * tabs.size()));
+    } else {
+      GB_CUDA(cudaMalloc(&d_clring, sizeof(double) * CL_RING * CL_SLOT * tabs.size()));
+      GB_CUDA(cudaMalloc(&d_clgsum, sizeof(double) * CL_MAXC * tabs.size()));
+      GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_constrain_cl<CL_MAXA, CL_MAXC>, CL_THREADS, 0));
+      coop_blocks_cl = std::max(1, std::min(bps * g.nsm, nblocks(n_clusters, CL_THREADS)));
+    }
   }
 }
 
@@ -702,6 +1076,18 @@ static void con_args(ConArgs& A) {
   A.flags = d_flags; A.sc = g.sc; A.blk = nullptr;
 }
 
+template <bool RATTLE>
+static void launch_small(ConArgs& A, double rstep) {
+  const ClusterTab* tabs = d_cltab;
+  const int* kind = d_clkind;
+  const ClKind* kinds = d_kinds;
+  int ncl = n_clusters;
+  float2* tbuf = d_clt;
+  double *fx = g.fx, *fy = g.fy, *fz = g.fz;
+  void* args[] = {&A, &tabs, &kind, &kinds, &ncl, &tbuf, &rstep, &fx, &fy, &fz};
+  GB_CUDA(cudaLaunchCooperativeKernel((void*)k_constrain_small<RATTLE>, coop_blocks_small, CS_THREADS, args, 0, g.stream));
+}
+
 // constraints_tags (constraints.F90:438-586): old bond vectors from the current positions
 void integ_con_tags() {
   if (g.ntcons <= 0) return;
@@ -719,21 +1105,25 @@ void integ_shake(int* iters, double* vircon, double* strcon) {
   cudaStream_t st = g.stream;
   const int n = g.natms;
   const double tstep = g.p.tstep, hstep = 0.5 * tstep, rstep = 1.0 / tstep;
-  k_copy3<<<nblocks(n, 256), 256, 0, st>>>(n, g.x, g.y, g.z, g.ox, g.oy, g.oz);
-  GB_LAUNCHED();
+  if (!cl_small) {
+    k_copy3<<<nblocks(n, 256), 256, 0, st>>>(n, g.x, g.y, g.z, g.ox, g.oy, g.oz);
+    GB_LAUNCHED();
+  }
   GB_CUDA(cudaMemsetAsync(d_flags, 0, sizeof(int) * (g.p.shake_maxit + CL_CHUNK + 2), st));
   ConArgs A;
   con_args(A);
-  const int nbs = n_clusters ? coop_blocks_cl : coop_blocks_shake;
+  const int nbs = cl_small ? coop_blocks_small : n_clusters ? coop_blocks_cl : coop_blocks_shake;
   A.blk = gb_blkacc(nbs * 6);
   prof_begin(P_SHAKE);
-  if (n_clusters) {
+  if (cl_small) {
+    launch_small<false>(A, rstep);
+  } else if (n_clusters) {
     const ClusterTab* tabs = d_cltab;
     int ncl = n_clusters, rattle = 0;
     double *ring = d_clring, *gsum = d_clgsum;
     GB_CUDA(cudaMemsetAsync(d_clgsum, 0, sizeof(double) * CL_MAXC * n_clusters, st));
     void* args[] = {&A, &tabs, &ncl, &ring, &gsum, &rattle};
-    GB_CUDA(cudaLaunchCooperativeKernel(cl_kernel, nbs, CL_THREADS, args, 0, st));
+    GB_CUDA(cudaLaunchCooperativeKernel((void*)k_constrain_cl<CL_MAXA, CL_MAXC>, nbs, CL_THREADS, args, 0, st));
   } else {
     void* args[] = {&A};
     GB_CUDA(cudaLaunchCooperativeKernel((void*)k_shake, nbs, 256, args, 0, st));
@@ -741,9 +1131,11 @@ void integ_shake(int* iters, double* vircon, double* strcon) {
   GB_LAUNCHED();
   prof_end(P_SHAKE);
   gb_reduce_blocks(A.blk, nbs, 6, &g.sc->acc[A_STRCON]);
-  k_shake_post<<<nblocks(n, 256), 256, 0, st>>>(n, g.acon_start, g.lfrzn, rstep, hstep, g.weight, g.x, g.y, g.z,
-                                                 g.ox, g.oy, g.oz, g.vx, g.vy, g.vz, g.fx, g.fy, g.fz);
-  GB_LAUNCHED();
+  if (!cl_small) {
+    k_shake_post<<<nblocks(n, 256), 256, 0, st>>>(n, g.acon_start, g.lfrzn, rstep, hstep, g.weight, g.x, g.y, g.z,
+                                                   g.ox, g.oy, g.oz, g.vx, g.vy, g.vz, g.fx, g.fy, g.fz);
+    GB_LAUNCHED();
+  }
   gb_sync_scalars();
   if (iters) *iters = g.hsc->shake_iters;
   const double* s = &g.hsc->acc[A_STRCON];
@@ -763,12 +1155,14 @@ void integ_rattle_launch() {
   ConArgs A;
   con_args(A);
   prof_begin(P_RATTLE);
-  if (n_clusters) {
+  if (cl_small) {
+    launch_small<true>(A, 0.0);
+  } else if (n_clusters) {
     const ClusterTab* tabs = d_cltab;
     int ncl = n_clusters, rattle = 1;
     double *ring = d_clring, *gsum = d_clgsum;
     void* args[] = {&A, &tabs, &ncl, &ring, &gsum, &rattle};
-    GB_CUDA(cudaLaunchCooperativeKernel(cl_kernel, coop_blocks_cl, CL_THREADS, args, 0, st));
+    GB_CUDA(cudaLaunchCooperativeKernel((void*)k_constrain_cl<CL_MAXA, CL_MAXC>, coop_blocks_cl, CL_THREADS, args, 0, st));
   } else {
     void* args[] = {&A};
     GB_CUDA(cudaLaunchCooperativeKernel((void*)k_rattle, coop_blocks_rattle, 256, args, 0, st));

@@ -1,0 +1,66 @@
+"""SHAKE/RATTLE on clusters of every kind that the scalar-form kernel takes (one, two and
+three constraints, frozen atoms), on clusters beyond it, and on more clusters than threads."""
+import numpy as np
+import pytest
+
+from dlpoly_gb300 import systems
+
+pytestmark = pytest.mark.gpu
+
+REL = 1e-9  # the trajectory bar of the other constraint tests
+
+
+def _mixed_clusters(tied):
+    """Water whose molecules keep 3, 2, 1 or no constraints; every 16th has a frozen oxygen.
+    tied: a molecule's oxygen is tied to another one's, a cluster of 4 atoms and 4 constraints."""
+    s = systems.spce_water(8)
+    lc = s.listcon.reshape(-1, 3, 3)
+    keep = {0: (0, 1, 2), 1: (0, 1), 2: (0,), 3: ()}
+    rows = [lc[m, k] for m in range(lc.shape[0]) for k in keep[m % 4]]
+    s.lfrzn = np.zeros(s.natms, np.int32)
+    s.lfrzn[0::3][8::16] = 1
+    frozen = s.lfrzn != 0
+    for v in (s.vx, s.vy, s.vz):
+        v[frozen] = 0.0
+    if tied:
+        o = 3 * 3  # the oxygen of molecule 3 (no constraints of its own), tied to molecule 0
+        pos = np.stack([s.x, s.y, s.z], 1)
+        d = pos[0] - pos[o]
+        d -= s.cell[0] * np.round(d / s.cell[0])
+        s.prmcon = np.append(s.prmcon, np.linalg.norm(d))
+        rows.append(np.array([3, 1, o + 1], np.int32))
+    s.listcon = np.concatenate(rows).astype(np.int32)
+    return s
+
+
+@pytest.mark.parametrize("tied", [False, True])
+def test_cluster_kinds_match_oracle(gpu_lib, oracle_lib, tied):
+    s = _mixed_clusters(tied)
+    out = []
+    for lib in (gpu_lib, oracle_lib):
+        lib.init(s)
+        lib.start()
+        out.append((lib.md_vv(3), lib.download()))
+    (sd, a), (sr, b) = out
+    assert [x.shake_iters for x in sd] == [x.shake_iters for x in sr]
+    assert [x.rattle_iters for x in sd] == [x.rattle_iters for x in sr]
+    for k in ("x", "y", "z", "vx", "vy", "vz"):
+        assert np.abs(a[k] - b[k]).max() <= REL * np.abs(b[k]).max(), k
+    for x, y in zip(sd, sr):
+        cs = np.abs(y.strcon[:]).max()
+        assert np.abs(np.array(x.strcon[:]) - np.array(y.strcon[:])).max() <= 1e-8 * cs
+
+
+def test_more_clusters_than_threads(gpu_lib, monkeypatch):
+    """64,000 molecules: a thread runs several clusters and keeps their scalars between chunks."""
+    s = systems.spce_water(40, kmax=128)
+    out = []
+    for glob in ("1", "0"):
+        monkeypatch.setenv("GB_SHAKE_GLOBAL", glob)
+        gpu_lib.init(s)
+        gpu_lib.start()
+        out.append((gpu_lib.md_vv(1), gpu_lib.download()))
+    (sg, a), (sc, b) = out
+    assert (sg[0].shake_iters, sg[0].rattle_iters) == (sc[0].shake_iters, sc[0].rattle_iters)
+    for k in ("x", "y", "z", "vx", "vy", "vz"):
+        assert np.abs(a[k] - b[k]).max() <= REL * np.abs(a[k]).max(), k
