@@ -438,10 +438,11 @@ int compute_forces(double* eng8, double* stress9, bool do_spme, bool do_real, bo
   return GB_OK;
 }
 
-int do_refresh(int32_t* update) {
+// build_follows: the caller builds the list when *update is set
+int do_refresh(int32_t* update, bool build_follows = false) {
   int upd = integ_vnl_check();
   if (update) *update = upd;
-  if (upd) return list_relocate_and_halo();
+  if (upd) return list_relocate_and_halo(!build_follows);
   return list_refresh_halo();
 }
 
@@ -1069,7 +1070,7 @@ static int md_run_deferred(int nsteps, gb_step_stats* stats) {
     const int32_t upd = integ_vnl_result();
     rebuilt[s] = upd;
     if (upd) {
-      int st = list_relocate_and_halo();
+      int st = list_relocate_and_halo(false);
       if (!st) st = list_build();
       if (st) { g.defer_scalars = false; return st; }
       compute_forces(nullptr, nullptr, true, true, true, nullptr);
@@ -1135,7 +1136,7 @@ int gb_md_run(int nsteps, gb_step_stats* stats) {
       S.shake_iters = it;
       GB_CUDA(cudaEventRecord(g.ev[1], g.stream));
       int32_t upd = 0;
-      int st = do_refresh(&upd);
+      int st = do_refresh(&upd, true);
       if (st) return st;
       S.list_rebuilt = upd;
       if (upd) {

@@ -31,7 +31,7 @@ enum : int {
 // Device-resident scalars: one small block so a single copy returns them all.
 struct DevScalars {
   int nlast;        // local + halo atoms
-  int nlast_prev;   // halo size before the current export direction
+  int nlast_prev;   // the same, as the last relocation left it
   int status;       // ST_* bits
   int ibig;         // largest list length seen (overflow report)
   int update;       // vnl_check decision
@@ -416,7 +416,9 @@ void side_join();                 // the first stream waits for the side stream 
 void run_side_hook();             // enqueue the pending side-stream work (g.side_hook), if any
 
 // module entry points (host)
-int list_relocate_and_halo();     // pbcshift + halo + vnl_set_check (gb_list.cu)
+// pbcshift + halo + vnl_set_check (gb_list.cu); wait = false leaves the halo's status to the
+// list_build that follows
+int list_relocate_and_halo(bool wait = true);
 int list_refresh_halo();          // refresh halo positions (gb_list.cu)
 int list_build();                 // binning + pairs (gb_list.cu)
 void list_setup();                // link-cell geometry (gb_list.cu)

@@ -14,21 +14,26 @@
 #include <cmath>
 #include <cstring>
 
+#include <cooperative_groups.h>
+
 #include "gb_common.cuh"
+
+namespace cg = cooperative_groups;
 
 namespace {
 
-constexpr int SCAN_BLOCK = 1024;
 constexpr int MAX_SBC = 1024;  // semi-ball offsets capacity
 
 __constant__ int c_off[MAX_SBC];   // linear cell offset of each semi-ball cell
 __constant__ int c_nix[MAX_SBC], c_niy[MAX_SBC], c_niz[MAX_SBC];
 __constant__ unsigned char c_nir[MAX_SBC];
-__constant__ unsigned char c_row[MAX_SBC];  // cell-tile row (dy, dz) of each semi-ball cell
-// The semi-ball cells in the reference order form, row by row, runs of consecutive cells
-// along x (contiguous sorted positions); a segment is such a run with one nir flag.
-__constant__ int c_seg_off0[MAX_SBC], c_seg_off1[MAX_SBC];  // linear offsets of its first and last cell
-__constant__ unsigned char c_seg_row[MAX_SBC], c_seg_nir[MAX_SBC];
+// for k_list_tiles, read a lane each: per semi-ball cell its linear offset and
+// (nix + 64) | (niy + 64) << 8 | (niz + 64) << 16 | nir << 24; and, as the semi-ball cells in
+// the reference order form, tile row (dy, dz) by tile row, runs of consecutive cells along x
+// (contiguous sorted positions), per run with one nir flag the linear offsets of its first
+// and last cell, its row and the flag
+__device__ int2 d_sbc[MAX_SBC];
+__device__ int4 d_seg[MAX_SBC];
 
 struct HaloGeom {
   double rc[9];
@@ -47,43 +52,17 @@ struct CellGeom {
 HaloGeom h_halo;
 CellGeom h_cg;
 double h_add[6][3];  // export add vectors for mdir -1,1,-2,2,-3,3
+int h_halo_blocks = 0;  // blocks of k_halo_build (GB_HALO_BLOCKS; 0: by size)
 
 // ---------------------------------------------------------------- kernels
-__global__ void k_pbcshift(int n, double* x, double* y, double* z, double a0, double a4, double a8,
-                           double c0, double c4, double c8, double half_minus) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  double xss = mul_rn(a0, x[i]), yss = mul_rn(a4, y[i]), zss = mul_rn(a8, z[i]);
-  xss = sub_rn(xss, round(xss)); if (xss >= half_minus) xss = -xss;
-  yss = sub_rn(yss, round(yss)); if (yss >= half_minus) yss = -yss;
-  zss = sub_rn(zss, round(zss)); if (zss >= half_minus) zss = -zss;
-  x[i] = mul_rn(c0, xss);
-  y[i] = mul_rn(c4, yss);
-  z[i] = mul_rn(c8, zss);
-}
+// The reduced coordinate rc(d) x + rc(d+3) y + rc(d+6) z of the reference: gb_init takes
+// cubic cells only, whose off-diagonal terms are zero and add nothing.
+__device__ __forceinline__ double red_coord(const double* rc, int d, double xd) { return mul_rn(rc[4 * d], xd); }
 
-__device__ __forceinline__ double red_coord(const double* rc, int d, double x, double y, double z) {
-  return add_rn(add_rn(mul_rn(rc[d], x), mul_rn(rc[d + 3], y)), mul_rn(rc[d + 6], z));
-}
-
-__global__ void k_halo_flags(int n, const double* x, const double* y, const double* z, HaloGeom hg,
-                             int* ixyz, int* src, int* shcode, DevScalars* sc) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i == 0) { sc->nlast = n; sc->nlast_prev = n; }
-  if (i >= n) return;
-  double xx = red_coord(hg.rc, 0, x[i], y[i], z[i]);
-  double yy = red_coord(hg.rc, 1, x[i], y[i], z[i]);
-  double zz = red_coord(hg.rc, 2, x[i], y[i], z[i]);
-  int v = 0;
-  if (xx <= hg.ecw[0]) v += 1;
-  if (xx >= hg.cw[0]) v += 2;
-  if (yy <= hg.ecw[1]) v += 10;
-  if (yy >= hg.cw[1]) v += 20;
-  if (zz <= hg.ecw[2]) v += 100;
-  if (zz >= hg.cw[2]) v += 200;
-  ixyz[i] = v;
-  src[i] = i;
-  shcode[i] = 13;
+// an integer that orders as the double does (an FP64 comparison takes the FP64 unit)
+__device__ __forceinline__ long long ordered(double v) {
+  const long long b = __double_as_longlong(v);
+  return b ^ ((b >> 63) & 0x7fffffffffffffffll);
 }
 
 __device__ __forceinline__ bool export_sel(int v, int kx, int ky, int kz, int jxyz) {
@@ -95,23 +74,170 @@ __device__ __forceinline__ bool export_sel(int v, int kx, int ky, int kz, int jx
   return (j == jxyz) || (j > jxyz && j % 3 == 0);
 }
 
-__global__ void k_export_count(const int* ixyz, const DevScalars* sc, int kx, int ky, int kz, int jxyz,
-                               int* blkcount) {
-  const int n = sc->nlast;
-  const int base = blockIdx.x * SCAN_BLOCK;
-  int cnt = 0;
-  for (int t = threadIdx.x; t < SCAN_BLOCK; t += blockDim.x) {
-    int i = base + t;
-    if (i < n && export_sel(ixyz[i], kx, ky, kz, jxyz)) ++cnt;
+
+// relocate_particles (pbcshift, numerics.F90:1886-1930), set_halo_particles (halo.F90:153-356)
+// and vnl_set_check (neighbours.F90:305-343) in one cooperative launch.  The images come
+// from six ordered exports (-x, +x, -y, +y, -z, +z), each a stable compaction of the atoms
+// and images so far: every block counts its run of them, a grid barrier, every block sums
+// the counts before its own and writes its images, a grid barrier.  The work is a few
+// microseconds; as 28 launches (count, scan, commit and write per export, and the passes
+// around them) it took 0.19 ms at 1,536 atoms and 0.21 ms at 175,616, latency of the
+// launches and of their serial loops; now 0.051 and 0.098 ms, latency of the 12 barriers
+// and of the dependent loads between them.
+constexpr int HALO_NT = 512, HALO_NK = 8;
+struct HaloArgs {
+  int n, mxatms;
+  double *x, *y, *z, *xb, *yb, *zb;
+  double a[3], c[3], half_minus;   // 1/L and L per dimension
+  HaloGeom hg;
+  double add[6][3];
+  int *ixyz, *src, *shcode, *ltg, *ltype, *lfrzn;
+  double *chge, *weight;
+  int* cnt;                        // one count per block and export
+  DevScalars* sc;
+};
+
+__device__ __forceinline__ double wrap1(double x, double a, double c, double half_minus) {
+  double s = mul_rn(a, x);
+  // |s| below half_minus (its bits): round(s) = 0
+  if ((__double_as_longlong(s) & 0x7fffffffffffffffll) >= __double_as_longlong(half_minus)) {
+    s = sub_rn(s, round(s));
+    if (s >= half_minus) s = -s;
   }
-  cnt = warp_sumi(cnt);
-  __shared__ int s[32];
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = cnt;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int tot = 0;
-    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) tot += s[w];
-    blkcount[blockIdx.x] = tot;
+  return mul_rn(c, s);
+}
+
+__global__ void __launch_bounds__(HALO_NT) k_halo_build(HaloArgs A) {
+  cg::grid_group grid = cg::this_grid();
+  const int nth = gridDim.x * blockDim.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  constexpr int NW = HALO_NT / 32, NK = HALO_NK;
+  __shared__ int s_w[NK * NW], s_tot[2];  // selected per sub-run of 512 and warp, then their exclusive sums
+  long long lo_b[3], hi_b[3];
+  for (int d = 0; d < 3; ++d) { lo_b[d] = ordered(A.hg.ecw[d]); hi_b[d] = ordered(A.hg.cw[d]); }
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += nth) {
+    const double x = wrap1(A.x[i], A.a[0], A.c[0], A.half_minus), y = wrap1(A.y[i], A.a[1], A.c[1], A.half_minus),
+                 z = wrap1(A.z[i], A.a[2], A.c[2], A.half_minus);
+    A.x[i] = x; A.y[i] = y; A.z[i] = z;
+    A.xb[i] = x; A.yb[i] = y; A.zb[i] = z;
+    const long long xx = ordered(red_coord(A.hg.rc, 0, x)), yy = ordered(red_coord(A.hg.rc, 1, y)),
+                    zz = ordered(red_coord(A.hg.rc, 2, z));
+    int v = 0;
+    if (xx <= lo_b[0]) v += 1;
+    if (xx >= hi_b[0]) v += 2;
+    if (yy <= lo_b[1]) v += 10;
+    if (yy >= hi_b[1]) v += 20;
+    if (zz <= lo_b[2]) v += 100;
+    if (zz >= hi_b[2]) v += 200;
+    A.ixyz[i] = v;
+    A.src[i] = i;
+    A.shcode[i] = 13;
+  }
+  grid.sync();
+  int n = A.n;
+  bool over = false;
+  for (int m = 0; m < 6; ++m) {
+    const int kx = m < 2 ? 1 : 0, ky = (m >> 1) == 1 ? 1 : 0, kz = m >= 4 ? 1 : 0;
+    const int unit = m < 2 ? 1 : m < 4 ? 10 : 100, jxyz = (m & 1) ? 2 * unit : unit, kxyz = 3 * unit;
+    const int dshift = (m & 1 ? -1 : 1) * (m < 2 ? 1 : m < 4 ? 3 : 9);
+    // this block's run of the atoms and images so far, NK x 512 of them at a time
+    const int per = (n + gridDim.x - 1) / gridDim.x;
+    const int lo = min(n, (int)blockIdx.x * per), hi = min(n, lo + per);
+    const bool once = per <= NK * HALO_NT;
+    int v[NK];
+    unsigned bal[NK];
+    auto look = [&](int i0) {
+#pragma unroll
+      for (int k = 0; k < NK; ++k) {
+        const int i = i0 + k * HALO_NT + threadIdx.x;
+        v[k] = i < hi ? A.ixyz[i] : 0;
+      }
+#pragma unroll
+      for (int k = 0; k < NK; ++k) bal[k] = __ballot_sync(0xffffffffu, export_sel(v[k], kx, ky, kz, jxyz));
+    };
+    int cnt = 0;
+    for (int i0 = lo; i0 < hi; i0 += NK * HALO_NT) {
+      look(i0);
+#pragma unroll
+      for (int k = 0; k < NK; ++k) cnt += __popc(bal[k]);
+    }
+    if (lane == 0) s_w[wid] = cnt;
+    __syncthreads();
+    if (wid == 0) {
+      const int s = __reduce_add_sync(0xffffffffu, lane < NW ? s_w[lane] : 0);
+      if (lane == 0) A.cnt[m * gridDim.x + blockIdx.x] = s;
+    }
+    grid.sync();
+    if (wid == 0) {  // images before this block's, and all of them
+      int before = 0, all = 0;
+      for (int b = lane; b < (int)gridDim.x; b += 32) {
+        const int c = __ldcg(&A.cnt[m * gridDim.x + b]);
+        all += c;
+        before += b < (int)blockIdx.x ? c : 0;
+      }
+      before = __reduce_add_sync(0xffffffffu, before);
+      all = __reduce_add_sync(0xffffffffu, all);
+      if (lane == 0) { s_tot[0] = before; s_tot[1] = all; }
+    }
+    __syncthreads();
+    int base = n + s_tot[0];
+    const int all = s_tot[1];
+    for (int i0 = lo; i0 < hi; i0 += NK * HALO_NT) {
+      if (!once) look(i0);
+      if (lane == 0) {
+#pragma unroll
+        for (int k = 0; k < NK; ++k) s_w[k * NW + wid] = __popc(bal[k]);
+      }
+      __syncthreads();
+      if (wid == 0) {  // exclusive sums over the NK x NW counts, NK * NW / 32 per lane
+        constexpr int PL = NK * NW / 32;
+        int c[PL], s = 0;
+#pragma unroll
+        for (int e = 0; e < PL; ++e) { c[e] = s_w[lane * PL + e]; s += c[e]; }
+        int inc = s;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int u = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= o) inc += u;
+        }
+        if (lane == 31) s_tot[0] = inc;
+        int run = inc - s;
+#pragma unroll
+        for (int e = 0; e < PL; ++e) { s_w[lane * PL + e] = run; run += c[e]; }
+      }
+      __syncthreads();
+#pragma unroll
+      for (int k = 0; k < NK; ++k) {
+        const int dst = base + s_w[k * NW + wid] + __popc(bal[k] & ((1u << lane) - 1u));
+        if (((bal[k] >> lane) & 1u) && dst < A.mxatms) {
+          const int i = i0 + k * HALO_NT + threadIdx.x, s = A.src[i];
+          A.x[dst] = add_rn(A.x[i], A.add[m][0]);
+          A.y[dst] = add_rn(A.y[i], A.add[m][1]);
+          A.z[dst] = add_rn(A.z[i], A.add[m][2]);
+          A.src[dst] = s;
+          A.shcode[dst] = A.shcode[i] + dshift;
+          const int ix = v[k] % 10, iy = (v[k] - ix) % 100, iz = (v[k] - (ix + iy)) % 1000;
+          const int j = ix * kx + iy * ky + iz * kz;
+          A.ixyz[dst] = v[k] - (j == jxyz ? jxyz : kxyz);
+          // the source atom's properties
+          A.ltg[dst] = A.ltg[s];
+          A.ltype[dst] = A.ltype[s];
+          A.chge[dst] = A.chge[s];
+          A.weight[dst] = A.weight[s];
+          A.lfrzn[dst] = A.lfrzn[s];
+        }
+      }
+      base += s_tot[0];
+      __syncthreads();
+    }
+    // images beyond mxatms are neither written nor counted
+    if (all > A.mxatms - n) { over = true; n = A.mxatms; }
+    else n += all;
+    if (m < 5) grid.sync();
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    A.sc->nlast = n;
+    A.sc->nlast_prev = n;
+    if (over) A.sc->status |= ST_HALO_OVERFLOW;
   }
 }
 
@@ -137,76 +263,6 @@ __global__ void k_scan_single(const int* in, int* out, int n, int* total) {
   if (threadIdx.x == T - 1 && total) *total = part[T - 1];
 }
 
-__global__ void k_export_commit(const int* blkcount, int nblk, int* blkoff, DevScalars* sc, int mxatms) {
-  // single thread: offsets were produced by k_scan_single into blkoff; grow nlast
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  int tot = blkoff[nblk - 1] + blkcount[nblk - 1];
-  int n = sc->nlast;
-  sc->nlast_prev = n;
-  if (n + tot > mxatms) {
-    sc->status |= ST_HALO_OVERFLOW;
-    tot = mxatms - n;
-  }
-  sc->nlast = n + tot;
-}
-
-__global__ void k_export_write(double* x, double* y, double* z, int* ltg, int* src, int* shcode, int* ixyz,
-                               const int* blkoff, const DevScalars* sc, int kx, int ky, int kz, int jxyz,
-                               int kxyz, double ax, double ay, double az, int dshift, int mxatms) {
-  const int n = sc->nlast_prev;
-  const int base = blockIdx.x * SCAN_BLOCK;
-  __shared__ int wsum[32];
-  __shared__ int chunk_base;
-  if (threadIdx.x == 0) chunk_base = 0;
-  __syncthreads();
-  // process the block's 1024 items in chunks of blockDim, preserving order
-  for (int c = 0; c < SCAN_BLOCK; c += blockDim.x) {
-    int i = base + c + threadIdx.x;
-    int v = (i < n && c + threadIdx.x < SCAN_BLOCK) ? ixyz[i] : 0;
-    bool sel = (i < n) && export_sel(v, kx, ky, kz, jxyz);
-    unsigned m = __ballot_sync(0xffffffffu, sel);
-    int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    int pre = __popc(m & ((1u << lane) - 1u));
-    if (lane == 0) wsum[w] = __popc(m);
-    __syncthreads();
-    int wpre = 0;
-    for (int k = 0; k < w; ++k) wpre += wsum[k];
-    if (sel) {
-      int dst = n + blkoff[blockIdx.x] + chunk_base + wpre + pre;
-      if (dst < mxatms) {
-        x[dst] = add_rn(x[i], ax);
-        y[dst] = add_rn(y[i], ay);
-        z[dst] = add_rn(z[i], az);
-        ltg[dst] = ltg[i];
-        src[dst] = src[i];
-        shcode[dst] = shcode[i] + dshift;
-        int ix = v % 10, iy = (v - ix) % 100, iz = (v - (ix + iy)) % 1000;
-        int j = ix * kx + iy * ky + iz * kz;
-        ixyz[dst] = v - (j == jxyz ? jxyz : kxyz);
-      }
-    }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      int t = 0;
-      for (int k = 0; k < (int)(blockDim.x >> 5); ++k) t += wsum[k];
-      chunk_base += t;
-    }
-    __syncthreads();
-  }
-}
-
-// halo properties from the local source atom
-__global__ void k_halo_props(int natms, const DevScalars* sc, const int* src, int* ltype, double* chge,
-                             double* weight, int* lfrzn) {
-  int i = natms + blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= sc->nlast) return;
-  int s = src[i];
-  ltype[i] = ltype[s];
-  chge[i] = chge[s];
-  weight[i] = weight[s];
-  lfrzn[i] = lfrzn[s];
-}
-
 // refresh_halo_positions: the same export chain applied to the source position
 __global__ void k_halo_refresh(int natms, const DevScalars* sc, const int* src, const int* shcode, double* x,
                                double* y, double* z, const double* adds /*6x3*/) {
@@ -222,22 +278,15 @@ __global__ void k_halo_refresh(int natms, const DevScalars* sc, const int* src, 
   x[i] = xx; y[i] = yy; z[i] = zz;
 }
 
-__global__ void k_set_check(int n, const double* x, const double* y, const double* z, double* xb, double* yb,
-                            double* zb) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  xb[i] = x[i]; yb[i] = y[i]; zb[i] = z[i];
-}
-
 // ----------------------------------------------------------------- binning
 __global__ void k_bin(int natms, const DevScalars* sc, const double* x, const double* y, const double* z,
                       CellGeom cg, int* which_cell, int* count) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int nlast = sc->nlast;
   if (i >= nlast) return;
-  const double xx = red_coord(cg.rc, 0, x[i], y[i], z[i]);
-  const double yy = red_coord(cg.rc, 1, x[i], y[i], z[i]);
-  const double zz = red_coord(cg.rc, 2, x[i], y[i], z[i]);
+  const double xx = red_coord(cg.rc, 0, x[i]);
+  const double yy = red_coord(cg.rc, 1, y[i]);
+  const double zz = red_coord(cg.rc, 2, z[i]);
   const int nlp = cg.nlp, jx0 = nlp, jy0 = nlp, jz0 = nlp;
   const int nlx0e = nlp - 1, nly0e = nlp - 1, nlz0e = nlp - 1;
   const int nlx1s = cg.nlx + nlp, nly1s = cg.nly + nlp, nlz1s = cg.nlz + nlp;
@@ -476,7 +525,11 @@ __global__ void k_tile_rows(TilePlan tp, CellGeom cg, const int* __restrict__ st
 // ballot compaction.  Beside list(k, i) the kernel writes spos(k, i): the partner's
 // sorted position, or -1 for the entries of the backward halo pass (pass 2), whose
 // pairs the partner atom's forward pass also lists, so that the pair kernels evaluate
-// each pair once, from its forward copy.
+// each pair once, from its forward copy.  Bound by issue in pass 1 and by the latency of
+// its loads in pass 2, whose cells are read from global memory: with the bounds of 32 cells
+// or runs loaded at once and pass 2's members taken as one sequence, a build takes 0.37
+// instead of 0.54 ms (98,304-atom water), 0.48 instead of 0.81 ms (175,616 ions) and 0.047
+// instead of 0.145 ms (1,536 atoms, where seven CTAs share a tile).
 __global__ void __launch_bounds__(256) k_list_tiles(int natms, CellGeom cg, TilePlan tp, int nsbcll, int nseg,
                                                     const int* __restrict__ tile_ids, int cap,
                                                     const int* __restrict__ tile_rows, const int* __restrict__ tile_info,
@@ -512,7 +565,7 @@ __global__ void __launch_bounds__(256) k_list_tiles(int natms, CellGeom cg, Tile
   const int nlx0e = nlp - 1, nly0e = nlp - 1, nlz0e = nlp - 1;
   const int nlx1s = cg.nlx + nlp, nly1s = cg.nly + nlp, nlz1s = cg.nlz + nlp;
   int ncand64 = 0, nfwd = 0, nbwd = 0;
-  for (int p = ip0 + warp; p < ip1; p += nw) {
+  for (int p = ip0 + warp + nw * blockIdx.y; p < ip1; p += nw * gridDim.y) {
     const int i0s = s_base[tp.r00] - s_first[tp.r00];
     const int i = s_at[p + i0s];
     const int ic = which_cell[i];
@@ -525,13 +578,28 @@ __global__ void __launch_bounds__(256) k_list_tiles(int natms, CellGeom cg, Tile
     int* li = list + (size_t)i * ld + 3;  // li[k] == list(k, i)
     int* si = spos + (size_t)i * ldt;
     int count = 0;
+    int l_s0 = 0, l_e = 0, l_sl = 0;
+    unsigned l_nir = 0;
     // pass 1: the forward half shell, all of it staged, one run of cells at a time
-    for (int sg = 0; sg < nseg; ++sg) {
-      const int r = c_seg_row[sg];
-      const int sl0 = s_base[r] - s_first[r];  // slot = sorted position + sl0
-      const int s0 = sg == 0 ? p + 1 : start[ic + c_seg_off0[sg]];  // segment 0 starts with the own cell
-      const int e = start[ic + c_seg_off1[sg] + 1];
-      const bool nir = c_seg_nir[sg] != 0;
+    // (the bounds of 32 runs are loaded at once, a lane each)
+    for (int q = 0; q < nseg; ++q) {
+      if ((q & 31) == 0) {
+        const int sg = q + lane;
+        int row = 0, nr = 0;
+        l_s0 = l_e = 0;
+        if (sg < nseg) {
+          const int4 d = d_seg[sg];
+          l_s0 = sg == 0 ? p + 1 : start[ic + d.x];  // segment 0 starts with the own cell
+          l_e = start[ic + d.y + 1];
+          row = d.z;
+          nr = d.w;
+        }
+        l_sl = s_base[row] - s_first[row];  // slot = sorted position + l_sl
+        l_nir = __ballot_sync(0xffffffffu, nr != 0);
+      }
+      const int s0 = __shfl_sync(0xffffffffu, l_s0, q & 31), e = __shfl_sync(0xffffffffu, l_e, q & 31),
+                sl0 = __shfl_sync(0xffffffffu, l_sl, q & 31);
+      const bool nir = (l_nir >> (q & 31)) & 1u;
       for (int b = s0; b < e; b += 32) {
         const int jj = b + lane;
         bool acc = false;
@@ -572,17 +640,42 @@ __global__ void __launch_bounds__(256) k_list_tiles(int natms, CellGeom cg, Tile
     const bool border = (ix1 >= 1 && ix1 <= nlp) || (ix2 <= -1 && ix2 >= -nlp) || (iy1 >= 1 && iy1 <= nlp) ||
                         (iy2 <= -1 && iy2 >= -nlp) || (iz1 >= 1 && iz1 <= nlp) || (iz2 <= -1 && iz2 >= -nlp);
     if (border) {
-      for (int kk = 1; kk < nsbcll; ++kk) {
-        const int jx = ix - c_nix[kk], jy = iy - c_niy[kk], jz = iz - c_niz[kk];
-        if (!(jx <= nlx0e || jx >= nlx1s || jy <= nly0e || jy >= nly1s || jz <= nlz0e || jz >= nlz1s)) continue;
-        const int jc = ic - c_off[kk];
-        const int s0 = start[jc], e = start[jc + 1];
-        const bool nir = c_nir[kk] != 0;
-        for (int b = s0; b < e; b += 32) {
-          const int jj = b + lane;
+      // 32 cells at a time, a lane each: their bounds, then their members as one sequence
+      // (lane L of a step takes the member q, of the last cell that starts at or before q);
+      // cell by cell each step had a chain of two dependent loads for a dozen members
+      for (int k0 = 1; k0 < nsbcll; k0 += 32) {
+        int c_s0 = 0, c_n = 0, c_nr = 0;
+        if (k0 + lane < nsbcll) {
+          const int2 d = d_sbc[k0 + lane];
+          const int jx = ix - ((d.y & 255) - 64), jy = iy - (((d.y >> 8) & 255) - 64), jz = iz - (((d.y >> 16) & 255) - 64);
+          if (jx <= nlx0e || jx >= nlx1s || jy <= nly0e || jy >= nly1s || jz <= nlz0e || jz >= nlz1s) {
+            const int jc = ic - d.x;
+            c_s0 = start[jc];
+            c_n = start[jc + 1] - c_s0;
+            c_nr = d.y >> 24;
+          }
+        }
+        int inc = c_n;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, inc, o);
+          if (lane >= o) inc += v;
+        }
+        const int tot = __shfl_sync(0xffffffffu, inc, 31);
+        const int c_off0 = c_s0 - (inc - c_n);  // sorted position of member q of the sequence: q + c_off0
+        const unsigned nirs = __ballot_sync(0xffffffffu, c_nr != 0);
+        for (int b = 0; b < tot; b += 32) {
+          const int q = b + lane;
+          int L = 0;  // cells whose members all precede q
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) {
+            const int v = __shfl_sync(0xffffffffu, inc, L + o - 1);
+            if (v <= q) L += o;
+          }
+          const int jj = q + __shfl_sync(0xffffffffu, c_off0, L & 31);
           bool acc = false;
-          if (jj < e) {
-            if (nir) {
+          if (q < tot) {
+            if ((nirs >> L) & 1u) {
               acc = true;
             } else {
               const float4 xj = xsf[jj];
@@ -636,56 +729,75 @@ __global__ void __launch_bounds__(256) k_list_tiles(int natms, CellGeom cg, Tile
   }
 }
 
-// Frozen (neighbours.F90:1198-1225) and excluded (:1229-1306) reordering, one
-// thread per atom, sequential exactly as the reference swaps.
-// The sorted positions in spos follow their list entries through every swap.
-__global__ void k_list_reorder(int natms, int* list, int ld, int* spos, int ldt, const int* lfrzn,
-                               const int* ltg, const int* list_excl, int ldx, int megfrz, int lbook) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= natms) return;
-  int* li = list + (size_t)i * ld + 3;
-  int* ti = spos + (size_t)i * ldt;
-  int l_end = li[0], m_end = l_end;
-  if (megfrz > 1 && lfrzn[i] > 0) {
-    for (int kk = l_end; kk >= 1; --kk) {
-      int j = li[kk];
-      if (lfrzn[j - 1] > 0) {
-        if (kk < m_end) {
-          li[kk] = li[m_end]; li[m_end] = j;
-          const int tk = ti[kk]; ti[kk] = ti[m_end]; ti[m_end] = tk;
+// Frozen (neighbours.F90:1198-1225) and excluded (:1229-1306) reordering, one warp per
+// atom.  The reference walks the list from its end and swaps each hit with the last entry
+// of the kept part; every entry between the hit and that one has been kept, so only the
+// hits act.  The warp finds them, 128 entries' loads in flight together, and lane 0 swaps
+// them in descending order, spos following.  (One thread per atom took 0.30 ms for 1,536
+// atoms and 0.36 ms for 98,304, a dependent load per entry; this takes 0.010 and 0.066 ms.)
+template <typename Hit>
+__device__ __forceinline__ int list_move_hits(int* li, int* ti, int n, Hit hit) {
+  const int lane = threadIdx.x & 31;
+  int m_end = n;
+  for (int b = (n - 1) & ~127; b >= 0 && n > 0; b -= 128) {
+    int j[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int kk = b + 32 * u + lane + 1;
+      j[u] = kk <= n ? li[kk] : 0;
+    }
+    unsigned hits[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) hits[u] = __ballot_sync(0xffffffffu, j[u] != 0 && hit(j[u]));
+#pragma unroll
+    for (int u = 3; u >= 0; --u) {
+      for (unsigned m = hits[u]; m; --m_end) {
+        const int bit = 31 - __clz((int)m);
+        m ^= 1u << bit;
+        const int k = b + 32 * u + bit + 1;
+        if (lane == 0 && k < m_end) {
+          const int jk = li[k], tk = ti[k];
+          li[k] = li[m_end]; li[m_end] = jk;
+          ti[k] = ti[m_end]; ti[m_end] = tk;
         }
-        --m_end;
       }
     }
   }
-  li[-2] = li[0];
-  li[0] = m_end;
+  return m_end;
+}
+
+__global__ void __launch_bounds__(256) k_list_reorder(int natms, int* list, int ld, int* spos, int ldt,
+                                                      const int* __restrict__ lfrzn, const int* __restrict__ ltg,
+                                                      const int* __restrict__ list_excl, int ldx, int megfrz,
+                                                      int lbook) {
+  const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (i >= natms) return;
+  int* li = list + (size_t)i * ld + 3;
+  int* ti = spos + (size_t)i * ldt;
+  const int n0 = li[0];
+  int n1 = n0;
+  if (megfrz > 1 && lfrzn[i] > 0) n1 = list_move_hits(li, ti, n0, [&](int j) { return lfrzn[j - 1] > 0; });
+  int n2 = n1;
   if (lbook) {
-    l_end = li[0];
-    m_end = l_end;
     const int* ex = list_excl + (size_t)i * ldx;
-    int ii = ex[0];
+    const int ii = ex[0];
     if (ii > 0) {
-      for (int kk = l_end; kk >= 1; --kk) {
-        int j = li[kk];
-        int jj = ltg[j - 1];
-        bool hit = false;
-        for (int t = 1; t <= ii; ++t) hit |= (ex[t] == jj);
-        if (hit) {
-          if (kk < m_end) {
-            li[kk] = li[m_end]; li[m_end] = j;
-            const int tk = ti[kk]; ti[kk] = ti[m_end]; ti[m_end] = tk;
-          }
-          --m_end;
-        }
-      }
+      __syncwarp();  // lane 0's swaps above
+      const int e1 = ex[1], e2 = ii > 1 ? ex[2] : e1;
+      n2 = list_move_hits(li, ti, n1, [&](int j) {
+        const int jj = j <= natms ? j : ltg[j - 1];  // a local atom's global id is its index
+        bool h = e1 == jj || e2 == jj;
+        for (int t = 3; t <= ii; ++t) h |= ex[t] == jj;
+        return h;
+      });
     }
-    li[-1] = li[0];
-    li[0] = m_end;
-    li[-3] = li[0];
-  } else {
-    li[-1] = li[0];
-    li[-3] = li[0];
+  }
+  __syncwarp();
+  if (lane == 0) {
+    li[-2] = n0;
+    li[-1] = n1;
+    li[0] = n2;
+    li[-3] = n2;
   }
 }
 
@@ -762,6 +874,8 @@ void list_setup() {
     h_add[m][2] = c[2] * u + c[5] * v + c[8] * w;
   }
   upload_adds();
+  const char* hb = getenv("GB_HALO_BLOCKS");
+  h_halo_blocks = hb ? std::max(0, atoi(hb)) : 0;
   // link-cell geometry (neighbours.F90:396-463)
   double cut2 = g.rcutx + 1.0e-6;
   double disp[3] = {1.0 * cp[6] / cut2, 1.0 * cp[7] / cut2, 1.0 * cp[8] / cut2};
@@ -821,23 +935,19 @@ void list_setup() {
     }
     tp.r00 = row[0];  // offset (0, 0, 0) comes first; its row starts at dx = 0
     if (nix[0] != 0 || niy[0] != 0 || niz[0] != 0 || tp.dxlo[tp.r00] != 0) throw (int)GB_ERR_ARG;
-    GB_CUDA(cudaMemcpyToSymbol(c_row, row.data(), row.size()));
     // segments: consecutive semi-ball cells of one row, adjacent along x, with one nir flag
-    std::vector<int> s0, s1;
-    std::vector<unsigned char> srow, snir;
+    std::vector<int4> seg;
+    std::vector<int2> sbc(off.size());
     for (size_t k = 0; k < off.size(); ++k) {
+      sbc[k] = make_int2(off[k], (nix[k] + 64) | (niy[k] + 64) << 8 | (niz[k] + 64) << 16 | (int)nir[k] << 24);
       const bool joins = k > 0 && row[k] == row[k - 1] && nix[k] == nix[k - 1] + 1 && nir[k] == nir[k - 1];
-      if (joins) {
-        s1.back() = off[k];
-      } else {
-        s0.push_back(off[k]); s1.push_back(off[k]); srow.push_back(row[k]); snir.push_back(nir[k]);
-      }
+      if (joins) seg.back().y = off[k];
+      else seg.push_back(make_int4(off[k], off[k], row[k], nir[k]));
     }
-    g.nseg = (int)s0.size();
-    GB_CUDA(cudaMemcpyToSymbol(c_seg_off0, s0.data(), sizeof(int) * s0.size()));
-    GB_CUDA(cudaMemcpyToSymbol(c_seg_off1, s1.data(), sizeof(int) * s1.size()));
-    GB_CUDA(cudaMemcpyToSymbol(c_seg_row, srow.data(), srow.size()));
-    GB_CUDA(cudaMemcpyToSymbol(c_seg_nir, snir.data(), snir.size()));
+    if (nlp > 63) throw (int)GB_ERR_ARG;  // beyond MAX_SBC long before
+    g.nseg = (int)seg.size();
+    GB_CUDA(cudaMemcpyToSymbol(d_seg, seg.data(), sizeof(int4) * seg.size()));
+    GB_CUDA(cudaMemcpyToSymbol(d_sbc, sbc.data(), sizeof(int2) * sbc.size()));
     // tile width: the widest run of cells whose staged set stays near the capacity the
     // pair kernel's shared memory allows at two CTAs per SM
     const double apc = (double)g.natms / ((double)nlx * nly * nlz);
@@ -897,48 +1007,32 @@ void list_setup() {
   }
 }
 
-int list_relocate_and_halo() {
+int list_relocate_and_halo(bool wait) {
   const int n = g.natms;
   g.spos_valid = false;  // new halo images: the sorted positions of the list are stale until the next build
-  const int T = 256;
-  cudaStream_t st = g.stream;
   prof_begin(P_HALO);
-  // relocate_particles in serial: pbcshift (deport_data.F90:3190)
-  {
-    double a0 = 1.0 / g.cell[0], a4 = 1.0 / g.cell[4], a8 = 1.0 / g.cell[8];
-    if (g.cubic) { a4 = a0; a8 = a0; }
-    double c4 = g.cubic ? g.cell[0] : g.cell[4], c8 = g.cubic ? g.cell[0] : g.cell[8];
-    k_pbcshift<<<nblocks(n, T), T, 0, st>>>(n, g.x, g.y, g.z, a0, a4, a8, g.cell[0], c4, c8,
-                                            std::nextafter(0.5, 0.0));
-    GB_LAUNCHED();
+  HaloArgs A;
+  A.n = n; A.mxatms = g.mxatms;
+  A.x = g.x; A.y = g.y; A.z = g.z; A.xb = g.xbg; A.yb = g.ybg; A.zb = g.zbg;
+  for (int d = 0; d < 3; ++d) {
+    const int k = g.cubic ? 0 : 4 * d;
+    A.a[d] = 1.0 / g.cell[k];
+    A.c[d] = g.cell[k];
   }
-  k_halo_flags<<<nblocks(n, T), T, 0, st>>>(n, g.x, g.y, g.z, h_halo, g.ixyz, g.src, g.shcode, g.sc);
-  GB_LAUNCHED();
-  const int nblk = nblocks(g.mxatms, SCAN_BLOCK);
-  int* blkcount = gb_scan_scratch(2 * nblk + 2);
-  int* blkoff = blkcount + nblk + 1;
-  const int mdirs[6][5] = {{1, 0, 0, 1, 3}, {1, 0, 0, 2, 3}, {0, 1, 0, 10, 30},
-                           {0, 1, 0, 20, 30}, {0, 0, 1, 100, 300}, {0, 0, 1, 200, 300}};
-  const int dsh[6] = {+1, -1, +3, -3, +9, -9};
-  for (int m = 0; m < 6; ++m) {
-    const int* md = mdirs[m];
-    k_export_count<<<nblk, 256, 0, st>>>(g.ixyz, g.sc, md[0], md[1], md[2], md[3], blkcount);
-    GB_LAUNCHED();
-    k_scan_single<<<1, 1024, 0, st>>>(blkcount, blkoff, nblk, nullptr);
-    GB_LAUNCHED();
-    k_export_commit<<<1, 32, 0, st>>>(blkcount, nblk, blkoff, g.sc, g.mxatms);
-    GB_LAUNCHED();
-    k_export_write<<<nblk, 256, 0, st>>>(g.x, g.y, g.z, g.ltg, g.src, g.shcode, g.ixyz, blkoff, g.sc, md[0], md[1],
-                                          md[2], md[3], md[4], h_add[m][0], h_add[m][1], h_add[m][2], dsh[m],
-                                          g.mxatms);
-    GB_LAUNCHED();
-  }
-  k_halo_props<<<nblocks(g.mxatms - n, T), T, 0, st>>>(n, g.sc, g.src, g.ltype, g.chge, g.weight, g.lfrzn);
-  GB_LAUNCHED();
-  // vnl_set_check (neighbours.F90:305-343): local positions are the checkpoint
-  k_set_check<<<nblocks(n, T), T, 0, st>>>(n, g.x, g.y, g.z, g.xbg, g.ybg, g.zbg);
+  A.half_minus = std::nextafter(0.5, 0.0);
+  A.hg = h_halo;
+  std::memcpy(A.add, h_add, sizeof(h_add));
+  A.ixyz = g.ixyz; A.src = g.src; A.shcode = g.shcode; A.ltg = g.ltg; A.ltype = g.ltype; A.lfrzn = g.lfrzn;
+  A.chge = g.chge; A.weight = g.weight;
+  A.sc = g.sc;
+  // one resident block per SM at most; a small box has several images per atom
+  const int nb = std::max(1, std::min(h_halo_blocks ? h_halo_blocks : nblocks(g.mxatms, HALO_NT), g.nsm));
+  A.cnt = gb_scan_scratch(6 * nb);
+  void* args[] = {&A};
+  GB_CUDA(cudaLaunchCooperativeKernel((void*)k_halo_build, nb, HALO_NT, args, 0, g.stream));
   GB_LAUNCHED();
   prof_end(P_HALO);
+  if (!wait) return GB_OK;  // list_build, which follows, reports ST_HALO_OVERFLOW
   gb_sync_scalars();
   if (g.hsc->status & ST_HALO_OVERFLOW) return GB_ERR_HALO;
   return GB_OK;
@@ -1025,45 +1119,62 @@ int list_build() {
     GB_LAUNCHED();
   }
   prof_end(P_BIN);
-  GB_CUDA(cudaMemsetAsync(&g.sc->ibig, 0, sizeof(int), st));
-  GB_CUDA(cudaMemsetAsync(&g.sc->tile_over, 0, 4 * sizeof(int), st));  // tile_over, tile_max, halo_fwd, halo_bwd
   prof_begin(P_LIST);
   const TilePlan& tp = g.tp;
   const int cap = g.tile_cap_list;
-  k_tile_rows<<<nblocks(tp.ntiles, 128), 128, 0, st>>>(tp, h_cg, g.cell_start, g.tile_rows, g.tile_info, cap,
-                                                        g.tile_over, g.sc);
-  GB_LAUNCHED();
+  // few tiles: several CTAs share a tile's atoms (each stages its whole shell), so that
+  // the device has about three CTAs per SM
+  const int split = std::max(1, std::min(8, 3 * g.nsm / std::max(tp.ntiles, 1)));
   GB_CUDA(cudaFuncSetAttribute(k_list_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, 20 * TILE_CAP_MAX));
-  k_list_tiles<<<tp.ntiles, 256, (size_t)cap * 20, st>>>(g.natms, h_cg, tp, g.nsbcll, g.nseg, nullptr, cap,
-                                                          g.tile_rows, g.tile_info, g.at_list, g.which_cell,
-                                                          g.cell_start, g.xs, g.xsf, g.list, g.ld, g.spos, g.ldt,
-                                                          g.p.max_list, g.sc);
-  GB_LAUNCHED();
-  gb_sync_scalars();
-  g.n_tile_over = g.hsc->tile_over;
-  g.tile_max_staged = g.hsc->tile_max;
-  if (g.n_tile_over > 0 && g.tile_max_staged <= TILE_CAP_MAX) {
-    // the tiles above the capacity, with shared memory for the largest of them
-    k_list_tiles<<<g.n_tile_over, 256, (size_t)g.tile_max_staged * 20, st>>>(
-        g.natms, h_cg, tp, g.nsbcll, g.nseg, g.tile_over, g.tile_max_staged, g.tile_rows, g.tile_info, g.at_list,
-        g.which_cell, g.cell_start, g.xs, g.xsf, g.list, g.ld, g.spos, g.ldt, g.p.max_list, g.sc);
+  // The host waits once, after the last kernel, unless the previous build had tiles above
+  // the first launch's capacity: then it looks before the second launch.  The first build
+  // that meets such tiles runs its kernels again with that launch.
+  for (;;) {
+    GB_CUDA(cudaMemsetAsync(&g.sc->ibig, 0, sizeof(int), st));
+    GB_CUDA(cudaMemsetAsync(&g.sc->tile_over, 0, 4 * sizeof(int), st));  // tile_over, tile_max, halo_fwd, halo_bwd
+    k_tile_rows<<<nblocks(tp.ntiles, 128), 128, 0, st>>>(tp, h_cg, g.cell_start, g.tile_rows, g.tile_info, cap,
+                                                          g.tile_over, g.sc);
     GB_LAUNCHED();
-  } else if (g.n_tile_over > 0) {
-    // a tile too dense for one CTA's shared memory: the whole list from the per-atom kernel
-    GB_CUDA(cudaMemsetAsync(&g.sc->halo_fwd, 0, 2 * sizeof(int), st));
-    k_list_pairs<<<nblocks((long long)mx * 32, T), T, 0, st>>>(g.natms, g.sc, h_cg, g.nsbcll, g.at_list,
-                                                               g.which_cell, g.cell_start, g.xs, g.xsf, g.list, g.ld,
-                                                               g.spos, g.ldt, g.p.max_list, g.sc);
+    k_list_tiles<<<dim3(tp.ntiles, split), 256, (size_t)cap * 20, st>>>(
+        g.natms, h_cg, tp, g.nsbcll, g.nseg, nullptr, cap, g.tile_rows, g.tile_info, g.at_list, g.which_cell,
+        g.cell_start, g.xs, g.xsf, g.list, g.ld, g.spos, g.ldt, g.p.max_list, g.sc);
     GB_LAUNCHED();
-  }
-  if (g.lbook || g.megfrz > 1) {
-    k_list_reorder<<<nblocks(g.natms, 128), 128, 0, st>>>(g.natms, g.list, g.ld, g.spos, g.ldt, g.lfrzn, g.ltg,
-                                                          g.list_excl, g.p.max_exclude + 1, g.megfrz,
-                                                          g.lbook ? 1 : 0);
-    GB_LAUNCHED();
+    const bool looked = g.n_tile_over > 0;
+    if (looked) {
+      gb_sync_scalars();
+      g.n_tile_over = g.hsc->tile_over;
+      g.tile_max_staged = g.hsc->tile_max;
+      if (g.n_tile_over > 0 && g.tile_max_staged <= TILE_CAP_MAX) {
+        // the tiles above the capacity, with shared memory for the largest of them
+        k_list_tiles<<<g.n_tile_over, 256, (size_t)g.tile_max_staged * 20, st>>>(
+            g.natms, h_cg, tp, g.nsbcll, g.nseg, g.tile_over, g.tile_max_staged, g.tile_rows, g.tile_info, g.at_list,
+            g.which_cell, g.cell_start, g.xs, g.xsf, g.list, g.ld, g.spos, g.ldt, g.p.max_list, g.sc);
+        GB_LAUNCHED();
+      } else if (g.n_tile_over > 0) {
+        // a tile too dense for one CTA's shared memory: the whole list from the per-atom kernel
+        GB_CUDA(cudaMemsetAsync(&g.sc->halo_fwd, 0, 2 * sizeof(int), st));
+        k_list_pairs<<<nblocks((long long)mx * 32, T), T, 0, st>>>(g.natms, g.sc, h_cg, g.nsbcll, g.at_list,
+                                                                   g.which_cell, g.cell_start, g.xs, g.xsf, g.list,
+                                                                   g.ld, g.spos, g.ldt, g.p.max_list, g.sc);
+        GB_LAUNCHED();
+      }
+    }
+    if (g.lbook || g.megfrz > 1) {  // (lists of tiles not built yet hold valid older entries, or none)
+      k_list_reorder<<<nblocks((long long)g.natms * 32, 256), 256, 0, st>>>(g.natms, g.list, g.ld, g.spos, g.ldt,
+                                                                            g.lfrzn, g.ltg, g.list_excl,
+                                                                            g.p.max_exclude + 1, g.megfrz,
+                                                                            g.lbook ? 1 : 0);
+      GB_LAUNCHED();
+    }
+    gb_sync_scalars();
+    if (looked || g.hsc->tile_over == 0) {
+      g.tile_max_staged = g.hsc->tile_max;
+      break;
+    }
+    g.n_tile_over = g.hsc->tile_over;
   }
   prof_end(P_LIST);
-  gb_sync_scalars();
+  if (g.hsc->status & ST_HALO_OVERFLOW) return GB_ERR_HALO;  // (list_relocate_and_halo without its wait)
   if (g.hsc->status & ST_LIST_OVERFLOW) return GB_ERR_LIST_OVERFLOW;
   // every pair across the periodic boundary is listed from both of its atoms, once in a
   // forward pass and once in the backward halo pass; the sorted-position pair kernels

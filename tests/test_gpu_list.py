@@ -1,0 +1,49 @@
+"""Verlet list, bit for bit, where its kernels take other branches: frozen and excluded
+atoms moved to the end of the lists, and halo exports longer than a block's registers hold."""
+import numpy as np
+import pytest
+
+from dlpoly_gb300 import systems
+
+pytestmark = pytest.mark.gpu
+
+
+def _lists(gpu_lib, oracle_lib, s):
+    out = []
+    for lib in (gpu_lib, oracle_lib):
+        lib.init(s)
+        lib.relocate()
+        out.append(lib.link_cell_pairs())
+    return out
+
+
+def _same(a, b):
+    """list(-3:0) and the listed entries, with the frozen and excluded ones beyond list(0)."""
+    assert np.array_equal(a[:, :4], b[:, :4])
+    k = np.arange(a.shape[1] - 4)[None, :]
+    used = k < b[:, 1:2]  # list(-2): before the reordering
+    assert np.array_equal(np.where(used, a[:, 4:], 0), np.where(used, b[:, 4:], 0))
+
+
+@pytest.mark.parametrize("frozen", [0, 1, 2, 40, "many"])
+def test_frozen_and_excluded_entries(gpu_lib, oracle_lib, frozen):
+    s = systems.spce_water(8)
+    s.lfrzn = np.zeros(s.natms, np.int32)
+    if frozen == "many":
+        s.lfrzn[np.arange(s.natms) % 3 != 0] = 1
+    else:
+        s.lfrzn[:3 * frozen:3] = 1
+    _same(*_lists(gpu_lib, oracle_lib, s))
+
+
+@pytest.mark.parametrize("blocks", [1, 2, 7])
+def test_halo_runs_longer_than_a_pass(gpu_lib, oracle_lib, monkeypatch, blocks):
+    monkeypatch.setenv("GB_HALO_BLOCKS", str(blocks))
+    _same(*_lists(gpu_lib, oracle_lib, systems.nacl_melt(16)))
+    monkeypatch.delenv("GB_HALO_BLOCKS")
+
+
+@pytest.mark.parametrize("make", [lambda: systems.nacl_melt(10, kmax=30), lambda: systems.eam_alloy(5),
+                                  lambda: systems.nacl_melt(22, kmax=64)])
+def test_small_and_ragged_boxes(gpu_lib, oracle_lib, make):
+    _same(*_lists(gpu_lib, oracle_lib, make()))
