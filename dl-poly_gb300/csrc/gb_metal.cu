@@ -24,6 +24,7 @@
 #include <vector>
 
 #include "gb_common.cuh"
+#include "gb_dfr.cuh"
 
 namespace {
 
@@ -43,6 +44,9 @@ struct MetTab {
   int listed;     // pair tables: the FIELD 'metal' directive lists this type pair (keypot 0)
   double nr0rdr;  // -r0 * rdr: x = r * rdr + nr0rdr
   long long b_lo, b_hi;  // r <= rmax decided on rsq bits outside [rmax^2 (1 -+ 1e-12)]
+  // double-float kernels: r <= rmax decided on rsq outside [f_lo, f_hi] (1e-6 around
+  // rmax^2; -1 without a table), and rdr, nr0rdr as double-floats
+  float f_lo, f_hi, rdr_h, rdr_l, nr_h, nr_l;
 };
 
 // r <= rmax as the reference decides it (correctly rounded sqrt), from the bits of rsq
@@ -350,6 +354,462 @@ __global__ void __launch_bounds__(256, 3) k_metal_forces(int natms, const DevSca
   block_reduce_store<MACC>(acc, blk);
 }
 
+// ------------------------------------------------------- sorted-position kernels
+// Both passes over the list's partners in cell order (spos, as the pair kernels walk it),
+// in double-float on the FP32 pipes.  The FP64 kernels above are bound by the FP64 unit
+// (1/64 of the FP32 rate): 95 FP64 instructions per 32 list entries, executed for whole
+// warps although a fifth of the entries lie beyond the cutoff.  Here an FP32 test of the
+// high parts queues the entries that may be inside, and 32 queued pairs at a time are
+// evaluated with every lane busy.  256,000 atoms: density 1.97 -> DENS ms, forces 4.35 ->
+// FORC ms.
+//   positions   int64 in units of 2^-48 A (exact for |x| >= 16 A): the separation is an
+//               exact integer difference
+//   r           relative error about 1e-14 (an FP32 square root and the first-order
+//               remainder; the FP64 kernels' one Newton step from an FP32 seed: 8e-14)
+//   tables      l by the nearest integer of the double-float coordinate, so that a pair
+//               takes the interval that the FP64 kernels take
+// A pair near a cutoff, at an end of its table, with a negative density or outside the
+// FP32 range takes the FP64 formulas of the kernels above (metal_density_slow,
+// metal_force_slow).  Densities and forces are summed in FP64 per sorted position and
+// folded onto the atoms (a halo image's onto its source) afterwards.
+struct __align__(16) MetRec {
+  long long x, y, z;
+  int type, pad;
+};
+
+struct __align__(16) CoefF {
+  float c0h, c0l, c1h, c1l;
+  float c2h, c2l, pad0, pad1;
+};
+
+struct MetSorted {
+  int natms;
+  const int *at_list, *loc_sp, *list, *spos;
+  int ld, ldt;
+  const float4* xhs;
+  const MetRec* rec;
+  const double *x, *y, *z, *rho;   // FP64 by atom index, for the slow path
+  const CoefF *fv, *fd;            // quadratic coefficients of the values and derivatives
+  const float2* fp;                // F'(rho) per sorted position
+  float f_pre, f_rc_lo, f_rc_hi;
+  double *s0, *s1, *s2;            // sums per sorted position
+  double* blk;
+  int* status;
+  unsigned long long* cnt;
+};
+
+constexpr double MET_POS_SCALE = 281474976710656.0;  // 2^48
+constexpr int MET_NT = 256, MET_U = 4;
+
+__global__ void k_metal_records(const DevScalars* sc, const int* __restrict__ sorted_pos, const double* __restrict__ x,
+                                const double* __restrict__ y, const double* __restrict__ z,
+                                const int* __restrict__ ltype, MetRec* __restrict__ rec) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= sc->nlast) return;
+  MetRec r;
+  r.x = __double2ll_rn(x[i] * MET_POS_SCALE);
+  r.y = __double2ll_rn(y[i] * MET_POS_SCALE);
+  r.z = __double2ll_rn(z[i] * MET_POS_SCALE);
+  r.type = ltype[i];
+  r.pad = 0;
+  rec[sorted_pos[i]] = r;
+}
+
+// (a - b) 2^-48 for |a - b| < 2^52, as a double-float
+__device__ __forceinline__ df pos_diff(long long a, long long b) {
+  const long long d = a - b;
+  const float h = __int2float_rn((int)(d >> 28)) * 9.5367431640625e-07f;                             // 2^-20
+  const float l = __int2float_rn((int)((unsigned)d & 0x0FFFFFFFu)) * 3.552713678800501e-15f;  // 2^-48
+  return quick_two_sum(h, l);
+}
+
+// exact double of a finite float by integer operations (0 below the normal range)
+__device__ __forceinline__ double flt_dbl(float f) {
+  const unsigned u = __float_as_uint(f), a = u & 0x7FFFFFFFu;
+  const unsigned hi = (u & 0x80000000u) | ((a >> 3) + 0x38000000u);
+  return a < 0x00800000u ? 0.0 : __hiloint2double((int)hi, (int)(a << 29));
+}
+
+// r and 1/r^2 of a double-float r^2 in the normal range
+__device__ __forceinline__ df met_dist(df r2, df* inv) {
+  const float rs = rsqrtf(r2.hi);
+  const float s = __fmul_rn(r2.hi, rs);
+  const df ss = two_prod(s, s);
+  const float e = __fadd_rn(__fsub_rn(__fsub_rn(r2.hi, ss.hi), ss.lo), r2.lo);
+  if (inv) {
+    const float q = __fmul_rn(rs, rs);
+    const float g = __fmaf_rn(-r2.lo, q, __fmaf_rn(-r2.hi, q, 1.f));  // 1 - r2 q, about 2^-21
+    *inv = quick_two_sum(q, __fmul_rn(q, __fmaf_rn(g, g, g)));
+  }
+  return quick_two_sum(s, __fmul_rn(__fmul_rn(0.5f, rs), e));
+}
+
+// table point l and fraction p in [-0.5, 0.5] of a double-float r; false at a table's ends
+__device__ __forceinline__ bool met_coord(const MetTab& t, df r, int* l, df* p) {
+  float k = rintf(__fmaf_rn(r.hi, t.rdr_h, t.nr_h));
+  const df pr = two_prod(r.hi, t.rdr_h);
+  const float e = __fmaf_rn(r.hi, t.rdr_l, __fmaf_rn(r.lo, t.rdr_h, pr.lo));
+  const df c = two_sum(t.nr_h, -k);
+  const df s = two_sum(pr.hi, c.hi);
+  df d = quick_two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(e, __fadd_rn(c.lo, t.nr_l))));
+  if (fabsf(d.hi) > 0.5f) {  // the FP32 nearest integer was the other neighbour
+    const float o = copysignf(1.f, d.hi);
+    k += o;
+    d = quick_two_sum(__fsub_rn(d.hi, o), d.lo);
+  }
+  *l = (int)k;
+  *p = d;
+  return k > 5.f && k < (float)(t.n - 1);
+}
+
+__device__ __forceinline__ df met_poly(const CoefF* __restrict__ c, int l, df p) {
+  const float4 a = *reinterpret_cast<const float4*>(&c[l].c0h);
+  const float2 b = *reinterpret_cast<const float2*>(&c[l].c2h);
+  const df t = df_fma(p, df_make(b.x, b.y), df_make(a.z, a.w));
+  return df_fma(p, t, df_make(a.x, a.y));
+}
+
+// +1 inside a table's reach, 0 beyond it, -1 too near its end for FP32
+__device__ __forceinline__ int met_in(const MetTab& t, float r2) { return r2 < t.f_lo ? 1 : r2 > t.f_hi ? 0 : -1; }
+
+__device__ __forceinline__ bool met_plain(float r2) { return r2 > 1e-10f && r2 < 1e10f; }
+
+// FP64 terms of one pair, as the atom-index kernels form them
+__device__ __noinline__ void metal_density_slow(const MetArgs& A, const MetTab& ti, const MetTab& tj, bool same, double dx,
+                                                double dy, double dz, double* to_i, double* to_j, bool* bad) {
+  const double rsq = dx * dx + dy * dy + dz * dz;
+  const long long rb = __double_as_longlong(rsq);
+  *to_i = *to_j = 0.0;
+  const bool in_j = tj.n > 5 && within(rb, tj.b_lo, tj.b_hi, rsq, tj.rmax);
+  const bool in_i = !same && ti.n > 5 && within(rb, ti.b_lo, ti.b_hi, rsq, ti.rmax);
+  if (!in_j && !in_i) return;
+  double rinv;
+  const double r = dist_from(rsq, rb, &rinv);
+  int l = 0;
+  double p = 0.0;
+  if (in_j) {
+    if (!qindex(tj, r, &l, &p)) *bad = true;
+    *to_i = density_at(A, tj, l, p);
+    if (same) *to_j = *to_i;
+  }
+  if (in_i) {
+    if (!qindex(ti, r, &l, &p)) *bad = true;
+    *to_j = density_at(A, ti, l, p);
+  }
+}
+
+// false beyond the cutoff; num = gamma r^2
+__device__ __noinline__ bool metal_force_slow(const MetArgs& A, const MetTab& tp, const MetTab& ti, const MetTab& tj,
+                                              bool same, double dx, double dy, double dz, double fi, double fj,
+                                              double* num, double* gamma, double* eng, bool* bad) {
+  const double rsq = dx * dx + dy * dy + dz * dz;
+  const long long rb = __double_as_longlong(rsq);
+  *num = *gamma = *eng = 0.0;
+  if (!within(rb, A.b_rc_lo, A.b_rc_hi, rsq, A.rcut)) return false;
+  double rinv, gamma1 = 0.0, gamma2 = 0.0, gamma3 = 0.0, p = 0.0;
+  const double r = dist_from(rsq, rb, &rinv);
+  int l = 0;
+  if (tp.n > 0 && within(rb, tp.b_lo, tp.b_hi, rsq, tp.rmax)) {
+    if (!qindex(tp, r, &l, &p)) *bad = true;
+    gamma1 = qeval_full(A.cd + tp.off, A.d + tp.off, l, p);
+    *eng = qeval_full(A.cv + tp.off, A.v + tp.off, l, p);
+  }
+  if (tj.n > 0 && ti.n > 5 && within(rb, tj.b_lo, tj.b_hi, rsq, tj.rmax)) {
+    if (!qindex(tj, r, &l, &p)) *bad = true;
+    gamma2 = qeval_full(A.cd + tj.off, A.d + tj.off, l, p);
+  }
+  if (same) {
+    gamma3 = gamma2;
+  } else if (ti.n > 5 && within(rb, ti.b_lo, ti.b_hi, rsq, ti.rmax)) {
+    if (!qindex(ti, r, &l, &p)) *bad = true;
+    gamma3 = qeval_full(A.cd + ti.off, A.d + ti.off, l, p);
+  }
+  *num = gamma1 + (gamma2 * fi + gamma3 * fj);
+  *gamma = *num * (rinv * rinv);
+  return true;
+}
+
+// The partners of the atom at sorted position p (list row i), 32 MET_U entries at a time
+// through the FP32 test, then 32 at a time through eval(j).
+template <typename Eval>
+__device__ __forceinline__ void met_walk(const MetSorted& S, int i, float4 pi, int* q, Eval eval) {
+  const int lane = threadIdx.x & 31;
+  const unsigned lt = (1u << lane) - 1u;
+  const int n = S.list[(size_t)i * S.ld + 3];
+  const int* sp = S.spos + (size_t)i * S.ldt;
+  int nq = 0;
+  for (int base = 0;; base += 32 * MET_U) {
+    const bool more = base < n;
+    if (more) {
+      int jv[MET_U];
+      float4 pv[MET_U];
+#pragma unroll
+      for (int u = 0; u < MET_U; ++u) {
+        const int m = base + 32 * u + lane + 1;
+        jv[u] = m <= n ? sp[m] : -1;
+      }
+#pragma unroll
+      for (int u = 0; u < MET_U; ++u) pv[u] = jv[u] >= 0 ? S.xhs[jv[u]] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+      for (int u = 0; u < MET_U; ++u) {
+        const float ex = pi.x - pv[u].x, ey = pi.y - pv[u].y, ez = pi.z - pv[u].z;
+        const bool keep = jv[u] >= 0 && fmaf(ex, ex, fmaf(ey, ey, ez * ez)) <= S.f_pre;
+        const unsigned b = __ballot_sync(0xffffffffu, keep);
+        if (keep) q[nq + __popc(b & lt)] = jv[u];
+        nq += __popc(b);
+      }
+      __syncwarp();
+    }
+    while (nq >= 32 || (!more && nq > 0)) {
+      const int take = min(nq, 32);
+      if (lane < take) eval(q[nq - take + lane]);
+      nq -= take;
+      __syncwarp();  // the taken slots are read before the next pass appends over them
+    }
+    if (!more) break;
+  }
+}
+
+__device__ __forceinline__ dacc dacc_xor(dacc a, int o) {
+  const float s = __shfl_xor_sync(0xffffffffu, a.s, o), c = __shfl_xor_sync(0xffffffffu, a.c, o);
+  const df u = two_sum(a.s, s);
+  dacc r;
+  r.s = u.hi;
+  r.c = __fadd_rn(__fadd_rn(a.c, c), u.lo);
+  return r;
+}
+
+__global__ void __launch_bounds__(MET_NT) k_metal_density_sorted(MetSorted S, MetArgs A) {
+  __shared__ MetTab tabs[MAX_TAB];
+  __shared__ int queue[MET_NT / 32][32 * (MET_U + 1)];
+  stage_tables(A, tabs);
+  const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
+  bool bad = false;
+  const int per = (S.natms + gridDim.x - 1) / gridDim.x;
+  const int a_end = min(S.natms, (int)(blockIdx.x + 1) * per);
+  for (int a = blockIdx.x * per + wq; a < a_end; a += MET_NT / 32) {
+    const int p = S.loc_sp[a], i = S.at_list[p];
+    const MetRec ri = S.rec[p];
+    const int ai = ri.type;
+    const MetTab& ti = tabs[A.nkey + ai - 1];
+    dacc rho = {0.f, 0.f};
+    met_walk(S, i, S.xhs[p], queue[wq], [&](int j) {
+      const MetRec rj = S.rec[j];
+      const bool same = rj.type == ai;
+      const MetTab& tj = tabs[A.nkey + rj.type - 1];
+      const df dx = pos_diff(ri.x, rj.x), dy = pos_diff(ri.y, rj.y), dz = pos_diff(ri.z, rj.z);
+      const df r2 = df_norm2(dx, dy, dz);
+      const int in_j = met_in(tj, r2.hi), in_i = same ? in_j : met_in(ti, r2.hi);
+      if (in_j == 0 && in_i == 0) return;
+      bool slow = in_j < 0 || in_i < 0 || !met_plain(r2.hi);
+      df to_i = df_make(0.f, 0.f), to_j = to_i;
+      if (!slow) {
+        const df r = met_dist(r2, nullptr);
+        int l = 0;
+        df f;
+        if (in_j) {
+          slow = !met_coord(tj, r, &l, &f);
+          if (!slow) {
+            to_i = met_poly(S.fv + tj.off, l, f);
+            slow = to_i.hi < 0.f;
+          }
+          if (same) to_j = to_i;
+        }
+        if (!same && in_i && !slow) {
+          if (!(in_j && ti.grid == tj.grid)) slow = !met_coord(ti, r, &l, &f);
+          if (!slow) {
+            to_j = met_poly(S.fv + ti.off, l, f);
+            slow = to_j.hi < 0.f;
+          }
+        }
+      }
+      double dj;
+      if (slow) {
+        const int jj = S.at_list[j];
+        double di;
+        metal_density_slow(A, ti, tj, same, S.x[i] - S.x[jj], S.y[i] - S.y[jj], S.z[i] - S.z[jj], &di, &dj, &bad);
+        df_split(di, &to_i.hi, &to_i.lo);
+      } else {
+        dj = flt_dbl(to_j.hi) + flt_dbl(to_j.lo);
+      }
+      dacc_add(rho, to_i);
+      if (__double_as_longlong(dj) != 0) atomicAdd(&S.s0[j], dj);
+    });
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) rho = dacc_xor(rho, o);
+    if (lane == 0) atomicAdd(&S.s0[p], dacc_value(rho));
+  }
+  if (bad) atomicOr(S.status, ST_METAL_TABLE);
+}
+
+// densities per sorted position onto the atoms
+__global__ void k_metal_rho_fold(int natms, const DevScalars* sc, const int* __restrict__ at_list,
+                                 const int* __restrict__ src, const double* __restrict__ s0, double* rho) {
+  const int p = blockIdx.x * blockDim.x + threadIdx.x;
+  if (p >= sc->nlast) return;
+  const double v = s0[p];
+  if (__double_as_longlong(v) == 0) return;
+  const int a = at_list[p];
+  atomicAdd(&rho[a < natms ? a : src[a]], v);
+}
+
+// metal_ld_set_halo per sorted position: F'(rho) of the atom or of an image's source
+__global__ void k_metal_fp(const DevScalars* sc, const int* __restrict__ src, const int* __restrict__ sorted_pos,
+                           const double* __restrict__ rho, float2* __restrict__ fp) {
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= sc->nlast) return;
+  float h, l;
+  df_split(rho[src[i]], &h, &l);
+  fp[sorted_pos[i]] = make_float2(h, l);
+}
+
+__global__ void __launch_bounds__(MET_NT) k_metal_forces_sorted(MetSorted S, MetArgs A) {
+  __shared__ MetTab tabs[MAX_TAB];
+  __shared__ int queue[MET_NT / 32][32 * (MET_U + 1)];
+  stage_tables(A, tabs);
+  const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
+  dacc e_eng = {0.f, 0.f}, e_vir = {0.f, 0.f};
+  bool bad = false;
+  unsigned long long n_list = 0;
+  int n_rc = 0;
+  const int per = (S.natms + gridDim.x - 1) / gridDim.x;
+  const int a_end = min(S.natms, (int)(blockIdx.x + 1) * per);
+  for (int a = blockIdx.x * per + wq; a < a_end; a += MET_NT / 32) {
+    const int p = S.loc_sp[a], i = S.at_list[p];
+    const MetRec ri = S.rec[p];
+    const int ai = ri.type;
+    const float2 f2 = S.fp[p];
+    const df fpi = df_make(f2.x, f2.y);
+    const MetTab& ti = tabs[A.nkey + ai - 1];
+    dacc fx = {0.f, 0.f}, fy = fx, fz = fx;
+    n_list += (unsigned long long)S.list[(size_t)i * S.ld + 3];
+    met_walk(S, i, S.xhs[p], queue[wq], [&](int j) {
+      const MetRec rj = S.rec[j];
+      const int aj = rj.type;
+      const MetTab& tp = tabs[(ai > aj ? ai * (ai - 1) / 2 + aj : aj * (aj - 1) / 2 + ai) - 1];
+      if (!tp.listed) return;  // keypot = -1
+      const df dx = pos_diff(ri.x, rj.x), dy = pos_diff(ri.y, rj.y), dz = pos_diff(ri.z, rj.z);
+      const df r2 = df_norm2(dx, dy, dz);
+      if (r2.hi > S.f_rc_hi) return;
+      const bool same = aj == ai;
+      const MetTab& tj = tabs[A.nkey + aj - 1];
+      const int in_p = met_in(tp, r2.hi), in_j = ti.n > 5 ? met_in(tj, r2.hi) : 0,
+                in_i = same ? in_j : met_in(ti, r2.hi);
+      bool slow = r2.hi > S.f_rc_lo || in_p < 0 || in_j < 0 || in_i < 0 || !met_plain(r2.hi);
+      const float2 fq = S.fp[j];
+      df gam = df_make(0.f, 0.f), num = gam, eng = gam;
+      if (!slow) {
+        df inv, f;
+        const df r = met_dist(r2, &inv);
+        int l = 0, gl = -1;
+        if (in_p) {
+          slow = !met_coord(tp, r, &l, &f);
+          gl = tp.grid;
+          if (!slow) {
+            num = met_poly(S.fd + tp.off, l, f);
+            eng = met_poly(S.fv + tp.off, l, f);
+          }
+        }
+        df g = df_make(0.f, 0.f);
+        if (in_j && !slow) {
+          if (tj.grid != gl) slow = !met_coord(tj, r, &l, &f);
+          gl = tj.grid;
+          if (!slow) {
+            g = met_poly(S.fd + tj.off, l, f);
+            // one table for both when the types are equal: g (F'_i + F'_j)
+            num = df_fma(g, same ? df_add(fpi, df_make(fq.x, fq.y)) : fpi, num);
+          }
+        }
+        if (!same && in_i && !slow) {
+          if (ti.grid != gl) slow = !met_coord(ti, r, &l, &f);
+          if (!slow) {
+            g = met_poly(S.fd + ti.off, l, f);
+            num = df_fma(g, df_make(fq.x, fq.y), num);
+          }
+        }
+        gam = df_mul(num, inv);
+        slow = slow || !(fabsf(num.hi) < 1e30f && fabsf(gam.hi) < 1e25f);
+      }
+      if (slow) {
+        const int jj = S.at_list[j];
+        double n64, g64, e64;
+        const double x = S.x[i] - S.x[jj], y = S.y[i] - S.y[jj], z = S.z[i] - S.z[jj];
+        if (!metal_force_slow(A, tp, ti, tj, same, x, y, z, S.rho[i],
+                              (double)fq.x + (double)fq.y, &n64, &g64, &e64, &bad)) return;
+        ++n_rc;
+        // summed in FP64, whatever their size
+        df_split(e64, &eng.hi, &eng.lo);
+        df_split(n64, &num.hi, &num.lo);
+        atomicAdd(&S.s0[p], g64 * x); atomicAdd(&S.s1[p], g64 * y); atomicAdd(&S.s2[p], g64 * z);
+        atomicAdd(&S.s0[j], -g64 * x); atomicAdd(&S.s1[j], -g64 * y); atomicAdd(&S.s2[j], -g64 * z);
+        dacc_add(e_eng, eng);
+        dacc_add(e_vir, df_neg(num));
+        return;
+      }
+      ++n_rc;
+      dacc_add(e_eng, eng);
+      dacc_add(e_vir, df_neg(num));
+      // the products as an exact high part and the sum of the rest
+      auto term = [&](df d, dacc& s, double* slot) {
+        const df t = two_prod(gam.hi, d.hi);
+        const float c = __fmaf_rn(gam.hi, d.lo, __fmaf_rn(gam.lo, d.hi, t.lo));
+        const df u = two_sum(s.s, t.hi);
+        s.s = u.hi;
+        s.c = __fadd_rn(s.c, __fadd_rn(u.lo, c));
+        atomicAdd(&slot[j], -(flt_dbl(t.hi) + flt_dbl(c)));
+      };
+      term(dx, fx, S.s0);
+      term(dy, fy, S.s1);
+      term(dz, fz, S.s2);
+    });
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      fx = dacc_xor(fx, o);
+      fy = dacc_xor(fy, o);
+      fz = dacc_xor(fz, o);
+    }
+    if (lane == 0) {
+      atomicAdd(&S.s0[p], dacc_value(fx));
+      atomicAdd(&S.s1[p], dacc_value(fy));
+      atomicAdd(&S.s2[p], dacc_value(fz));
+    }
+  }
+  if (bad) atomicOr(S.status, ST_METAL_TABLE);
+  if (S.cnt) {
+    n_rc = warp_sumi(n_rc);
+    if (lane == 0) {
+      atomicAdd(&S.cnt[0], n_list);
+      atomicAdd(&S.cnt[1], (unsigned long long)n_rc);
+    }
+  }
+  dfr out[2] = {to_dfr(two_sum(e_eng.s, e_eng.c)), to_dfr(two_sum(e_vir.s, e_vir.c))};
+  block_reduce_store<2>(out, S.blk);
+}
+
+// stress (sum over slots of x (x) F, every halo image at its own position) and each slot's
+// force onto its atom, as the pair kernels' k_slot_stress_fold
+__global__ void k_metal_force_fold(int natms, const DevScalars* sc, const int* __restrict__ at_list,
+                                   const int* __restrict__ src, const double* __restrict__ x,
+                                   const double* __restrict__ y, const double* __restrict__ z,
+                                   const double* __restrict__ s0, const double* __restrict__ s1,
+                                   const double* __restrict__ s2, double* fx, double* fy, double* fz, double* blk) {
+  const int nlast = sc->nlast;
+  double st[6] = {0, 0, 0, 0, 0, 0};
+  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < nlast; p += gridDim.x * blockDim.x) {
+    const double fa = s0[p], fb = s1[p], fc = s2[p];
+    if ((__double_as_longlong(fa) | __double_as_longlong(fb) | __double_as_longlong(fc)) == 0) continue;
+    const int a = at_list[p];
+    const double xa = x[a], ya = y[a], za = z[a];
+    st[0] = fma(xa, fa, st[0]); st[1] = fma(xa, fb, st[1]); st[2] = fma(xa, fc, st[2]);
+    st[3] = fma(ya, fb, st[3]); st[4] = fma(ya, fc, st[4]); st[5] = fma(za, fc, st[5]);
+    const int tgt = a < natms ? a : src[a];
+    atomicAdd(&fx[tgt], fa);
+    atomicAdd(&fy[tgt], fb);
+    atomicAdd(&fz[tgt], fc);
+  }
+  block_reduce_store<6>(st, blk);
+}
+
 // ------------------------------------------------------------------- host state
 MetTab* d_tab = nullptr;
 double* d_val = nullptr;
@@ -359,6 +819,13 @@ Coef* d_cd = nullptr;
 int* d_listed = nullptr;
 double* d_rho = nullptr;
 int n_key = 0, n_tab = 0, occ_dens = 0, occ_force = 0;
+// sorted-position kernels
+CoefF *d_fv = nullptr, *d_fd = nullptr;
+MetRec* d_rec = nullptr;
+float2* d_fp = nullptr;
+double* d_slot = nullptr;     // 3 x mxatms: density or force sums per sorted position
+int occ_dens_s = 0, occ_force_s = 0;
+double max_rmax = 0.0;        // largest reach of a density table
 
 // metal_table_derivatives: five-point derivative on the normalised neighbours
 void table_derivatives(const std::vector<double>& buf, std::vector<double>& der) {
@@ -400,11 +867,12 @@ void table_derivatives(const std::vector<double>& buf, std::vector<double>& der)
 }  // namespace
 
 void metal_free() {
-  void* p[] = {d_tab, d_val, d_der, d_cv, d_cd, d_listed, d_rho};
+  void* p[] = {d_tab, d_val, d_der, d_cv, d_cd, d_listed, d_rho, d_fv, d_fd, d_rec, d_fp, d_slot};
   for (void* q : p)
     if (q) cudaFree(q);
   d_tab = nullptr; d_val = nullptr; d_der = nullptr; d_cv = nullptr; d_cd = nullptr; d_listed = nullptr;
   d_rho = nullptr;
+  d_fv = d_fd = nullptr; d_rec = nullptr; d_fp = nullptr; d_slot = nullptr;
   n_key = n_tab = 0;
   g.has_metal = false;
 }
@@ -417,6 +885,7 @@ bool metal_active() { return g.has_metal; }
 int metal_setup(int ntab, const int32_t* kind, const int32_t* t1, const int32_t* t2, const int32_t* ngrid,
                 const double* start, const double* finish, const double* values, const int32_t* listed) {
   metal_free();
+  max_rmax = 0.0;
   const int nt = g.p.ntypes;
   n_key = nt * (nt + 1) / 2;
   n_tab = n_key + 2 * nt;
@@ -425,6 +894,8 @@ int metal_setup(int ntab, const int32_t* kind, const int32_t* t1, const int32_t*
   for (auto& t : tab) {
     t.n = 0; t.off = 0; t.r0 = t.rmax = t.dr = t.rdr = t.nr0rdr = 0.0; t.grid = -1; t.listed = 0;
     t.b_lo = t.b_hi = 0;
+    t.f_lo = t.f_hi = -1.f;
+    t.rdr_h = t.rdr_l = t.nr_h = t.nr_l = 0.f;
   }
   std::vector<double> val(1, 0.0), der(1, 0.0);
   size_t pos = 0;
@@ -500,7 +971,36 @@ int metal_setup(int ntab, const int32_t* kind, const int32_t* t1, const int32_t*
     t.nr0rdr = -t.r0 * t.rdr;
     t.b_lo = bits(t.rmax * t.rmax * (1.0 - 1e-12));
     t.b_hi = bits(t.rmax * t.rmax * (1.0 + 1e-12));
+    if (id < n_key + nt) {  // tables of r
+      t.f_lo = (float)(t.rmax * t.rmax * (1.0 - 1e-6));
+      t.f_hi = (float)(t.rmax * t.rmax * (1.0 + 1e-6));
+      df_split(t.rdr, &t.rdr_h, &t.rdr_l);
+      df_split(t.nr0rdr, &t.nr_h, &t.nr_l);
+      if (id >= n_key) max_rmax = std::max(max_rmax, t.rmax);
+    }
   }
+  auto split_coef = [](const std::vector<Coef>& c) {
+    std::vector<CoefF> f(c.size());
+    for (size_t k = 0; k < c.size(); ++k) {
+      CoefF& o = f[k];
+      df_split(c[k].c0, &o.c0h, &o.c0l);
+      df_split(c[k].c1, &o.c1h, &o.c1l);
+      df_split(c[k].c2, &o.c2h, &o.c2l);
+      o.pad0 = o.pad1 = 0.f;
+    }
+    return f;
+  };
+  const std::vector<CoefF> fv = split_coef(cv), fd = split_coef(cd);
+  const size_t mx = std::max(g.mxatms, 1);
+  GB_CUDA(cudaMalloc(&d_fv, sizeof(CoefF) * fv.size()));
+  GB_CUDA(cudaMalloc(&d_fd, sizeof(CoefF) * fd.size()));
+  GB_CUDA(cudaMemcpy(d_fv, fv.data(), sizeof(CoefF) * fv.size(), cudaMemcpyHostToDevice));
+  GB_CUDA(cudaMemcpy(d_fd, fd.data(), sizeof(CoefF) * fd.size(), cudaMemcpyHostToDevice));
+  GB_CUDA(cudaMalloc(&d_rec, sizeof(MetRec) * mx));
+  GB_CUDA(cudaMalloc(&d_fp, sizeof(float2) * mx));
+  GB_CUDA(cudaMalloc(&d_slot, sizeof(double) * 3 * mx));
+  GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_dens_s, k_metal_density_sorted, MET_NT, 0));
+  GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_force_s, k_metal_forces_sorted, MET_NT, 0));
   GB_CUDA(cudaMalloc(&d_tab, sizeof(MetTab) * n_tab));
   GB_CUDA(cudaMalloc(&d_val, sizeof(double) * val.size()));
   GB_CUDA(cudaMalloc(&d_der, sizeof(double) * der.size()));
@@ -520,18 +1020,78 @@ int metal_setup(int ntab, const int32_t* kind, const int32_t* t1, const int32_t*
   return GB_OK;
 }
 
-// both passes; adds forces into g.fx/fy/fz and stress into stress9; returns
-// engmet, virmet (pair part) and engden, virden (embedding part) in e4
-void metal_forces(double* e4, double* stress9) {
+// The double-float kernels where the list pairs every halo entry with its backward copy and
+// the fixed-point positions and separations hold (the list's reach below 16 A, the box
+// and its halo below 2^14 A); the FP64 form by instructions keeps the FP64 kernels.
+static bool use_sorted_metal() {
+  return g.spos_valid && g.use_sorted && !g.fp64_native && g.rcutx < 15.9 && 1.5 * g.cell[0] < 16384.0 &&
+         max_rmax < 1.0e4;
+}
+
+static void metal_forces_sorted(const MetArgs& A, unsigned long long* cnt) {
   cudaStream_t st = g.stream;
-  MetArgs A;
-  A.tab = d_tab; A.v = d_val; A.d = d_der; A.cv = d_cv; A.cd = d_cd; A.listed = d_listed;
-  A.nkey = n_key; A.ntypes = g.p.ntypes; A.ntab = n_tab; A.rcut = g.p.rcut;
-  {
-    const double rc2 = g.p.rcut * g.p.rcut, lo = rc2 * (1.0 - 1e-12), hi = rc2 * (1.0 + 1e-12);
-    std::memcpy(&A.b_rc_lo, &lo, 8);
-    std::memcpy(&A.b_rc_hi, &hi, 8);
-  }
+  const int T = 256, mx = g.mxatms, nbm = nblocks(mx, T);
+  MetSorted S;
+  S.natms = g.natms;
+  S.at_list = g.at_list; S.loc_sp = g.loc_sp; S.list = g.list; S.spos = g.spos; S.ld = g.ld; S.ldt = g.ldt;
+  S.xhs = g.xhs; S.rec = d_rec;
+  S.x = g.x; S.y = g.y; S.z = g.z; S.rho = d_rho;
+  S.fv = d_fv; S.fd = d_fd; S.fp = d_fp;
+  S.s0 = d_slot; S.s1 = d_slot + mx; S.s2 = d_slot + 2 * (size_t)mx;
+  S.status = &g.sc->status;
+  const double rc2 = g.p.rcut * g.p.rcut;
+  S.f_rc_lo = (float)(rc2 * (1.0 - 1e-6));
+  S.f_rc_hi = (float)(rc2 * (1.0 + 1e-6));
+  // the FP32 test of the high parts: coordinates below R have rounding errors below u
+  auto pre = [](double r2) {
+    const double u = std::ldexp(1.0, std::ilogb(1.5 * g.cell[0]) - 23), D = std::sqrt(r2) + 1.0;
+    const double dlt = 2.0 * u + std::ldexp(1.0, -23) * (D + 2.0 * u);
+    const double band = 4.0 * (2.0 * std::sqrt(3.0) * D * dlt + 3.0 * dlt * dlt) + 8.0 * std::ldexp(1.0, -23) * D * D;
+    return std::nextafter((float)(r2 + band), 3.0e38f);
+  };
+  // short-lived CTAs of at most 16 atoms per warp, in runs of consecutive sorted positions;
+  // a small system keeps one CTA per resident slot
+  auto blocks = [&](int occ) {
+    const int per = std::max(1, std::min(16, g.natms / ((MET_NT / 32) * std::max(1, occ) * g.nsm)));
+    return std::max(1, nblocks(g.natms, (MET_NT / 32) * per));
+  };
+  const int nbd = blocks(occ_dens_s), nbf = blocks(occ_force_s), nbe = nblocks(g.natms, T),
+            nbs = std::max(1, std::min(nbm, 4 * g.nsm));
+  double* blk = gb_blkacc(nbe + 2 * nbf + 6 * nbs);
+  double *blk2 = blk + nbe, *blk3 = blk2 + 2 * (size_t)nbf;
+  S.blk = blk2;
+  S.cnt = cnt;
+  prof_begin(P_METAL_DENSITY);
+  k_metal_records<<<nbm, T, 0, st>>>(g.sc, g.sorted_pos, g.x, g.y, g.z, g.ltype, d_rec);
+  GB_LAUNCHED();
+  GB_CUDA(cudaMemsetAsync(d_slot, 0, sizeof(double) * (size_t)mx, st));
+  GB_CUDA(cudaMemsetAsync(d_rho, 0, sizeof(double) * (size_t)g.natms, st));
+  S.f_pre = pre(max_rmax * max_rmax * (1.0 + 1e-6));
+  k_metal_density_sorted<<<nbd, MET_NT, 0, st>>>(S, A);
+  GB_LAUNCHED();
+  k_metal_rho_fold<<<nbm, T, 0, st>>>(g.natms, g.sc, g.at_list, g.src, d_slot, d_rho);
+  GB_LAUNCHED();
+  k_metal_embed<<<nbe, T, 0, st>>>(g.natms, g.ltype, A, d_rho, blk, &g.sc->status);
+  GB_LAUNCHED();
+  gb_reduce_blocks(blk, nbe, 1, &g.sc->acc[A_METAL + 8]);
+  k_metal_fp<<<nbm, T, 0, st>>>(g.sc, g.src, g.sorted_pos, d_rho, d_fp);
+  GB_LAUNCHED();
+  prof_end(P_METAL_DENSITY);
+  prof_begin(P_METAL_FORCES);
+  GB_CUDA(cudaMemsetAsync(d_slot, 0, sizeof(double) * 3 * (size_t)mx, st));
+  S.f_pre = pre(rc2 * (1.0 + 1e-6));
+  k_metal_forces_sorted<<<nbf, MET_NT, 0, st>>>(S, A);
+  GB_LAUNCHED();
+  k_metal_force_fold<<<nbs, T, 0, st>>>(g.natms, g.sc, g.at_list, g.src, g.x, g.y, g.z, S.s0, S.s1, S.s2, g.fx, g.fy,
+                                        g.fz, blk3);
+  GB_LAUNCHED();
+  gb_reduce_blocks(blk2, nbf, 2, &g.sc->acc[A_METAL]);
+  gb_reduce_blocks(blk3, nbs, 6, &g.sc->acc[A_METAL + 2]);
+  prof_end(P_METAL_FORCES);
+}
+
+static void metal_forces_fp64(const MetArgs& A, unsigned long long* cnt) {
+  cudaStream_t st = g.stream;
   const int T = 256;
   GB_CUDA(cudaMemsetAsync(d_rho, 0, sizeof(double) * g.mxatms, st));
   prof_begin(P_METAL_DENSITY);
@@ -550,16 +1110,31 @@ void metal_forces(double* e4, double* stress9) {
   prof_begin(P_METAL_FORCES);
   nb = std::max(1, std::min(nblocks((long long)g.mxatms * 32, T), occ_force * g.nsm));
   double* blk2 = blk + std::max(nbe, 1);
-  unsigned long long* cnt = nullptr;
-  if (!g.has_coul && !g.has_vdw) {  // the pair kernel did not run: count here
-    GB_CUDA(cudaMemsetAsync(&g.sc->npairs_list, 0, 2 * sizeof(unsigned long long), st));
-    cnt = &g.sc->npairs_list;
-  }
   k_metal_forces<<<nb, T, 0, st>>>(g.natms, g.sc, g.at_list, g.list, g.ld, g.x, g.y, g.z, g.ltype, g.ltg, g.src, A,
                                    d_rho, g.fx, g.fy, g.fz, blk2, &g.sc->status, cnt);
   GB_LAUNCHED();
   gb_reduce_blocks(blk2, nb, MACC, &g.sc->acc[A_METAL]);
   prof_end(P_METAL_FORCES);
+}
+
+// both passes; adds forces into g.fx/fy/fz and stress into stress9; returns
+// engmet, virmet (pair part) and engden, virden (embedding part) in e4
+void metal_forces(double* e4, double* stress9) {
+  MetArgs A;
+  A.tab = d_tab; A.v = d_val; A.d = d_der; A.cv = d_cv; A.cd = d_cd; A.listed = d_listed;
+  A.nkey = n_key; A.ntypes = g.p.ntypes; A.ntab = n_tab; A.rcut = g.p.rcut;
+  {
+    const double rc2 = g.p.rcut * g.p.rcut, lo = rc2 * (1.0 - 1e-12), hi = rc2 * (1.0 + 1e-12);
+    std::memcpy(&A.b_rc_lo, &lo, 8);
+    std::memcpy(&A.b_rc_hi, &hi, 8);
+  }
+  unsigned long long* cnt = nullptr;
+  if (!g.has_coul && !g.has_vdw) {  // the pair kernel did not run: count here
+    GB_CUDA(cudaMemsetAsync(&g.sc->npairs_list, 0, 2 * sizeof(unsigned long long), g.stream));
+    cnt = &g.sc->npairs_list;
+  }
+  if (use_sorted_metal()) metal_forces_sorted(A, cnt);
+  else metal_forces_fp64(A, cnt);
   gb_sync_scalars();
   if (g.hsc->status & ST_METAL_DENSITY) throw (int)GB_ERR_METAL_DENSITY;
   if (g.hsc->status & ST_METAL_TABLE) throw (int)GB_ERR_METAL_TABLE;
