@@ -360,8 +360,9 @@ __global__ void __launch_bounds__(256, 3) k_metal_forces(int natms, const DevSca
 // (1/64 of the FP32 rate): 95 FP64 instructions per 32 list entries, executed for whole
 // warps although a fifth of the entries lie beyond the cutoff.  Here an FP32 test of the
 // high parts queues the entries that may be inside, and 32 queued pairs at a time are
-// evaluated with every lane busy.  256,000 atoms: density 1.97 -> DENS ms, forces 4.35 ->
-// FORC ms.
+// evaluated with every lane busy.  256,000 atoms: density 1.97 -> 0.42 ms, forces 4.35 ->
+// 0.83 ms (1.04 with 102 registers, two CTAs per SM; a fourth CTA spills and gains
+// nothing); latency of the partners and tables, at a third of the issue slots.
 //   positions   int64 in units of 2^-48 A (exact for |x| >= 16 A): the separation is an
 //               exact integer difference
 //   r           relative error about 1e-14 (an FP32 square root and the first-order
@@ -663,7 +664,7 @@ __global__ void k_metal_fp(const DevScalars* sc, const int* __restrict__ src, co
   fp[sorted_pos[i]] = make_float2(h, l);
 }
 
-__global__ void __launch_bounds__(MET_NT) k_metal_forces_sorted(MetSorted S, MetArgs A) {
+__global__ void __launch_bounds__(MET_NT, 3) k_metal_forces_sorted(MetSorted S, MetArgs A) {
   __shared__ MetTab tabs[MAX_TAB];
   __shared__ int queue[MET_NT / 32][32 * (MET_U + 1)];
   stage_tables(A, tabs);
@@ -1050,9 +1051,9 @@ static void metal_forces_sorted(const MetArgs& A, unsigned long long* cnt) {
     return std::nextafter((float)(r2 + band), 3.0e38f);
   };
   // short-lived CTAs of at most 16 atoms per warp, in runs of consecutive sorted positions;
-  // a small system keeps one CTA per resident slot
+  // a small system has at most one CTA per resident slot
   auto blocks = [&](int occ) {
-    const int per = std::max(1, std::min(16, g.natms / ((MET_NT / 32) * std::max(1, occ) * g.nsm)));
+    const int per = std::max(1, std::min(16, nblocks(g.natms, (MET_NT / 32) * std::max(1, occ) * g.nsm)));
     return std::max(1, nblocks(g.natms, (MET_NT / 32) * per));
   };
   const int nbd = blocks(occ_dens_s), nbf = blocks(occ_force_s), nbe = nblocks(g.natms, T),
