@@ -757,7 +757,7 @@ struct PairSortedArgs {
   const double* vsig;
   int ntypes;
   float rc2, rv2, alpha, a2rp, scaling;  // mixed form
-  unsigned long long* fixs;
+  unsigned long long *f0, *f1, *f2;  // fixed-point x, y, z forces per sorted position
   double* blk;
   unsigned long long* cnt;
   const DevScalars* sc;
@@ -1005,9 +1005,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_pair_sorted(PairSortedArgs A,
           if (hit) {
             ++n_rc;
             sx += ix; sy += iy; sz += iz;
-            atomicAdd(&A.fixs[3 * (size_t)j + 0], (unsigned long long)(-ix));
-            atomicAdd(&A.fixs[3 * (size_t)j + 1], (unsigned long long)(-iy));
-            atomicAdd(&A.fixs[3 * (size_t)j + 2], (unsigned long long)(-iz));
+            atomicAdd(&A.f0[j], (unsigned long long)(-ix));
+            atomicAdd(&A.f1[j], (unsigned long long)(-iy));
+            atomicAdd(&A.f2[j], (unsigned long long)(-iz));
           }
         }
         nq -= take;
@@ -1026,9 +1026,9 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_pair_sorted(PairSortedArgs A,
       sz += __shfl_xor_sync(0xffffffffu, sz, o);
     }
     if (lane == 0) {
-      atomicAdd(&A.fixs[3 * (size_t)p + 0], (unsigned long long)sx);
-      atomicAdd(&A.fixs[3 * (size_t)p + 1], (unsigned long long)sy);
-      atomicAdd(&A.fixs[3 * (size_t)p + 2], (unsigned long long)sz);
+      atomicAdd(&A.f0[p], (unsigned long long)sx);
+      atomicAdd(&A.f1[p], (unsigned long long)sy);
+      atomicAdd(&A.f2[p], (unsigned long long)sz);
       n_list += (unsigned long long)n;
     }
   }
@@ -1049,12 +1049,13 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_pair_sorted(PairSortedArgs A,
 __global__ void k_slot_stress_fold(int natms, const DevScalars* sc, const int* __restrict__ at_list,
                                    const int* __restrict__ src, const double* __restrict__ x,
                                    const double* __restrict__ y, const double* __restrict__ z,
-                                   const long long* __restrict__ fixs, unsigned long long* fixp, double* blk) {
+                                   const long long* __restrict__ s0, const long long* __restrict__ s1,
+                                   const long long* __restrict__ s2, unsigned long long* fixp, double* blk) {
   const int nlast = sc->nlast;
   const double s = 1.0 / 1099511627776.0;
   double st[6] = {0, 0, 0, 0, 0, 0};
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < nlast; p += gridDim.x * blockDim.x) {
-    const long long f0 = fixs[3 * (size_t)p], f1 = fixs[3 * (size_t)p + 1], f2 = fixs[3 * (size_t)p + 2];
+    const long long f0 = s0[p], f1 = s1[p], f2 = s2[p];
     if ((f0 | f1 | f2) == 0) continue;
     const int a = at_list[p];
     const double fa = (double)f0 * s, fb = (double)f1 * s, fc = (double)f2 * s;
@@ -1161,7 +1162,9 @@ void pair_forces_sorted(PairGeom& pg, int nb2) {
   A.rc2 = (float)pg.rc2; A.rv2 = (float)pg.rv2; A.alpha = (float)g.p.alpha;
   A.a2rp = (float)(g.p.alpha * 2.0 / std::sqrt(3.14159265358979323846264338327950288));
   A.scaling = (float)pg.scaling;
-  A.fixs = (unsigned long long*)g.fixs;
+  A.f0 = (unsigned long long*)g.fixs;
+  A.f1 = A.f0 + g.mxatms;
+  A.f2 = A.f1 + g.mxatms;
   A.cnt = &g.sc->npairs_list;
   A.sc = g.sc;
   // four list entries per lane in the filter pass (measured at 262,144 ions, pair time
@@ -1204,7 +1207,8 @@ void pair_forces_sorted(PairGeom& pg, int nb2) {
   GB_LAUNCHED();
   run_side_hook();  // side-stream work enqueued behind the pair kernel's launch
   side_join();  // the reciprocal-space forces are in place before the pair forces join them
-  k_slot_stress_fold<<<nbs, 256, 0, st>>>(g.natms, g.sc, g.at_list, g.src, g.x, g.y, g.z, g.fixs,
+  k_slot_stress_fold<<<nbs, 256, 0, st>>>(g.natms, g.sc, g.at_list, g.src, g.x, g.y, g.z, (const long long*)A.f0,
+                                          (const long long*)A.f1, (const long long*)A.f2,
                                           (unsigned long long*)g.fixp, blks);
   GB_LAUNCHED();
   if (!mixed) {
