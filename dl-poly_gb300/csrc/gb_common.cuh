@@ -188,7 +188,8 @@ struct Dev {
   float4* xls = nullptr;       // per sorted position: remainders (x, y, z, q) of the FP64 values
   unsigned char* tys = nullptr;  // per sorted position: atom type
   uint2* xlh = nullptr;        // mixed form, per sorted position: remainders x 2^20 as half floats, and the type
-  long long* fixs = nullptr;   // 3 x mxatms fixed-point pair forces per sorted position
+  long long* fixs = nullptr;   // 3 x mxatms fixed-point pair forces per sorted position, and the pair kernel's counter
+  float2* eat = nullptr;       // 4 x natms: pair energies and virials per local atom, in sorted order
   double metal_e4[4] = {0, 0, 0, 0};  // engmet, virmet, engden, virden of the last evaluation
   // thermostat of the VV stages (gb_thermostat.cu)
   int ens = 0;                 // GB_NVE, GB_NVT_BERENDSEN, GB_NVT_NOSE_HOOVER, GB_NVT_LANGEVIN

@@ -727,11 +727,14 @@ __global__ void __launch_bounds__(PAIR_DF_NT, 4) k_pair_df64(int natms, const De
 // are contiguous runs that L1 holds, not gathers by atom index.  Pair forces go to
 // per-sorted-position int64 fixed-point sums (64-bit integer reductions: the result does
 // not depend on their order); k_slot_stress_fold sums the stress and moves them to atoms.
-// CTA size by form (measured at 262,144 ions, each CTA on a contiguous run of the local
-// atoms; pair time per launch and MD step with SPME on the side stream, 1024-thread CTAs
-// (one per SM) / 256-thread CTAs (four per SM)): double-float 1.192 / 1.285 ms, step 2.77 /
-// 2.84 ms; mixed 0.687 / 0.687 ms, step 1.52 / 1.48 ms (the side stream's kernels find room
-// beside the smaller CTAs).  GB_PAIR_NT=256 or 1024 sets it for both forms.
+// CTA size by form (one resident set of CTAs; 262,144 ions, 10 MD steps with their start, 1024-
+// thread CTAs (one per SM) / 256-thread CTAs (four per SM)): double-float 25.9 / 27.7 ms,
+// mixed 14.1 / 14.0 ms (the side stream's kernels find room beside the smaller CTAs).
+// GB_PAIR_NT=256 or 1024 sets it for both forms.
+// The double-float pair is bound by FP32 issue: 0.845 ms per launch at 262,144 ions (1.084
+// with renormalised products and quotients and equal runs of atoms per CTA and warp, whose
+// last warps left a tenth of the SMs' time idle); the mixed one by the latency of its
+// partner loads: 0.470 ms (0.555 with equal runs).
 constexpr int PAIR_SORTED_NT = 1024;
 
 struct PairSortedArgs {
@@ -758,63 +761,85 @@ struct PairSortedArgs {
   int ntypes;
   float rc2, rv2, alpha, a2rp, scaling;  // mixed form
   unsigned long long *f0, *f1, *f2;  // fixed-point x, y, z forces per sorted position
-  double* blk;
+  float2* eat;               // per local atom (in sorted order) its energy and virial sums, 4 x natms
+  unsigned long long* pool;  // next atom of the shared eighth, or null
   unsigned long long* cnt;
   const DevScalars* sc;
 };
 
-// The FP64 form's terms of one pair (the arithmetic of pair_terms_df64, partner data
-// passed in); jp is the partner's sorted position, whose atom index the exact FP64
-// evaluation near a cutoff looks up.
+// c0 + d (c1 + d c2) as an unnormalised pair (the low part up to two FP32 ulps of the high
+// one): 23 FP32 operations instead of poly_df's 28
+__device__ __forceinline__ df poly_pair(float4 c01, float c2h, float c2l, df d) {
+  const df p = two_prod(d.hi, c2h);
+  const df t = two_sum(c01.z, p.hi);
+  const float tl = __fadd_rn(__fadd_rn(t.lo, c01.w), __fmaf_rn(d.hi, c2l, __fmaf_rn(d.lo, c2h, p.lo)));
+  const df q = two_prod(d.hi, t.hi);
+  const df s = two_sum(c01.x, q.hi);
+  return df_make(s.hi, __fadd_rn(__fadd_rn(s.lo, c01.y), __fmaf_rn(d.hi, tl, __fmaf_rn(d.lo, t.hi, q.lo))));
+}
+
+// a * b as an unnormalised pair
+__device__ __forceinline__ df prod_pair(df a, df b) {
+  const df p = two_prod(a.hi, b.hi);
+  return df_make(p.hi, __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.lo, b.hi, p.lo)));
+}
+
+// r (relative error about 1e-14: an FP32 root and the first-order remainder) and 1/r^2
+// (3e-14) of a double-float r^2
+__device__ __forceinline__ df dist_inv2(df r2, df* inv) {
+  const float rs = rsqrtf(r2.hi);
+  const float s = __fmul_rn(r2.hi, rs);
+  const df ss = two_prod(s, s);
+  const float e = __fadd_rn(__fsub_rn(__fsub_rn(r2.hi, ss.hi), ss.lo), r2.lo);
+  const float q = __fmul_rn(rs, rs);
+  const float g = __fmaf_rn(-r2.lo, q, __fmaf_rn(-r2.hi, q, 1.f));  // 1 - r2 q
+  *inv = df_make(q, __fmul_rn(q, __fmaf_rn(g, g, g)));
+  return quick_two_sum(s, __fmul_rn(__fmul_rn(0.5f, rs), e));
+}
+
+// The FP64 form's terms of one pair (the formulas of pair_terms_df64, partner data
+// passed in; key: the pair's vdW table or -1); jp is the partner's sorted position, whose
+// atom index the exact FP64 evaluation near a cutoff looks up.
 // Returns false when the pair exerts no force.
 __device__ __forceinline__ bool pair_df64_eval(const PairGeom& pg, const PairSortedArgs& A, const float4* etab,
-                                               int i, int jp, int ai,
-                                               int aj, df qi, bool qi_on, float qjh, float qjl, df dx, df dy, df dz,
+                                               int i, int jp, int ai, int aj, int key,
+                                               df qi, bool qi_on, float qjh, float qjl, df dx, df dy, df dz,
                                                df rsq, dacc (&acc)[NACC_DF], long long& ix, long long& iy,
                                                long long& iz) {
   const bool band = (rsq.hi >= pg.f_rc2_lo && rsq.hi <= pg.f_rc2_hi) ||
                     (rsq.hi >= pg.f_rv2_lo && rsq.hi <= pg.f_rv2_hi);
   const bool in_c = qi_on && qjh != 0.0f && rsq.hi < pg.f_rc2_lo;
-  int key = -1;
-  if (rsq.hi < pg.f_rv2_lo) {
-    key = vkey(ai, aj) - 1;
-    if (A.vkind[key] == 0) key = -1;
-  }
-  // wv: the vdW virial term -gvv r^2 (-G(r) of the table itself on the fast path)
-  df gam = df_make(0.f, 0.f), ee = gam, ev = gam, gvc = gam, gvv = gam, wv = gam;
-  bool slow = band;
+  if (!(rsq.hi < pg.f_rv2_lo)) key = -1;
+  df gam = df_make(0.f, 0.f);
+  // (an r^2 whose square root or reciprocal FP32 cannot hold is in the first table interval)
+  bool slow = band || (pg.vdw_direct && key >= 0) || !(rsq.hi > 1e-30f);
   if (!slow && (in_c || key >= 0)) {
-    const df rinv = df_rsqrt(rsq);
-    const df rrr = df_mul(rsq, rinv);
+    df inv;
+    const df rrr = dist_inv2(rsq, &inv);
     df d;
     const int k = table_coord(rrr, pg.erdr_hi, pg.erdr_lo, &d);
     int kv = k;
     df dv = d;
     if (!pg.same_grid && key >= 0) kv = table_coord(rrr, pg.vrdr_hi, pg.vrdr_lo, &dv);
-    if (k == 0 || (key >= 0 && kv == 0)) {
-      slow = true;  // first interval: the exact three-point formula, in FP64
-    } else {
+    slow = k == 0 || (key >= 0 && kv == 0);  // first interval: the exact three-point formula, in FP64
+    if (!slow) {
       if (in_c) {
         const float4* c = etab + k * 3;
         const float4 e01 = c[0], d01 = c[1], c2 = c[2];
         const df pre = df_mul(qi, df_make(qjh, qjl));
-        gvc = df_mul(pre, poly_df(d01, c2.z, c2.w, d));
-        ee = df_mul(pre, poly_df(e01, c2.x, c2.y, d));
-        gam = gvc;
+        gam = prod_pair(pre, poly_pair(d01, c2.z, c2.w, d));
+        dacc_add_prod(acc[2], pre, poly_pair(e01, c2.x, c2.y, d));
+        dacc_add_prod(acc[3], df_neg(gam), rsq);
       }
       if (key >= 0) {
-        const df r_rsq = df_sqr(rinv);
-        if (pg.vdw_direct) {
-          slow = true;
-        } else {
-          const float4* c = A.vtab + (size_t)key * ((pg.max_grid + 3) * 3) + (size_t)kv * 3;
-          const float4 f01 = c[0], v01 = c[1], c2 = c[2];
-          const df G = poly_df(f01, c2.x, c2.y, dv);
-          gvv = df_mul(G, r_rsq);
-          wv = df_neg(G);
-          ev = poly_df(v01, c2.z, c2.w, dv);
-          gam = df_add(gam, gvv);
-        }
+        const float4* c = A.vtab + (size_t)key * ((pg.max_grid + 3) * 3) + (size_t)kv * 3;
+        const float4 f01 = c[0], v01 = c[1], c2 = c[2];
+        const df G = poly_pair(f01, c2.x, c2.y, dv);
+        const df gvv = prod_pair(G, inv);
+        const df s = two_sum(gam.hi, gvv.hi);
+        gam = df_make(s.hi, __fadd_rn(s.lo, __fadd_rn(gam.lo, gvv.lo)));
+        dacc_add(acc[0], poly_pair(v01, c2.z, c2.w, dv));
+        dacc_add(acc[1], df_neg(G));  // -gvv r^2 is the table value itself
       }
     }
   }
@@ -825,23 +850,23 @@ __device__ __forceinline__ bool pair_df64_eval(const PairGeom& pg, const PairSor
     pair_terms_fp64(pg, A.x[i] - A.x[j], A.y[i] - A.y[j], A.z[i] - A.z[j], A.q[i] * pg.scaling, A.q[j], ai, aj,
                     A.ecoef, A.vcoef, A.vkind, A.veps, A.vsig, &g64, &e64c, &e64v, &gc64, &gv64, &any);
     if (!any) return false;
-    float h, l;
-    df_split(g64, &h, &l); gam = df_make(h, l);
-    df_split(e64c, &h, &l); ee = df_make(h, l);
-    df_split(e64v, &h, &l); ev = df_make(h, l);
-    df_split(gc64, &h, &l); gvc = df_make(h, l);
-    df_split(gv64, &h, &l); gvv = df_make(h, l);
-    wv = df_neg(df_mul(gvv, rsq));
+    df ee, ev, gvc, gvv;
+    df_split(g64, &gam.hi, &gam.lo);
+    df_split(e64c, &ee.hi, &ee.lo);
+    df_split(e64v, &ev.hi, &ev.lo);
+    df_split(gc64, &gvc.hi, &gvc.lo);
+    df_split(gv64, &gvv.hi, &gvv.lo);
+    dacc_add(acc[0], ev);
+    dacc_add_prod(acc[1], df_neg(gvv), rsq);
+    dacc_add(acc[2], ee);
+    dacc_add_prod(acc[3], df_neg(gvc), rsq);
   } else if (!in_c && key < 0) {
     return false;
   }
-  ix = fix40_prod(gam, dx);
-  iy = fix40_prod(gam, dy);
-  iz = fix40_prod(gam, dz);
-  dacc_add(acc[0], ev);
-  dacc_add(acc[1], wv);
-  dacc_add(acc[2], ee);
-  dacc_add_prod(acc[3], df_neg(gvc), rsq);
+  const df g40 = df_make(__fmul_rn(gam.hi, 1099511627776.0f), __fmul_rn(gam.lo, 1099511627776.0f));
+  ix = fix_prod(g40, dx);
+  iy = fix_prod(g40, dy);
+  iz = fix_prod(g40, dz);
   return true;
 }
 
@@ -899,32 +924,65 @@ struct PairQueueN {
   int j[N];
 };
 
+__device__ __forceinline__ dacc dacc_shfl(dacc v, int o) {
+  dacc r;
+  r.s = __shfl_xor_sync(0xffffffffu, v.s, o);
+  r.c = __shfl_xor_sync(0xffffffffu, v.c, o);
+  return r;
+}
+
+// the sum of two compensated sums (commutative: both lanes of an exchange get the same bits)
+__device__ __forceinline__ dacc dacc_join(dacc a, dacc b) {
+  const df u = two_sum(a.s, b.s);
+  dacc r;
+  r.s = u.hi;
+  r.c = __fadd_rn(__fadd_rn(a.c, b.c), u.lo);
+  return r;
+}
+
 template <int MIXED, int U, int NT>
 __global__ void __launch_bounds__(NT, 1024 / NT) k_pair_sorted(PairSortedArgs A, PairGeom pg) {
   __shared__ PairQueueN<32 * (U + 1)> pq[NT / 32];
   __shared__ float4 s_lj[MIXED ? MAX_TYPES * MAX_TYPES : 1];
+  __shared__ short s_key[MIXED ? 1 : MAX_TYPES * MAX_TYPES];  // FP64 form: a type pair's vdW table, or -1
+  __shared__ int s_next;
   extern __shared__ float4 s_etab[];  // FP64 form: the double-float erfc table
   if (MIXED) {
     for (int e = threadIdx.x; e < A.ntypes * A.ntypes; e += blockDim.x) {
       const int ai = e / A.ntypes + 1, aj = e % A.ntypes + 1;
       s_lj[e] = c_lj[vkey(ai, aj) - 1];
     }
-    __syncthreads();
   } else {
     for (int e = threadIdx.x; e < A.netab; e += blockDim.x) s_etab[e] = A.etab[e];
-    __syncthreads();
+    for (int e = threadIdx.x; e < min(A.ntypes * A.ntypes, MAX_TYPES * MAX_TYPES); e += blockDim.x) {
+      const int key = vkey(e / A.ntypes + 1, e % A.ntypes + 1) - 1;
+      s_key[e] = (short)(A.vkind[key] != 0 ? key : -1);
+    }
   }
   const int lane = threadIdx.x & 31, wq = threadIdx.x >> 5;
-  dacc acc[NACC_DF];
-#pragma unroll
-  for (int k = 0; k < NACC_DF; ++k) { acc[k].s = 0.f; acc[k].c = 0.f; }
   unsigned long long n_list = 0, n_rc = 0;
-  // Each CTA takes an equal, contiguous run of the local atoms in sorted (cell) order, its
-  // warps NT / 32 consecutive atoms at a time: the partners of the atoms in flight are the
-  // same few link cells, and the next atoms' mostly the same, which the SM's L1 holds.
-  const int per = (A.natms + gridDim.x - 1) / gridDim.x;
-  const int a_end = min(A.natms, (int)(blockIdx.x + 1) * per);
-  for (int a = blockIdx.x * per + wq; a < a_end; a += NT / 32) {
+  // Each CTA takes an equal, contiguous run of the first M local atoms in sorted (cell)
+  // order, its warps the next atom of the run at a time: the partners of the atoms in flight
+  // are the same few link cells, and the next atoms' mostly the same, which the SM's L1
+  // holds.  With one resident set of CTAs the last eighth of the atoms goes to whichever warp
+  // is free (the lists of border atoms are short, so equal runs are unequal work).  The
+  // sums of an atom (its energies in eat) do not depend on the warp that forms them.
+  const int M = A.pool ? A.natms - A.natms / 8 : A.natms;
+  const int per = (M + gridDim.x - 1) / gridDim.x;
+  const int a_end = min(M, (int)(blockIdx.x + 1) * per);
+  if (threadIdx.x == 0) s_next = blockIdx.x * per;
+  __syncthreads();
+  for (;;) {
+    int a = 0;
+    if (lane == 0) {
+      a = atomicAdd(&s_next, 1);
+      if (a >= a_end) a = A.pool ? M + (int)atomicAdd(A.pool, 1ull) : A.natms;
+    }
+    a = __shfl_sync(0xffffffffu, a, 0);
+    if (a >= A.natms) break;
+    dacc acc[NACC_DF];
+#pragma unroll
+    for (int k = 0; k < NACC_DF; ++k) { acc[k].s = 0.f; acc[k].c = 0.f; }
     const int p = A.loc_sp[a];
     const int i = A.at_list[p];
     const float4 pi = A.xhs[p];
@@ -999,7 +1057,14 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_pair_sorted(PairSortedArgs A,
             const df dy = quick_two_sum(ey.hi, __fadd_rn(ey.lo, __fsub_rn(li.y, lj.y)));
             const df dz = quick_two_sum(ez.hi, __fadd_rn(ez.lo, __fsub_rn(li.z, lj.z)));
             const df rsq = df_norm2(dx, dy, dz);
-            hit = rsq.hi <= pg.f_hi && pair_df64_eval(pg, A, s_etab, i, j, ai, aj, qi, qi_on, pj.w, lj.w, dx,
+            int key;
+            if (A.ntypes <= MAX_TYPES) {
+              key = s_key[ljrow + aj];
+            } else {
+              key = vkey(ai, aj) - 1;
+              if (A.vkind[key] == 0) key = -1;
+            }
+            hit = rsq.hi <= pg.f_hi && pair_df64_eval(pg, A, s_etab, i, j, ai, aj, key, qi, qi_on, pj.w, lj.w, dx,
                                                       dy, dz, rsq, acc, ix, iy, iz);
           }
           if (hit) {
@@ -1017,7 +1082,19 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_pair_sorted(PairSortedArgs A,
     }
     if (MIXED) {
 #pragma unroll
-      for (int q = 0; q < 4; ++q) dacc_add(acc[q], df_make(e4[q], 0.f));
+      for (int q = 0; q < 4; ++q) acc[q].s = e4[q];
+    }
+    // the atom's four energy and virial sums by a reduce-scatter over the warp: two values a
+    // lane after the first level, one after the second, left in lanes 0, 8, 16, 24
+    {
+      const bool up16 = lane & 16, up8 = lane & 8;
+      dacc k0 = up16 ? acc[2] : acc[0], k1 = up16 ? acc[3] : acc[1];
+      k0 = dacc_join(k0, dacc_shfl(up16 ? acc[0] : acc[2], 16));
+      k1 = dacc_join(k1, dacc_shfl(up16 ? acc[1] : acc[3], 16));
+      dacc r = dacc_join(up8 ? k1 : k0, dacc_shfl(up8 ? k0 : k1, 8));
+#pragma unroll
+      for (int o = 4; o > 0; o >>= 1) r = dacc_join(r, dacc_shfl(r, o));
+      if ((lane & 7) == 0) A.eat[(size_t)(lane >> 3) * A.natms + a] = make_float2(r.s, r.c);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -1032,29 +1109,39 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_pair_sorted(PairSortedArgs A,
       n_list += (unsigned long long)n;
     }
   }
-  dfr out[NACC_DF];
-#pragma unroll
-  for (int k = 0; k < NACC_DF; ++k) out[k] = to_dfr(two_sum(acc[k].s, acc[k].c));
   n_rc = (unsigned long long)warp_sumi((int)n_rc);
   if (lane == 0) {
     if (n_list) atomicAdd(&A.cnt[0], n_list);
     if (n_rc) atomicAdd(&A.cnt[1], n_rc);
   }
-  block_reduce_store<NACC_DF>(out, A.blk);
 }
 
 // Pair stress from the per-sorted-position forces (sum over slots of x (x) F, every halo
 // image at its own position, in FP64 from the exact fixed-point forces), then each
 // slot's force onto its atom (a halo image's onto its source): integer sums.
+// The same launch sums the local atoms' energies and virials (eat), 4 values before the 6 of
+// the stress; the block sums are double-float, so that only the stress products and
+// running sums use the FP64 unit.
 __global__ void k_slot_stress_fold(int natms, const DevScalars* sc, const int* __restrict__ at_list,
                                    const int* __restrict__ src, const double* __restrict__ x,
                                    const double* __restrict__ y, const double* __restrict__ z,
                                    const long long* __restrict__ s0, const long long* __restrict__ s1,
-                                   const long long* __restrict__ s2, unsigned long long* fixp, double* blk) {
+                                   const long long* __restrict__ s2, const float2* __restrict__ eat,
+                                   unsigned long long* fixp, double* blk) {
   const int nlast = sc->nlast;
   const double s = 1.0 / 1099511627776.0;
   double st[6] = {0, 0, 0, 0, 0, 0};
+  dacc e[NACC_DF];
+#pragma unroll
+  for (int c = 0; c < NACC_DF; ++c) { e[c].s = 0.f; e[c].c = 0.f; }
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < nlast; p += gridDim.x * blockDim.x) {
+    if (p < natms) {
+#pragma unroll
+      for (int c = 0; c < NACC_DF; ++c) {
+        const float2 v = eat[(size_t)c * natms + p];
+        dacc_add(e[c], df_make(v.x, v.y));
+      }
+    }
     const long long f0 = s0[p], f1 = s1[p], f2 = s2[p];
     if ((f0 | f1 | f2) == 0) continue;
     const int a = at_list[p];
@@ -1067,7 +1154,12 @@ __global__ void k_slot_stress_fold(int natms, const DevScalars* sc, const int* _
     atomicAdd(&fixp[3 * tgt + 1], (unsigned long long)f1);
     atomicAdd(&fixp[3 * tgt + 2], (unsigned long long)f2);
   }
-  block_reduce_store<6>(st, blk);
+  dfr out[NACC_DF + 6];
+#pragma unroll
+  for (int c = 0; c < NACC_DF; ++c) out[c] = to_dfr(two_sum(e[c].s, e[c].c));
+#pragma unroll
+  for (int k = 0; k < 6; ++k) out[NACC_DF + k] = dfr(st[k]);
+  block_reduce_store<NACC_DF + 6>(out, blk);
 }
 
 // Pair stress of the double-float kernel from its per-slot forces: with every image's
@@ -1183,24 +1275,22 @@ void pair_forces_sorted(PairGeom& pg, int nb2) {
   if (dsm > 0) GB_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)dsm));
   int occ = 0;
   GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, nt, dsm));
-  // The CTAs take equal contiguous runs of the local atoms: one resident set of CTAs
-  // (the double-float form), or short-lived CTAs of 16 atoms per warp (the mixed form: they
-  // retire through the step, so the side stream's SPME kernels take their places and the
-  // last runs balance the load; measured at 262,144 ions, mixed pair 0.682 -> 0.646 ms and
-  // step 1.481 -> 1.460 ms; for the double-float form they were slower at every length).
-  // GB_PAIR_APW sets the atoms per warp (0: one resident set).
-  int apw = mixed ? 16 : 0;
+  // The CTAs take equal contiguous runs of the local atoms: one resident set of CTAs, whose
+  // free warps share the last atoms.  GB_PAIR_APW sets short-lived CTAs of that many atoms
+  // per warp instead (16 per warp: mixed 14.4 instead of 14.0 ms for 10 steps, double-float
+  // 26.0 instead of 25.9 ms).
+  int apw = 0;
   if (g.pair_apw >= 0) apw = g.pair_apw;
   // a small system keeps at least one CTA per resident slot (fewer atoms per warp)
   if (apw > 0) apw = std::max(1, std::min(apw, g.natms / ((nt / 32) * std::max(1, occ) * g.nsm)));
   const int nb = apw > 0 ? std::max(1, nblocks((long long)g.natms, (nt / 32) * apw))
                          : std::max(1, std::min(nblocks((long long)g.mxatms * 32, nt), occ * g.nsm));
   const int nbs = std::max(1, std::min(nblocks(g.mxatms, 256), 4 * g.nsm));  // stress blocks
-  double* blk = gb_blkacc(nb * NACC_DF + nbs * 6 + nb2 * 8);
-  double* blks = blk + (size_t)nb * NACC_DF;
-  double* blk2 = blks + (size_t)nbs * 6;
-  A.blk = blk;
-  GB_CUDA(cudaMemsetAsync(g.fixs, 0, sizeof(long long) * 3 * (size_t)g.mxatms, st));
+  double* blks = gb_blkacc(nbs * NACC + nb2 * 8);
+  double* blk2 = blks + (size_t)nbs * NACC;
+  A.eat = g.eat;
+  A.pool = apw > 0 ? nullptr : A.f2 + g.mxatms;
+  GB_CUDA(cudaMemsetAsync(g.fixs, 0, sizeof(long long) * (3 * (size_t)g.mxatms + 1), st));
   if (!mixed) GB_CUDA(cudaMemsetAsync(g.fixp, 0, sizeof(long long) * 3 * (size_t)g.mxatms, st));
   prof_begin(P_PAIR);
   kern<<<nb, nt, dsm, st>>>(A, pg);
@@ -1208,7 +1298,7 @@ void pair_forces_sorted(PairGeom& pg, int nb2) {
   run_side_hook();  // side-stream work enqueued behind the pair kernel's launch
   side_join();  // the reciprocal-space forces are in place before the pair forces join them
   k_slot_stress_fold<<<nbs, 256, 0, st>>>(g.natms, g.sc, g.at_list, g.src, g.x, g.y, g.z, (const long long*)A.f0,
-                                          (const long long*)A.f1, (const long long*)A.f2,
+                                          (const long long*)A.f1, (const long long*)A.f2, g.eat,
                                           (unsigned long long*)g.fixp, blks);
   GB_LAUNCHED();
   if (!mixed) {
@@ -1216,8 +1306,7 @@ void pair_forces_sorted(PairGeom& pg, int nb2) {
     GB_LAUNCHED();
   }
   prof_end(P_PAIR);
-  gb_reduce_blocks(blk, nb, NACC_DF, &g.sc->acc[A_PAIR]);
-  gb_reduce_blocks(blks, nbs, 6, &g.sc->acc[A_PAIR + NACC_DF]);
+  gb_reduce_blocks(blks, nbs, NACC, &g.sc->acc[A_PAIR]);
   if (g.lbook) {
     prof_begin(P_EXCL);
     k_excl_fp64<<<nb2, 128, 0, st>>>(g.natms, g.list, g.ld, g.x, g.y, g.z, g.chge, g.ltg, g.src, g.p.alpha,
