@@ -195,7 +195,7 @@ void free_all() {
                   g.lfrzn, g.ixyz, g.src, g.shcode, g.xbg, g.ybg, g.zbg, g.ox, g.oy, g.oz, g.which_cell,
                   g.cell_count, g.cell_start, g.cell_fill, g.at_list, g.sorted_pos, g.xs, g.xsf, g.list, g.blk,
                   g.list_excl, g.erfc_coef, g.erfc_coef_f, g.vdw_coef, g.vdw_coef_f,
-                  g.vdw_kind, g.vdw_eps, g.vdw_sig, g.erfc_df, g.vdw_df, g.qdf, g.spos, g.xhs, g.xls, g.tys, g.xlh, g.fixs, g.eat, g.loc_sp,
+                  g.vdw_kind, g.vdw_eps, g.vdw_sig, g.erfc_df, g.vdw_df, g.qdf, g.spos, g.xhs, g.rec, g.xlh, g.fixs, g.eat, g.loc_sp,
                   g.tile_rows, g.tile_info, g.tile_over, g.blkacc, g.con_i, g.con_j, g.con_d0, g.dxx, g.dyy,
                   g.dzz, g.dxt, g.dyt, g.dzt, g.dt2, g.gam, g.listot, g.acon_start, g.acon_list, g.sc, d_scratch,
                   d_scratch_s, g.blkacc_s};
@@ -632,6 +632,12 @@ int gb_init(const gb_params* prm, int natms, const int32_t* ltype, const double*
     invert_host(g.cell, g.rcell, &det);
     dcell_host(g.cell, g.celprp);
     g.volm = g.celprp[9];
+    {
+      // the box with its halo within 62 bits, listed separations within 52 (fix_diff)
+      const int box = (int)std::ceil(std::log2(1.5 * std::max(g.cell[0], 1.0)));
+      const int sep = (int)std::ceil(std::log2(prm->rcut + 2.0 * prm->rpad + 1.0));
+      g.pos_scale = std::ldexp(1.0, std::min(48, std::min(62 - box, 52 - sep)));
+    }
     g.cubic = (g.cell[0] == g.cell[4] && g.cell[0] == g.cell[8]);
     bool ortho = g.cell[1] == 0 && g.cell[2] == 0 && g.cell[3] == 0 && g.cell[5] == 0 && g.cell[6] == 0 && g.cell[7] == 0;
     if (!ortho || !g.cubic) { free_all(); return GB_ERR_ARG; }  // cubic cells (imcon 1) only
@@ -666,7 +672,7 @@ int gb_init(const gb_params* prm, int natms, const int32_t* ltype, const double*
     dalloc(&g.list, (size_t)g.ld * natms);
     g.ldt = ((prm->max_list + 1 + 3) / 4) * 4;  // spos(k, i), k = 1..max_list, rows 16-byte aligned
     dalloc(&g.spos, (size_t)g.ldt * natms);
-    dalloc(&g.xhs, mx); dalloc(&g.xls, mx); dalloc(&g.tys, mx); dalloc(&g.xlh, mx);
+    dalloc(&g.xhs, mx); dalloc(&g.rec, mx); dalloc(&g.xlh, mx);
     dalloc(&g.loc_sp, natms);
     dalloc(&g.fixs, 3 * (size_t)mx + 1);
     dalloc(&g.eat, 4 * (size_t)natms);
@@ -706,7 +712,11 @@ int gb_init(const gb_params* prm, int natms, const int32_t* ltype, const double*
     pair_setup();
     g.scaling = kR4pie0 / prm->epsq;
     double sq2 = 0.0;
-    for (int i = 0; i < natms; ++i) sq2 += chge[i] * chge[i];
+    g.qmax = 0.0;
+    for (int i = 0; i < natms; ++i) {
+      sq2 += chge[i] * chge[i];
+      g.qmax = std::max(g.qmax, std::fabs(chge[i]));
+    }
     g.self_interaction = -sq2 * (g.scaling * prm->alpha * (1.0 / 1.7724538509055161040) / 1.0);  // spme.F90:159-231
     g.ntcons = ntcons;
     if (ntcons > 0) integ_setup_constraints(listcon, prmcon);

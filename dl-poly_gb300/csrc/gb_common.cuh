@@ -88,6 +88,16 @@ enum ProfId {
 void prof_begin(int id);
 void prof_end(int id);
 
+// A sorted position's coordinates for the double-float kernels: int64 in units of
+// 1/pos_scale, whose differences are exact (the FP64 coordinate is rounded to them: at 48
+// bits, 2^-49 A, the FP64 rounding of a coordinate beyond 16 A), the low part of the
+// charge and the atom type.
+struct __align__(16) PosRec {
+  long long x, y, z;
+  float ql;
+  int type;
+};
+
 // All device pointers of the context.  Arrays of size mxatms hold local atoms
 // in [0, natms) followed by halo images in [natms, nlast).
 struct Dev {
@@ -185,8 +195,8 @@ struct Dev {
   int* dflag = nullptr;        // its device-side address
   int* loc_sp = nullptr;       // natms: the sorted positions of the local atoms, in sorted order
   float4* xhs = nullptr;       // per sorted position: FP32 high parts (x, y, z, q)
-  float4* xls = nullptr;       // per sorted position: remainders (x, y, z, q) of the FP64 values
-  unsigned char* tys = nullptr;  // per sorted position: atom type
+  PosRec* rec = nullptr;       // FP64 form, per sorted position: fixed-point coordinates, charge remainder, type
+  double pos_scale = 0;        // units per Angstrom of rec's coordinates (a power of two)
   uint2* xlh = nullptr;        // mixed form, per sorted position: remainders x 2^20 as half floats, and the type
   long long* fixs = nullptr;   // 3 x mxatms fixed-point pair forces per sorted position, and the pair kernel's counter
   float2* eat = nullptr;       // 4 x natms: pair energies and virials per local atom, in sorted order
@@ -213,6 +223,7 @@ struct Dev {
   std::vector<int> h_vdw_kind;
   std::vector<double> h_vdw_eps, h_vdw_sig;
   double elrc = 0, vlrc = 0, self_interaction = 0, scaling = 0;
+  double qmax = 0;               // largest |charge|
 
   // SPME grids live in gb_spme.cu (SpmeGrid); shared scratch here
   double* blkacc = nullptr;    // per-block partial accumulators

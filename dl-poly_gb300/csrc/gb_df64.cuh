@@ -148,4 +148,27 @@ __device__ __forceinline__ long long fix_prod(df a, df b) {
   return __float2ll_rz(p) + __float2ll_rz(t);
 }
 
+// (a - b) / scale of two fixed-point coordinates for |a - b| < 2^52: an exact integer
+// difference as a double-float; sh = 2^28 / scale, sl = 1 / scale
+__device__ __forceinline__ df fix_diff(long long a, long long b, float sh, float sl) {
+  const long long d = a - b;
+  const float h = __fmul_rn(__int2float_rn((int)(d >> 28)), sh);
+  const float l = __fmul_rn(__int2float_rn((int)((unsigned)d & 0x0FFFFFFFu)), sl);
+  return quick_two_sum(h, l);
+}
+
+// a += x * y where the running sum a.s carries a constant C added to it that exceeds the
+// sum and every product: |a.s| >= |x y|, so that t - a.s is exact and the second FMA gives
+// the rounding error of the first (Dekker's fast two-sum with the product unrounded).  Six
+// FP32 operations instead of dacc_add_prod's twelve; the sum's error is relative to C
+// (about 2^-48 C per term).  Start with (C, 0) and take the sum with off_value.
+__device__ __forceinline__ void off_add_prod(dacc& a, df x, df y) {
+  const float t = __fmaf_rn(x.hi, y.hi, a.s);
+  const float r = __fmaf_rn(x.hi, y.hi, -__fsub_rn(t, a.s));
+  a.c = __fmaf_rn(x.hi, y.lo, __fmaf_rn(x.lo, y.hi, __fadd_rn(a.c, r)));
+  a.s = t;
+}
+
+__device__ __forceinline__ df off_value(const dacc& a, float c) { return two_sum(__fsub_rn(a.s, c), a.c); }
+
 #endif

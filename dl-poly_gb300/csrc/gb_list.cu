@@ -810,11 +810,11 @@ __global__ void __launch_bounds__(256) k_list_reorder(int natms, int* list, int 
 // fourth word (bit pattern), so a pair reads everything about j in two 16-byte loads
 // Both records in one pass over the atoms (the FP64 values converted once): by atom index
 // (xf, xlo: the type in xlo.w) and, for the sorted-position pair kernels, per sorted
-// position sorted_pos[i] (xhs, xls: the charge's remainder in xls.w, tys)
+// position sorted_pos[i] (xhs, and rec or, in the mixed form, xlh)
 __global__ void k_pos_records(const DevScalars* sc, const int* __restrict__ sorted_pos, const double* __restrict__ x,
                               const double* __restrict__ y, const double* __restrict__ z, const double* __restrict__ q,
-                              const int* __restrict__ ltype, float4* xf, float4* xlo, float2* qdf, float4* xhs,
-                              float4* xls, unsigned char* tys, uint2* xlh) {
+                              const int* __restrict__ ltype, double pos_scale, float4* xf, float4* xlo, float2* qdf,
+                              float4* xhs, PosRec* rec, uint2* xlh) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= sc->nlast) return;
   const double xa = x[i], ya = y[i], za = z[i], qa = q[i];
@@ -831,8 +831,13 @@ __global__ void k_pos_records(const DevScalars* sc, const int* __restrict__ sort
     if (xlh) {  // the mixed form's 8-byte record (pair_lo_type decodes it)
       xlh[p] = pack_lo_type(lx, ly, lz, ta);
     } else {
-      xls[p] = make_float4(lx, ly, lz, lq);
-      tys[p] = (unsigned char)ta;
+      PosRec r;
+      r.x = __double2ll_rn(xa * pos_scale);
+      r.y = __double2ll_rn(ya * pos_scale);
+      r.z = __double2ll_rn(za * pos_scale);
+      r.ql = lq;
+      r.type = ta;
+      rec[p] = r;
     }
   }
 }
@@ -1186,8 +1191,8 @@ int list_build() {
 
 void list_pos_records(bool sorted) {
   k_pos_records<<<nblocks(g.mxatms, 256), 256, 0, g.stream>>>(
-      g.sc, g.sorted_pos, g.x, g.y, g.z, g.chge, g.ltype, g.xf, g.xlo, g.precision == GB_FP64 ? g.qdf : nullptr,
-      sorted ? g.xhs : nullptr, g.xls, g.tys, g.precision == GB_MIXED ? g.xlh : nullptr);
+      g.sc, g.sorted_pos, g.x, g.y, g.z, g.chge, g.ltype, g.pos_scale, g.xf, g.xlo, g.precision == GB_FP64 ? g.qdf : nullptr,
+      sorted ? g.xhs : nullptr, g.rec, g.precision == GB_MIXED ? g.xlh : nullptr);
   GB_LAUNCHED();
 }
 

@@ -363,8 +363,7 @@ __global__ void __launch_bounds__(256, 3) k_metal_forces(int natms, const DevSca
 // evaluated with every lane busy.  256,000 atoms: density 1.97 -> 0.42 ms, forces 4.35 ->
 // 0.83 ms (1.04 with 102 registers, two CTAs per SM; a fourth CTA spills and gains
 // nothing); latency of the partners and tables, at a third of the issue slots.
-//   positions   int64 in units of 2^-48 A (exact for |x| >= 16 A): the separation is an
-//               exact integer difference
+//   positions   fixed point (PosRec): the separation is an exact integer difference
 //   r           relative error about 1e-14 (an FP32 square root and the first-order
 //               remainder; the FP64 kernels' one Newton step from an FP32 seed: 8e-14)
 //   tables      l by the nearest integer of the double-float coordinate, so that a pair
@@ -373,11 +372,6 @@ __global__ void __launch_bounds__(256, 3) k_metal_forces(int natms, const DevSca
 // FP32 range takes the FP64 formulas of the kernels above (metal_density_slow,
 // metal_force_slow).  Densities and forces are summed in FP64 per sorted position and
 // folded onto the atoms (a halo image's onto its source) afterwards.
-struct __align__(16) MetRec {
-  long long x, y, z;
-  int type, pad;
-};
-
 struct __align__(16) CoefF {
   float c0h, c0l, c1h, c1l;
   float c2h, c2l, pad0, pad1;
@@ -388,7 +382,8 @@ struct MetSorted {
   const int *at_list, *loc_sp, *list, *spos;
   int ld, ldt;
   const float4* xhs;
-  const MetRec* rec;
+  const PosRec* rec;
+  float sh, sl;                    // scales of its coordinates (fix_diff)
   const double *x, *y, *z, *rho;   // FP64 by atom index, for the slow path
   const CoefF *fv, *fd;            // quadratic coefficients of the values and derivatives
   const float2* fp;                // F'(rho) per sorted position
@@ -399,30 +394,7 @@ struct MetSorted {
   unsigned long long* cnt;
 };
 
-constexpr double MET_POS_SCALE = 281474976710656.0;  // 2^48
 constexpr int MET_NT = 256, MET_U = 4;
-
-__global__ void k_metal_records(const DevScalars* sc, const int* __restrict__ sorted_pos, const double* __restrict__ x,
-                                const double* __restrict__ y, const double* __restrict__ z,
-                                const int* __restrict__ ltype, MetRec* __restrict__ rec) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= sc->nlast) return;
-  MetRec r;
-  r.x = __double2ll_rn(x[i] * MET_POS_SCALE);
-  r.y = __double2ll_rn(y[i] * MET_POS_SCALE);
-  r.z = __double2ll_rn(z[i] * MET_POS_SCALE);
-  r.type = ltype[i];
-  r.pad = 0;
-  rec[sorted_pos[i]] = r;
-}
-
-// (a - b) 2^-48 for |a - b| < 2^52, as a double-float
-__device__ __forceinline__ df pos_diff(long long a, long long b) {
-  const long long d = a - b;
-  const float h = __int2float_rn((int)(d >> 28)) * 9.5367431640625e-07f;                             // 2^-20
-  const float l = __int2float_rn((int)((unsigned)d & 0x0FFFFFFFu)) * 3.552713678800501e-15f;  // 2^-48
-  return quick_two_sum(h, l);
-}
 
 // exact double of a finite float by integer operations (0 below the normal range)
 __device__ __forceinline__ double flt_dbl(float f) {
@@ -590,15 +562,16 @@ __global__ void __launch_bounds__(MET_NT) k_metal_density_sorted(MetSorted S, Me
   const int a_end = min(S.natms, (int)(blockIdx.x + 1) * per);
   for (int a = blockIdx.x * per + wq; a < a_end; a += MET_NT / 32) {
     const int p = S.loc_sp[a], i = S.at_list[p];
-    const MetRec ri = S.rec[p];
+    const PosRec ri = S.rec[p];
     const int ai = ri.type;
     const MetTab& ti = tabs[A.nkey + ai - 1];
     dacc rho = {0.f, 0.f};
     met_walk(S, i, S.xhs[p], queue[wq], [&](int j) {
-      const MetRec rj = S.rec[j];
+      const PosRec rj = S.rec[j];
       const bool same = rj.type == ai;
       const MetTab& tj = tabs[A.nkey + rj.type - 1];
-      const df dx = pos_diff(ri.x, rj.x), dy = pos_diff(ri.y, rj.y), dz = pos_diff(ri.z, rj.z);
+      const df dx = fix_diff(ri.x, rj.x, S.sh, S.sl), dy = fix_diff(ri.y, rj.y, S.sh, S.sl),
+               dz = fix_diff(ri.z, rj.z, S.sh, S.sl);
       const df r2 = df_norm2(dx, dy, dz);
       const int in_j = met_in(tj, r2.hi), in_i = same ? in_j : met_in(ti, r2.hi);
       if (in_j == 0 && in_i == 0) return;
@@ -677,7 +650,7 @@ __global__ void __launch_bounds__(MET_NT, 3) k_metal_forces_sorted(MetSorted S, 
   const int a_end = min(S.natms, (int)(blockIdx.x + 1) * per);
   for (int a = blockIdx.x * per + wq; a < a_end; a += MET_NT / 32) {
     const int p = S.loc_sp[a], i = S.at_list[p];
-    const MetRec ri = S.rec[p];
+    const PosRec ri = S.rec[p];
     const int ai = ri.type;
     const float2 f2 = S.fp[p];
     const df fpi = df_make(f2.x, f2.y);
@@ -685,11 +658,12 @@ __global__ void __launch_bounds__(MET_NT, 3) k_metal_forces_sorted(MetSorted S, 
     dacc fx = {0.f, 0.f}, fy = fx, fz = fx;
     n_list += (unsigned long long)S.list[(size_t)i * S.ld + 3];
     met_walk(S, i, S.xhs[p], queue[wq], [&](int j) {
-      const MetRec rj = S.rec[j];
+      const PosRec rj = S.rec[j];
       const int aj = rj.type;
       const MetTab& tp = tabs[(ai > aj ? ai * (ai - 1) / 2 + aj : aj * (aj - 1) / 2 + ai) - 1];
       if (!tp.listed) return;  // keypot = -1
-      const df dx = pos_diff(ri.x, rj.x), dy = pos_diff(ri.y, rj.y), dz = pos_diff(ri.z, rj.z);
+      const df dx = fix_diff(ri.x, rj.x, S.sh, S.sl), dy = fix_diff(ri.y, rj.y, S.sh, S.sl),
+               dz = fix_diff(ri.z, rj.z, S.sh, S.sl);
       const df r2 = df_norm2(dx, dy, dz);
       if (r2.hi > S.f_rc_hi) return;
       const bool same = aj == ai;
@@ -822,7 +796,6 @@ double* d_rho = nullptr;
 int n_key = 0, n_tab = 0, occ_dens = 0, occ_force = 0;
 // sorted-position kernels
 CoefF *d_fv = nullptr, *d_fd = nullptr;
-MetRec* d_rec = nullptr;
 float2* d_fp = nullptr;
 double* d_slot = nullptr;     // 3 x mxatms: density or force sums per sorted position
 int occ_dens_s = 0, occ_force_s = 0;
@@ -868,12 +841,12 @@ void table_derivatives(const std::vector<double>& buf, std::vector<double>& der)
 }  // namespace
 
 void metal_free() {
-  void* p[] = {d_tab, d_val, d_der, d_cv, d_cd, d_listed, d_rho, d_fv, d_fd, d_rec, d_fp, d_slot};
+  void* p[] = {d_tab, d_val, d_der, d_cv, d_cd, d_listed, d_rho, d_fv, d_fd, d_fp, d_slot};
   for (void* q : p)
     if (q) cudaFree(q);
   d_tab = nullptr; d_val = nullptr; d_der = nullptr; d_cv = nullptr; d_cd = nullptr; d_listed = nullptr;
   d_rho = nullptr;
-  d_fv = d_fd = nullptr; d_rec = nullptr; d_fp = nullptr; d_slot = nullptr;
+  d_fv = d_fd = nullptr; d_fp = nullptr; d_slot = nullptr;
   n_key = n_tab = 0;
   g.has_metal = false;
 }
@@ -997,7 +970,6 @@ int metal_setup(int ntab, const int32_t* kind, const int32_t* t1, const int32_t*
   GB_CUDA(cudaMalloc(&d_fd, sizeof(CoefF) * fd.size()));
   GB_CUDA(cudaMemcpy(d_fv, fv.data(), sizeof(CoefF) * fv.size(), cudaMemcpyHostToDevice));
   GB_CUDA(cudaMemcpy(d_fd, fd.data(), sizeof(CoefF) * fd.size(), cudaMemcpyHostToDevice));
-  GB_CUDA(cudaMalloc(&d_rec, sizeof(MetRec) * mx));
   GB_CUDA(cudaMalloc(&d_fp, sizeof(float2) * mx));
   GB_CUDA(cudaMalloc(&d_slot, sizeof(double) * 3 * mx));
   GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_dens_s, k_metal_density_sorted, MET_NT, 0));
@@ -1021,13 +993,9 @@ int metal_setup(int ntab, const int32_t* kind, const int32_t* t1, const int32_t*
   return GB_OK;
 }
 
-// The double-float kernels where the list pairs every halo entry with its backward copy and
-// the fixed-point positions and separations hold (the list's reach below 16 A, the box
-// and its halo below 2^14 A); the FP64 form by instructions keeps the FP64 kernels.
-static bool use_sorted_metal() {
-  return g.spos_valid && g.use_sorted && !g.fp64_native && g.rcutx < 15.9 && 1.5 * g.cell[0] < 16384.0 &&
-         max_rmax < 1.0e4;
-}
+// The double-float kernels where the list pairs every halo entry with its backward copy;
+// the FP64 form by instructions keeps the FP64 kernels.
+static bool use_sorted_metal() { return g.spos_valid && g.use_sorted && !g.fp64_native; }
 
 static void metal_forces_sorted(const MetArgs& A, unsigned long long* cnt) {
   cudaStream_t st = g.stream;
@@ -1035,7 +1003,9 @@ static void metal_forces_sorted(const MetArgs& A, unsigned long long* cnt) {
   MetSorted S;
   S.natms = g.natms;
   S.at_list = g.at_list; S.loc_sp = g.loc_sp; S.list = g.list; S.spos = g.spos; S.ld = g.ld; S.ldt = g.ldt;
-  S.xhs = g.xhs; S.rec = d_rec;
+  S.xhs = g.xhs; S.rec = g.rec;
+  S.sh = (float)(268435456.0 / g.pos_scale);
+  S.sl = (float)(1.0 / g.pos_scale);
   S.x = g.x; S.y = g.y; S.z = g.z; S.rho = d_rho;
   S.fv = d_fv; S.fd = d_fd; S.fp = d_fp;
   S.s0 = d_slot; S.s1 = d_slot + mx; S.s2 = d_slot + 2 * (size_t)mx;
@@ -1063,8 +1033,6 @@ static void metal_forces_sorted(const MetArgs& A, unsigned long long* cnt) {
   S.blk = blk2;
   S.cnt = cnt;
   prof_begin(P_METAL_DENSITY);
-  k_metal_records<<<nbm, T, 0, st>>>(g.sc, g.sorted_pos, g.x, g.y, g.z, g.ltype, d_rec);
-  GB_LAUNCHED();
   GB_CUDA(cudaMemsetAsync(d_slot, 0, sizeof(double) * (size_t)mx, st));
   GB_CUDA(cudaMemsetAsync(d_rho, 0, sizeof(double) * (size_t)g.natms, st));
   S.f_pre = pre(max_rmax * max_rmax * (1.0 + 1e-6));

@@ -746,8 +746,8 @@ struct PairSortedArgs {
   const int* spos;
   int ldt;
   const float4* xhs;
-  const float4* xls;
-  const unsigned char* tys;
+  const PosRec* rec;   // FP64 form: fixed-point positions, charge remainder and type
+  float sh, sl;        // its scales (fix_diff)
   const uint2* xlh;  // mixed form: remainders and type in 8 bytes (pair_lo_type)
   const double *x, *y, *z, *q;  // FP64 by atom index: the exact pair evaluation near a cutoff
   const float4* etab;
@@ -986,14 +986,16 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_pair_sorted(PairSortedArgs A,
     const int p = A.loc_sp[a];
     const int i = A.at_list[p];
     const float4 pi = A.xhs[p];
-    float4 li;
+    float4 li = make_float4(0.f, 0.f, 0.f, 0.f);
+    PosRec ri;
     int ai;
     if (MIXED) {
       pair_lo_type(A.xlh[p], li.x, li.y, li.z, ai);
       li.w = 0.f;
     } else {
-      li = A.xls[p];
-      ai = A.tys[p];
+      ri = A.rec[p];
+      li.w = ri.ql;
+      ai = ri.type;
     }
     const df qi = df_mul(df_make(pi.w, li.w), df_make(pg.scal_hi, pg.scal_lo));  // q_i r4pie0/eps
     const bool qi_on = pi.w != 0.0f;
@@ -1036,26 +1038,20 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_pair_sorted(PairSortedArgs A,
         if (lane < take) {
           const int j = pq[wq].j[nq - take + lane];
           const float4 pj = A.xhs[j];
-          float4 lj;
-          int aj;
-          if (MIXED) {
-            pair_lo_type(A.xlh[j], lj.x, lj.y, lj.z, aj);
-            lj.w = 0.f;
-          } else {
-            lj = A.xls[j];
-            aj = A.tys[j];
-          }
           long long ix = 0, iy = 0, iz = 0;
           bool hit;
           if (MIXED) {
+            float4 lj;
+            int aj;
+            pair_lo_type(A.xlh[j], lj.x, lj.y, lj.z, aj);
             const float dx = (pi.x - pj.x) + (li.x - lj.x), dy = (pi.y - pj.y) + (li.y - lj.y),
                         dz = (pi.z - pj.z) + (li.z - lj.z);
             hit = pair_mixed_eval(A, s_lj, ljrow, aj, qi32, pj.w, dx, dy, dz, e4, ix, iy, iz);
           } else {
-            const df ex = two_sum(pi.x, -pj.x), ey = two_sum(pi.y, -pj.y), ez = two_sum(pi.z, -pj.z);
-            const df dx = quick_two_sum(ex.hi, __fadd_rn(ex.lo, __fsub_rn(li.x, lj.x)));
-            const df dy = quick_two_sum(ey.hi, __fadd_rn(ey.lo, __fsub_rn(li.y, lj.y)));
-            const df dz = quick_two_sum(ez.hi, __fadd_rn(ez.lo, __fsub_rn(li.z, lj.z)));
+            const PosRec rj = A.rec[j];
+            const int aj = rj.type;
+            const df dx = fix_diff(ri.x, rj.x, A.sh, A.sl), dy = fix_diff(ri.y, rj.y, A.sh, A.sl),
+                     dz = fix_diff(ri.z, rj.z, A.sh, A.sl);
             const df rsq = df_norm2(dx, dy, dz);
             int key;
             if (A.ntypes <= MAX_TYPES) {
@@ -1064,7 +1060,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_pair_sorted(PairSortedArgs A,
               key = vkey(ai, aj) - 1;
               if (A.vkind[key] == 0) key = -1;
             }
-            hit = rsq.hi <= pg.f_hi && pair_df64_eval(pg, A, s_etab, i, j, ai, aj, key, qi, qi_on, pj.w, lj.w, dx,
+            hit = rsq.hi <= pg.f_hi && pair_df64_eval(pg, A, s_etab, i, j, ai, aj, key, qi, qi_on, pj.w, rj.ql, dx,
                                                       dy, dz, rsq, acc, ix, iy, iz);
           }
           if (hit) {
@@ -1245,7 +1241,9 @@ void pair_forces_sorted(PairGeom& pg, int nb2) {
   A.at_list = g.at_list;
   A.loc_sp = g.loc_sp;
   A.list = g.list; A.ld = g.ld; A.spos = g.spos; A.ldt = g.ldt;
-  A.xhs = g.xhs; A.xls = g.xls; A.tys = g.tys; A.xlh = g.xlh;
+  A.xhs = g.xhs; A.rec = g.rec; A.xlh = g.xlh;
+  A.sh = (float)(268435456.0 / g.pos_scale);
+  A.sl = (float)(1.0 / g.pos_scale);
   A.x = g.x; A.y = g.y; A.z = g.z; A.q = g.chge;
   A.etab = g.erfc_df; A.vtab = g.vdw_df; A.ecoef = g.erfc_coef; A.vcoef = g.vdw_coef;
   A.netab = (g.nsamples + 1) * 3;
