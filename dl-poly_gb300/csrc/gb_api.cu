@@ -1057,10 +1057,7 @@ static int md_run_deferred(int nsteps, gb_step_stats* stats) {
   GB_CUDA(cudaEventRecord(g.ev[5], g.stream));
   g.defer_scalars = true;
   auto stage1 = [&]() {
-    GB_CUDA(cudaMemsetAsync(&g.sc->status, 0, sizeof(int), g.stream));
-    int it = 0;
-    integ_vv(1, nullptr, nullptr, &it, nullptr, nullptr);
-    integ_vnl_launch();
+    integ_stage1_check();
     GB_CUDA(cudaMemcpyAsync(g.hsc, g.sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, g.stream));
   };
   auto step_rest = [&]() {

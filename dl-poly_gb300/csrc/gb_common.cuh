@@ -32,9 +32,11 @@ enum : int {
 struct DevScalars {
   int nlast;        // local + halo atoms
   int nlast_prev;   // the same, as the last relocation left it
-  int status;       // ST_* bits
   int ibig;         // largest list length seen (overflow report)
+  unsigned count;   // blocks done, for grid_sum on the first stream (0 between launches)
+  int status;       // ST_* bits
   int update;       // vnl_check decision
+  double maxdisp;   // bits of the largest squared displacement since the last rebuild
   int shake_iters;
   int rattle_iters;
   int converged;    // constraint iteration flag
@@ -43,8 +45,7 @@ struct DevScalars {
   int tile_max;     // most staged atoms of any cell tile
   int halo_fwd;     // list entries with a halo image found in the forward half shell (evaluated)
   int halo_bwd;     // list entries with a halo image found in the backward halo pass (skipped)
-  int pad[3];
-  double maxdisp;   // largest displacement since the last rebuild
+  int pad[1];
   unsigned long long npairs_list;  // half-list entries walked by the pair kernel
   unsigned long long npairs_rc;    // unique pairs inside the cutoff
   double acc[96];   // energy / virial / stress accumulators
@@ -419,6 +420,53 @@ __device__ __forceinline__ void block_reduce_store(float (&v)[NV], double* out) 
   }
 }
 
+// Grid-wide sums of NV <= 8 doubles in one launch: each block's sums go to part[block], and
+// the block that counts last adds them up, in block order, and hands value k to put(k, sum)
+// (one thread per value).  A warp sums its eight values by a reduce-scatter (9 FP64 additions
+// instead of 5 per value).  count: a zero in device memory, zero again afterwards.  At
+// least 32 NV threads per block.
+template <int NV, typename Put>
+__device__ __forceinline__ void grid_sum(const double (&in)[NV], double* part, unsigned* count, Put put) {
+  static_assert(NV <= 8, "one value per lane after three exchanges");
+  __shared__ double red[32][8];
+  __shared__ bool s_last;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  double v[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) v[k] = k < NV ? in[k < NV ? k : 0] : 0.0;
+#pragma unroll
+  for (int h = 4, o = 16; h > 0; h >>= 1, o >>= 1) {
+    const bool up = lane & o;
+#pragma unroll
+    for (int k = 0; k < h; ++k) {
+      const double keep = up ? v[k + h] : v[k], send = up ? v[k] : v[k + h];
+      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
+  if ((lane & 3) == 0) red[wid][(lane & 16 ? 4 : 0) + (lane & 8 ? 2 : 0) + (lane & 4 ? 1 : 0)] = v[0];
+  __syncthreads();
+  if (threadIdx.x < NV) {
+    double s = 0.0;
+    for (int w = 0; w < nw; ++w) s += red[w][threadIdx.x];
+    part[(size_t)blockIdx.x * NV + threadIdx.x] = s;
+    __threadfence();
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) s_last = atomicAdd(count, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!s_last) return;
+  __threadfence();
+  if (wid < NV) {
+    double s = 0.0;
+    for (int b = lane; b < (int)gridDim.x; b += 32) s += __ldcg(&part[(size_t)b * NV + wid]);
+    s = warp_sum(s);
+    if (lane == 0) put(wid, s);
+  }
+  if (threadIdx.x == 0) *count = 0u;
+}
+
 // host helpers implemented in gb_api.cu
 void gb_sync_scalars();           // copy device scalars to the pinned mirror (synchronises)
 double* gb_blkacc(int n);         // per-block accumulator scratch with n doubles
@@ -456,7 +504,8 @@ void integ_con_tags();            // constraints_tags: old bond vectors from the
 void integ_shake(int* iters, double* vircon, double* strcon);  // apply_shake (throws GB_ERR_SHAKE)
 void integ_rattle_launch();       // apply_rattle, kit = 1 (status bit ST_RATTLE_FAIL)
 int integ_vnl_check();
-void integ_vnl_launch();          // the displacement check, its sums copied to the pinned scalars
+void integ_vnl_launch();          // the displacement check
+void integ_stage1_check();        // NVE stage 1 and the displacement check in one kernel, status cleared
 int integ_vnl_result();           // its decision from the copied scalars (after a wait)
 void integ_zero_forces();
 void integ_forces_to_fp64();      // mixed: fixed point -> FP64 forces

@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
+#include <cstddef>
 #include <cstdlib>
 #include <cstring>
 
@@ -37,6 +38,14 @@ inline int nblocks(long long n, int t) { return (int)((n + t - 1) / t); }
 __device__ __forceinline__ double image1(double d, double c, double a) {
   // images, cubic branch (numerics.F90:1527-1532): d - c*Anint(a*d)
   return sub_rn(d, mul_rn(c, round(mul_rn(a, d))));
+}
+
+__device__ __forceinline__ long long absbits(double v) { return __double_as_longlong(v) & 0x7fffffffffffffffll; }
+
+// d - c*Anint(a*d), skipping the FP64 work when |d| < quarter (bits) makes the shift zero
+__device__ __forceinline__ double image_short(double d, long long quarter_bits, double c, double a) {
+  if (absbits(d) < quarter_bits) return d;
+  return image1(d, c, a);
 }
 
 // Velocity Verlet stages (nve.F90:127-217).  hdw[i] = (tstep/2) / weight(i), formed once
@@ -72,30 +81,63 @@ __global__ void k_vv2(int n, const double* __restrict__ hdw, const double* __res
   }
 }
 
-// m v (x) v summed over the atoms (kinetics.F90:218-262): a grid-stride loop, so each
-// thread reduces its own atoms in registers and the FP64 block reduction runs once per
-// thread rather than once per atom (the FP64 unit bounds this kernel)
-__global__ void k_kinstress(int n, const double* w, const int* lfrzn, const double* vx, const double* vy,
-                            const double* vz, double* blk) {
+// m v (x) v summed over the atoms (kinetics.F90:218-262), after the second half kick of
+// k_vv2 when hdw is given: a grid-stride loop, so each thread reduces its own atoms in
+// registers and the FP64 sum over the grid runs once per thread rather than once per atom
+// (the FP64 unit bounds it).  Its last block adds up the blocks' sums: one launch where
+// the kick, the blocks' sums and their total took three (16 us at 4,096 atoms, now 8).
+constexpr int KIN_NT = 256;
+__global__ void __launch_bounds__(KIN_NT) k_kinstress(int n, const double* __restrict__ w,
+                                                      const int* __restrict__ lfrzn, const double* __restrict__ hdw,
+                                                      const double* __restrict__ fx, const double* __restrict__ fy,
+                                                      const double* __restrict__ fz, double* __restrict__ vx,
+                                                      double* __restrict__ vy, double* __restrict__ vz, double* part,
+                                                      DevScalars* sc) {
   double a[6] = {0, 0, 0, 0, 0, 0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    if (lfrzn[i] != 0) continue;
-    const double m = w[i], u = vx[i], v = vy[i], t = vz[i];
+    const double m = w[i];
+    double u = vx[i], v = vy[i], t = vz[i];
+    const bool frozen = lfrzn[i] != 0;
+    if (hdw) {
+      const double tmp = hdw[i];
+      if (tmp > 0.0) {
+        u = u + tmp * fx[i]; v = v + tmp * fy[i]; t = t + tmp * fz[i];
+        vx[i] = u; vy[i] = v; vz[i] = t;
+      }
+    }
+    if (frozen) continue;
     a[0] += m * u * u; a[1] += m * u * v; a[2] += m * u * t;
     a[3] += m * v * v; a[4] += m * v * t; a[5] += m * t * t;
   }
-  block_reduce_store<6>(a, blk);
+  grid_sum<6>(a, part, &sc->count, [&](int k, double s) { sc->acc[A_STRKIN + k] = s; });
 }
 
-// largest |r - r_checkpoint|^2 with minimum image, over a grid-stride loop; the caller takes
-// the square root of the maximum (the square root is monotone and correctly rounded, so
-// it equals the largest of the per-atom square roots); doubles >= 0 order as their bits
-__global__ void k_maxdisp(int n, const double* x, const double* y, const double* z, const double* xb,
-                          const double* yb, const double* zb, double c0, double a0, unsigned long long* out) {
+// largest |r - r_checkpoint|^2 with minimum image, over a grid-stride loop, after the first
+// half kick and the drift of k_vv1 when hdw is given; the caller takes the square root of
+// the maximum (the square root is monotone and correctly rounded, so it equals the largest
+// of the per-atom square roots); doubles >= 0 order as their bits
+__global__ void k_maxdisp(int n, const double* __restrict__ hdw, double tstep, const double* __restrict__ fx,
+                          const double* __restrict__ fy, const double* __restrict__ fz, double* __restrict__ vx,
+                          double* __restrict__ vy, double* __restrict__ vz, double* __restrict__ x,
+                          double* __restrict__ y, double* __restrict__ z, const double* __restrict__ xb,
+                          const double* __restrict__ yb, const double* __restrict__ zb, double c0, double a0,
+                          unsigned long long* out) {
   double r2 = 0.0;
+  const long long quarter = __double_as_longlong(0.25 * c0);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const double dx = image1(x[i] - xb[i], c0, a0), dy = image1(y[i] - yb[i], c0, a0),
-                 dz = image1(z[i] - zb[i], c0, a0);
+    double px = x[i], py = y[i], pz = z[i];
+    const double bx = xb[i], by = yb[i], bz = zb[i];
+    if (hdw) {
+      const double tmp = hdw[i];
+      if (tmp > 0.0) {
+        const double u = vx[i] + tmp * fx[i], v = vy[i] + tmp * fy[i], t = vz[i] + tmp * fz[i];
+        vx[i] = u; vy[i] = v; vz[i] = t;
+        px = px + tstep * u; py = py + tstep * v; pz = pz + tstep * t;
+        x[i] = px; y[i] = py; z[i] = pz;
+      }
+    }
+    const double dx = image_short(px - bx, quarter, c0, a0), dy = image_short(py - by, quarter, c0, a0),
+                 dz = image_short(pz - bz, quarter, c0, a0);
     r2 = fmax(r2, dx * dx + dy * dy + dz * dz);
   }
 #pragma unroll
@@ -293,14 +335,6 @@ __device__ __forceinline__ void warp_flag(bool fail, int* flag) {
   const unsigned m = __activemask();
   const unsigned b = __ballot_sync(m, fail);
   if (b && (threadIdx.x & 31) == __ffs(m) - 1) atomicOr(flag, 1);
-}
-
-__device__ __forceinline__ long long absbits(double v) { return __double_as_longlong(v) & 0x7fffffffffffffffll; }
-
-// d - c*Anint(a*d), skipping the FP64 work when |d| < quarter (bits) makes the shift zero
-__device__ __forceinline__ double image_short(double d, long long quarter_bits, double c, double a) {
-  if (absbits(d) < quarter_bits) return d;
-  return image1(d, c, a);
 }
 
 // register-array reads with a runtime index, as selects (no local-memory copy)
@@ -1050,11 +1084,28 @@ void integ_forces_to_fp64() {
   GB_LAUNCHED();
 }
 
+// The displacement check, with the NVE stage 1 in the same pass when stage1 is set.  The
+// caller has cleared maxdisp (integ_clear).
+static void launch_maxdisp(bool stage1) {
+  k_maxdisp<<<std::min(nblocks(g.natms, 128), 4 * g.nsm), 128, 0, g.stream>>>(
+      g.natms, stage1 ? g.hdw : nullptr, g.p.tstep, g.fx, g.fy, g.fz, g.vx, g.vy, g.vz, g.x, g.y, g.z, g.xbg, g.ybg,
+      g.zbg, g.cell[0], 1.0 / g.cell[0], (unsigned long long*)&g.sc->maxdisp);
+  GB_LAUNCHED();
+}
+
+// NVE without constraints: stage 1 and the displacement check as one kernel, behind one
+// clearing of the status and the maximum
+void integ_stage1_check() {
+  GB_CUDA(cudaMemsetAsync(&g.sc->status, 0, offsetof(DevScalars, maxdisp) + sizeof(double) - offsetof(DevScalars, status),
+                          g.stream));
+  prof_begin(P_VV);
+  launch_maxdisp(true);
+  prof_end(P_VV);
+}
+
 void integ_vnl_launch() {
   GB_CUDA(cudaMemsetAsync(&g.sc->maxdisp, 0, sizeof(double), g.stream));
-  k_maxdisp<<<std::min(nblocks(g.natms, 256), 2 * g.nsm), 256, 0, g.stream>>>(
-      g.natms, g.x, g.y, g.z, g.xbg, g.ybg, g.zbg, g.cell[0], 1.0 / g.cell[0], (unsigned long long*)&g.sc->maxdisp);
-  GB_LAUNCHED();
+  launch_maxdisp(false);
 }
 
 int integ_vnl_result() { return std::sqrt(g.hsc->maxdisp) >= std::nextafter(0.5, 0.0) * g.p.rpad ? 1 : 0; }
@@ -1171,6 +1222,14 @@ void integ_rattle_launch() {
   prof_end(P_RATTLE);
 }
 
+// kinetic stress into acc[A_STRKIN], after the second half kick when kick is set
+static void launch_kinstress(bool kick) {
+  const int nb = std::min(nblocks(g.natms, KIN_NT), 2 * g.nsm);
+  k_kinstress<<<nb, KIN_NT, 0, g.stream>>>(g.natms, g.weight, g.lfrzn, kick ? g.hdw : nullptr, g.fx, g.fy, g.fz, g.vx,
+                                           g.vy, g.vz, gb_blkacc(nb * 6), g.sc);
+  GB_LAUNCHED();
+}
+
 void integ_vv(int stage, double* strkin, double* engke, int* iters, double* vircon, double* strcon) {
   cudaStream_t st = g.stream;
   const int n = g.natms;
@@ -1186,17 +1245,17 @@ void integ_vv(int stage, double* strkin, double* engke, int* iters, double* virc
     prof_end(P_VV);
     integ_shake(iters, vircon, strcon);
   } else {
+    const bool fused = g.ntcons <= 0 && g.ens == GB_NVE;  // the kick and the kinetic stress in one pass
     prof_begin(P_VV);
-    k_vv2<<<nblocks(n, 256), 256, 0, st>>>(n, g.hdw, g.fx, g.fy, g.fz, g.vx, g.vy, g.vz);
-    GB_LAUNCHED();
+    if (!fused) {
+      k_vv2<<<nblocks(n, 256), 256, 0, st>>>(n, g.hdw, g.fx, g.fy, g.fz, g.vx, g.vy, g.vz);
+      GB_LAUNCHED();
+    }
+    if (fused) launch_kinstress(true);
     prof_end(P_VV);
     integ_rattle_launch();
     if (!thermo_vv2_finish(strkin, engke)) {
-      const int nb = std::min(nblocks(n, 256), 2 * g.nsm);
-      double* blk = gb_blkacc(nb * 6);
-      k_kinstress<<<nb, 256, 0, st>>>(n, g.weight, g.lfrzn, g.vx, g.vy, g.vz, blk);
-      GB_LAUNCHED();
-      gb_reduce_blocks(blk, nb, 6, &g.sc->acc[A_STRKIN]);
+      if (!fused) launch_kinstress(false);
       if (g.defer_scalars) return;  // the MD loop reads the sums after its last step
       gb_sync_scalars();
       kin_scalars(g.hsc, strkin, engke);

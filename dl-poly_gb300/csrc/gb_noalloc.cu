@@ -14,53 +14,43 @@
 namespace {
 
 constexpr int KIN_THREADS = 256;
-constexpr int KIN_MAX_BLOCKS = 4096;                              // 4096 * 256 = 1,048,576 atoms
-constexpr int KIN_MAX_ATOMS = KIN_MAX_BLOCKS * KIN_THREADS;
+constexpr int KIN_MAX_ATOMS = 1048576;
+constexpr int KIN_SLOTS = 4096;    // of 6 doubles: 196,608 B per device
+constexpr int KIN_BLOCKS = 304;    // two per SM: the partial sums of at most so many blocks are kept
 constexpr int KIN_MAX_DEVICES = 64;
 
-// 6 partial sums per block: 4096 * 6 * 8 B = 196,608 B per device.
-static __device__ __align__(256) double g_kin_scratch[KIN_MAX_BLOCKS * 6];
+// The blocks' partial sums in its first KIN_BLOCKS slots; its last word counts the blocks
+// that are done (0 between calls).
+static __device__ __align__(256) double g_kin_scratch[KIN_SLOTS * 6];
 
 // Host side: the device address of g_kin_scratch on each device, looked up
 // once per device.  (In host code the symbol name itself is only a host-side
 // stand-in, never a device address.)
 double* g_kin_scratch_addr[KIN_MAX_DEVICES] = {nullptr};
 
-__global__ void k_kin_partial(int n, const double* __restrict__ w, const int* __restrict__ lfrzn,
-                              const double* __restrict__ vx, const double* __restrict__ vy,
-                              const double* __restrict__ vz, double* part) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// A grid-stride loop whose last block adds up the blocks' sums: one launch instead of two,
+// and one reduction per thread instead of one per atom.  98,304 atoms: 22.5 -> 16.2 us a
+// call, the latency of the launch, of the loads and of the two stages of the sum.
+__global__ void __launch_bounds__(KIN_THREADS) k_kin_sum(int n, const double* __restrict__ w,
+                                                         const int* __restrict__ lfrzn, const double* __restrict__ vx,
+                                                         const double* __restrict__ vy, const double* __restrict__ vz,
+                                                         double* part, double* __restrict__ out) {
   double a[6] = {0, 0, 0, 0, 0, 0};
-  if (i < n && (lfrzn == nullptr || lfrzn[i] == 0)) {
-    const double m = w[i];
-    a[0] = m * vx[i] * vx[i]; a[1] = m * vx[i] * vy[i]; a[2] = m * vx[i] * vz[i];
-    a[3] = m * vy[i] * vy[i]; a[4] = m * vy[i] * vz[i]; a[5] = m * vz[i] * vz[i];
+  const int stride = gridDim.x * blockDim.x;
+#pragma unroll 4
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) {
+    const bool free_atom = lfrzn == nullptr || lfrzn[i] == 0;
+    const double m = w[i], u = vx[i], v = vy[i], t = vz[i];
+    if (!free_atom) continue;
+    const double mu = m * u, mv = m * v;
+    a[0] = fma(mu, u, a[0]); a[1] = fma(mu, v, a[1]); a[2] = fma(mu, t, a[2]);
+    a[3] = fma(mv, v, a[3]); a[4] = fma(mv, t, a[4]); a[5] = fma(m * t, t, a[5]);
   }
-  // every block writes its own 6 slots, so nothing has to be cleared first
-  block_reduce_store<6>(a, part);
-}
-
-__global__ void k_kin_final(int nb, const double* __restrict__ part, double* __restrict__ out) {
-  __shared__ double red[32][6];
-  double s[6] = {0, 0, 0, 0, 0, 0};
-  for (int b = threadIdx.x; b < nb; b += blockDim.x)
-    for (int k = 0; k < 6; ++k) s[k] += part[(size_t)b * 6 + k];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int k = 0; k < 6; ++k) s[k] = warp_sum(s[k]);
-  if (lane == 0)
-    for (int k = 0; k < 6; ++k) red[wid][k] = s[k];
-  __syncthreads();
-  if (wid == 0) {
-    for (int k = 0; k < 6; ++k) {
-      double t = lane < (int)(blockDim.x >> 5) ? red[lane][k] : 0.0;
-      s[k] = warp_sum(t);
-    }
-    if (lane == 0) {
-      out[0] = s[0]; out[1] = s[1]; out[2] = s[2];
-      out[3] = s[1]; out[4] = s[3]; out[5] = s[4];
-      out[6] = s[2]; out[7] = s[4]; out[8] = s[5];
-    }
-  }
+  grid_sum<6>(a, part, reinterpret_cast<unsigned*>(part + KIN_SLOTS * 6) - 1, [&](int k, double s) {
+    const int at[6] = {0, 1, 2, 4, 5, 8}, mirror[6] = {0, 3, 6, 4, 7, 8};
+    out[at[k]] = s;
+    out[mirror[k]] = s;
+  });
 }
 
 }  // namespace
@@ -77,12 +67,9 @@ extern "C" int gb_kinstress_noalloc(const double* vx, const double* vy, const do
     if (cudaGetSymbolAddress((void**)&p, g_kin_scratch) != cudaSuccess || !p) return GB_ERR_CUDA;
     g_kin_scratch_addr[dev] = p;
   }
-  double* part = g_kin_scratch_addr[dev];
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
   const int nb = n > 0 ? (n + KIN_THREADS - 1) / KIN_THREADS : 1;
-  k_kin_partial<<<nb, KIN_THREADS, 0, st>>>(n, weight, lfrzn, vx, vy, vz, part);
-  if (cudaGetLastError() != cudaSuccess) return GB_ERR_CUDA;
-  k_kin_final<<<1, 256, 0, st>>>(nb, part, strkin_out);
+  k_kin_sum<<<nb < KIN_BLOCKS ? nb : KIN_BLOCKS, KIN_THREADS, 0, static_cast<cudaStream_t>(stream)>>>(
+      n, weight, lfrzn, vx, vy, vz, g_kin_scratch_addr[dev], strkin_out);
   if (cudaGetLastError() != cudaSuccess) return GB_ERR_CUDA;
   return GB_OK;
 }

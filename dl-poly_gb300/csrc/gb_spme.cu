@@ -484,9 +484,9 @@ __global__ void k_spme_gather(int natms, const double* __restrict__ x, const dou
 // GATHER_AB atoms at a time: 3 x GATHER_AB lanes build their splines in parallel, and
 // the four per-atom sums are combined by a reduce-scatter that leaves the energy sum in
 // lane 0 and the x, y, z force sums in lanes 8, 16, 24.
-constexpr int GATHER_AB = 8;  // atoms per warp batch
+constexpr int GATHER_AB = 8;  // most atoms per warp batch (ab: fewer in a small system, see grid_run)
 template <int P>
-__global__ void __launch_bounds__(256, 4) k_spme_gather_f32(int natms, const float* __restrict__ q4, SpmeGeom sg,
+__global__ void __launch_bounds__(256, 4) k_spme_gather_f32(int natms, int ab, const float* __restrict__ q4, SpmeGeom sg,
                                                          const int* __restrict__ gidx, const float* __restrict__ gw,
                                                          const float* __restrict__ phi, float rk0, float rk1,
                                                          float rk2, float* __restrict__ fout, double* blk) {
@@ -495,9 +495,8 @@ __global__ void __launch_bounds__(256, 4) k_spme_gather_f32(int natms, const flo
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
   const int K0 = sg.K[0], K1 = sg.K[1], K2 = sg.K[2];
   float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * GATHER_AB; base < natms;
-       base += nwarps * GATHER_AB) {
-    if (lane < 3 * GATHER_AB) {
+  for (int base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * ab; base < natms; base += nwarps * ab) {
+    if (lane < 3 * ab) {
       const int a = lane / 3, d = lane - 3 * a, i = base + a;
       if (i < natms) {
         float m[PMAX], dm[PMAX];
@@ -507,7 +506,7 @@ __global__ void __launch_bounds__(256, 4) k_spme_gather_f32(int natms, const flo
       }
     }
     __syncwarp();
-    const int na = min(GATHER_AB, natms - base);
+    const int na = min(ab, natms - base);
     for (int a = 0; a < na; ++a) {
       const int i = base + a;
       const float qi = q4[4 * i + 3];
@@ -614,7 +613,7 @@ __device__ __forceinline__ df ld_df(const dfr* p) {
 // the second) that leaves them in lanes 0, 8, 16, 24.  No FP64 instruction: forces leave
 // as double-floats.
 template <int P>
-__global__ void __launch_bounds__(256, 6) k_spme_gather_wdf(int natms, SpmeGeom sg, const int* __restrict__ gidx,
+__global__ void __launch_bounds__(256, 6) k_spme_gather_wdf(int natms, int ab, SpmeGeom sg, const int* __restrict__ gidx,
                                                          const dfr* __restrict__ gsp,
                                                          const float2* __restrict__ gq, const dfr* __restrict__ phi,
                                                          float2 rk0, float2 rk1, float2 rk2, float qmax,
@@ -635,9 +634,8 @@ __global__ void __launch_bounds__(256, 6) k_spme_gather_wdf(int natms, SpmeGeom 
   dacc acc[4];
 #pragma unroll
   for (int c = 0; c < 4; ++c) { acc[c].s = 0.f; acc[c].c = 0.f; }
-  for (int base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * GATHER_AB; base < natms;
-       base += nwarps * GATHER_AB) {
-    const int na = min(GATHER_AB, natms - base);
+  for (int base = ((blockIdx.x * blockDim.x + threadIdx.x) >> 5) * ab; base < natms; base += nwarps * ab) {
+    const int na = min(ab, natms - base);
 #pragma unroll
     for (int e = lane; e < NS * GATHER_AB; e += 32) {
       const int c = e >> 3, a = e & 7;
@@ -876,14 +874,19 @@ SpmeGrid S_main, S_coarse;
 // GB_SPREAD_FIX=1 selects the int64 fixed-point spread with shared-memory atomics
 bool g_spread_fix = false;
 
-// Brick edge: a divisor of K of at least p-1 (a brick's atoms reach at most the
-// next brick).  Larger bricks cut the halo overlap (B+p-1)^3 / B^3 of the tiles
-// the fixed-order reduction reads back, so prefer one of at least bpref (BPREF for
-// the force grid; the coarse grid of the multiple-time-step form, with 8x fewer
-// points, prefers BPREF_COARSE so that its bricks hold as few atoms and are as many).
-constexpr int BPREF = 12, BPREF_COARSE = 8;
-int choose_brick(int K, int p, int bpref) {
-  for (int B = std::max(p - 1, bpref); B <= BMAX; ++B)
+// Brick edge: a divisor of K of at least p-1 (a brick's atoms reach at most the next
+// brick).  Larger bricks cut the halo overlap (B+p-1)^3 / B^3 of the tiles that the
+// fixed-order reduction reads back, but beyond 12 a tile leaves one CTA per SM (double-
+// float spread with its reduction, B = 16 against the rule's: 160^3 0.314 / 0.227 ms,
+// 128^3 0.161 / 0.123 ms), and a grid of few bricks leaves SMs idle (48^3, B = 12
+// against 8: 0.025 / 0.021 ms): the largest edge up to 12 that gives a hundred bricks, else
+// the smallest.  The coarse grid of the multiple-time-step form takes the smallest from 8.
+int choose_brick(int K, int p, bool coarse) {
+  if (!coarse) {
+    for (int B = 12; B >= p - 1; --B)
+      if (K % B == 0 && (long long)(K / B) * (K / B) * (K / B) >= 100) return B;
+  }
+  for (int B = coarse ? std::max(p - 1, 8) : p - 1; B <= BMAX; ++B)
     if (K % B == 0) return B;
   for (int B = p - 1; B <= BMAX; ++B)
     if (K % B == 0) return B;
@@ -949,7 +952,7 @@ void raise_fft(const SpmeGrid& S, int smem) {
   raise_smem(k.z_conv, smem);
 }
 
-void grid_setup(SpmeGrid& S, const int* Kin, int p, bool fp64, int bpref) {
+void grid_setup(SpmeGrid& S, const int* Kin, int p, bool fp64) {
   grid_free(S);
   if (p > PMAX || p < 3) throw (int)GB_ERR_ARG;
   for (int d = 0; d < 3; ++d) S.K[d] = Kin[d];
@@ -960,7 +963,7 @@ void grid_setup(SpmeGrid& S, const int* Kin, int p, bool fp64, int bpref) {
   S.planh = make_plan(S.K[0] / 2);
   S.Kx = S.K[0] / 2 + 1;
   for (int d = 0; d < 3; ++d) {
-    S.B[d] = choose_brick(S.K[d], p, bpref);
+    S.B[d] = choose_brick(S.K[d], p, !fp64);
     if (S.B[d] < 0) {
       // fall back to the whole dimension as one brick if it is small enough
       if (S.K[d] <= BMAX) S.B[d] = S.K[d];
@@ -1274,21 +1277,23 @@ void grid_run(SpmeGrid& S, bool coarse, float* rec, double* eng_rc, double* vir_
   if (!occ_g) GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_g, k_spme_gather_f32<8>, 256, 0));
   static int occ_gd = 0;
   if (DF && !occ_gd) GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_gd, k_spme_gather_wdf<8>, 256, 0));
-  const int nbg = warp_gather ? std::max(1, std::min((DF ? occ_gd : occ_g) * g.nsm,
-                                                     nblocks((long long)n * 32 / GATHER_AB, 256)))
-                              : nblocks(n, 128);
+  // atoms per warp: up to 8, fewer where that would leave resident warps without an atom
+  // (4,096 ions: one atom per warp, 0.012 instead of 0.041 ms)
+  const int slots = (DF ? occ_gd : occ_g) * g.nsm;
+  const int ab = std::max(1, std::min(GATHER_AB, n / (8 * std::max(1, slots))));
+  const int nbg = warp_gather ? std::max(1, std::min(slots, nblocks((long long)nblocks(n, ab) * 32, 256))) : nblocks(n, 128);
   double* blkg = blkz + (size_t)nbz * 6;
   prof_begin(pid(P_SPME_GATHER));
   if (warp_gather && DF) {
     auto kern = p == 8 ? k_spme_gather_wdf<8> : k_spme_gather_wdf<6>;
     float2 rkd[3];
     for (int a = 0; a < 3; ++a) df_split(rk[a], &rkd[a].x, &rkd[a].y);
-    kern<<<nbg, 256, 0, st>>>(n, S.sg, S.gidx, reinterpret_cast<const dfr*>(S.gsp),
+    kern<<<nbg, 256, 0, st>>>(n, ab, S.sg, S.gidx, reinterpret_cast<const dfr*>(S.gsp),
                               reinterpret_cast<const float2*>(S.gw + 6 * (size_t)n), reinterpret_cast<const dfr*>(Q),
                               rkd[0], rkd[1], rkd[2], S.qmax, vmax, reinterpret_cast<float2*>(S.fspme), blkg);
   } else if (warp_gather) {
     auto kern = p == 8 ? k_spme_gather_f32<8> : k_spme_gather_f32<6>;
-    kern<<<nbg, 256, 0, st>>>(n, reinterpret_cast<const float*>(g.xf), S.sg, S.gidx, S.gw,
+    kern<<<nbg, 256, 0, st>>>(n, ab, reinterpret_cast<const float*>(g.xf), S.sg, S.gidx, S.gw,
                               reinterpret_cast<const float*>(Q), (float)rk[0], (float)rk[1], (float)rk[2], S.fout_f,
                               blkg);
   } else {
@@ -1344,7 +1349,7 @@ void spme_scalars(const DevScalars* h, double* eng_rc, double* vir_rc, double* s
 void spme_setup() {
   const char* e = getenv("GB_SPREAD_FIX");
   g_spread_fix = e && e[0] == '1';
-  grid_setup(S_main, g.p.kmax, g.p.nsplines, true, BPREF);
+  grid_setup(S_main, g.p.kmax, g.p.nsplines, true);
 }
 
 void spme_free() {
@@ -1359,7 +1364,7 @@ void spme_forces(double* eng_rc, double* vir_rc, double* stress9) {
   else grid_run<float, float2>(S_main, false, rec, eng_rc, vir_rc, stress9);
 }
 
-void spme_coarse_setup(const int* K, int p) { grid_setup(S_coarse, K, p, false, BPREF_COARSE); }
+void spme_coarse_setup(const int* K, int p) { grid_setup(S_coarse, K, p, false); }
 
 bool spme_coarse_ready() { return S_coarse.ready; }
 
