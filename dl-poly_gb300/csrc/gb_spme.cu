@@ -81,6 +81,17 @@ __device__ __forceinline__ void bspline_vals(T w, int p_rt, T* m /*p*/, T* dm /*
   for (int t = 0; t < p; ++t) m[t] = z[t + 1];
 }
 
+// The atoms of the spread's bricks: cap slots per brick filled by the preparation kernel,
+// atoms beyond a brick's slots in one overflow list of (brick, atom).
+struct SpreadBins {
+  int cap;
+  int* count;              // atoms per brick
+  int* bucket;             // nbricks x cap, or null
+  int2* ovf;
+  int *ovf_count, *pool;   // entries of ovf; integers taken from a and b
+  int *a, *b;              // natms each, for bricks with more atoms than slots
+};
+
 // Splines and brick binning: a CTA takes PREP_AT atoms with one thread per atom and
 // dimension (threads d * PREP_AT + a), so that each thread builds one spline; the
 // dimension-0 threads then combine the three brick coordinates through shared memory.
@@ -89,7 +100,7 @@ template <typename T, int P>
 __global__ void __launch_bounds__(3 * PREP_AT, std::is_same<T, dfr>::value ? 5 : 0) k_spme_prep(int natms, const double* __restrict__ x,
                                                            const double* __restrict__ y, const double* __restrict__ z,
                                                            const double* __restrict__ q, SpmeGeom sg, T* spl,
-                                                           int* nidx, int* brick_of, int* brick_count, int* gidx,
+                                                           int* nidx, int* brick_of, SpreadBins bins, int* gidx,
                                                            float* gw, float2* gq, T* gsp) {
   __shared__ int bsh[3][PREP_AT];
   const int d = threadIdx.x / PREP_AT, a = threadIdx.x - d * PREP_AT;
@@ -143,11 +154,19 @@ __global__ void __launch_bounds__(3 * PREP_AT, std::is_same<T, dfr>::value ? 5 :
     if (b >= 0) df_split(q[i], &h, &l);
     gq[i] = make_float2(h, l);
   }
-  brick_of[i] = b;
   // the lanes of a warp that share a brick add their count with one atomic (atoms of
-  // nearby index are near each other in the lattice start); counts are order-independent
-  const unsigned grp = __match_any_sync(__activemask(), b);
-  if (b >= 0 && (int)(threadIdx.x & 31) == __ffs(grp) - 1) atomicAdd(&brick_count[b], __popc(grp));
+  // nearby index are near each other in the lattice start) and take consecutive slots
+  const unsigned act = __activemask(), grp = __match_any_sync(act, b);
+  const int lane = threadIdx.x & 31, leader = __ffs(grp) - 1;
+  int slot = 0;
+  if (b >= 0 && lane == leader) slot = atomicAdd(&bins.count[b], __popc(grp));
+  slot = __shfl_sync(act, slot, leader) + __popc(grp & ((1u << lane) - 1u));
+  if (!bins.bucket) {  // the fixed-point spread sorts the bricks by a scan of the counts
+    brick_of[i] = b;
+  } else if (b >= 0) {
+    if (slot < bins.cap) bins.bucket[(size_t)b * bins.cap + slot] = i;
+    else bins.ovf[atomicAdd(bins.ovf_count, 1)] = make_int2(b, i);
+  }
 }
 
 // atoms into their bricks' ranges; the lanes of a warp that share a brick take
@@ -166,21 +185,9 @@ __global__ void k_brick_scatter(int natms, const int* brick_of, const int* start
   tmp[start[b] + base + __popc(grp & ((1u << lane) - 1u))] = i;
 }
 
-__global__ void k_brick_sort(int nbricks, const int* start, const int* tmp, int* out) {
-  int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (warp >= nbricks) return;
-  int s = start[warp], n = start[warp + 1] - s;
-  for (int a = lane; a < n; a += 32) {
-    int v = tmp[s + a], r = 0;
-    for (int b = 0; b < n; ++b) r += tmp[s + b] < v;
-    out[s + r] = v;
-  }
-}
-
 // ------------------------------------------------------------- spreading
-constexpr int SPREAD_CH = 32;
+constexpr int SPREAD_CH = 16;
 constexpr int SPREAD_NT = 512;             // threads of a tile-spread CTA
-constexpr int SPREAD_NW = SPREAD_NT / 32;  // its warps (a power of two: plane owner = z & (NW - 1))
 constexpr int BMAX = 16;
 
 // tile point += a * b.  Double-float tiles hold unnormalised compensated pairs: the exact
@@ -201,18 +208,30 @@ __device__ __forceinline__ void tile_acc(T* dst, T a, T b) { *dst = tile_upd(*ds
 
 // Tile scatter: CTA = one brick and the atoms whose floor(u) lies in it.  The
 // CTA owns a (B+p-1)^3 shared-memory tile covering the brick plus the p-1
-// points below it that its atoms reach; atoms are scattered one after another
-// (one FMA per grid point, no atomics; each warp owns every nw-th z plane of the
-// tile, so a chunk of atoms needs one barrier; launched with SPREAD_NT threads),
+// points below it that its atoms reach; atoms are scattered one after another, in index
+// order (one FMA per grid point, no atomics; each warp owns every nw-th z plane of the
+// tile, so a chunk of atoms needs two barriers; launched with SPREAD_NT threads),
 // then the tile is written to its own slot of `ext` for the halo reduction below.
 // Per chunk atom the set-up stores Mx, the p x p products My (Mz q) and the atom's
-// tile offset with its z and y offsets (one 16-byte read per atom in the scatter).
+// tile offset with its z and y offsets (one 16-byte read per atom in the scatter); the next
+// chunk's splines are copied asynchronously into `raw` while this chunk is scattered.
 // NT = 256 (order 8): warp w owns the tile planes z = w (mod 8) and takes the whole plane
 // of each atom, two points per lane (rows k and k + 4), two independent updates.
+__host__ __device__ inline size_t tile_bytes(size_t tsize, size_t esz, int cap) {  // holds cap integers too
+  const size_t t = tsize * esz, c = sizeof(int) * (((size_t)cap + 1) & ~(size_t)1);
+  return t > c ? t : c;
+}
+
+template <int BYTES>
+__device__ __forceinline__ void copy_async(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+               "n"(BYTES)
+               : "memory");
+}
+
 template <typename T, int P, int NT = SPREAD_NT>
-__global__ void k_spme_spread_tile(SpmeGeom sg, const int* __restrict__ bstart, const int* __restrict__ batoms,
-                                   const T* __restrict__ spl, const int* __restrict__ nidx,
-                                   const double* __restrict__ q, T* __restrict__ ext) {
+__global__ void k_spme_spread_tile(SpmeGeom sg, SpreadBins bins, const T* __restrict__ spl,
+                                   const int* __restrict__ nidx, T* __restrict__ ext) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   const int p = P ? P : sg.p;
   const int b = blockIdx.x;
@@ -221,32 +240,88 @@ __global__ void k_spme_spread_tile(SpmeGeom sg, const int* __restrict__ bstart, 
   const int TXd = sg.B[0] + p - 1, TYd = sg.B[1] + p - 1, TZd = sg.B[2] + p - 1;
   const int PL = TXd * TYd;
   const int tsize = PL * TZd;
+  const int p2 = p * p, p3 = 3 * p;
   int4* info = reinterpret_cast<int4*>(smem_raw);  // [SPREAD_CH] tile offset, z offset, y offset, x offset
   T* Pkl = reinterpret_cast<T*>(info + SPREAD_CH);  // [SPREAD_CH][p*p] My(k) * q Mz(l)
-  T* Mx = Pkl + SPREAD_CH * p * p;                   // [SPREAD_CH][p]
+  T* raw = Pkl + SPREAD_CH * p2;                     // [SPREAD_CH][3*p] splines of the next chunk
+  T* Mx = raw + SPREAD_CH * p3;                      // [SPREAD_CH][p]
   T* tile = Mx + SPREAD_CH * p;
-  for (int e = threadIdx.x; e < tsize; e += blockDim.x) tile[e] = (T)0;
-  const int s0 = bstart[b], s1 = bstart[b + 1];
-  const int p2 = p * p;
+  // [SPREAD_CH][3] grid indices of the next chunk, after the tile's space
+  int* rawn = reinterpret_cast<int*>(reinterpret_cast<unsigned char*>(tile) + tile_bytes(tsize, sizeof(T), bins.cap));
+  int* order = rawn + 3 * SPREAD_CH;                 // [cap] the brick's atoms in index order
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  for (int c = s0; c < s1; c += SPREAD_CH) {
-    const int nc = min(SPREAD_CH, s1 - c);
+  const int na = bins.count[b];
+  const int* atoms = order;
+  if (na <= bins.cap) {  // rank sort in shared memory; the tile's space holds the unsorted atoms
+    int* un = reinterpret_cast<int*>(tile);
+    const int* bucket = bins.bucket + (size_t)b * bins.cap;
+    for (int e = threadIdx.x; e < na; e += blockDim.x) un[e] = bucket[e];
+    __syncthreads();
+    for (int e = threadIdx.x; e < na; e += blockDim.x) {
+      const int v = un[e];
+      int r = 0;
+      for (int k = 0; k < na; ++k) r += un[k] < v;
+      order[r] = v;
+    }
+  } else {  // the brick's slots and its entries of the overflow list, sorted in global memory
+    __shared__ int s_base, s_n;
+    if (threadIdx.x == 0) {
+      s_base = atomicAdd(bins.pool, na);
+      s_n = bins.cap;
+    }
+    __syncthreads();
+    int *un = bins.a + s_base, *so = bins.b + s_base;
+    for (int e = threadIdx.x; e < bins.cap; e += blockDim.x) un[e] = bins.bucket[(size_t)b * bins.cap + e];
+    const int no = *bins.ovf_count;
+    for (int e = threadIdx.x; e < no; e += blockDim.x) {
+      const int2 o = bins.ovf[e];
+      if (o.x == b) un[atomicAdd(&s_n, 1)] = o.y;
+    }
+    __syncthreads();
+    for (int e = threadIdx.x; e < na; e += blockDim.x) {
+      const int v = un[e];
+      int r = 0;
+      for (int k = 0; k < na; ++k) r += un[k] < v;
+      so[r] = v;
+    }
+    atoms = so;
+  }
+  __syncthreads();
+  auto fetch = [&](int c) {  // the splines and grid indices of the chunk at c
+    const int nc = min(SPREAD_CH, na - c);
+    if constexpr (P != 0) {
+      constexpr int U = 3 * P * (int)sizeof(T) / 8;  // 8-byte units per atom
+      for (int e = threadIdx.x; e < nc * U; e += blockDim.x) {
+        const int a = e / U, u = e - a * U;
+        copy_async<8>(reinterpret_cast<char*>(raw + a * p3) + 8 * u,
+                      reinterpret_cast<const char*>(spl + (size_t)atoms[c + a] * p3) + 8 * u);
+      }
+      for (int e = threadIdx.x; e < nc * 3; e += blockDim.x) copy_async<4>(rawn + e, nidx + 3 * (size_t)atoms[c + e / 3] + e % 3);
+    } else {
+      for (int e = threadIdx.x; e < nc * p3; e += blockDim.x) raw[e] = spl[(size_t)atoms[c + e / p3] * p3 + e % p3];
+      for (int e = threadIdx.x; e < nc * 3; e += blockDim.x) rawn[e] = nidx[3 * (size_t)atoms[c + e / 3] + e % 3];
+    }
+  };
+  if (na > 0) fetch(0);
+  for (int e = threadIdx.x; e < tsize; e += blockDim.x) tile[e] = (T)0;
+  for (int c = 0; c < na; c += SPREAD_CH) {
+    const int nc = min(SPREAD_CH, na - c);
+    if constexpr (P != 0) asm volatile("cp.async.wait_all;" ::: "memory");
     __syncthreads();
     for (int e = threadIdx.x; e < nc * p; e += blockDim.x) {
       const int a = e / p, t = e - a * p;
-      const int i = batoms[c + a];
-      Mx[a * p + t] = spl[((size_t)i * 3 + 0) * p + t];
+      Mx[e] = raw[a * p3 + t];
       if (t == 0) {
-        const int ox = nidx[3 * i + 0] - g0x, oy = nidx[3 * i + 1] - g0y, oz = nidx[3 * i + 2] - g0z;
+        const int ox = rawn[3 * a] - g0x, oy = rawn[3 * a + 1] - g0y, oz = rawn[3 * a + 2] - g0z;
         info[a] = make_int4(oz * PL + oy * TXd + ox, oz, oy, ox);
       }
     }
     for (int e = threadIdx.x; e < nc * p2; e += blockDim.x) {
       const int a = e / p2, kl = e - a * p2, k = kl % p, l = kl / p;
-      const int i = batoms[c + a];
-      Pkl[a * p2 + kl] = spl[((size_t)i * 3 + 1) * p + k] * spl[((size_t)i * 3 + 2) * p + l];  // My (Mz q)
+      Pkl[e] = raw[a * p3 + p + k] * raw[a * p3 + 2 * p + l];  // My (Mz q)
     }
     __syncthreads();
+    if (c + SPREAD_CH < na) fetch(c + SPREAD_CH);
     // every tile point is only ever written by one warp, in atom order, so the warps run
     // through the chunk without a barrier per atom.  Orders up to 8: the points of tile
     // plane z and row y belong to warp (z mod 8) + 8 (y mod 2), so every warp takes one
@@ -407,9 +482,10 @@ __global__ void k_spme_tile_reduce(SpmeGeom sg, const T* __restrict__ ext, T* __
   Q[((size_t)gz * sg.K[1] + gy) * sg.K[0] + gx] = tile_sum<T, T>(sg, ext, gx, gy, gz);
 }
 
-inline size_t spread_smem(int B0, int B1, int B2, int p, size_t esz) {
+inline size_t spread_smem(int B0, int B1, int B2, int p, size_t esz, int cap) {
   const size_t tsize = (size_t)(B0 + p - 1) * (B1 + p - 1) * (B2 + p - 1);
-  return esz * (tsize + (size_t)SPREAD_CH * p * p + (size_t)SPREAD_CH * p) + sizeof(int4) * SPREAD_CH;
+  return tile_bytes(tsize, esz, cap) + esz * ((size_t)SPREAD_CH * p * p + (size_t)SPREAD_CH * 4 * p) +
+         (sizeof(int4) + 3 * sizeof(int)) * SPREAD_CH + sizeof(int) * (size_t)cap;
 }
 
 // --------------------------------------------------------------- gather
@@ -842,6 +918,10 @@ struct SpmeGrid {
   int* nidx = nullptr;         // natms * 3 grid indices
   int *brick_of = nullptr, *brick_count = nullptr, *brick_start = nullptr, *brick_fill = nullptr,
       *brick_atoms = nullptr;
+  // the spread's bricks (SpreadBins): slots per brick, slots, overflow list, second sort buffer
+  int cap = 0;
+  int *bucket = nullptr, *brick_sort = nullptr;
+  int2* ovf = nullptr;
   double* Q = nullptr;
   double2* G = nullptr;
   float* Qf = nullptr;
@@ -934,7 +1014,7 @@ void grid_free(SpmeGrid& S) {
   void* ptrs[] = {S.spl, S.nidx, S.brick_of, S.brick_count, S.brick_start, S.brick_fill, S.brick_atoms, S.Q, S.G,
                   S.Qf, S.Gf, S.theta, S.psi, S.theta_f, S.psi_f, S.tw[0], S.tw[1], S.tw[2], S.twf[0], S.twf[1],
                   S.twf[2], S.twh, S.twhf, S.fspme, S.spread_ext, S.gidx, S.gw, S.gsp, S.fout_f, S.theta_d, S.psi_d,
-                  S.tw_d[0], S.tw_d[1], S.tw_d[2], S.twh_d};
+                  S.tw_d[0], S.tw_d[1], S.tw_d[2], S.twh_d, S.bucket, S.brick_sort, S.ovf};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   S = SpmeGrid();
@@ -989,7 +1069,13 @@ void grid_setup(SpmeGrid& S, const int* Kin, int p, bool fp64) {
   GB_CUDA(cudaMalloc(&S.spl, sizeof(double) * n * 3 * p));
   GB_CUDA(cudaMalloc(&S.nidx, sizeof(int) * 3 * n));
   GB_CUDA(cudaMalloc(&S.brick_of, sizeof(int) * n));
-  GB_CUDA(cudaMalloc(&S.brick_count, sizeof(int) * (S.nbricks + 2)));
+  // after the counts: one unused, then the largest |potential|, the overflow entries, the pool
+  GB_CUDA(cudaMalloc(&S.brick_count, sizeof(int) * (S.nbricks + 4)));
+  // slots for three times the mean and some; at most 2,048 (their sorted copy is in shared memory)
+  S.cap = std::min(2048, (int)std::min<size_t>(n, 3 * (n / S.nbricks) + 32));
+  GB_CUDA(cudaMalloc(&S.bucket, sizeof(int) * (size_t)S.nbricks * S.cap));
+  GB_CUDA(cudaMalloc(&S.brick_sort, sizeof(int) * n));
+  GB_CUDA(cudaMalloc(&S.ovf, sizeof(int2) * n));
   GB_CUDA(cudaMalloc(&S.brick_start, sizeof(int) * (S.nbricks + 2)));
   GB_CUDA(cudaMalloc(&S.brick_fill, sizeof(int) * (S.nbricks + 2)));
   GB_CUDA(cudaMalloc(&S.brick_atoms, sizeof(int) * n));
@@ -1007,15 +1093,15 @@ void grid_setup(SpmeGrid& S, const int* Kin, int p, bool fp64) {
   {
     const size_t tsize = (size_t)(S.B[0] + p - 1) * (S.B[1] + p - 1) * (S.B[2] + p - 1);
     GB_CUDA(cudaMalloc(&S.spread_ext, sizeof(double) * tsize * S.nbricks));
-    raise_smem(k_spme_spread_tile<double, 8>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(double)));
-    raise_smem(k_spme_spread_tile<double, 0>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(double)));
-    raise_smem(k_spme_spread_tile<dfr, 8>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(dfr)));
-    raise_smem(k_spme_spread_tile<dfr, 0>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(dfr)));
-    raise_smem(k_spme_spread_tile<float, 8, 256>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(float)));
-    raise_smem(k_spme_spread_tile<float, 6>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(float)));
-    raise_smem(k_spme_spread_tile<double, 6>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(double)));
-    raise_smem(k_spme_spread_tile<dfr, 6>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(dfr)));
-    raise_smem(k_spme_spread_tile<float, 0>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(float)));
+    raise_smem(k_spme_spread_tile<double, 8>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(double), S.cap));
+    raise_smem(k_spme_spread_tile<double, 0>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(double), S.cap));
+    raise_smem(k_spme_spread_tile<dfr, 8>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(dfr), S.cap));
+    raise_smem(k_spme_spread_tile<dfr, 0>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(dfr), S.cap));
+    raise_smem(k_spme_spread_tile<float, 8, 256>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(float), S.cap));
+    raise_smem(k_spme_spread_tile<float, 6>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(float), S.cap));
+    raise_smem(k_spme_spread_tile<double, 6>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(double), S.cap));
+    raise_smem(k_spme_spread_tile<dfr, 6>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(dfr), S.cap));
+    raise_smem(k_spme_spread_tile<float, 0>, (int)spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(float), S.cap));
     raise_smem(k_spme_spread_fix<8>, (int)(tsize * sizeof(long long)));
     raise_smem(k_spme_spread_fix<6>, (int)(tsize * sizeof(long long)));
     raise_smem(k_spme_spread_fix<0>, (int)(tsize * sizeof(long long)));
@@ -1173,29 +1259,31 @@ void grid_run(SpmeGrid& S, bool coarse, float* rec, double* eng_rc, double* vir_
                      : (F64 ? reinterpret_cast<const T2*>(S.tw[2]) : reinterpret_cast<const T2*>(S.twf[2]));
   const int K1 = S.K[0], K2 = S.K[1], K3 = S.K[2];
   // splines + brick binning
-  GB_CUDA(cudaMemsetAsync(S.brick_count, 0, sizeof(int) * (S.nbricks + 2), st));
-  GB_CUDA(cudaMemsetAsync(S.brick_fill, 0, sizeof(int) * (S.nbricks + 2), st));
+  GB_CUDA(cudaMemsetAsync(S.brick_count, 0, sizeof(int) * (S.nbricks + 4), st));
+  // the tile spread adds a brick's atoms in ascending index order (deterministic sums); the
+  // fixed-point spread of the mixed form (GB_SPREAD_FIX=1) does not depend on it
+  const bool tile_spread = F64 || !g_spread_fix;
+  SpreadBins bins;
+  bins.cap = S.cap;
+  bins.count = S.brick_count;
+  bins.bucket = tile_spread ? S.bucket : nullptr;
+  bins.ovf = S.ovf;
+  bins.ovf_count = S.brick_count + S.nbricks + 2;
+  bins.pool = S.brick_count + S.nbricks + 3;
+  bins.a = S.brick_atoms;
+  bins.b = S.brick_sort;
   prof_begin(pid(P_SPME_PREP));
   const bool warp_gather = (!F64 || DF) && (p == 8 || p == 6);
   auto prep = p == 8 ? k_spme_prep<T, 8> : (p == 6 ? k_spme_prep<T, 6> : k_spme_prep<T, 0>);
-  prep<<<nblocks(n, PREP_AT), 3 * PREP_AT, 0, st>>>(n, g.x, g.y, g.z, g.chge, S.sg, spl, S.nidx, S.brick_of, S.brick_count,
+  prep<<<nblocks(n, PREP_AT), 3 * PREP_AT, 0, st>>>(n, g.x, g.y, g.z, g.chge, S.sg, spl, S.nidx, S.brick_of, bins,
                                          warp_gather ? S.gidx : nullptr, warp_gather && !DF ? S.gw : nullptr,
                                          warp_gather && DF ? reinterpret_cast<float2*>(S.gw + 6 * (size_t)n) : nullptr,
                                          warp_gather && DF ? reinterpret_cast<T*>(S.gsp) : nullptr);
   GB_LAUNCHED();
 
-  scan_exclusive(S.brick_count, S.brick_start, S.nbricks + 1);
-  // the tile spread adds a brick's atoms in ascending index order (deterministic sums);
-  // the fixed-point spread of the mixed form (GB_SPREAD_FIX=1) does not depend on it
-  const bool tile_spread = F64 || !g_spread_fix;
-  if (tile_spread) {
-    int* tmp = gb_scan_scratch(n + 1);
-    k_brick_scatter<<<nblocks(n, 256), 256, 0, st>>>(n, S.brick_of, S.brick_start, S.brick_fill, tmp);
-    GB_LAUNCHED();
-    k_brick_sort<<<nblocks((long long)S.nbricks * 32, 256), 256, 0, st>>>(S.nbricks, S.brick_start, tmp,
-                                                                          S.brick_atoms);
-    GB_LAUNCHED();
-  } else {  // fixed-point sums do not depend on the order of a brick's atoms
+  if (!tile_spread) {
+    GB_CUDA(cudaMemsetAsync(S.brick_fill, 0, sizeof(int) * (S.nbricks + 2), st));
+    scan_exclusive(S.brick_count, S.brick_start, S.nbricks + 1);
     k_brick_scatter<<<nblocks(n, 256), 256, 0, st>>>(n, S.brick_of, S.brick_start, S.brick_fill, S.brick_atoms);
     GB_LAUNCHED();
   }
@@ -1203,8 +1291,7 @@ void grid_run(SpmeGrid& S, bool coarse, float* rec, double* eng_rc, double* vir_
   // spreading: tile scatter per brick, then the fixed-order halo reduction
   {
     T* ext = reinterpret_cast<T*>(S.spread_ext);
-    const size_t smem = spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(T));
-    const size_t NG = (size_t)K1 * K2 * K3;
+    const size_t smem = spread_smem(S.B[0], S.B[1], S.B[2], p, sizeof(T), S.cap);
     const int red_nt = std::min(256, (K1 + 31) / 32 * 32);  // halo reduction: x in the block, y and z in the grid
     const dim3 red_grid((unsigned)nblocks(K1, red_nt), (unsigned)K2, (unsigned)K3);
     prof_begin(pid(P_SPME_SPREAD));
@@ -1215,8 +1302,7 @@ void grid_run(SpmeGrid& S, bool coarse, float* rec, double* eng_rc, double* vir_
       constexpr bool EIGHT = std::is_same<T, float>::value;
       constexpr int NT8 = EIGHT ? 256 : SPREAD_NT;
       auto spread = p == 8 ? k_spme_spread_tile<T, 8, NT8> : (p == 6 ? k_spme_spread_tile<T, 6> : k_spme_spread_tile<T, 0>);
-      spread<<<S.nbricks, p == 8 ? NT8 : SPREAD_NT, smem, st>>>(S.sg, S.brick_start, S.brick_atoms, spl, S.nidx, g.chge,
-                                                              ext);
+      spread<<<S.nbricks, p == 8 ? NT8 : SPREAD_NT, smem, st>>>(S.sg, bins, spl, S.nidx, ext);
       GB_LAUNCHED();
       k_spme_tile_reduce<T><<<red_grid, red_nt, 0, st>>>(S.sg, ext, Q);
       GB_LAUNCHED();
