@@ -157,6 +157,37 @@ __device__ __forceinline__ df fix_diff(long long a, long long b, float sh, float
   return quick_two_sum(h, l);
 }
 
+// double to double-float by integer operations (an FP64 conversion would take the FP64
+// unit): the top 24 bits, then the other 29; 0 below 2^-60, infinite above 2^100
+__device__ __forceinline__ df dbl_split(double v) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+  const unsigned h = (unsigned)(b >> 32), l = (unsigned)b, s = h & 0x80000000u;
+  const int e = (int)((h >> 20) & 0x7FFu) - 1023;
+  if (e < -60) return df_make(0.f, 0.f);
+  if (e > 100) return df_make(__uint_as_float(s | 0x7F800000u), 0.f);
+  const float hi = __uint_as_float(s | ((unsigned)(e + 127) << 23) | ((h & 0xFFFFFu) << 3) | (l >> 29));
+  const float lo = __uint2float_rn(l & 0x1FFFFFFFu) * __uint_as_float((unsigned)(e - 52 + 127) << 23);
+  return quick_two_sum(hi, __uint_as_float(__float_as_uint(lo) ^ s));
+}
+
+// exact double of a float by integer operations (0 below the normal range)
+__device__ __forceinline__ double flt_dbl(float f) {
+  const unsigned u = __float_as_uint(f), a = u & 0x7FFFFFFFu;
+  const unsigned hi = (u & 0x80000000u) | ((a >> 3) + 0x38000000u);
+  return a < 0x00800000u ? 0.0 : __hiloint2double((int)hi, (int)(a << 29));
+}
+
+// fix_diff to the last of the 48 bits: the integer's low 28 bits in two exact parts (their
+// conversion in fix_diff rounds to 2^-45 of the range of |a - b|)
+__device__ __forceinline__ df fix_diff_full(long long a, long long b, float sh, float sl) {
+  const long long d = a - b;
+  const unsigned u = (unsigned)d;
+  const float h = __fmul_rn(__int2float_rn((int)(d >> 28)), sh);
+  const float m = __fmul_rn(__int2float_rn((int)((u >> 14) & 0x3FFFu)), __fmul_rn(sl, 16384.f));
+  const df s = quick_two_sum(h, m);
+  return quick_two_sum(s.hi, __fmaf_rn(__int2float_rn((int)(u & 0x3FFFu)), sl, s.lo));
+}
+
 // a += x * y where the running sum a.s carries a constant C added to it that exceeds the
 // sum and every product: |a.s| >= |x y|, so that t - a.s is exact and the second FMA gives
 // the rounding error of the first (Dekker's fast two-sum with the product unrounded).  Six

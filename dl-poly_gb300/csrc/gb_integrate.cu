@@ -581,19 +581,6 @@ struct ClKind {        // clusters with equal masses, lengths and topology share
   double wh[CL_MAXA];                   // weight / hstep, 0: frozen
 };
 
-// double to double-float by integer operations (an FP64 conversion would take the FP64
-// unit): the top 24 bits, then the other 29; 0 below 2^-60, infinite above 2^100
-__device__ __forceinline__ df dbl_split(double v) {
-  const unsigned long long b = (unsigned long long)__double_as_longlong(v);
-  const unsigned h = (unsigned)(b >> 32), l = (unsigned)b, s = h & 0x80000000u;
-  const int e = (int)((h >> 20) & 0x7FFu) - 1023;
-  if (e < -60) return df_make(0.f, 0.f);
-  if (e > 100) return df_make(__uint_as_float(s | 0x7F800000u), 0.f);
-  const float hi = __uint_as_float(s | ((unsigned)(e + 127) << 23) | ((h & 0xFFFFFu) << 3) | (l >> 29));
-  const float lo = __uint2float_rn(l & 0x1FFFFFFFu) * __uint_as_float((unsigned)(e - 52 + 127) << 23);
-  return quick_two_sum(hi, __uint_as_float(__float_as_uint(lo) ^ s));
-}
-
 __device__ __forceinline__ df df_of(float2 a) { return df_make(a.x, a.y); }
 
 __device__ __forceinline__ df df_dot(const df (&a)[3], const df (&b)[3]) {

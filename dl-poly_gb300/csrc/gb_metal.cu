@@ -360,21 +360,22 @@ __global__ void __launch_bounds__(256, 3) k_metal_forces(int natms, const DevSca
 // (1/64 of the FP32 rate): 95 FP64 instructions per 32 list entries, executed for whole
 // warps although a fifth of the entries lie beyond the cutoff.  Here an FP32 test of the
 // high parts queues the entries that may be inside, and 32 queued pairs at a time are
-// evaluated with every lane busy.  256,000 atoms: density 1.97 -> 0.42 ms, forces 4.35 ->
-// 0.83 ms (1.04 with 102 registers, two CTAs per SM; a fourth CTA spills and gains
+// evaluated with every lane busy.  256,000 atoms: density 1.97 -> 0.45 ms, forces 4.35 ->
+// 0.89 ms (1.04 with 102 registers, two CTAs per SM; a fourth CTA spills and gains
 // nothing); latency of the partners and tables, at a third of the issue slots.
 //   positions   fixed point (PosRec): the separation is an exact integer difference
-//   r           relative error about 1e-14 (an FP32 square root and the first-order
-//               remainder; the FP64 kernels' one Newton step from an FP32 seed: 8e-14)
-//   tables      l by the nearest integer of the double-float coordinate, so that a pair
-//               takes the interval that the FP64 kernels take
+//   r           to the last of 48 bits, and its fraction of a table interval from the r of
+//               the table's point; an atom's force is summed in FP64 (errors of forces
+//               against 64 bits 1.2e-13, the FP64 kernels 0.8e-13: both from r, on which
+//               the difference of a pair's terms depends forty times over; energies and
+//               stress are nearer than the FP64 kernels')
 // A pair near a cutoff, at an end of its table, with a negative density or outside the
 // FP32 range takes the FP64 formulas of the kernels above (metal_density_slow,
 // metal_force_slow).  Densities and forces are summed in FP64 per sorted position and
 // folded onto the atoms (a halo image's onto its source) afterwards.
 struct __align__(16) CoefF {
   float c0h, c0l, c1h, c1l;
-  float c2h, c2l, pad0, pad1;
+  float c2h, c2l, rh, rl;  // r of the point (in the tables of the values)
 };
 
 struct MetSorted {
@@ -396,14 +397,20 @@ struct MetSorted {
 
 constexpr int MET_NT = 256, MET_U = 4;
 
-// exact double of a finite float by integer operations (0 below the normal range)
-__device__ __forceinline__ double flt_dbl(float f) {
-  const unsigned u = __float_as_uint(f), a = u & 0x7FFFFFFFu;
-  const unsigned hi = (u & 0x80000000u) | ((a >> 3) + 0x38000000u);
-  return a < 0x00800000u ? 0.0 : __hiloint2double((int)hi, (int)(a << 29));
+// df_norm2 with the squares of the low parts
+__device__ __forceinline__ df met_norm2(df x, df y, df z) {
+  const df px = two_prod(x.hi, x.hi), py = two_prod(y.hi, y.hi), pz = two_prod(z.hi, z.hi);
+  const float cx = __fmaf_rn(__fadd_rn(x.hi, x.hi), x.lo, __fmaf_rn(x.lo, x.lo, px.lo));
+  const float cy = __fmaf_rn(__fadd_rn(y.hi, y.hi), y.lo, __fmaf_rn(y.lo, y.lo, py.lo));
+  const float cz = __fmaf_rn(__fadd_rn(z.hi, z.hi), z.lo, __fmaf_rn(z.lo, z.lo, pz.lo));
+  const df s1 = two_sum(px.hi, py.hi);
+  const df s2 = two_sum(s1.hi, pz.hi);
+  return quick_two_sum(s2.hi, __fadd_rn(__fadd_rn(__fadd_rn(cx, cy), __fadd_rn(cz, s1.lo)), s2.lo));
 }
 
-// r and 1/r^2 of a double-float r^2 in the normal range
+// r and 1/r^2 (3e-14) of a double-float r^2 in the normal range.  The force of a metal pair is a
+// difference of terms that changes forty times as fast as r, so r gets the last bits: an
+// FP32 root s and the remainder (r^2 - s^2) / 2s with 1/s refined from the root's seed.
 __device__ __forceinline__ df met_dist(df r2, df* inv) {
   const float rs = rsqrtf(r2.hi);
   const float s = __fmul_rn(r2.hi, rs);
@@ -414,25 +421,31 @@ __device__ __forceinline__ df met_dist(df r2, df* inv) {
     const float g = __fmaf_rn(-r2.lo, q, __fmaf_rn(-r2.hi, q, 1.f));  // 1 - r2 q, about 2^-21
     *inv = quick_two_sum(q, __fmul_rn(q, __fmaf_rn(g, g, g)));
   }
-  return quick_two_sum(s, __fmul_rn(__fmul_rn(0.5f, rs), e));
+  const float y = __fmaf_rn(rs, __fmaf_rn(-s, rs, 1.f), rs);
+  return quick_two_sum(s, __fmul_rn(__fmul_rn(0.5f, y), e));
 }
 
-// table point l and fraction p in [-0.5, 0.5] of a double-float r; false at a table's ends
-__device__ __forceinline__ bool met_coord(const MetTab& t, df r, int* l, df* p) {
+// table point l and fraction p in [-0.5, 0.5] of a double-float r; false at a table's ends.
+// p = (r - r_l) / dr from the point's own r: the product r / dr would be rounded at 2^-48 of
+// a coordinate of some thousand.
+__device__ __forceinline__ bool met_coord(const MetTab& t, const CoefF* __restrict__ c, df r, int* l, df* p) {
   float k = rintf(__fmaf_rn(r.hi, t.rdr_h, t.nr_h));
-  const df pr = two_prod(r.hi, t.rdr_h);
-  const float e = __fmaf_rn(r.hi, t.rdr_l, __fmaf_rn(r.lo, t.rdr_h, pr.lo));
-  const df c = two_sum(t.nr_h, -k);
-  const df s = two_sum(pr.hi, c.hi);
-  df d = quick_two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(e, __fadd_rn(c.lo, t.nr_l))));
-  if (fabsf(d.hi) > 0.5f) {  // the FP32 nearest integer was the other neighbour
-    const float o = copysignf(1.f, d.hi);
-    k += o;
-    d = quick_two_sum(__fsub_rn(d.hi, o), d.lo);
+  if (!(k > 5.f && k < (float)(t.n - 1))) return false;
+  int i = (int)k;
+  df d;
+  for (;;) {
+    const float2 rk = *reinterpret_cast<const float2*>(&c[i].rh);
+    const df s = two_sum(r.hi, -rk.x);
+    const df q = quick_two_sum(s.hi, __fadd_rn(s.lo, __fsub_rn(r.lo, rk.y)));
+    d = df_mul(q, df_make(t.rdr_h, t.rdr_l));
+    // (the FP32 nearest integer may have been the other neighbour of a midpoint)
+    if (d.hi > 0.5f && i + 1 == (int)k + 1) ++i;
+    else if (d.hi < -0.5f && i - 1 == (int)k - 1) --i;
+    else break;
   }
-  *l = (int)k;
+  *l = i;
   *p = d;
-  return k > 5.f && k < (float)(t.n - 1);
+  return i > 5 && i < t.n - 1;
 }
 
 __device__ __forceinline__ df met_poly(const CoefF* __restrict__ c, int l, df p) {
@@ -570,9 +583,9 @@ __global__ void __launch_bounds__(MET_NT) k_metal_density_sorted(MetSorted S, Me
       const PosRec rj = S.rec[j];
       const bool same = rj.type == ai;
       const MetTab& tj = tabs[A.nkey + rj.type - 1];
-      const df dx = fix_diff(ri.x, rj.x, S.sh, S.sl), dy = fix_diff(ri.y, rj.y, S.sh, S.sl),
-               dz = fix_diff(ri.z, rj.z, S.sh, S.sl);
-      const df r2 = df_norm2(dx, dy, dz);
+      const df dx = fix_diff_full(ri.x, rj.x, S.sh, S.sl), dy = fix_diff_full(ri.y, rj.y, S.sh, S.sl),
+               dz = fix_diff_full(ri.z, rj.z, S.sh, S.sl);
+      const df r2 = met_norm2(dx, dy, dz);
       const int in_j = met_in(tj, r2.hi), in_i = same ? in_j : met_in(ti, r2.hi);
       if (in_j == 0 && in_i == 0) return;
       bool slow = in_j < 0 || in_i < 0 || !met_plain(r2.hi);
@@ -582,7 +595,7 @@ __global__ void __launch_bounds__(MET_NT) k_metal_density_sorted(MetSorted S, Me
         int l = 0;
         df f;
         if (in_j) {
-          slow = !met_coord(tj, r, &l, &f);
+          slow = !met_coord(tj, S.fv + tj.off, r, &l, &f);
           if (!slow) {
             to_i = met_poly(S.fv + tj.off, l, f);
             slow = to_i.hi < 0.f;
@@ -590,7 +603,7 @@ __global__ void __launch_bounds__(MET_NT) k_metal_density_sorted(MetSorted S, Me
           if (same) to_j = to_i;
         }
         if (!same && in_i && !slow) {
-          if (!(in_j && ti.grid == tj.grid)) slow = !met_coord(ti, r, &l, &f);
+          if (!(in_j && ti.grid == tj.grid)) slow = !met_coord(ti, S.fv + ti.off, r, &l, &f);
           if (!slow) {
             to_j = met_poly(S.fv + ti.off, l, f);
             slow = to_j.hi < 0.f;
@@ -655,16 +668,16 @@ __global__ void __launch_bounds__(MET_NT, 3) k_metal_forces_sorted(MetSorted S, 
     const float2 f2 = S.fp[p];
     const df fpi = df_make(f2.x, f2.y);
     const MetTab& ti = tabs[A.nkey + ai - 1];
-    dacc fx = {0.f, 0.f}, fy = fx, fz = fx;
+    double fx = 0.0, fy = 0.0, fz = 0.0;
     n_list += (unsigned long long)S.list[(size_t)i * S.ld + 3];
     met_walk(S, i, S.xhs[p], queue[wq], [&](int j) {
       const PosRec rj = S.rec[j];
       const int aj = rj.type;
       const MetTab& tp = tabs[(ai > aj ? ai * (ai - 1) / 2 + aj : aj * (aj - 1) / 2 + ai) - 1];
       if (!tp.listed) return;  // keypot = -1
-      const df dx = fix_diff(ri.x, rj.x, S.sh, S.sl), dy = fix_diff(ri.y, rj.y, S.sh, S.sl),
-               dz = fix_diff(ri.z, rj.z, S.sh, S.sl);
-      const df r2 = df_norm2(dx, dy, dz);
+      const df dx = fix_diff_full(ri.x, rj.x, S.sh, S.sl), dy = fix_diff_full(ri.y, rj.y, S.sh, S.sl),
+               dz = fix_diff_full(ri.z, rj.z, S.sh, S.sl);
+      const df r2 = met_norm2(dx, dy, dz);
       if (r2.hi > S.f_rc_hi) return;
       const bool same = aj == ai;
       const MetTab& tj = tabs[A.nkey + aj - 1];
@@ -678,7 +691,7 @@ __global__ void __launch_bounds__(MET_NT, 3) k_metal_forces_sorted(MetSorted S, 
         const df r = met_dist(r2, &inv);
         int l = 0, gl = -1;
         if (in_p) {
-          slow = !met_coord(tp, r, &l, &f);
+          slow = !met_coord(tp, S.fv + tp.off, r, &l, &f);
           gl = tp.grid;
           if (!slow) {
             num = met_poly(S.fd + tp.off, l, f);
@@ -687,7 +700,7 @@ __global__ void __launch_bounds__(MET_NT, 3) k_metal_forces_sorted(MetSorted S, 
         }
         df g = df_make(0.f, 0.f);
         if (in_j && !slow) {
-          if (tj.grid != gl) slow = !met_coord(tj, r, &l, &f);
+          if (tj.grid != gl) slow = !met_coord(tj, S.fv + tj.off, r, &l, &f);
           gl = tj.grid;
           if (!slow) {
             g = met_poly(S.fd + tj.off, l, f);
@@ -696,7 +709,7 @@ __global__ void __launch_bounds__(MET_NT, 3) k_metal_forces_sorted(MetSorted S, 
           }
         }
         if (!same && in_i && !slow) {
-          if (ti.grid != gl) slow = !met_coord(ti, r, &l, &f);
+          if (ti.grid != gl) slow = !met_coord(ti, S.fv + ti.off, r, &l, &f);
           if (!slow) {
             g = met_poly(S.fd + ti.off, l, f);
             num = df_fma(g, df_make(fq.x, fq.y), num);
@@ -724,29 +737,29 @@ __global__ void __launch_bounds__(MET_NT, 3) k_metal_forces_sorted(MetSorted S, 
       ++n_rc;
       dacc_add(e_eng, eng);
       dacc_add(e_vir, df_neg(num));
-      // the products as an exact high part and the sum of the rest
-      auto term = [&](df d, dacc& s, double* slot) {
+      // the products as an exact high part and the sum of the rest; summed in FP64 (the forces
+      // of an atom's neighbours cancel to a small part of each)
+      auto term = [&](df d, double& s, double* slot) {
         const df t = two_prod(gam.hi, d.hi);
-        const float c = __fmaf_rn(gam.hi, d.lo, __fmaf_rn(gam.lo, d.hi, t.lo));
-        const df u = two_sum(s.s, t.hi);
-        s.s = u.hi;
-        s.c = __fadd_rn(s.c, __fadd_rn(u.lo, c));
-        atomicAdd(&slot[j], -(flt_dbl(t.hi) + flt_dbl(c)));
+        const double v = flt_dbl(t.hi) + flt_dbl(__fmaf_rn(gam.hi, d.lo, __fmaf_rn(gam.lo, d.hi, t.lo)));
+        s += v;
+        atomicAdd(&slot[j], -v);
       };
       term(dx, fx, S.s0);
       term(dy, fy, S.s1);
       term(dz, fz, S.s2);
     });
+    {
+      // reduce-scatter of three values over the warp: x in lane 0, y in 8, z in 16
+      const bool up16 = lane & 16, up8 = lane & 8;
+      double k0 = up16 ? fz : fx, k1 = up16 ? 0.0 : fy;
+      k0 += __shfl_xor_sync(0xffffffffu, up16 ? fx : fz, 16);
+      k1 += __shfl_xor_sync(0xffffffffu, up16 ? fy : 0.0, 16);
+      double r = up8 ? k1 : k0;
+      r += __shfl_xor_sync(0xffffffffu, up8 ? k0 : k1, 8);
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      fx = dacc_xor(fx, o);
-      fy = dacc_xor(fy, o);
-      fz = dacc_xor(fz, o);
-    }
-    if (lane == 0) {
-      atomicAdd(&S.s0[p], dacc_value(fx));
-      atomicAdd(&S.s1[p], dacc_value(fy));
-      atomicAdd(&S.s2[p], dacc_value(fz));
+      for (int o = 4; o > 0; o >>= 1) r += __shfl_xor_sync(0xffffffffu, r, o);
+      if ((lane & 7) == 0 && lane < 24) atomicAdd(&(lane == 0 ? S.s0 : lane == 8 ? S.s1 : S.s2)[p], r);
     }
   }
   if (bad) atomicOr(S.status, ST_METAL_TABLE);
@@ -960,11 +973,16 @@ int metal_setup(int ntab, const int32_t* kind, const int32_t* t1, const int32_t*
       df_split(c[k].c0, &o.c0h, &o.c0l);
       df_split(c[k].c1, &o.c1h, &o.c1l);
       df_split(c[k].c2, &o.c2h, &o.c2l);
-      o.pad0 = o.pad1 = 0.f;
+      o.rh = o.rl = 0.f;
     }
     return f;
   };
-  const std::vector<CoefF> fv = split_coef(cv), fd = split_coef(cd);
+  std::vector<CoefF> fv = split_coef(cv), fd = split_coef(cd);
+  for (int id = 0; id < n_key + nt; ++id)
+    for (int l = 5; l <= tab[id].n - 1; ++l) {
+      CoefF& o = fv[tab[id].off + l];
+      df_split(tab[id].r0 + (double)l / tab[id].rdr, &o.rh, &o.rl);
+    }
   const size_t mx = std::max(g.mxatms, 1);
   GB_CUDA(cudaMalloc(&d_fv, sizeof(CoefF) * fv.size()));
   GB_CUDA(cudaMalloc(&d_fd, sizeof(CoefF) * fd.size()));
