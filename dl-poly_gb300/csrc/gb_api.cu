@@ -1041,15 +1041,52 @@ int gb_metal_rho(double* out) {
   });
 }
 
-// The NVE loop without constraints, thermostat, metals or learned MTS: the host
-// waits only for the Verlet-list decision of each step (vnl_check); each step's
-// energy, virial and stress sums are copied to a pinned ring with the step's other
-// work and turned into gb_step_stats after the last step.  With 3 or more steps the
-// steps run as two CUDA graphs each: stage 1 with the displacement check (its sums
-// copied to the pinned scalars), then, after the host's decision, either the rebuild
-// step launched kernel by kernel or the graph of a step without rebuild (halo refresh,
-// forces with SPME forked to the side stream, stage 2), captured again after every
-// rebuild.  The per-region timings of gb_last_timings are not taken on this path (the
+// the DL_POLY or library code of the status bits that a step's kernels set (0: none)
+static int md_status(int status) {
+  if (status & ST_SHAKE_FAIL) return GB_ERR_SHAKE;
+  if (status & ST_METAL_DENSITY) return GB_ERR_METAL_DENSITY;
+  if (status & ST_METAL_TABLE) return GB_ERR_METAL_TABLE;
+  if (status & ST_RATTLE_FAIL) return GB_ERR_RATTLE;
+  if (status & ST_RNG) return GB_ERR_RNG;
+  return GB_OK;
+}
+
+static void md_step_stats(const DevScalars* h, int32_t rebuilt, gb_step_stats& S) {
+  std::memset(&S, 0, sizeof(S));
+  double st[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, e6[6] = {0, 0, 0, 0, 0, 0}, m4[4] = {0, 0, 0, 0};
+  if (g.has_coul) spme_scalars(h, &S.engcpe_rc, &S.vircpe_rc, st);
+  if (g.has_coul || g.has_vdw) pair_scalars(h, e6, st);
+  if (g.has_metal) metal_scalars(h, m4, st);
+  S.engcpe_rl = e6[0]; S.vircpe_rl = e6[1]; S.engcpe_ex = e6[2]; S.vircpe_ex = e6[3];
+  S.engvdw = e6[4]; S.virvdw = e6[5];
+  S.engmet = m4[0] + m4[2];
+  S.virmet = m4[1] + m4[3];
+  for (int k = 0; k < 9; ++k) S.stress[k] = st[k];
+  kin_scalars(h, S.strkin, &S.engke);
+  if (g.ens == GB_NVT_NOSE_HOOVER) {
+    S.engke = h->th[6];
+    S.consv = h->th[7];
+  }
+  if (g.ntcons > 0) {
+    con_scalars(h, &S.vircon, S.strcon);
+    S.shake_iters = h->shake_iters;
+    S.rattle_iters = h->rattle_iters;
+  }
+  S.list_rebuilt = rebuilt;
+  S.mts_full = 1;
+}
+
+// The loop without learned MTS: the host waits only for the Verlet-list decision of each
+// step (vnl_check), where it also sees the status bits set since the last one (a RATTLE
+// or metal table failure of a step thus ends the call at the next step's decision, after
+// that step's stage 1, with the same code); each step's energy, virial and stress sums are
+// copied to a pinned ring with the step's other work and turned into gb_step_stats after
+// the last step.  With 3 or more steps the steps run as two CUDA graphs: stage 1 with the
+// displacement check (its sums copied to the pinned scalars), then, after the host's
+// decision and the halo refresh or the list rebuild that it calls for, the forces (SPME
+// forked to the side stream) and stage 2; the second is captured again when a rebuild
+// changes the kernels that walk the list.  Langevin's stage 1 is launched (its noise is keyed
+// on the step).  The per-region timings of gb_last_timings are not taken on this path (the
 // total is).
 static int md_run_deferred(int nsteps, gb_step_stats* stats) {
   if (g.ring_cap < nsteps) {
@@ -1061,75 +1098,86 @@ static int md_run_deferred(int nsteps, gb_step_stats* stats) {
   }
   std::vector<int32_t> rebuilt(nsteps, 0);
   GB_CUDA(cudaEventRecord(g.ev[5], g.stream));
+  gb_blkacc(9 * nblocks(g.natms, 256) + 4096);  // (no allocation inside a capture)
+  GB_CUDA(cudaMemsetAsync(&g.sc->status, 0, sizeof(int), g.stream));
   g.defer_scalars = true;
+  const bool plain = g.ntcons == 0 && g.ens == GB_NVE;
   auto stage1 = [&]() {
-    integ_stage1_check();
+    if (plain) {
+      integ_stage1_check();
+    } else {
+      int it = 0;
+      integ_vv(1, nullptr, nullptr, &it, nullptr, nullptr);
+      integ_vnl_launch();
+    }
     GB_CUDA(cudaMemcpyAsync(g.hsc, g.sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, g.stream));
   };
   auto step_rest = [&]() {
-    list_refresh_halo();
     compute_forces(nullptr, nullptr, true, true, true, nullptr);
     int it = 0;
     integ_vv(2, nullptr, nullptr, &it, nullptr, nullptr);
   };
   bool graphs = g.use_graphs && !g.prof_on && nsteps >= 3;
-  if (graphs) graphs = capture_graph(&g.gx_vv1, &g.gl_vv1, stage1);
-  bool step_ok = false;  // gx_step holds a step of the current list
-  for (int s = 0; s < nsteps; ++s) {
+  const bool graph1 = graphs && g.ens != GB_NVT_LANGEVIN && capture_graph(&g.gx_vv1, &g.gl_vv1, stage1);
+  if (graphs && g.ens != GB_NVT_LANGEVIN && !graph1) graphs = false;
+  bool step_ok = false, step_spos = false;  // gx_step holds the step's rest for this kind of list
+  int code = GB_OK, done = 0;
+  for (int s = 0; s < nsteps && code == GB_OK; ++s) {
     ++g.nstep;
-    if (graphs) launch_graph(g.gx_vv1, g.gl_vv1);
+    if (graph1) launch_graph(g.gx_vv1, g.gl_vv1);
     else stage1();
     GB_CUDA(cudaStreamSynchronize(g.stream));
     if (g.prof_on) gb_sync_scalars();  // resolves the pending profile events
+    code = md_status(g.hsc->status);
+    if (code != GB_OK) {
+      done = (g.hsc->status & ST_SHAKE_FAIL) ? s : std::max(0, s - 1);
+      break;
+    }
+    done = s;
     const int32_t upd = integ_vnl_result();
     rebuilt[s] = upd;
     if (upd) {
-      int st = list_relocate_and_halo(false);
-      if (!st) st = list_build();
-      if (st) { g.defer_scalars = false; return st; }
-      compute_forces(nullptr, nullptr, true, true, true, nullptr);
-      int it = 0;
-      integ_vv(2, nullptr, nullptr, &it, nullptr, nullptr);
-      step_ok = false;
+      code = list_relocate_and_halo(false);
+      if (!code) code = list_build();
+      if (code) break;
     } else {
-      if (graphs && !step_ok) step_ok = capture_graph(&g.gx_step, &g.gl_step, step_rest);
-      if (graphs && step_ok) launch_graph(g.gx_step, g.gl_step);
-      else step_rest();
+      list_refresh_halo();
     }
+    if (graphs && !(step_ok && step_spos == g.spos_valid)) {
+      step_ok = capture_graph(&g.gx_step, &g.gl_step, step_rest);
+      step_spos = g.spos_valid;
+    }
+    if (graphs && step_ok) launch_graph(g.gx_step, g.gl_step);
+    else step_rest();
     GB_CUDA(cudaMemcpyAsync(&g.ring[s], g.sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, g.stream));
+    done = s + 1;
   }
   g.defer_scalars = false;
   GB_CUDA(cudaEventRecord(g.ev[6], g.stream));
   GB_CUDA(cudaEventSynchronize(g.ev[6]));
+  if (code == GB_OK && nsteps > 0) {
+    code = md_status(g.ring[nsteps - 1].status);
+    if (code != GB_OK) done = nsteps - 1;
+  }
   float span = 0.f;
   cudaEventElapsedTime(&span, g.ev[5], g.ev[6]);
   for (int k = 0; k < 5; ++k) g.last_ms[k] = 0.0;
   g.last_ms[4] = span;
   g.last_ms[5] = span;
-  if (stats) {
-    for (int s = 0; s < nsteps; ++s) {
-      gb_step_stats S;
-      std::memset(&S, 0, sizeof(S));
-      const DevScalars* h = &g.ring[s];
-      double strec[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0}, e6[6] = {0, 0, 0, 0, 0, 0};
-      if (g.has_coul) spme_scalars(h, &S.engcpe_rc, &S.vircpe_rc, strec);
-      if (g.has_coul || g.has_vdw) pair_scalars(h, e6, strec);
-      S.engcpe_rl = e6[0]; S.vircpe_rl = e6[1]; S.engcpe_ex = e6[2]; S.vircpe_ex = e6[3];
-      S.engvdw = e6[4]; S.virvdw = e6[5];
-      for (int k = 0; k < 9; ++k) S.stress[k] = strec[k];
-      kin_scalars(h, S.strkin, &S.engke);
-      S.list_rebuilt = rebuilt[s];
-      S.mts_full = 1;
-      stats[s] = S;
-    }
+  if (stats)
+    for (int s = 0; s < done; ++s) md_step_stats(&g.ring[s], rebuilt[s], stats[s]);
+  for (int k = 0; k < 4; ++k) g.metal_e4[k] = 0.0;
+  if (g.has_metal && done > 0) {
+    double st[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+    metal_scalars(&g.ring[done - 1], g.metal_e4, st);
   }
-  return (int)GB_OK;
+  return code;
 }
 
 int gb_md_run(int nsteps, gb_step_stats* stats) {
   return guarded([&]() {
     if (nsteps < 0) return (int)GB_ERR_ARG;
-    if (nsteps > 0 && g.use_deferred && g.ntcons == 0 && g.ens == GB_NVE && !g.has_metal && !mts_active()) {
+    if (nsteps > 0 && g.use_deferred && !mts_active()) {
       try {
         return md_run_deferred(nsteps, stats);
       } catch (int e) {

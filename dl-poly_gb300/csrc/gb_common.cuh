@@ -175,15 +175,14 @@ struct Dev {
   int n_tile_over = 0, tile_max_staged = 0;   // from the last list build
   bool spos_valid = false;     // the last list pairs every halo entry with its backward copy
   bool use_sorted = true;      // sorted-position pair kernels (GB_PAIR_SORTED=0: the atom-index kernels)
-  // NVE MD loop without constraints, thermostat, metals or learned MTS: the energy,
-  // virial and stress sums of each step are copied to a pinned ring and read after the
-  // last step, so the host waits only for the Verlet-list decision of each step
+  // MD loop without learned MTS: the energy, virial and stress sums of each step are copied
+  // to a pinned ring and read after the last step, so the host waits only for the
+  // Verlet-list decision of each step
   bool defer_scalars = false;
   bool use_deferred = true;    // GB_MD_DEFER=0 keeps the per-step read-back
   // that loop as CUDA graphs (GB_GRAPHS=0: every kernel launched by the host): stage 1 with
-  // the Verlet-list check, and a step without a list rebuild (halo refresh, forces, stage
-  // 2), captured once per call and again after each rebuild; the launch counter adds each
-  // graph's kernels per launch
+  // the Verlet-list check, and the forces with stage 2, captured once per call; the launch
+  // counter adds each graph's kernels per launch
   bool use_graphs = true;
   cudaGraphExec_t gx_vv1 = nullptr, gx_step = nullptr;
   int64_t gl_vv1 = 0, gl_step = 0;
@@ -500,12 +499,14 @@ void integ_vv(int stage, double* strkin, double* engke, int* iters, double* virc
 void spme_scalars(const DevScalars* h, double* eng_rc, double* vir_rc, double* stress9);
 void pair_scalars(const DevScalars* h, double* eng6, double* stress9);
 void kin_scalars(const DevScalars* h, double* strkin, double* engke);
+void con_scalars(const DevScalars* h, double* vircon, double* strcon);
+void metal_scalars(const DevScalars* h, double* e4, double* stress9);  // stress9 accumulates
 void integ_con_tags();            // constraints_tags: old bond vectors from the current positions
 void integ_shake(int* iters, double* vircon, double* strcon);  // apply_shake (throws GB_ERR_SHAKE)
 void integ_rattle_launch();       // apply_rattle, kit = 1 (status bit ST_RATTLE_FAIL)
 int integ_vnl_check();
 void integ_vnl_launch();          // the displacement check
-void integ_stage1_check();        // NVE stage 1 and the displacement check in one kernel, status cleared
+void integ_stage1_check();        // NVE stage 1 and the displacement check in one kernel
 int integ_vnl_result();           // its decision from the copied scalars (after a wait)
 void integ_zero_forces();
 void integ_forces_to_fp64();      // mixed: fixed point -> FP64 forces

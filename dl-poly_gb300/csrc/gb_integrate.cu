@@ -19,7 +19,6 @@
 #include <algorithm>
 #include <cfloat>
 #include <cmath>
-#include <cstddef>
 #include <cstdlib>
 #include <cstring>
 
@@ -1072,7 +1071,7 @@ void integ_forces_to_fp64() {
 }
 
 // The displacement check, with the NVE stage 1 in the same pass when stage1 is set.  The
-// caller has cleared maxdisp (integ_clear).
+// caller has cleared maxdisp.
 static void launch_maxdisp(bool stage1) {
   k_maxdisp<<<std::min(nblocks(g.natms, 128), 4 * g.nsm), 128, 0, g.stream>>>(
       g.natms, stage1 ? g.hdw : nullptr, g.p.tstep, g.fx, g.fy, g.fz, g.vx, g.vy, g.vz, g.x, g.y, g.z, g.xbg, g.ybg,
@@ -1080,11 +1079,9 @@ static void launch_maxdisp(bool stage1) {
   GB_LAUNCHED();
 }
 
-// NVE without constraints: stage 1 and the displacement check as one kernel, behind one
-// clearing of the status and the maximum
+// NVE without constraints: stage 1 and the displacement check as one kernel
 void integ_stage1_check() {
-  GB_CUDA(cudaMemsetAsync(&g.sc->status, 0, offsetof(DevScalars, maxdisp) + sizeof(double) - offsetof(DevScalars, status),
-                          g.stream));
+  GB_CUDA(cudaMemsetAsync(&g.sc->maxdisp, 0, sizeof(double), g.stream));
   prof_begin(P_VV);
   launch_maxdisp(true);
   prof_end(P_VV);
@@ -1174,12 +1171,10 @@ void integ_shake(int* iters, double* vircon, double* strcon) {
                                                    g.ox, g.oy, g.oz, g.vx, g.vy, g.vz, g.fx, g.fy, g.fz);
     GB_LAUNCHED();
   }
+  if (g.defer_scalars) return;  // the MD loop reads the sums and the status
   gb_sync_scalars();
   if (iters) *iters = g.hsc->shake_iters;
-  const double* s = &g.hsc->acc[A_STRCON];
-  double str[9] = {s[0], s[1], s[2], s[1], s[3], s[4], s[2], s[4], s[5]};
-  if (strcon) for (int k = 0; k < 9; ++k) strcon[k] = str[k];
-  if (vircon) *vircon = -(str[0] + str[4] + str[8]);
+  con_scalars(g.hsc, vircon, strcon);
   if (g.hsc->status & ST_SHAKE_FAIL) throw (int)GB_ERR_SHAKE;
 }
 
@@ -1247,11 +1242,20 @@ void integ_vv(int stage, double* strkin, double* engke, int* iters, double* virc
       gb_sync_scalars();
       kin_scalars(g.hsc, strkin, engke);
     }
+    if (g.defer_scalars) return;
     if (iters && g.ntcons > 0) *iters = g.hsc->rattle_iters;
     if (g.ntcons > 0 && (g.hsc->status & ST_RATTLE_FAIL)) throw (int)GB_ERR_RATTLE;
     if (g.hsc->status & ST_RNG) throw (int)GB_ERR_RNG;
     if (g.hsc->status & ST_DEVICE_WAIT) throw (int)GB_ERR_DEVICE_WAIT;
   }
+}
+
+// virial and stress (symmetric 3x3) of the SHAKE stage from the device sums
+void con_scalars(const DevScalars* h, double* vircon, double* strcon) {
+  const double* s = &h->acc[A_STRCON];
+  const double str[9] = {s[0], s[1], s[2], s[1], s[3], s[4], s[2], s[4], s[5]};
+  if (strcon) for (int k = 0; k < 9; ++k) strcon[k] = str[k];
+  if (vircon) *vircon = -(str[0] + str[4] + str[8]);
 }
 
 // kinetic stress (symmetric 3x3) and kinetic energy from the device sums

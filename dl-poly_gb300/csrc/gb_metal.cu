@@ -1122,10 +1122,16 @@ void metal_forces(double* e4, double* stress9) {
   }
   if (use_sorted_metal()) metal_forces_sorted(A, cnt);
   else metal_forces_fp64(A, cnt);
+  if (g.defer_scalars) return;  // the MD loop reads the sums and the status
   gb_sync_scalars();
   if (g.hsc->status & ST_METAL_DENSITY) throw (int)GB_ERR_METAL_DENSITY;
   if (g.hsc->status & ST_METAL_TABLE) throw (int)GB_ERR_METAL_TABLE;
-  const double* a = &g.hsc->acc[A_METAL];
+  metal_scalars(g.hsc, e4, stress9);
+}
+
+// engmet, virmet, engden, virden and the stress from the device sums
+void metal_scalars(const DevScalars* h, double* e4, double* stress9) {
+  const double* a = &h->acc[A_METAL];
   e4[0] = a[0];
   e4[1] = a[1];
   e4[2] = a[8];

@@ -375,6 +375,7 @@ bool thermo_vv2_finish(double* strkin, double* engke) {
     k_berendsen_final<<<1, 1, 0, g.stream>>>(g.sc, g.p.tstep, g.tau_t, g.sigma);
     GB_LAUNCHED();
   }
+  if (g.defer_scalars) return true;  // the MD loop reads the sums
   gb_sync_scalars();
   const double* s = &g.hsc->acc[A_STRKIN];
   double sk[9] = {s[0], s[1], s[2], s[1], s[3], s[4], s[2], s[4], s[5]};

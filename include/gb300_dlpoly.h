@@ -210,9 +210,10 @@ int gb_rattle(int32_t* iters);
 
 /* Resident MD loop (md_vv, drivers.F90:2059-2288): nsteps of VV1+SHAKE,
  * refresh, forces, VV2+RATTLE with no host round trip; stats[nsteps] may be NULL.
- * Each step first advances the step counter (gb_set_step).  In NVE without
- * constraints, thermostat, metals or learned MTS, a call of 3 or more steps replays
- * each step as CUDA graphs captured inside the call (same kernels and results). */
+ * Each step first advances the step counter (gb_set_step).  Without learned MTS a call
+ * of 3 or more steps replays each step as CUDA graphs captured inside the call (same
+ * kernels and results), and a step's failure that its forces or stage 2 set ends the call
+ * at the next step's list decision, with that step's code. */
 int gb_md_run(int nsteps, gb_step_stats* stats);
 
 /* Ensemble of the VV stages: the dispatch on thermo%ensemble (drivers.F90:1132-1175)
@@ -305,7 +306,9 @@ int gb_set_precision(int precision);
 
 /* Device time (ms) of the last gb_md_run per region, CUDA events on the
  * library stream: [0] list+halo, [1] real-space, [2] SPME, [3] integrate,
- * [4] total.  n = number of slots to copy. */
+ * [4] total.  Without learned MTS the total alone is taken ([0] to [3] are 0;
+ * GB_MD_DEFER=0 in the environment at gb_init takes them all, with a wait per
+ * step).  n = number of slots to copy. */
 int gb_last_timings(double* ms, int n);
 
 /* Number of kernels the library launched since gb_init (its own count). */

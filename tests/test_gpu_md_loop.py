@@ -1,0 +1,66 @@
+"""The MD loop that reads a step's sums after its last step, launched or replayed as CUDA graphs,
+against the loop that reads them at every step: constraints, thermostats and metals."""
+import numpy as np
+import pytest
+
+from dlpoly_gb300 import systems
+
+pytestmark = pytest.mark.gpu
+
+RUNS = {
+    "water": (lambda: systems.spce_water(8), 0, "nve", 1e-12),
+    "water_mixed_nose_hoover": (lambda: systems.spce_water(8), 1, "nose-hoover", 1e-12),
+    "water_berendsen": (lambda: systems.spce_water(8), 0, "berendsen", 1e-12),
+    "nacl_langevin": (lambda: systems.nacl_melt(16), 0, "langevin", 1e-12),
+    "eam": (lambda: systems.eam_alloy(8), 0, "nve", 1e-9),  # FP64 atomics: their order varies
+}
+FIELDS = ("engcpe_rc", "vircpe_rc", "engcpe_rl", "vircpe_rl", "engcpe_ex", "vircpe_ex", "engvdw", "virvdw", "engke",
+          "vircon", "consv", "engmet", "virmet")
+
+
+@pytest.mark.parametrize("name", RUNS)
+def test_deferred_loop_matches_per_step_readback(gpu_lib, monkeypatch, name):
+    make, precision, ens, tol = RUNS[name]
+    s = make()
+    out = []
+    for defer, graphs in (("0", "0"), ("1", "0"), ("1", "1")):
+        monkeypatch.setenv("GB_MD_DEFER", defer)
+        monkeypatch.setenv("GB_GRAPHS", graphs)
+        gpu_lib.init(s, precision=precision)
+        if ens != "nve":
+            gpu_lib.set_ensemble(ens, temp=300.0, tau_t=0.05, chi=5.0)
+        gpu_lib.start()
+        st = gpu_lib.md_vv(9)
+        met = gpu_lib.metal_energies() if s.eam else {}
+        out.append((st, gpu_lib.download(), gpu_lib.thermostat_state(), met))
+    monkeypatch.delenv("GB_MD_DEFER")
+    monkeypatch.delenv("GB_GRAPHS")
+    sa, a, ta, ma = out[0]
+    for sb, b, tb, mb in out[1:]:
+        for k in a:
+            assert np.abs(a[k] - b[k]).max() <= tol * np.abs(a[k]).max(), k
+        for x, y in zip(sa, sb):
+            assert (x.list_rebuilt, x.shake_iters, x.rattle_iters) == (y.list_rebuilt, y.shake_iters, y.rattle_iters)
+            for f in FIELDS:
+                scale = max(abs(getattr(x, f)), 1e-3 * abs(x.engke))
+                assert abs(getattr(x, f) - getattr(y, f)) <= 10 * tol * scale, f
+            for f in ("stress", "strkin", "strcon"):
+                u, v = np.array(getattr(x, f)[:]), np.array(getattr(y, f)[:])
+                assert np.abs(u - v).max() <= 10 * tol * max(np.abs(u).max(), 1e-30), f
+        for k in ta:
+            assert abs(ta[k] - tb[k]) <= 10 * tol * max(abs(ta[k]), 1e-30), k
+        for k in ma:
+            assert mb[k] == pytest.approx(ma[k], rel=10 * tol), k
+
+
+def test_failing_step_ends_the_call_with_its_code(gpu_lib):
+    """SHAKE beyond its sweeps ends a run of several steps with 105; the steps before it are reported."""
+    s = systems.spce_water(8)
+    gpu_lib.init(s, shake_maxit=20)
+    gpu_lib.start()
+    with pytest.raises(Exception) as e:
+        gpu_lib.md_vv(5)
+    assert getattr(e.value, "code", None) == 105
+    gpu_lib.init(s)
+    gpu_lib.start()
+    assert all(x.shake_iters > 20 for x in gpu_lib.md_vv(5))
