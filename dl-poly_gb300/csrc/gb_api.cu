@@ -960,7 +960,7 @@ int gb_shake(int32_t* iters, double* vircon, double* strcon) {
 int gb_rattle(int32_t* iters) {
   return guarded([&]() {
     GB_CUDA(cudaMemsetAsync(&g.sc->status, 0, sizeof(int), g.stream));
-    integ_rattle_launch();
+    integ_rattle_launch(false);
     gb_sync_scalars();
     if (iters) *iters = g.ntcons > 0 ? g.hsc->rattle_iters : 0;
     if (g.ntcons > 0 && (g.hsc->status & ST_RATTLE_FAIL)) return (int)GB_ERR_RATTLE;

@@ -503,7 +503,7 @@ void con_scalars(const DevScalars* h, double* vircon, double* strcon);
 void metal_scalars(const DevScalars* h, double* e4, double* stress9);  // stress9 accumulates
 void integ_con_tags();            // constraints_tags: old bond vectors from the current positions
 void integ_shake(int* iters, double* vircon, double* strcon);  // apply_shake (throws GB_ERR_SHAKE)
-void integ_rattle_launch();       // apply_rattle, kit = 1 (status bit ST_RATTLE_FAIL)
+void integ_rattle_launch(bool tags);  // apply_rattle, kit = 1 (status bit ST_RATTLE_FAIL)
 int integ_vnl_check();
 void integ_vnl_launch();          // the displacement check
 void integ_stage1_check();        // NVE stage 1 and the displacement check in one kernel

@@ -178,6 +178,7 @@ struct ConArgs {
   const double* w;
   double tstep, tol, c0, a0;
   int* flags;      // maxit+1 ints, zeroed
+  bool tags;       // RATTLE of k_constrain_small: form the bond vectors from the positions (and store them)
   DevScalars* sc;
   double* blk;     // per-block stress partials (6)
 };
@@ -562,21 +563,30 @@ __global__ void __launch_bounds__(128) k_constrain_cl(ConArgs A, const ClusterTa
 // form's, whose coordinates carry the rounding of the box's size (7e-15 A at 50 A).
 // An FP64 instruction takes 16 issue slots of an SM sub-partition here: the FP64 form of
 // the sweep (~110 FP64 instructions with 3 divisions, k_constrain_cl) took 0.83 ms a call
-// for 32,768 waters (~67 sweeps) and 0.52 ms for 2,197; the scalar form takes 0.133 (SHAKE)
-// and 0.055 ms (RATTLE), and 0.090 and 0.043 ms, bound by FP32 issue at two warps per
-// scheduler and by the dependent operations of a sweep.
-// Sweeps run in chunks of CS_CHUNK between grid barriers; a cluster keeps the scalars of
-// the chunk's start and repeats the chunk's committed sweeps once the last one is known.
-constexpr int CS_THREADS = 64, CS_CHUNK = 16, CS_MAXC = 3;
+// for 32,768 waters (~67 sweeps) and 0.52 ms for 2,197.
+// A lane holds one constraint (3 lanes a cluster, 10 clusters a warp) and exchanges its
+// scalar by shuffles: a sweep is a chain of dependent operations, which one lane per
+// cluster ran at two warps a scheduler (0.133 and 0.090 ms).  q_c is evaluated as c0 +
+// sum_i t_i (l_i + sum_j q_ij t_j); the inner sums run over an added constant
+// (off_add_prod), and the scalars of a chunk's sweeps are kept in shared memory, so that
+// none is repeated.  It takes 0.090 ms (SHAKE) and 0.053 ms (RATTLE, which forms the bond
+// vectors too) for 32,768 waters, 0.047 and 0.027 ms for 2,197: the operations of a sweep in
+// order, the FP64 set-up and epilogue, and five grid barriers.
+// Sweeps run in chunks of CS_CHUNK between grid barriers (20 steps of 2,197 molecules:
+// 8.6 ms with chunks of 8, 8.3 with 16 and with 31, which doubles the shared memory).
+constexpr int CS_CHUNK = 16, CS_MAXC = 3, CS_PERWARP = 10;
+constexpr int CS_THREADS = 704;  // one block per SM: 22 warps of at most 88 registers
+constexpr int CS_POLY = 14;      // float2 of the polynomials of a lane
 
 struct ClKind {        // clusters with equal masses, lengths and topology share one
   int na, nc;
   int li[CS_MAXC], lj[CS_MAXC];         // local ends of the constraints
   float2 K[CS_MAXC][CS_MAXC];           // double-float
   float2 tol_s[CS_MAXC], tol_r;         // bounds on |q| (2 tol d0) and |g| (2 tol / tstep)
+  float2 two_m[CS_MAXC];                // gamma sum = two_m * t (SHAKE), double-float
+  float off;                            // 8 max(d0^2) rounded up to a power of two: exceeds |l| and its sums
   double W[CL_MAXA][CS_MAXC];
   double d0sq[CS_MAXC];
-  double two_m[CS_MAXC];                // gamma sum = two_m * t (SHAKE)
   double wh[CL_MAXA];                   // weight / hstep, 0: frozen
 };
 
@@ -597,210 +607,280 @@ __device__ __forceinline__ bool df_abs_less(df a, float2 b) {
   return h < b.x || (h == b.x && l < b.y);
 }
 
+__device__ __forceinline__ df df_shfl(df a, int lane) {
+  return df_make(__shfl_sync(0xffffffffu, a.hi, lane), __shfl_sync(0xffffffffu, a.lo, lane));
+}
+
+// The polynomials of a lane's constraint; index r is the constraint of the cluster r places
+// after its own, cyclically; q in the order 00, 01, 02, 11, 12, 22.
 struct ClPoly {
-  df c0[CS_MAXC], l[CS_MAXC][CS_MAXC], q[CS_MAXC][6];  // q_c or g_c (l only)
-  df p0[CS_MAXC], p[CS_MAXC][CS_MAXC];                 // p_c
+  df c0, l[CS_MAXC];  // l over the constant off (SHAKE)
+  df q[6];
+  df p0, p[CS_MAXC];
 };
 
+// c: constraint of the lane, on: it has one; n1, n2: lanes of the next two constraints
 template <bool RATTLE>
-__device__ __forceinline__ void cs_setup(const ConArgs& A, const ClusterTab& T, const ClKind& D, long long quarter,
-                                         ClPoly& P) {
-  df b[CS_MAXC][3], u[CS_MAXC][3], B[CS_MAXC][CS_MAXC], K[CS_MAXC][CS_MAXC];
+__device__ __forceinline__ void cs_setup(const ConArgs& A, const ClusterTab& T, const ClKind& D, int c, bool on, int n1,
+                                         int n2, long long quarter, ClPoly& P) {
+  df b[CS_MAXC][3], u[3], B[6], K[CS_MAXC];
+  P.c0 = df_make(0.f, 0.f);
 #pragma unroll
-  for (int c = 0; c < CS_MAXC; ++c) {
-#pragma unroll
-    for (int k = 0; k < 3; ++k) b[c][k] = u[c][k] = df_make(0.f, 0.f);
-    P.c0[c] = df_make(0.f, 0.f);
-    if (c < D.nc) {
-      const int k = T.con[c], i = T.atom[D.li[c]], j = T.atom[D.lj[c]];
-      double bx = A.dxx[k], by = A.dyy[k], bz = A.dzz[k];
-      if (RATTLE) {
-        const double b2 = bx * bx + by * by + bz * bz;
-        double r = rsqrt_seeded(b2);
-        r = r * fma(-0.5 * b2 * r, r, 1.5);
-        bx *= r; by *= r; bz *= r;
-      }
-      b[c][0] = dbl_split(bx); b[c][1] = dbl_split(by); b[c][2] = dbl_split(bz);
-      if (RATTLE) {
-        const double dx = A.vx[i] - A.vx[j], dy = A.vy[i] - A.vy[j], dz = A.vz[i] - A.vz[j];
-        P.c0[c] = dbl_split(bx * dx + by * dy + bz * dz);
-      } else {
-        const double dx = image_short(A.x[i] - A.x[j], quarter, A.c0, A.a0);
-        const double dy = image_short(A.y[i] - A.y[j], quarter, A.c0, A.a0);
-        const double dz = image_short(A.z[i] - A.z[j], quarter, A.c0, A.a0);
-        u[c][0] = dbl_split(dx); u[c][1] = dbl_split(dy); u[c][2] = dbl_split(dz);
-        P.c0[c] = dbl_split(dx * dx + dy * dy + dz * dz - D.d0sq[c]);
-      }
+  for (int k = 0; k < 3; ++k) b[0][k] = u[k] = P.c0;
+  if (on) {
+    const int k = T.con[c], i = T.atom[D.li[c]], j = T.atom[D.lj[c]];
+    double bx, by, bz;
+    if (RATTLE && A.tags) {
+      bx = image_short(A.x[i] - A.x[j], quarter, A.c0, A.a0);
+      by = image_short(A.y[i] - A.y[j], quarter, A.c0, A.a0);
+      bz = image_short(A.z[i] - A.z[j], quarter, A.c0, A.a0);
+      A.dxx[k] = bx; A.dyy[k] = by; A.dzz[k] = bz;
+    } else {
+      bx = A.dxx[k]; by = A.dyy[k]; bz = A.dzz[k];
     }
-#pragma unroll
-    for (int k = 0; k < CS_MAXC; ++k) K[c][k] = df_of(D.K[c][k]);
+    if (RATTLE) {
+      const double b2 = bx * bx + by * by + bz * bz;
+      double r = rsqrt_seeded(b2);
+      r = r * fma(-0.5 * b2 * r, r, 1.5);
+      bx *= r; by *= r; bz *= r;
+      const double dx = A.vx[i] - A.vx[j], dy = A.vy[i] - A.vy[j], dz = A.vz[i] - A.vz[j];
+      P.c0 = dbl_split(bx * dx + by * dy + bz * dz);
+    } else {
+      const double dx = image_short(A.x[i] - A.x[j], quarter, A.c0, A.a0);
+      const double dy = image_short(A.y[i] - A.y[j], quarter, A.c0, A.a0);
+      const double dz = image_short(A.z[i] - A.z[j], quarter, A.c0, A.a0);
+      u[0] = dbl_split(dx); u[1] = dbl_split(dy); u[2] = dbl_split(dz);
+      P.c0 = dbl_split(dx * dx + dy * dy + dz * dz - D.d0sq[c]);
+    }
+    b[0][0] = dbl_split(bx); b[0][1] = dbl_split(by); b[0][2] = dbl_split(bz);
   }
 #pragma unroll
-  for (int c = 0; c < CS_MAXC; ++c)
+  for (int k = 0; k < 3; ++k) {
+    b[1][k] = df_shfl(b[0][k], n1);
+    b[2][k] = df_shfl(b[0][k], n2);
+  }
+  const int c1 = c == 2 ? 0 : c + 1, c2 = c == 0 ? 2 : c - 1;
+  K[0] = df_of(D.K[c][c]); K[1] = df_of(D.K[c][c1]); K[2] = df_of(D.K[c][c2]);
+  B[0] = df_dot(b[0], b[0]);
+  B[1] = df_dot(b[0], b[1]);
+  B[2] = df_shfl(B[1], n2);  // 2 . 0
+  B[3] = df_shfl(B[0], n1);
+  B[4] = df_shfl(B[1], n1);  // 1 . 2
+  B[5] = df_shfl(B[0], n2);
+  if (!on) K[0] = K[1] = K[2] = df_make(0.f, 0.f);
 #pragma unroll
-    for (int k = c; k < CS_MAXC; ++k) B[c][k] = B[k][c] = df_dot(b[c], b[k]);
-#pragma unroll
-  for (int c = 0; c < CS_MAXC; ++c) {
+  for (int k = 0; k < CS_MAXC; ++k) {
+    P.p[k] = df_mul(K[k], B[k]);
+    if (RATTLE) continue;
+    const df w = df_mul(K[k], df_dot(u, b[k]));
+    const df s = two_sum(D.off, 2.f * w.hi);
+    P.l[k] = df_make(s.hi, s.lo + 2.f * w.lo);
+  }
+  if (!RATTLE) {
+    P.p0 = on ? df_dot(u, b[0]) : df_make(1.f, 0.f);
     int m = 0;
 #pragma unroll
-    for (int k = 0; k < CS_MAXC; ++k) {
-      P.p[c][k] = df_mul(K[c][k], B[c][k]);
-      if (RATTLE) {
-        P.l[c][k] = P.p[c][k];
-        continue;
-      }
-      const df w = df_mul(K[c][k], df_dot(u[c], b[k]));
-      P.l[c][k] = df_make(2.f * w.hi, 2.f * w.lo);
+    for (int k = 0; k < CS_MAXC; ++k)
 #pragma unroll
       for (int n = k; n < CS_MAXC; ++n, ++m) {
-        const df e = df_mul(df_mul(K[c][k], K[c][n]), B[k][n]);
+        const df e = df_mul(df_mul(K[k], K[n]), B[m]);
         const float f = n == k ? 1.f : 2.f;
-        P.q[c][m] = df_make(f * e.hi, f * e.lo);
+        P.q[m] = df_make(f * e.hi, f * e.lo);
       }
-    }
-    if (!RATTLE) {
-      P.p0[c] = df_dot(u[c], b[c]);
-      if (c >= D.nc) P.p0[c] = df_make(1.f, 0.f);
-    }
   }
 }
 
-// one sweep from the scalars t: true when a constraint fails its test; t updated
+// one sweep from the scalars t (own first): true when the constraint fails its test; the new
+// scalars in t
 template <bool RATTLE>
-__device__ __forceinline__ bool cs_sweep(const ClKind& D, const ClPoly& P, df (&t)[CS_MAXC]) {
-  bool fail = false;
-  df m[6];
-  if (!RATTLE) {
-    int k = 0;
+__device__ __forceinline__ bool cs_sweep(const ClPoly& P, float off, float2 tol, int n1, int n2, df (&t)[CS_MAXC]) {
+  dacc a = {P.c0.hi, P.c0.lo};
+  df step;
+  bool fail;
+  if constexpr (RATTLE) {
 #pragma unroll
-    for (int i = 0; i < CS_MAXC; ++i)
+    for (int i = 0; i < CS_MAXC; ++i) dacc_add_prod(a, P.p[i], t[i]);
+    step = quick_two_sum(a.s, a.c);
+    fail = !df_abs_less(step, tol);
+  } else {
+    dacc e = {P.p0.hi, P.p0.lo};  // p exceeds its corrections
 #pragma unroll
-      for (int j = i; j < CS_MAXC; ++j, ++k) m[k] = df_mul(t[i], t[j]);
-  }
-  df step[CS_MAXC];
+    for (int i = 0; i < CS_MAXC; ++i) off_add_prod(e, P.p[i], t[i]);
+    // 1/p: FP32 reciprocal and the first-order remainder (relative error about 2^-46)
+    const float r = __frcp_rn(e.s);
+    const float h = __fmaf_rn(-e.c, r, __fmaf_rn(-e.s, r, 1.f));
+    int m = 0;
 #pragma unroll
-  for (int c = 0; c < CS_MAXC; ++c) {
-    dacc a = {P.c0[c].hi, P.c0[c].lo};
+    for (int i = 0; i < CS_MAXC; ++i) {
+      dacc v = {P.l[i].hi, P.l[i].lo};
 #pragma unroll
-    for (int i = 0; i < CS_MAXC; ++i) dacc_add_prod(a, P.l[c][i], t[i]);
-    if constexpr (RATTLE) {
-      step[c] = quick_two_sum(a.s, a.c);
-      if (c < D.nc && !df_abs_less(step[c], D.tol_r)) fail = true;
-    } else {
-#pragma unroll
-      for (int i = 0; i < 6; ++i) dacc_add_prod(a, P.q[c][i], m[i]);
-      const df q = quick_two_sum(a.s, a.c);
-      if (c < D.nc && !df_abs_less(q, D.tol_s[c])) fail = true;
-      dacc e = {P.p0[c].hi, P.p0[c].lo};
-#pragma unroll
-      for (int i = 0; i < CS_MAXC; ++i) dacc_add_prod(e, P.p[c][i], t[i]);
-      const df p = quick_two_sum(e.s, e.c);
-      // 1/p: FP32 reciprocal and the first-order remainder (relative error about 2^-46)
-      const float r = __frcp_rn(p.hi);
-      const float h = __fmaf_rn(-p.lo, r, __fmaf_rn(-p.hi, r, 1.f));
-      const df s = df_mul(q, df_make(r, r * h));
-      step[c] = df_make(0.5f * s.hi, 0.5f * s.lo);
+      for (int j = i; j < CS_MAXC; ++j, ++m) off_add_prod(v, P.q[m], t[j]);
+      dacc_add_prod(a, df_make(__fsub_rn(v.s, off), v.c), t[i]);
     }
+    const df q = quick_two_sum(a.s, a.c);
+    fail = !df_abs_less(q, tol);
+    const df s = df_mul(q, df_make(r, r * h));
+    step = df_make(0.5f * s.hi, 0.5f * s.lo);
   }
-#pragma unroll
-  for (int c = 0; c < CS_MAXC; ++c) t[c] = df_add(t[c], step[c]);
+  t[0] = df_add(t[0], step);
+  t[1] = df_shfl(t[0], n1);
+  t[2] = df_shfl(t[0], n2);
   return fail;
 }
 
-// SHAKE with its epilogue (apply_shake: v += dr/dt, f += dr/dt m/(dt/2)) or RATTLE.  tbuf: the
-// scalars between chunks when a thread has several clusters (ncl > threads), 2 x 3 per cluster.
+// The polynomials of a lane to and from pbuf (more clusters than resident lanes).
+template <bool RATTLE, bool STORE>
+__device__ __forceinline__ void cs_poly_io(float2* __restrict__ pbuf, size_t ld, ClPoly& P) {
+  auto io = [&](int slot, df& v) {
+    if (STORE)
+      pbuf[slot * ld] = make_float2(v.hi, v.lo);
+    else
+      v = df_of(pbuf[slot * ld]);
+  };
+  io(0, P.c0);
+#pragma unroll
+  for (int k = 0; k < 3; ++k) io(1 + k, P.p[k]);
+  if (RATTLE) return;
+#pragma unroll
+  for (int k = 0; k < 3; ++k) io(4 + k, P.l[k]);
+#pragma unroll
+  for (int k = 0; k < 6; ++k) io(7 + k, P.q[k]);
+  io(13, P.p0);
+}
+
+// SHAKE with its epilogue (apply_shake: v += dr/dt, f += dr/dt m/(dt/2)) or RATTLE.  pbuf: when
+// there are more clusters than resident lanes, the polynomials of a lane and its scalar
+// at the start and the end of the chunk ([CS_POLY + 2][3 ncl]; L2 traffic of a few microseconds
+// a chunk); such a cluster repeats the last chunk's committed sweeps.
 template <bool RATTLE>
 __global__ void __launch_bounds__(CS_THREADS) k_constrain_small(ConArgs A, const ClusterTab* __restrict__ tabs,
                                                                const int* __restrict__ kind_of,
                                                                const ClKind* __restrict__ kinds, int ncl,
-                                                               float2* __restrict__ tbuf, double rstep, double* fx,
+                                                               float2* __restrict__ pbuf, double rstep, double* fx,
                                                                double* fy, double* fz) {
+  extern __shared__ float2 cs_hist[];  // [CS_CHUNK][blockDim.x]: the scalar before each sweep of the chunk
   cg::grid_group grid = cg::this_grid();
-  const int tid = blockIdx.x * blockDim.x + threadIdx.x;
-  const int nth = gridDim.x * blockDim.x;
+  const int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const int wstep = ((gridDim.x * blockDim.x) >> 5) * CS_PERWARP;
+  const int sub = lane / 3, c = lane - 3 * sub;
+  const int n1 = 3 * sub + (c == 2 ? 0 : c + 1), n2 = 3 * sub + (c == 0 ? 2 : c - 1);
   const long long quarter = __double_as_longlong(0.25 * A.c0);
-  const bool multi = ncl > nth;
+  const bool multi = ncl > wstep;
+  const size_t ld = 3 * (size_t)ncl;
   ClPoly P;
-  df t[CS_MAXC], tb[CS_MAXC];
+  df t[CS_MAXC];
 #pragma unroll
-  for (int c = 0; c < CS_MAXC; ++c) t[c] = tb[c] = df_make(0.f, 0.f);
+  for (int r = 0; r < CS_MAXC; ++r) t[r] = df_make(0.f, 0.f);
   int it0 = 0, nfinal = -1, last = 0;
+  bool done = false;
   for (int ch = 0;; ++ch) {
     unsigned bad = 0;
     const int n = min(CS_CHUNK, A.maxit - it0);
-    for (int cl = tid; cl < ncl; cl += nth) {
+    for (int cl0 = warp * CS_PERWARP; cl0 < ncl; cl0 += wstep) {
+      const bool in = lane < 3 * CS_PERWARP && cl0 + sub < ncl;
+      const int cl = in ? cl0 + sub : cl0;
       const ClKind& D = kinds[kind_of[cl]];
-      if (multi || it0 == 0) cs_setup<RATTLE>(A, tabs[cl], D, quarter, P);
-#pragma unroll
-      for (int c = 0; c < CS_MAXC; ++c) {
-        if (multi) t[c] = it0 ? df_of(tbuf[(size_t)(2 * c) * ncl + cl]) : df_make(0.f, 0.f);
-        tb[c] = t[c];
-        if (multi) tbuf[(size_t)(2 * c + 1) * ncl + cl] = make_float2(t[c].hi, t[c].lo);
+      const bool on = in && c < D.nc;
+      float2* pb = pbuf + (size_t)3 * cl + c;
+      if (it0 == 0) {
+        cs_setup<RATTLE>(A, tabs[cl], D, c, on, n1, n2, quarter, P);
+        if (multi && in) cs_poly_io<RATTLE, true>(pb, ld, P);
+        t[0] = t[1] = t[2] = df_make(0.f, 0.f);
+      } else if (multi) {
+        cs_poly_io<RATTLE, false>(pb, ld, P);
+        t[0] = df_of(pb[(CS_POLY + 1) * ld]);
+        t[1] = df_shfl(t[0], n1);
+        t[2] = df_shfl(t[0], n2);
       }
-      for (int s = 0; s < n; ++s)
-        if (cs_sweep<RATTLE>(D, P, t)) bad |= 1u << s;
-      if (multi) {
-#pragma unroll
-        for (int c = 0; c < CS_MAXC; ++c) tbuf[(size_t)(2 * c) * ncl + cl] = make_float2(t[c].hi, t[c].lo);
+      if (multi && in) pb[CS_POLY * ld] = make_float2(t[0].hi, t[0].lo);
+      const float off = D.off;
+      const float2 tol = RATTLE ? D.tol_r : D.tol_s[c];
+      unsigned b = 0;
+      for (int s = 0; s < n; ++s) {
+        cs_hist[s * blockDim.x + threadIdx.x] = make_float2(t[0].hi, t[0].lo);
+        if (cs_sweep<RATTLE>(P, off, tol, n1, n2, t)) b |= 1u << s;
       }
+      if (on) bad |= b;
+      if (multi && in) pb[(CS_POLY + 1) * ld] = make_float2(t[0].hi, t[0].lo);
     }
     bad = __reduce_or_sync(0xffffffffu, bad);
-    if (bad && (threadIdx.x & 31) == 0) atomicOr(&A.flags[ch], (int)bad);
+    if (bad && lane == 0) atomicOr(&A.flags[ch], (int)bad);
     grid.sync();
-    const unsigned f = ~(unsigned)__ldcg(&A.flags[ch]) & ((n == 32) ? 0xffffffffu : (1u << n) - 1u);
+    const unsigned f = ~(unsigned)__ldcg(&A.flags[ch]) & ((1u << n) - 1u);
     last = n;  // committed sweeps of this chunk: all, or those before the first that nobody failed
     if (f) {
       last = __ffs((int)f) - 1;
       nfinal = it0 + last + 1;
-      break;
+      done = true;
     }
-    if (it0 + n >= A.maxit) break;
+    if (done || it0 + n >= A.maxit) break;
     it0 += n;
   }
-  if (tid == 0) {
+  if (warp == 0 && lane == 0) {
     (RATTLE ? A.sc->rattle_iters : A.sc->shake_iters) = nfinal > 0 ? nfinal : A.maxit;
     if (nfinal < 0) A.sc->status |= RATTLE ? ST_RATTLE_FAIL : ST_SHAKE_FAIL;
   }
-  double st[6] = {0, 0, 0, 0, 0, 0};
-  for (int cl = tid; cl < ncl; cl += nth) {
+  df st[6];
+#pragma unroll
+  for (int k = 0; k < 6; ++k) st[k] = df_make(0.f, 0.f);
+  for (int cl0 = warp * CS_PERWARP; cl0 < ncl; cl0 += wstep) {
+    const bool in = lane < 3 * CS_PERWARP && cl0 + sub < ncl;
+    const int cl = in ? cl0 + sub : cl0;
     const ClusterTab& T = tabs[cl];
     const ClKind& D = kinds[kind_of[cl]];
+    const bool on = in && c < D.nc;
     if (multi) {
-      cs_setup<RATTLE>(A, T, D, quarter, P);
-#pragma unroll
-      for (int c = 0; c < CS_MAXC; ++c) tb[c] = df_of(tbuf[(size_t)(2 * c + 1) * ncl + cl]);
+      const float2* pb = pbuf + (size_t)3 * cl + c;
+      cs_poly_io<RATTLE, false>(pbuf + (size_t)3 * cl + c, ld, P);
+      t[0] = df_of(pb[CS_POLY * ld]);
+      t[1] = df_shfl(t[0], n1);
+      t[2] = df_shfl(t[0], n2);
+      const float2 tol = RATTLE ? D.tol_r : D.tol_s[c];
+      for (int s = 0; s < last; ++s) cs_sweep<RATTLE>(P, D.off, tol, n1, n2, t);
+    } else if (done) {
+      t[0] = df_of(cs_hist[last * blockDim.x + threadIdx.x]);
     }
-    for (int s = 0; s < last; ++s) cs_sweep<RATTLE>(D, P, tb);
-    double tt[CS_MAXC], b[CS_MAXC][3];
-#pragma unroll
-    for (int c = 0; c < CS_MAXC; ++c) {
-      tt[c] = b[c][0] = b[c][1] = b[c][2] = 0.0;
-      if (c >= D.nc) continue;
+    double v[3] = {0.0, 0.0, 0.0};  // t b of the lane's constraint
+    if (on) {
       const int k = T.con[c];
-      tt[c] = df_to_double(tb[c]);
-      b[c][0] = A.dxx[k]; b[c][1] = A.dyy[k]; b[c][2] = A.dzz[k];
+      const double b[3] = {A.dxx[k], A.dyy[k], A.dzz[k]};
+      double tt = df_to_double(t[0]);
       if (RATTLE) {
-        const double b2 = b[c][0] * b[c][0] + b[c][1] * b[c][1] + b[c][2] * b[c][2];
+        const double b2 = b[0] * b[0] + b[1] * b[1] + b[2] * b[2];
         double r = rsqrt_seeded(b2);
         r = r * fma(-0.5 * b2 * r, r, 1.5);
-        tt[c] *= r;  // unit bond vectors
+        tt *= r;  // unit bond vectors
       } else {
-        const double g = D.two_m[c] * tt[c];
-        const double gx = g * b[c][0], gy = g * b[c][1], gz = g * b[c][2];
-        st[0] -= gx * b[c][0]; st[1] -= gx * b[c][1]; st[2] -= gx * b[c][2];
-        st[3] -= gy * b[c][1]; st[4] -= gy * b[c][2]; st[5] -= gz * b[c][2];
-      }
-    }
+        const df g = df_mul(df_of(D.two_m[c]), t[0]);
+        const df bd[3] = {dbl_split(b[0]), dbl_split(b[1]), dbl_split(b[2])};
+        int m = 0;
 #pragma unroll
-    for (int a = 0; a < CL_MAXA; ++a) {
-      if (a >= D.na || __double_as_longlong(D.wh[a]) == 0) continue;
+        for (int p = 0; p < 3; ++p) {
+          const df gb = df_mul(g, bd[p]);
+#pragma unroll
+          for (int q = p; q < 3; ++q, ++m) {
+            const df e = df_mul(gb, bd[q]);
+            st[m] = df_add(st[m], df_make(-e.hi, -e.lo));
+          }
+        }
+      }
+#pragma unroll
+      for (int p = 0; p < 3; ++p) v[p] = tt * b[p];
+    }
+    double w[CS_MAXC][3];
+#pragma unroll
+    for (int k = 0; k < CS_MAXC; ++k)
+#pragma unroll
+      for (int p = 0; p < 3; ++p) w[k][p] = __shfl_sync(0xffffffffu, v[p], 3 * sub + k);
+    if (!in) continue;
+    for (int a = c; a < D.na; a += CS_MAXC) {
+      if (__double_as_longlong(D.wh[a]) == 0) continue;
       double dx = 0.0, dy = 0.0, dz = 0.0;
 #pragma unroll
-      for (int c = 0; c < CS_MAXC; ++c) {
-        const double w = D.W[a][c];
-        if (__double_as_longlong(w) == 0) continue;
-        const double f = w * tt[c];
-        dx = fma(f, b[c][0], dx); dy = fma(f, b[c][1], dy); dz = fma(f, b[c][2], dz);
+      for (int k = 0; k < CS_MAXC; ++k) {
+        const double f = D.W[a][k];
+        if (__double_as_longlong(f) == 0) continue;
+        dx = fma(f, w[k][0], dx); dy = fma(f, w[k][1], dy); dz = fma(f, w[k][2], dz);
       }
       const int i = T.atom[a];
       if (RATTLE) {
@@ -818,7 +898,7 @@ __global__ void __launch_bounds__(CS_THREADS) k_constrain_small(ConArgs A, const
   if (!RATTLE) {
     dfr sd[6];
 #pragma unroll
-    for (int k = 0; k < 6; ++k) sd[k] = to_dfr(dbl_split(st[k]));
+    for (int k = 0; k < 6; ++k) sd[k] = to_dfr(st[k]);
     block_reduce_store<6>(sd, A.blk);
   }
 }
@@ -853,9 +933,9 @@ constexpr int CL_THREADS = 128;  // small blocks spread the clusters over every 
 // clusters of at most 3 constraints (k_constrain_small)
 int* d_clkind = nullptr;     // kind of each cluster
 ClKind* d_kinds = nullptr;
-float2* d_clt = nullptr;     // scalars between chunks, when there are more clusters than resident threads
+float2* d_clt = nullptr;     // polynomials and scalars, when there are more clusters than resident lanes
 bool cl_small = false;
-int coop_blocks_small = 0;
+int coop_blocks_small = 0, cs_threads = 32;
 
 // connected constraint clusters; false when one exceeds CL_MAXA atoms or CL_MAXC constraints
 bool build_clusters(const std::vector<int>& ci, const std::vector<int>& cj, std::vector<ClusterTab>& out) {
@@ -954,7 +1034,8 @@ bool build_kinds(const std::vector<ClusterTab>& tabs, const std::vector<double>&
       W[D.li[c]][c] -= iw[D.li[c]] / m;
       W[D.lj[c]][c] += iw[D.lj[c]] / m;
       D.d0sq[c] = len * len;
-      D.two_m[c] = 2.0 / (m * dt * dt);
+      D.two_m[c] = split(2.0 / (m * dt * dt));
+      D.off = std::max(D.off, std::ldexp(1.f, std::ilogb(len * len) + 4));
       D.tol_s[c] = split(2.0 * (tol * len));
     }
     D.tol_r = split(tol / (0.5 * dt));
@@ -1041,12 +1122,15 @@ void integ_setup_constraints(const int32_t* listcon, const double* prmcon) {
       GB_CUDA(cudaMemcpy(d_clkind, kind_of.data(), sizeof(int) * kind_of.size(), cudaMemcpyHostToDevice));
       GB_CUDA(cudaMalloc(&d_kinds, sizeof(ClKind) * kinds.size()));
       GB_CUDA(cudaMemcpy(d_kinds, kinds.data(), sizeof(ClKind) * kinds.size(), cudaMemcpyHostToDevice));
-      int b0 = 0, b1 = 0;
-      GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b0, k_constrain_small<false>, CS_THREADS, 0));
-      GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b1, k_constrain_small<true>, CS_THREADS, 0));
-      coop_blocks_small = std::max(1, std::min(std::min(b0, b1) * g.nsm, nblocks(n_clusters, CS_THREADS)));
-      if ((long long)coop_blocks_small * CS_THREADS < n_clusters)
-        GB_CUDA(cudaMalloc(&d_clt, sizeof(float2) * 2 * CS_MAXC * tabs.size()));
+      // one block per SM (the fewest to meet at a grid barrier), wide enough for all clusters
+      const int nwarp = (n_clusters + CS_PERWARP - 1) / CS_PERWARP;
+      cs_threads = 32 * std::min((nwarp + g.nsm - 1) / g.nsm, CS_THREADS / 32);
+      coop_blocks_small = std::min(g.nsm, nblocks(nwarp, cs_threads / 32));
+      const int smem = (int)sizeof(float2) * CS_CHUNK * CS_THREADS;
+      GB_CUDA(cudaFuncSetAttribute(k_constrain_small<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      GB_CUDA(cudaFuncSetAttribute(k_constrain_small<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+      if (coop_blocks_small * (cs_threads / 32) < nwarp)
+        GB_CUDA(cudaMalloc(&d_clt, sizeof(float2) * (CS_POLY + 2) * CS_MAXC * tabs.size()));
     } else {
       GB_CUDA(cudaMalloc(&d_clring, sizeof(double) * CL_RING * CL_SLOT * tabs.size()));
       GB_CUDA(cudaMalloc(&d_clgsum, sizeof(double) * CL_MAXC * tabs.size()));
@@ -1108,7 +1192,7 @@ static void con_args(ConArgs& A) {
   A.dt2 = g.dt2; A.gam = g.gam;
   A.x = g.x; A.y = g.y; A.z = g.z; A.vx = g.vx; A.vy = g.vy; A.vz = g.vz; A.w = g.weight;
   A.tstep = g.p.tstep; A.tol = g.p.shake_tol; A.c0 = g.cell[0]; A.a0 = 1.0 / g.cell[0];
-  A.flags = d_flags; A.sc = g.sc; A.blk = nullptr;
+  A.flags = d_flags; A.sc = g.sc; A.blk = nullptr; A.tags = false;
 }
 
 template <bool RATTLE>
@@ -1120,7 +1204,8 @@ static void launch_small(ConArgs& A, double rstep) {
   float2* tbuf = d_clt;
   double *fx = g.fx, *fy = g.fy, *fz = g.fz;
   void* args[] = {&A, &tabs, &kind, &kinds, &ncl, &tbuf, &rstep, &fx, &fy, &fz};
-  GB_CUDA(cudaLaunchCooperativeKernel((void*)k_constrain_small<RATTLE>, coop_blocks_small, CS_THREADS, args, 0, g.stream));
+  GB_CUDA(cudaLaunchCooperativeKernel((void*)k_constrain_small<RATTLE>, coop_blocks_small, cs_threads, args,
+                                      sizeof(float2) * CS_CHUNK * cs_threads, g.stream));
 }
 
 // constraints_tags (constraints.F90:438-586): old bond vectors from the current positions
@@ -1179,14 +1264,17 @@ void integ_shake(int* iters, double* vircon, double* strcon) {
 }
 
 // apply_rattle with kit = 1 (constraints.F90:1032-1069 -> constraints_rattle :587-775) on
-// the current velocities, against the bond vectors of the last integ_con_tags.  The
+// the current velocities, against the bond vectors of the last integ_con_tags or, with
+// tags, of the current positions (constraints_tags as part of the kernel).  The
 // status is read by the caller (ST_RATTLE_FAIL).
-void integ_rattle_launch() {
+void integ_rattle_launch(bool tags) {
   if (g.ntcons <= 0) return;
   cudaStream_t st = g.stream;
   GB_CUDA(cudaMemsetAsync(d_flags, 0, sizeof(int) * (g.p.shake_maxit + CL_CHUNK + 2), st));
   ConArgs A;
   con_args(A);
+  if (tags && !cl_small) integ_con_tags();
+  A.tags = tags;
   prof_begin(P_RATTLE);
   if (cl_small) {
     launch_small<true>(A, 0.0);
@@ -1217,8 +1305,8 @@ void integ_vv(int stage, double* strkin, double* engke, int* iters, double* virc
   const int n = g.natms;
   const double tstep = g.p.tstep, hstep = 0.5 * tstep;
   if (iters) *iters = 0;
-  integ_con_tags();
   if (stage == 1) {
+    integ_con_tags();
     prof_begin(P_VV);
     if (!thermo_vv1(hstep, tstep)) {
       k_vv1<<<nblocks(n, 256), 256, 0, st>>>(n, g.hdw, tstep, g.fx, g.fy, g.fz, g.vx, g.vy, g.vz, g.x, g.y, g.z);
@@ -1235,7 +1323,7 @@ void integ_vv(int stage, double* strkin, double* engke, int* iters, double* virc
     }
     if (fused) launch_kinstress(true);
     prof_end(P_VV);
-    integ_rattle_launch();
+    integ_rattle_launch(true);
     if (!thermo_vv2_finish(strkin, engke)) {
       if (!fused) launch_kinstress(false);
       if (g.defer_scalars) return;  // the MD loop reads the sums after its last step
