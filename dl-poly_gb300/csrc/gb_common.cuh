@@ -145,7 +145,7 @@ struct Dev {
   int* which_cell = nullptr;   // mxatms
   int* cell_count = nullptr;   // ncells+2
   int* cell_start = nullptr;   // ncells+2 (0-based start)
-  int* cell_fill = nullptr;    // ncells+2
+  int* cell_lstart = nullptr;  // ncells+2: local atoms in the cells before
   int* at_list = nullptr;      // mxatms (sorted atom ids)
   int* sorted_pos = nullptr;   // mxatms: position of atom in at_list
   double4_32a* xs = nullptr;       // mxatms sorted FP64 coordinates (x,y,z,pad)

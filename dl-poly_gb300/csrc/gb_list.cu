@@ -52,7 +52,7 @@ struct CellGeom {
 HaloGeom h_halo;
 CellGeom h_cg;
 double h_add[6][3];  // export add vectors for mdir -1,1,-2,2,-3,3
-int h_halo_blocks = 0;  // blocks of k_halo_build (GB_HALO_BLOCKS; 0: by size)
+int h_halo_blocks = 0;  // blocks of k_halo_count and k_halo_write (GB_HALO_BLOCKS; 0: by size)
 
 // ---------------------------------------------------------------- kernels
 // The reduced coordinate rc(d) x + rc(d+3) y + rc(d+6) z of the reference: gb_init takes
@@ -65,37 +65,35 @@ __device__ __forceinline__ long long ordered(double v) {
   return b ^ ((b >> 63) & 0x7fffffffffffffffll);
 }
 
-__device__ __forceinline__ bool export_sel(int v, int kx, int ky, int kz, int jxyz) {
-  if (v <= 0) return false;
-  int ix = v % 10;
-  int iy = (v - ix) % 100;
-  int iz = (v - (ix + iy)) % 1000;
-  int j = ix * kx + iy * ky + iz * kz;
-  return (j == jxyz) || (j > jxyz && j % 3 == 0);
-}
-
-
 // relocate_particles (pbcshift, numerics.F90:1886-1930), set_halo_particles (halo.F90:153-356)
-// and vnl_set_check (neighbours.F90:305-343) in one cooperative launch.  The images come
+// and vnl_set_check (neighbours.F90:305-343) in two launches.  The reference's images come
 // from six ordered exports (-x, +x, -y, +y, -z, +z), each a stable compaction of the atoms
-// and images so far: every block counts its run of them, a grid barrier, every block sums
-// the counts before its own and writes its images, a grid barrier.  The work is a few
-// microseconds; as 28 launches (count, scan, commit and write per export, and the passes
-// around them) it took 0.19 ms at 1,536 atoms and 0.21 ms at 175,616, latency of the
-// launches and of their serial loops; now 0.051 and 0.098 ms, latency of the 12 barriers
-// and of the dependent loads between them.
-constexpr int HALO_NT = 512, HALO_NK = 8;
+// and images so far, and an image is not exported again along its own dimension.  So an
+// image is an atom and a class, ox + 3 oy + 9 oz with o = 0 (not exported), 1 (-) or 2 (+)
+// per dimension, an atom has the classes that its three 2-bit codes allow, and the images
+// stand in the order of their class, then of their atom.  One launch wraps the atoms and counts
+// each class per block, the next sums the counts before its own and writes the images.
+// As six compactions between the barriers of one cooperative kernel it took 0.055 ms at
+// 4,096 atoms; the two launches take 0.016, latency of the dependent loads.
+constexpr int HALO_NT = 256, HALO_NC = 27;
 struct HaloArgs {
   int n, mxatms;
   double *x, *y, *z, *xb, *yb, *zb;
   double a[3], c[3], half_minus;   // 1/L and L per dimension
   HaloGeom hg;
   double add[6][3];
-  int *ixyz, *src, *shcode, *ltg, *ltype, *lfrzn;
+  int *code, *src, *shcode, *ltg, *ltype, *lfrzn;
   double *chge, *weight;
-  int* cnt;                        // one count per block and export
+  int* cnt;                        // [HALO_NC][blocks]
   DevScalars* sc;
 };
+
+// code: the 2-bit codes of x, y, z (bit 0: exported by -, bit 1: by +)
+__device__ __forceinline__ bool has_class(int code, int c) {
+  const int ox = c % 3, oy = (c / 3) % 3, oz = c / 9;
+  return (ox == 0 || (code >> (ox - 1)) & 1) && (oy == 0 || (code >> (oy + 1)) & 1) &&
+         (oz == 0 || (code >> (oz + 3)) & 1);
+}
 
 __device__ __forceinline__ double wrap1(double x, double a, double c, double half_minus) {
   double s = mul_rn(a, x);
@@ -107,160 +105,177 @@ __device__ __forceinline__ double wrap1(double x, double a, double c, double hal
   return mul_rn(c, s);
 }
 
-__global__ void __launch_bounds__(HALO_NT) k_halo_build(HaloArgs A) {
-  cg::grid_group grid = cg::this_grid();
-  const int nth = gridDim.x * blockDim.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  constexpr int NW = HALO_NT / 32, NK = HALO_NK;
-  __shared__ int s_w[NK * NW], s_tot[2];  // selected per sub-run of 512 and warp, then their exclusive sums
+__global__ void __launch_bounds__(HALO_NT) k_halo_count(HaloArgs A) {
+  __shared__ int s_cnt[HALO_NC];
+  const int lane = threadIdx.x & 31;
   long long lo_b[3], hi_b[3];
   for (int d = 0; d < 3; ++d) { lo_b[d] = ordered(A.hg.ecw[d]); hi_b[d] = ordered(A.hg.cw[d]); }
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < A.n; i += nth) {
-    const double x = wrap1(A.x[i], A.a[0], A.c[0], A.half_minus), y = wrap1(A.y[i], A.a[1], A.c[1], A.half_minus),
-                 z = wrap1(A.z[i], A.a[2], A.c[2], A.half_minus);
-    A.x[i] = x; A.y[i] = y; A.z[i] = z;
-    A.xb[i] = x; A.yb[i] = y; A.zb[i] = z;
-    const long long xx = ordered(red_coord(A.hg.rc, 0, x)), yy = ordered(red_coord(A.hg.rc, 1, y)),
-                    zz = ordered(red_coord(A.hg.rc, 2, z));
+  if (threadIdx.x < HALO_NC) s_cnt[threadIdx.x] = 0;
+  __syncthreads();
+  const int per = (A.n + gridDim.x - 1) / gridDim.x;
+  const int lo = min(A.n, (int)blockIdx.x * per), hi = min(A.n, lo + per);
+  int cnt = 0;  // lane c: class c
+  for (int i0 = lo; i0 < hi; i0 += HALO_NT) {
+    const int i = i0 + threadIdx.x;
     int v = 0;
-    if (xx <= lo_b[0]) v += 1;
-    if (xx >= hi_b[0]) v += 2;
-    if (yy <= lo_b[1]) v += 10;
-    if (yy >= hi_b[1]) v += 20;
-    if (zz <= lo_b[2]) v += 100;
-    if (zz >= hi_b[2]) v += 200;
-    A.ixyz[i] = v;
-    A.src[i] = i;
-    A.shcode[i] = 13;
+    if (i < hi) {
+      const double x = wrap1(A.x[i], A.a[0], A.c[0], A.half_minus), y = wrap1(A.y[i], A.a[1], A.c[1], A.half_minus),
+                   z = wrap1(A.z[i], A.a[2], A.c[2], A.half_minus);
+      A.x[i] = x; A.y[i] = y; A.z[i] = z;
+      A.xb[i] = x; A.yb[i] = y; A.zb[i] = z;
+      const long long xx = ordered(red_coord(A.hg.rc, 0, x)), yy = ordered(red_coord(A.hg.rc, 1, y)),
+                      zz = ordered(red_coord(A.hg.rc, 2, z));
+      v = (xx <= lo_b[0] ? 1 : 0) | (xx >= hi_b[0] ? 2 : 0) | (yy <= lo_b[1] ? 4 : 0) | (yy >= hi_b[1] ? 8 : 0) |
+          (zz <= lo_b[2] ? 16 : 0) | (zz >= hi_b[2] ? 32 : 0);
+      A.code[i] = v;
+      A.src[i] = i;
+      A.shcode[i] = 13;
+    }
+    if (!__any_sync(0xffffffffu, v != 0)) continue;
+#pragma unroll
+    for (int c = 1; c < HALO_NC; ++c) {
+      const int k = __popc(__ballot_sync(0xffffffffu, has_class(v, c)));
+      if (lane == c) cnt += k;
+    }
   }
-  grid.sync();
-  int n = A.n;
-  bool over = false;
-  for (int m = 0; m < 6; ++m) {
-    const int kx = m < 2 ? 1 : 0, ky = (m >> 1) == 1 ? 1 : 0, kz = m >= 4 ? 1 : 0;
-    const int unit = m < 2 ? 1 : m < 4 ? 10 : 100, jxyz = (m & 1) ? 2 * unit : unit, kxyz = 3 * unit;
-    const int dshift = (m & 1 ? -1 : 1) * (m < 2 ? 1 : m < 4 ? 3 : 9);
-    // this block's run of the atoms and images so far, NK x 512 of them at a time
-    const int per = (n + gridDim.x - 1) / gridDim.x;
-    const int lo = min(n, (int)blockIdx.x * per), hi = min(n, lo + per);
-    const bool once = per <= NK * HALO_NT;
-    int v[NK];
-    unsigned bal[NK];
-    auto look = [&](int i0) {
+  if (lane < HALO_NC && cnt) atomicAdd(&s_cnt[lane], cnt);
+  __syncthreads();
+  if (threadIdx.x < HALO_NC) A.cnt[threadIdx.x * gridDim.x + blockIdx.x] = s_cnt[threadIdx.x];
+}
+
+__global__ void __launch_bounds__(HALO_NT) k_halo_write(HaloArgs A) {
+  constexpr int NW = HALO_NT / 32;
+  __shared__ int s_before[HALO_NC], s_all[HALO_NC], s_w[NW][32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nb = gridDim.x;
+  for (int c = 1 + wid; c < HALO_NC; c += NW) {  // images of the class before this block's, and all of them
+    int before = 0, all = 0;
+    for (int b = lane; b < nb; b += 32) {
+      const int k = A.cnt[c * nb + b];
+      all += k;
+      before += b < (int)blockIdx.x ? k : 0;
+    }
+    before = __reduce_add_sync(0xffffffffu, before);
+    all = __reduce_add_sync(0xffffffffu, all);
+    if (lane == 0) { s_before[c] = before; s_all[c] = all; }
+  }
+  __syncthreads();
+  const bool cls = lane >= 1 && lane < HALO_NC;
+  const int all = cls ? s_all[lane] : 0;
+  int inc = all;
 #pragma unroll
-      for (int k = 0; k < NK; ++k) {
-        const int i = i0 + k * HALO_NT + threadIdx.x;
-        v[k] = i < hi ? A.ixyz[i] : 0;
-      }
-#pragma unroll
-      for (int k = 0; k < NK; ++k) bal[k] = __ballot_sync(0xffffffffu, export_sel(v[k], kx, ky, kz, jxyz));
-    };
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += u;
+  }
+  int base = A.n + (inc - all) + (cls ? s_before[lane] : 0);  // lane c: place of the next image of class c
+  if (blockIdx.x == 0 && threadIdx.x == 31) {  // images beyond mxatms are neither written nor counted
+    const int nlast = min(A.n + inc, A.mxatms);
+    A.sc->nlast = nlast;
+    A.sc->nlast_prev = nlast;
+    if (A.n + inc > A.mxatms) A.sc->status |= ST_HALO_OVERFLOW;
+  }
+  const int per = (A.n + nb - 1) / nb;
+  const int lo = min(A.n, (int)blockIdx.x * per), hi = min(A.n, lo + per);
+  for (int i0 = lo; i0 < hi; i0 += HALO_NT) {
+    const int i = i0 + threadIdx.x;
+    const int v = i < hi ? A.code[i] : 0;
+    unsigned present = 0;  // classes that an atom of the warp has
     int cnt = 0;
-    for (int i0 = lo; i0 < hi; i0 += NK * HALO_NT) {
-      look(i0);
+    if (__any_sync(0xffffffffu, v != 0)) {
 #pragma unroll
-      for (int k = 0; k < NK; ++k) cnt += __popc(bal[k]);
-    }
-    if (lane == 0) s_w[wid] = cnt;
-    __syncthreads();
-    if (wid == 0) {
-      const int s = __reduce_add_sync(0xffffffffu, lane < NW ? s_w[lane] : 0);
-      if (lane == 0) A.cnt[m * gridDim.x + blockIdx.x] = s;
-    }
-    grid.sync();
-    if (wid == 0) {  // images before this block's, and all of them
-      int before = 0, all = 0;
-      for (int b = lane; b < (int)gridDim.x; b += 32) {
-        const int c = __ldcg(&A.cnt[m * gridDim.x + b]);
-        all += c;
-        before += b < (int)blockIdx.x ? c : 0;
+      for (int c = 1; c < HALO_NC; ++c) {
+        const int k = __popc(__ballot_sync(0xffffffffu, has_class(v, c)));
+        if (lane == c) cnt = k;
       }
-      before = __reduce_add_sync(0xffffffffu, before);
-      all = __reduce_add_sync(0xffffffffu, all);
-      if (lane == 0) { s_tot[0] = before; s_tot[1] = all; }
+      present = __ballot_sync(0xffffffffu, cnt != 0);
+    }
+    s_w[wid][lane] = cnt;
+    __syncthreads();
+    int pre = base;
+    for (int w = 0; w < NW; ++w) {
+      const int k = s_w[w][lane];
+      if (w < wid) pre += k;
+      base += k;
     }
     __syncthreads();
-    int base = n + s_tot[0];
-    const int all = s_tot[1];
-    for (int i0 = lo; i0 < hi; i0 += NK * HALO_NT) {
-      if (!once) look(i0);
-      if (lane == 0) {
-#pragma unroll
-        for (int k = 0; k < NK; ++k) s_w[k * NW + wid] = __popc(bal[k]);
-      }
-      __syncthreads();
-      if (wid == 0) {  // exclusive sums over the NK x NW counts, NK * NW / 32 per lane
-        constexpr int PL = NK * NW / 32;
-        int c[PL], s = 0;
-#pragma unroll
-        for (int e = 0; e < PL; ++e) { c[e] = s_w[lane * PL + e]; s += c[e]; }
-        int inc = s;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int u = __shfl_up_sync(0xffffffffu, inc, o);
-          if (lane >= o) inc += u;
-        }
-        if (lane == 31) s_tot[0] = inc;
-        int run = inc - s;
-#pragma unroll
-        for (int e = 0; e < PL; ++e) { s_w[lane * PL + e] = run; run += c[e]; }
-      }
-      __syncthreads();
-#pragma unroll
-      for (int k = 0; k < NK; ++k) {
-        const int dst = base + s_w[k * NW + wid] + __popc(bal[k] & ((1u << lane) - 1u));
-        if (((bal[k] >> lane) & 1u) && dst < A.mxatms) {
-          const int i = i0 + k * HALO_NT + threadIdx.x, s = A.src[i];
-          A.x[dst] = add_rn(A.x[i], A.add[m][0]);
-          A.y[dst] = add_rn(A.y[i], A.add[m][1]);
-          A.z[dst] = add_rn(A.z[i], A.add[m][2]);
-          A.src[dst] = s;
-          A.shcode[dst] = A.shcode[i] + dshift;
-          const int ix = v[k] % 10, iy = (v[k] - ix) % 100, iz = (v[k] - (ix + iy)) % 1000;
-          const int j = ix * kx + iy * ky + iz * kz;
-          A.ixyz[dst] = v[k] - (j == jxyz ? jxyz : kxyz);
-          // the source atom's properties
-          A.ltg[dst] = A.ltg[s];
-          A.ltype[dst] = A.ltype[s];
-          A.chge[dst] = A.chge[s];
-          A.weight[dst] = A.weight[s];
-          A.lfrzn[dst] = A.lfrzn[s];
-        }
-      }
-      base += s_tot[0];
-      __syncthreads();
+    if (!present) continue;
+    double x = 0.0, y = 0.0, z = 0.0, q = 0.0, wt = 0.0;
+    int tg = 0, ty = 0, fr = 0;
+    if (v) {
+      x = A.x[i]; y = A.y[i]; z = A.z[i];
+      q = A.chge[i]; wt = A.weight[i];
+      tg = A.ltg[i]; ty = A.ltype[i]; fr = A.lfrzn[i];
     }
-    // images beyond mxatms are neither written nor counted
-    if (all > A.mxatms - n) { over = true; n = A.mxatms; }
-    else n += all;
-    if (m < 5) grid.sync();
-  }
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    A.sc->nlast = n;
-    A.sc->nlast_prev = n;
-    if (over) A.sc->status |= ST_HALO_OVERFLOW;
+    for (unsigned m = present; m; m &= m - 1) {
+      const int c = __ffs((int)m) - 1;
+      const bool on = has_class(v, c);
+      const unsigned bal = __ballot_sync(0xffffffffu, on);
+      const int dst = __shfl_sync(0xffffffffu, pre, c) + __popc(bal & ((1u << lane) - 1u));
+      if (!on || dst >= A.mxatms) continue;
+      const int o[3] = {c % 3, (c / 3) % 3, c / 9};
+      double xi = x, yi = y, zi = z;
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        if (o[d] == 0) continue;
+        const double* ad = A.add[2 * d + o[d] - 1];
+        xi = add_rn(xi, ad[0]); yi = add_rn(yi, ad[1]); zi = add_rn(zi, ad[2]);
+      }
+      A.x[dst] = xi; A.y[dst] = yi; A.z[dst] = zi;
+      A.src[dst] = i;
+      A.shcode[dst] = 13 + (o[0] == 0 ? 0 : o[0] == 1 ? 1 : -1) + (o[1] == 0 ? 0 : o[1] == 1 ? 3 : -3) +
+                      (o[2] == 0 ? 0 : o[2] == 1 ? 9 : -9);
+      A.ltg[dst] = tg;
+      A.ltype[dst] = ty;
+      A.chge[dst] = q;
+      A.weight[dst] = wt;
+      A.lfrzn[dst] = fr;
+    }
   }
 }
 
-// Exclusive scan of n ints in a single block (n up to a few million).
-__global__ void k_scan_single(const int* in, int* out, int n, int* total) {
-  __shared__ int part[1024];
-  const int T = blockDim.x;
-  const int per = (n + T - 1) / T;
-  const int b = threadIdx.x * per;
-  int s = 0;
-  for (int k = 0; k < per; ++k) if (b + k < n) s += in[b + k];
-  part[threadIdx.x] = s;
-  __syncthreads();
-  for (int o = 1; o < T; o <<= 1) {
-    int v = threadIdx.x >= o ? part[threadIdx.x - o] : 0;
-    __syncthreads();
-    part[threadIdx.x] += v;
-    __syncthreads();
+// Exclusive scan of the cells' counts (block 0: all cells, into start; block 1: the domain's
+// cells, which hold the local atoms, into lstart) and the zeros that the list's kernels
+// count from.  A warp takes 1/32 of the cells, 32 at a time.
+__global__ void __launch_bounds__(1024) k_cell_scan(int n, CellGeom cg, const int* __restrict__ count, int* start,
+                                                    int* lstart, DevScalars* sc) {
+  __shared__ int s_w[32];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    sc->ibig = 0;
+    sc->tile_over = sc->tile_max = sc->halo_fwd = sc->halo_bwd = 0;
   }
-  int run = part[threadIdx.x] - s;
-  for (int k = 0; k < per; ++k)
-    if (b + k < n) { out[b + k] = run; run += in[b + k]; }
-  if (threadIdx.x == T - 1 && total) *total = part[T - 1];
+  const bool local = blockIdx.x == 1;
+  const int per = ((n + 1023) / 1024) * 32, lo = min(n, wid * per), hi = min(n, lo + per);
+  auto get = [&](int c) {
+    if (c >= hi) return 0;
+    if (local) {
+      const int a = c - 1, iz = a / (cg.NX * cg.NY), iy = a / cg.NX - cg.NY * iz, ix = a % cg.NX;
+      if (a < 0 || ix < cg.nlp || ix >= cg.nlp + cg.nlx || iy < cg.nlp || iy >= cg.nlp + cg.nly || iz < cg.nlp ||
+          iz >= cg.nlp + cg.nlz)
+        return 0;
+    }
+    return count[c];
+  };
+  int t = 0;
+#pragma unroll 4
+  for (int b = lo; b < hi; b += 32) t += get(b + lane);
+  t = __reduce_add_sync(0xffffffffu, t);
+  if (lane == 0) s_w[wid] = t;
+  __syncthreads();
+  int run = __reduce_add_sync(0xffffffffu, lane < wid ? s_w[lane] : 0);
+  int* out = local ? lstart : start;
+#pragma unroll 4
+  for (int b = lo; b < hi; b += 32) {
+    const int k = get(b + lane);
+    int inc = k;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, inc, o);
+      if (lane >= o) inc += u;
+    }
+    if (b + lane < hi) out[b + lane] = run + inc - k;
+    run += __shfl_sync(0xffffffffu, inc, 31);
+  }
 }
 
 // refresh_halo_positions: the same export chain applied to the source position
@@ -339,33 +354,54 @@ __global__ void k_bin(int natms, const DevScalars* sc, const double* x, const do
   atomicAdd(&count[icell], 1);
 }
 
-__global__ void k_cell_scatter(const DevScalars* sc, const int* which_cell, const int* start, int* fill,
+// (counts the cells back down to zero, for the next build)
+__global__ void k_cell_scatter(const DevScalars* sc, const int* which_cell, const int* start, int* count,
                                int* tmp) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= sc->nlast) return;
   int c = which_cell[i];
-  int slot = atomicAdd(&fill[c], 1);
+  int slot = atomicSub(&count[c], 1) - 1;
   tmp[start[c] + slot] = i;
 }
 
+__device__ __forceinline__ void tile_row(int t, const TilePlan& tp, const CellGeom& cg, const int* __restrict__ start,
+                                         int* __restrict__ tile_rows, int* __restrict__ tile_info, int cap,
+                                         int* __restrict__ tile_over, DevScalars* sc);
+
 // Stable order inside each cell (ascending atom index, as the reference's
-// counting sort over i = 1..nlast): rank of each member by counting.
-__global__ void k_cell_sort(int ncells_p1, const int* start, const int* tmp, int* at_list, int* sorted_pos,
-                            const double* x, const double* y, const double* z, double4_32a* xs, float4* xsf) {
-  int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  int lane = threadIdx.x & 31;
-  if (warp >= ncells_p1) return;
-  int s = start[warp], e = start[warp + 1], n = e - s;
-  if (warp == 0) {  // residual halo cell: never a neighbour cell, order irrelevant
-    for (int a = lane; a < n; a += 32) {
-      int v = tmp[s + a];
-      at_list[s + a] = v;
-      sorted_pos[v] = s + a;
-      xs[s + a] = make_double4_32a(x[v], y[v], z[v], 0.0);
-      xsf[s + a] = make_float4((float)x[v], (float)y[v], (float)z[v], 0.0f);
+// counting sort over i = 1..nlast): rank of each member by counting.  A local atom's
+// sorted position goes to loc_sp too, in sorted order (a domain cell holds local atoms only).
+// The blocks after the cells' take the residual halo cell (one warp took 0.065 ms for it
+// where it is large: 6,591-atom water; 0.006 so), the blocks after those the tiles' rows.
+constexpr int SORT_NT = 256, RESID_BLOCKS = 32;
+__global__ void __launch_bounds__(SORT_NT) k_cell_sort(int ncells_p1, int natms, const int* start, const int* lstart,
+                                                       const int* tmp, int* at_list, int* sorted_pos, int* loc_sp,
+                                                       const double* x, const double* y, const double* z,
+                                                       double4_32a* xs, float4* xsf, TilePlan tp, CellGeom cg,
+                                                       int* tile_rows, int* tile_info, int cap, int* tile_over,
+                                                       DevScalars* sc) {
+  const int ncb = (ncells_p1 + SORT_NT / 32 - 1) / (SORT_NT / 32);
+  if ((int)blockIdx.x >= ncb) {
+    const int rb = blockIdx.x - ncb;
+    if (rb >= RESID_BLOCKS) {
+      tile_row((rb - RESID_BLOCKS) * SORT_NT + threadIdx.x, tp, cg, start, tile_rows, tile_info, cap, tile_over, sc);
+      return;
+    }
+    // residual halo cell: never a neighbour cell, order irrelevant
+    const int s = start[0], e = start[1];
+    for (int a = s + rb * SORT_NT + threadIdx.x; a < e; a += RESID_BLOCKS * SORT_NT) {
+      const int v = tmp[a];
+      at_list[a] = v;
+      sorted_pos[v] = a;
+      const double xv = x[v], yv = y[v], zv = z[v];
+      xs[a] = make_double4_32a(xv, yv, zv, 0.0);
+      xsf[a] = make_float4((float)xv, (float)yv, (float)zv, 0.0f);
     }
     return;
   }
+  const int cell = (blockIdx.x * SORT_NT + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (cell >= ncells_p1 || cell == 0) return;
+  const int s = start[cell], n = start[cell + 1] - s, ls = lstart[cell];
   for (int a = lane; a < n; a += 32) {
     int v = tmp[s + a];
     int r = 0;
@@ -373,6 +409,7 @@ __global__ void k_cell_sort(int ncells_p1, const int* start, const int* tmp, int
     int pos = s + r;
     at_list[pos] = v;
     sorted_pos[v] = pos;
+    if (v < natms) loc_sp[ls + r] = pos;
     double xv = x[v], yv = y[v], zv = z[v];
     xs[pos] = make_double4_32a(xv, yv, zv, 0.0);
     xsf[pos] = make_float4((float)xv, (float)yv, (float)zv, 0.0f);
@@ -492,9 +529,9 @@ __global__ void __launch_bounds__(256) k_list_pairs(int natms, const DevScalars*
 // of cells and its slot base in the tile's staged set; per tile the staged total and the
 // sorted-position range of its own (i) atoms.  Tiles above the capacity of the first
 // launches go to tile_over for a second launch with more shared memory.
-__global__ void k_tile_rows(TilePlan tp, CellGeom cg, const int* __restrict__ start, int* __restrict__ tile_rows,
-                            int* __restrict__ tile_info, int cap, int* __restrict__ tile_over, DevScalars* sc) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void tile_row(int t, const TilePlan& tp, const CellGeom& cg, const int* __restrict__ start,
+                                         int* __restrict__ tile_rows, int* __restrict__ tile_info, int cap,
+                                         int* __restrict__ tile_over, DevScalars* sc) {
   if (t >= tp.ntiles) return;
   const int tx = t % tp.ntx, ty = (t / tp.ntx) % tp.nty, tz = t / (tp.ntx * tp.nty);
   const int nlp = cg.nlp;
@@ -516,6 +553,11 @@ __global__ void k_tile_rows(TilePlan tp, CellGeom cg, const int* __restrict__ st
   tile_info[4 * t + 3] = 0;
   if (base > cap) tile_over[atomicAdd(&sc->tile_over, 1)] = t;
   atomicMax(&sc->tile_max, base);
+}
+
+__global__ void k_tile_rows(TilePlan tp, CellGeom cg, const int* __restrict__ start, int* __restrict__ tile_rows,
+                            int* __restrict__ tile_info, int cap, int* __restrict__ tile_over, DevScalars* sc) {
+  tile_row(blockIdx.x * blockDim.x + threadIdx.x, tp, cg, start, tile_rows, tile_info, cap, tile_over, sc);
 }
 
 // Half-shell Verlet list (neighbours.F90:876-1184), one CTA per cell tile: the tile's
@@ -1004,10 +1046,11 @@ void list_setup() {
   h_cg.rcsq_hi = (float)(h_cg.rcsq + band);
   h_cg.half_plus = std::nextafter(0.5, 1.0);
   if (g.cells_alloc < g.ncells + 2) {
-    cudaFree(g.cell_count); cudaFree(g.cell_start); cudaFree(g.cell_fill);
+    cudaFree(g.cell_count); cudaFree(g.cell_start); cudaFree(g.cell_lstart);
     GB_CUDA(cudaMalloc(&g.cell_count, sizeof(int) * (g.ncells + 2)));
     GB_CUDA(cudaMalloc(&g.cell_start, sizeof(int) * (g.ncells + 2)));
-    GB_CUDA(cudaMalloc(&g.cell_fill, sizeof(int) * (g.ncells + 2)));
+    GB_CUDA(cudaMalloc(&g.cell_lstart, sizeof(int) * (g.ncells + 2)));
+    GB_CUDA(cudaMemset(g.cell_count, 0, sizeof(int) * (g.ncells + 2)));
     g.cells_alloc = g.ncells + 2;
   }
 }
@@ -1027,14 +1070,14 @@ int list_relocate_and_halo(bool wait) {
   A.half_minus = std::nextafter(0.5, 0.0);
   A.hg = h_halo;
   std::memcpy(A.add, h_add, sizeof(h_add));
-  A.ixyz = g.ixyz; A.src = g.src; A.shcode = g.shcode; A.ltg = g.ltg; A.ltype = g.ltype; A.lfrzn = g.lfrzn;
+  A.code = g.ixyz; A.src = g.src; A.shcode = g.shcode; A.ltg = g.ltg; A.ltype = g.ltype; A.lfrzn = g.lfrzn;
   A.chge = g.chge; A.weight = g.weight;
   A.sc = g.sc;
-  // one resident block per SM at most; a small box has several images per atom
-  const int nb = std::max(1, std::min(h_halo_blocks ? h_halo_blocks : nblocks(g.mxatms, HALO_NT), g.nsm));
-  A.cnt = gb_scan_scratch(6 * nb);
-  void* args[] = {&A};
-  GB_CUDA(cudaLaunchCooperativeKernel((void*)k_halo_build, nb, HALO_NT, args, 0, g.stream));
+  const int nb = std::max(1, h_halo_blocks ? h_halo_blocks : std::min(nblocks(n, HALO_NT), 2 * g.nsm));
+  A.cnt = gb_scan_scratch(HALO_NC * nb);
+  k_halo_count<<<nb, HALO_NT, 0, g.stream>>>(A);
+  GB_LAUNCHED();
+  k_halo_write<<<nb, HALO_NT, 0, g.stream>>>(A);
   GB_LAUNCHED();
   prof_end(P_HALO);
   if (!wait) return GB_OK;  // list_build, which follows, reports ST_HALO_OVERFLOW
@@ -1062,71 +1105,26 @@ int list_refresh_halo() {
   return GB_OK;
 }
 
-// The sorted positions of the local atoms, in sorted (cell) order: loc_sp[0, natms).  Per
-// block of 1024 positions a count, then (after a scan of the counts) each block's local
-// positions at its offset, ranked by a ballot prefix within each warp.
-constexpr int LOC_NT = 1024;
-__global__ void __launch_bounds__(LOC_NT) k_local_count(int natms, int mx, const DevScalars* sc,
-                                                        const int* __restrict__ at_list, int* blkcount) {
-  __shared__ int s[LOC_NT / 32];
-  const int p = blockIdx.x * LOC_NT + threadIdx.x;
-  const bool loc = p < min(sc->nlast, mx) && at_list[p] < natms;
-  const unsigned b = __ballot_sync(0xffffffffu, loc);
-  if ((threadIdx.x & 31) == 0) s[threadIdx.x >> 5] = __popc(b);
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int t = 0;
-    for (int w = 0; w < LOC_NT / 32; ++w) t += s[w];
-    blkcount[blockIdx.x] = t;
-  }
-}
-
-__global__ void __launch_bounds__(LOC_NT) k_local_scatter(int natms, int mx, const DevScalars* sc,
-                                                          const int* __restrict__ at_list,
-                                                          const int* __restrict__ blkoff, int* loc_sp) {
-  __shared__ int s[LOC_NT / 32];
-  const int p = blockIdx.x * LOC_NT + threadIdx.x, lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-  const bool loc = p < min(sc->nlast, mx) && at_list[p] < natms;
-  const unsigned b = __ballot_sync(0xffffffffu, loc);
-  if (lane == 0) s[w] = __popc(b);
-  __syncthreads();
-  int before = 0;
-  for (int k = 0; k < w; ++k) before += s[k];
-  const int r = blkoff[blockIdx.x] + before + __popc(b & ((1u << lane) - 1u));
-  if (loc && r < natms) loc_sp[r] = p;
-}
-
 int list_build() {
   const int T = 256;
   cudaStream_t st = g.stream;
   const int mx = g.mxatms;
-  GB_CUDA(cudaMemsetAsync(g.cell_count, 0, sizeof(int) * (g.ncells + 2), st));
-  GB_CUDA(cudaMemsetAsync(g.cell_fill, 0, sizeof(int) * (g.ncells + 2), st));
+  const TilePlan& tp = g.tp;
+  const int cap = g.tile_cap_list;
   prof_begin(P_BIN);
   k_bin<<<nblocks(mx, T), T, 0, st>>>(g.natms, g.sc, g.x, g.y, g.z, h_cg, g.which_cell, g.cell_count);
   GB_LAUNCHED();
-  k_scan_single<<<1, 1024, 0, st>>>(g.cell_count, g.cell_start, g.ncells + 2, nullptr);
+  k_cell_scan<<<2, 1024, 0, st>>>(g.ncells + 2, h_cg, g.cell_count, g.cell_start, g.cell_lstart, g.sc);
   GB_LAUNCHED();
   int* tmp = gb_scan_scratch(mx + 1);
-  k_cell_scatter<<<nblocks(mx, T), T, 0, st>>>(g.sc, g.which_cell, g.cell_start, g.cell_fill, tmp);
+  k_cell_scatter<<<nblocks(mx, T), T, 0, st>>>(g.sc, g.which_cell, g.cell_start, g.cell_count, tmp);
   GB_LAUNCHED();
-  k_cell_sort<<<nblocks((long long)(g.ncells + 1) * 32, T), T, 0, st>>>(g.ncells + 1, g.cell_start, tmp, g.at_list,
-                                                                       g.sorted_pos, g.x, g.y, g.z, g.xs, g.xsf);
+  k_cell_sort<<<nblocks(g.ncells + 1, SORT_NT / 32) + RESID_BLOCKS + nblocks(tp.ntiles, SORT_NT), SORT_NT, 0, st>>>(
+      g.ncells + 1, g.natms, g.cell_start, g.cell_lstart, tmp, g.at_list, g.sorted_pos, g.loc_sp, g.x, g.y, g.z, g.xs,
+      g.xsf, tp, h_cg, g.tile_rows, g.tile_info, cap, g.tile_over, g.sc);
   GB_LAUNCHED();
-  {
-    const int nb = nblocks(mx, LOC_NT);
-    int* cnt = gb_scan_scratch(2 * nb + 2);
-    k_local_count<<<nb, LOC_NT, 0, st>>>(g.natms, mx, g.sc, g.at_list, cnt);
-    GB_LAUNCHED();
-    k_scan_single<<<1, 1024, 0, st>>>(cnt, cnt + nb + 1, nb, nullptr);
-    GB_LAUNCHED();
-    k_local_scatter<<<nb, LOC_NT, 0, st>>>(g.natms, mx, g.sc, g.at_list, cnt + nb + 1, g.loc_sp);
-    GB_LAUNCHED();
-  }
   prof_end(P_BIN);
   prof_begin(P_LIST);
-  const TilePlan& tp = g.tp;
-  const int cap = g.tile_cap_list;
   // few tiles: several CTAs share a tile's atoms (each stages its whole shell), so that
   // the device has about three CTAs per SM
   const int split = std::max(1, std::min(8, 3 * g.nsm / std::max(tp.ntiles, 1)));
@@ -1134,12 +1132,14 @@ int list_build() {
   // The host waits once, after the last kernel, unless the previous build had tiles above
   // the first launch's capacity: then it looks before the second launch.  The first build
   // that meets such tiles runs its kernels again with that launch.
-  for (;;) {
-    GB_CUDA(cudaMemsetAsync(&g.sc->ibig, 0, sizeof(int), st));
-    GB_CUDA(cudaMemsetAsync(&g.sc->tile_over, 0, 4 * sizeof(int), st));  // tile_over, tile_max, halo_fwd, halo_bwd
-    k_tile_rows<<<nblocks(tp.ntiles, 128), 128, 0, st>>>(tp, h_cg, g.cell_start, g.tile_rows, g.tile_info, cap,
-                                                          g.tile_over, g.sc);
-    GB_LAUNCHED();
+  for (bool again = false;; again = true) {
+    if (again) {
+      GB_CUDA(cudaMemsetAsync(&g.sc->ibig, 0, sizeof(int), st));
+      GB_CUDA(cudaMemsetAsync(&g.sc->tile_over, 0, 4 * sizeof(int), st));  // tile_over, tile_max, halo_fwd, halo_bwd
+      k_tile_rows<<<nblocks(tp.ntiles, 128), 128, 0, st>>>(tp, h_cg, g.cell_start, g.tile_rows, g.tile_info, cap,
+                                                            g.tile_over, g.sc);
+      GB_LAUNCHED();
+    }
     k_list_tiles<<<dim3(tp.ntiles, split), 256, (size_t)cap * 20, st>>>(
         g.natms, h_cg, tp, g.nsbcll, g.nseg, nullptr, cap, g.tile_rows, g.tile_info, g.at_list, g.which_cell,
         g.cell_start, g.xs, g.xsf, g.list, g.ld, g.spos, g.ldt, g.p.max_list, g.sc);
