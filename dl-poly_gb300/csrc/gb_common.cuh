@@ -33,7 +33,7 @@ struct DevScalars {
   int nlast;        // local + halo atoms
   int nlast_prev;   // the same, as the last relocation left it
   int ibig;         // largest list length seen (overflow report)
-  unsigned count;   // blocks done, for grid_sum on the first stream (0 between launches)
+  unsigned count;   // blocks done, for grid_finish on the first stream (0 between launches)
   int status;       // ST_* bits
   int update;       // vnl_check decision
   double maxdisp;   // bits of the largest squared displacement since the last rebuild
@@ -45,7 +45,7 @@ struct DevScalars {
   int tile_max;     // most staged atoms of any cell tile
   int halo_fwd;     // list entries with a halo image found in the forward half shell (evaluated)
   int halo_bwd;     // list entries with a halo image found in the backward halo pass (skipped)
-  int pad[1];
+  unsigned count_s; // the same on the side stream
   unsigned long long npairs_list;  // half-list entries walked by the pair kernel
   unsigned long long npairs_rc;    // unique pairs inside the cutoff
   double acc[96];   // energy / virial / stress accumulators
@@ -372,98 +372,89 @@ __device__ __forceinline__ double rsqrt_seeded(double v) {
   return r * fma(-0.5 * v * r, r, 1.5);
 }
 
-// Block-wide reduction of NV doubles into per-block slots out[blockIdx.x*NV + k].
-template <int NV>
-__device__ __forceinline__ void block_reduce_store(double (&v)[NV], double* out) {
-  __shared__ double red[32][NV];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < NV; ++k) v[k] = warp_sum(v[k]);
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) red[wid][k] = v[k];
-  }
-  __syncthreads();
-  if (wid == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      double t = lane < nw ? red[lane][k] : 0.0;
-      t = warp_sum(t);
-      if (lane == 0) out[(size_t)blockIdx.x * NV + k] = t;
-    }
-  }
-}
+template <typename T>
+__device__ __forceinline__ T shfl_xor_t(T v, int o) { return __shfl_xor_sync(0xffffffffu, v, o); }
 
-// FP32 variant: sums in FP32 and converts only the NV block totals (one thread)
-// to FP64, so an FP32 kernel issues no FP64 instruction per warp.
-template <int NV>
-__device__ __forceinline__ void block_reduce_store(float (&v)[NV], double* out) {
-  __shared__ float redf[32][NV];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int k = 0; k < NV; ++k) v[k] = warp_sumf(v[k]);
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) redf[wid][k] = v[k];
-  }
-  __syncthreads();
-  if (wid == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      float t = lane < nw ? redf[lane][k] : 0.f;
-      t = warp_sumf(t);
-      if (lane == 0) out[(size_t)blockIdx.x * NV + k] = (double)t;
-    }
-  }
-}
-
-// Grid-wide sums of NV <= 8 doubles in one launch: each block's sums go to part[block], and
-// the block that counts last adds them up, in block order, and hands value k to put(k, sum)
-// (one thread per value).  A warp sums its eight values by a reduce-scatter (9 FP64 additions
-// instead of 5 per value).  count: a zero in device memory, zero again afterwards.  At
-// least 32 NV threads per block.
-template <int NV, typename Put>
-__device__ __forceinline__ void grid_sum(const double (&in)[NV], double* part, unsigned* count, Put put) {
-  static_assert(NV <= 8, "one value per lane after three exchanges");
-  __shared__ double red[32][8];
-  __shared__ bool s_last;
+// Block-wide sums of NV values (double, float or double-float) into per-block slots
+// out[blockIdx.x * NV + k].  A warp sums its values by a reduce-scatter, which leaves value k
+// with the lanes k * 32 / P2 onwards: for eight values 9 additions instead of 40.  The sums
+// run in the values' own type; only the block totals are converted to FP64.
+template <int NV, typename T>
+__device__ __forceinline__ void block_reduce_store(const T (&in)[NV], double* out) {
+  constexpr int P2 = NV <= 1 ? 1 : NV <= 2 ? 2 : NV <= 4 ? 4 : NV <= 8 ? 8 : 16, G = 32 / P2;
+  static_assert(NV <= 16, "reduce-scatter of up to 16 values");
+  __shared__ T red[32][P2];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
-  double v[8];
+  T v[P2];
 #pragma unroll
-  for (int k = 0; k < 8; ++k) v[k] = k < NV ? in[k < NV ? k : 0] : 0.0;
+  for (int k = 0; k < P2; ++k) v[k] = k < NV ? in[k < NV ? k : 0] : T(0);
 #pragma unroll
-  for (int h = 4, o = 16; h > 0; h >>= 1, o >>= 1) {
+  for (int h = P2 / 2, o = 16; h > 0; h >>= 1, o >>= 1) {
     const bool up = lane & o;
 #pragma unroll
     for (int k = 0; k < h; ++k) {
-      const double keep = up ? v[k + h] : v[k], send = up ? v[k] : v[k + h];
-      v[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+      const T keep = up ? v[k + h] : v[k], send = up ? v[k] : v[k + h];
+      v[k] = keep + shfl_xor_t(send, o);
     }
   }
-  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
-  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 1);
-  if ((lane & 3) == 0) red[wid][(lane & 16 ? 4 : 0) + (lane & 8 ? 2 : 0) + (lane & 4 ? 1 : 0)] = v[0];
+#pragma unroll
+  for (int o = G / 2; o > 0; o >>= 1) v[0] = v[0] + shfl_xor_t(v[0], o);
+  if (lane % G == 0) red[wid][lane / G] = v[0];
   __syncthreads();
-  if (threadIdx.x < NV) {
-    double s = 0.0;
-    for (int w = 0; w < nw; ++w) s += red[w][threadIdx.x];
-    part[(size_t)blockIdx.x * NV + threadIdx.x] = s;
+  if (wid == 0) {
+    const int k = lane % P2;
+    T s = T(0);
+    for (int w = lane / P2; w < nw; w += G) s = s + red[w][k];
+#pragma unroll
+    for (int o = P2; o < 32; o <<= 1) s = s + shfl_xor_t(s, o);
+    if (lane < NV) out[(size_t)blockIdx.x * NV + lane] = (double)s;
+  }
+}
+
+// The sums over a grid's blocks as the end of the kernel that made the block sums (part, by
+// block_reduce_store): the block that counts last adds them in a fixed order, a launch less
+// than gb_reduce_blocks.  True in that block (all threads), with the sums in gs.out.
+// gs.count: a zero in device memory, zero again afterwards; null: nothing is done here.
+struct GridSum {
+  unsigned* count;
+  double* out;
+};
+template <int NV>
+__device__ __forceinline__ bool grid_finish(const double* part, GridSum gs) {
+  if (!gs.count) return false;
+  constexpr int P2 = NV <= 1 ? 1 : NV <= 2 ? 2 : NV <= 4 ? 4 : NV <= 8 ? 8 : 16, G = 32 / P2;
+  __shared__ double s_sum[32][P2];
+  __shared__ bool s_last;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+  if (wid == 0) {  // the warp that wrote this block's sums
     __threadfence();
+    __syncwarp();
+    if (lane == 0) s_last = atomicAdd(gs.count, 1u) == gridDim.x - 1;
   }
   __syncthreads();
-  if (threadIdx.x == 0) s_last = atomicAdd(count, 1u) == gridDim.x - 1;
-  __syncthreads();
-  if (!s_last) return;
+  if (!s_last) return false;
   __threadfence();
-  if (wid < NV) {
-    double s = 0.0;
-    for (int b = lane; b < (int)gridDim.x; b += 32) s += __ldcg(&part[(size_t)b * NV + wid]);
-    s = warp_sum(s);
-    if (lane == 0) put(wid, s);
+  // lane: value lane % P2 of every (nw G)-th block
+  const int k = lane % P2;
+  double s = 0.0;
+  if (k < NV) {
+#pragma unroll 16
+    for (int b = wid * G + lane / P2; b < (int)gridDim.x; b += nw * G) s += __ldcg(&part[(size_t)b * NV + k]);
   }
-  if (threadIdx.x == 0) *count = 0u;
+#pragma unroll
+  for (int o = P2; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+  if (lane < P2) s_sum[wid][lane] = s;
+  __syncthreads();
+  if (wid == 0) {
+    s = 0.0;
+    for (int w = lane / P2; w < nw; w += G) s += s_sum[w][k];
+#pragma unroll
+    for (int o = P2; o < 32; o <<= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (lane < NV) gs.out[lane] = s;
+  }
+  if (threadIdx.x == 0) *gs.count = 0u;
+  __syncthreads();
+  return true;
 }
 
 // host helpers implemented in gb_api.cu
@@ -471,6 +462,9 @@ void gb_sync_scalars();           // copy device scalars to the pinned mirror (s
 double* gb_blkacc(int n);         // per-block accumulator scratch with n doubles
 void gb_reduce_blocks(const double* blk, int nblocks, int nv, double* out_dev);  // sums into out_dev[0..nv)
 int* gb_scan_scratch(int n);
+// nv sums over nb blocks of nt threads by the kernel itself (grid_finish), or by a launch behind it
+GridSum gb_grid_sum(int nb, int nt, int nv, double* out_dev);
+void gb_grid_sum_done(const GridSum& gs, const double* blk, int nb, int nv);
 void side_join();                 // the first stream waits for the side stream (no-op without a fork)
 void run_side_hook();             // enqueue the pending side-stream work (g.side_hook), if any
 
@@ -481,7 +475,7 @@ int list_relocate_and_halo(bool wait = true);
 int list_refresh_halo();          // refresh halo positions (gb_list.cu)
 int list_build();                 // binning + pairs (gb_list.cu)
 void list_setup();                // link-cell geometry (gb_list.cu)
-void list_pos_records(bool sorted);  // FP32 hi/lo positions by atom index and (sorted) per sorted position
+void list_pos_records(bool sorted);  // FP32 hi/lo positions by atom index and (sorted) per sorted position; clears the force sums
 void scan_exclusive(const int* in, int* out, int n);
 void pair_forces(double* eng6, double* stress9);  // gb_pair.cu (adds into forces)
 void pair_setup();                // gb_pair.cu: per-key constants
@@ -508,7 +502,7 @@ int integ_vnl_check();
 void integ_vnl_launch();          // the displacement check
 void integ_stage1_check();        // NVE stage 1 and the displacement check in one kernel
 int integ_vnl_result();           // its decision from the copied scalars (after a wait)
-void integ_zero_forces();
+void integ_zero_forces();         // of the FP64 form by instructions; list_pos_records clears the others'
 void integ_forces_to_fp64();      // mixed: fixed point -> FP64 forces
 void integ_setup_constraints(const int32_t* listcon, const double* prmcon);
 // thermostats (gb_thermostat.cu)

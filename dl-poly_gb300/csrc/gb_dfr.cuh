@@ -50,32 +50,7 @@ __device__ __forceinline__ dfr shfl_xor_dfr(dfr v, int o) {
   return dfr(__shfl_xor_sync(0xffffffffu, v.hi, o), __shfl_xor_sync(0xffffffffu, v.lo, o));
 }
 
-// block sums of double-float values: reduced in double-float (no FP64 instruction per
-// thread), one thread converts the NV block totals to FP64
-template <int NV>
-__device__ __forceinline__ void block_reduce_store(dfr (&v)[NV], double* out) {
-  __shared__ dfr redd[32][NV];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) v[k] += shfl_xor_dfr(v[k], o);
-  }
-  if (lane == 0) {
-#pragma unroll
-    for (int k = 0; k < NV; ++k) redd[wid][k] = v[k];
-  }
-  __syncthreads();
-  if (wid == 0) {
-    const int nw = (blockDim.x + 31) >> 5;
-#pragma unroll
-    for (int k = 0; k < NV; ++k) {
-      dfr t = lane < nw ? redd[lane][k] : dfr();
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) t += shfl_xor_dfr(t, o);
-      if (lane == 0) out[(size_t)blockIdx.x * NV + k] = (double)t;
-    }
-  }
-}
+// for block_reduce_store
+__device__ __forceinline__ dfr shfl_xor_t(dfr v, int o) { return shfl_xor_dfr(v, o); }
 
 #endif

@@ -40,7 +40,7 @@ struct FftKernels {
   void (*x_inv)(const T2*, T*, FftPlan, const T2*, const T2*, int, int, unsigned*);
   void (*y_fwd)(T2*, int, int, FftPlan, const T2*);
   void (*y_inv)(T2*, int, int, FftPlan, const T2*);
-  void (*z_conv)(T2*, int, int, int, FftPlan, const T2*, const T*, const T*, SpmeGeom, double*);
+  void (*z_conv)(T2*, int, int, int, FftPlan, const T2*, const T*, const T*, SpmeGeom, double*, GridSum);
 };
 
 // kernels for an x pass of half length M and y, z passes of lengths K2, K3:
@@ -369,7 +369,8 @@ __global__ void k_fft_y(T2* __restrict__ G, int Kx, int K2_, FftPlan pl, const T
 // themselves and their conjugate mirror, so they count twice in the stress
 template <typename T, typename T2, int NC>
 __global__ void k_fft_z_conv(T2* __restrict__ G, int K1, int K2, int K3_, FftPlan pl, const T2* __restrict__ tw,
-                             const T* __restrict__ theta, const T* __restrict__ psi, SpmeGeom sg, double* blk) {
+                             const T* __restrict__ theta, const T* __restrict__ psi, SpmeGeom sg, double* blk,
+                             GridSum gs) {
   extern __shared__ unsigned char smem_raw[];
   const int K3 = NC ? NC : K3_;
   T2* a = reinterpret_cast<T2*>(smem_raw);
@@ -455,6 +456,7 @@ __global__ void k_fft_z_conv(T2* __restrict__ G, int K1, int K2, int K3_, FftPla
     if (t < nt) base[(size_t)zz * plane + t] = r2[t * K3 + zz];
   }
   block_reduce_store<6>(st, blk);
+  grid_finish<6>(blk, gs);
 }
 
 

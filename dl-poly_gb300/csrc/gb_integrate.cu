@@ -91,7 +91,7 @@ __global__ void __launch_bounds__(KIN_NT) k_kinstress(int n, const double* __res
                                                       const double* __restrict__ fx, const double* __restrict__ fy,
                                                       const double* __restrict__ fz, double* __restrict__ vx,
                                                       double* __restrict__ vy, double* __restrict__ vz, double* part,
-                                                      DevScalars* sc) {
+                                                      GridSum gs) {
   double a[6] = {0, 0, 0, 0, 0, 0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double m = w[i];
@@ -108,7 +108,8 @@ __global__ void __launch_bounds__(KIN_NT) k_kinstress(int n, const double* __res
     a[0] += m * u * u; a[1] += m * u * v; a[2] += m * u * t;
     a[3] += m * v * v; a[4] += m * v * t; a[5] += m * t * t;
   }
-  grid_sum<6>(a, part, &sc->count, [&](int k, double s) { sc->acc[A_STRKIN + k] = s; });
+  block_reduce_store<6>(a, part);
+  grid_finish<6>(part, gs);
 }
 
 // largest |r - r_checkpoint|^2 with minimum image, over a grid-stride loop, after the first
@@ -178,6 +179,7 @@ struct ConArgs {
   const double* w;
   double tstep, tol, c0, a0;
   int* flags;      // maxit+1 ints, zeroed
+  GridSum gs;      // of k_constrain_small's stress
   bool tags;       // RATTLE of k_constrain_small: form the bond vectors from the positions (and store them)
   DevScalars* sc;
   double* blk;     // per-block stress partials (6)
@@ -900,6 +902,7 @@ __global__ void __launch_bounds__(CS_THREADS) k_constrain_small(ConArgs A, const
 #pragma unroll
     for (int k = 0; k < 6; ++k) sd[k] = to_dfr(st[k]);
     block_reduce_store<6>(sd, A.blk);
+    grid_finish<6>(A.blk, A.gs);
   }
 }
 
@@ -1141,12 +1144,8 @@ void integ_setup_constraints(const int32_t* listcon, const double* prmcon) {
 }
 
 void integ_zero_forces() {
-  if (g.precision == GB_FP64) {
-    k_zero3<<<nblocks(g.natms, 256), 256, 0, g.stream>>>(g.natms, g.fx, g.fy, g.fz);
-    GB_LAUNCHED();
-  } else {
-    GB_CUDA(cudaMemsetAsync(g.fixp, 0, sizeof(long long) * 3 * (size_t)g.natms, g.stream));
-  }
+  k_zero3<<<nblocks(g.natms, 256), 256, 0, g.stream>>>(g.natms, g.fx, g.fy, g.fz);
+  GB_LAUNCHED();
 }
 
 void integ_forces_to_fp64() {
@@ -1192,7 +1191,7 @@ static void con_args(ConArgs& A) {
   A.dt2 = g.dt2; A.gam = g.gam;
   A.x = g.x; A.y = g.y; A.z = g.z; A.vx = g.vx; A.vy = g.vy; A.vz = g.vz; A.w = g.weight;
   A.tstep = g.p.tstep; A.tol = g.p.shake_tol; A.c0 = g.cell[0]; A.a0 = 1.0 / g.cell[0];
-  A.flags = d_flags; A.sc = g.sc; A.blk = nullptr; A.tags = false;
+  A.flags = d_flags; A.sc = g.sc; A.blk = nullptr; A.gs = {nullptr, nullptr}; A.tags = false;
 }
 
 template <bool RATTLE>
@@ -1234,6 +1233,7 @@ void integ_shake(int* iters, double* vircon, double* strcon) {
   con_args(A);
   const int nbs = cl_small ? coop_blocks_small : n_clusters ? coop_blocks_cl : coop_blocks_shake;
   A.blk = gb_blkacc(nbs * 6);
+  if (cl_small) A.gs = gb_grid_sum(nbs, cs_threads, 6, &g.sc->acc[A_STRCON]);
   prof_begin(P_SHAKE);
   if (cl_small) {
     launch_small<false>(A, rstep);
@@ -1250,7 +1250,7 @@ void integ_shake(int* iters, double* vircon, double* strcon) {
   }
   GB_LAUNCHED();
   prof_end(P_SHAKE);
-  gb_reduce_blocks(A.blk, nbs, 6, &g.sc->acc[A_STRCON]);
+  if (!A.gs.count) gb_reduce_blocks(A.blk, nbs, 6, &g.sc->acc[A_STRCON]);
   if (!cl_small) {
     k_shake_post<<<nblocks(n, 256), 256, 0, st>>>(n, g.acon_start, g.lfrzn, rstep, hstep, g.weight, g.x, g.y, g.z,
                                                    g.ox, g.oy, g.oz, g.vx, g.vy, g.vz, g.fx, g.fy, g.fz);
@@ -1295,9 +1295,12 @@ void integ_rattle_launch(bool tags) {
 // kinetic stress into acc[A_STRKIN], after the second half kick when kick is set
 static void launch_kinstress(bool kick) {
   const int nb = std::min(nblocks(g.natms, KIN_NT), 2 * g.nsm);
+  const GridSum gs = gb_grid_sum(nb, KIN_NT, 6, &g.sc->acc[A_STRKIN]);
+  double* part = gb_blkacc(nb * 6);
   k_kinstress<<<nb, KIN_NT, 0, g.stream>>>(g.natms, g.weight, g.lfrzn, kick ? g.hdw : nullptr, g.fx, g.fy, g.fz, g.vx,
-                                           g.vy, g.vz, gb_blkacc(nb * 6), g.sc);
+                                           g.vy, g.vz, part, gs);
   GB_LAUNCHED();
+  gb_grid_sum_done(gs, part, nb, 6);
 }
 
 void integ_vv(int stage, double* strkin, double* engke, int* iters, double* vircon, double* strcon) {

@@ -852,13 +852,28 @@ __global__ void __launch_bounds__(256) k_list_reorder(int natms, int* list, int 
 // fourth word (bit pattern), so a pair reads everything about j in two 16-byte loads
 // Both records in one pass over the atoms (the FP64 values converted once): by atom index
 // (xf, xlo: the type in xlo.w) and, for the sorted-position pair kernels, per sorted
-// position sorted_pos[i] (xhs, and rec or, in the mixed form, xlh)
+// position sorted_pos[i] (xhs, and rec or, in the mixed form, xlh).  The same pass clears the
+// force sums of the evaluation that follows (one launch for up to four; at 4,096 ions a
+// fill takes 2 us and a gap).
+struct ForceZero {
+  int natms, mxatms;
+  double *fx, *fy, *fz;      // FP64 forces (null in the mixed form)
+  long long *fixp, *fixs;    // fixed-point sums by atom and by sorted position, with the pool's counter (or null)
+};
 __global__ void k_pos_records(const DevScalars* sc, const int* __restrict__ sorted_pos, const double* __restrict__ x,
                               const double* __restrict__ y, const double* __restrict__ z, const double* __restrict__ q,
                               const int* __restrict__ ltype, double pos_scale, float4* xf, float4* xlo, float2* qdf,
-                              float4* xhs, PosRec* rec, uint2* xlh) {
+                              float4* xhs, PosRec* rec, uint2* xlh, ForceZero Z) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < Z.natms) {
+    if (Z.fx) { Z.fx[i] = 0.0; Z.fy[i] = 0.0; Z.fz[i] = 0.0; }
+    if (Z.fixp) { Z.fixp[3 * i] = 0; Z.fixp[3 * i + 1] = 0; Z.fixp[3 * i + 2] = 0; }
+  }
   if (i >= sc->nlast) return;
+  if (Z.fixs) {
+    Z.fixs[i] = 0; Z.fixs[Z.mxatms + i] = 0; Z.fixs[2 * (size_t)Z.mxatms + i] = 0;
+    if (i == 0) Z.fixs[3 * (size_t)Z.mxatms] = 0;
+  }
   const double xa = x[i], ya = y[i], za = z[i], qa = q[i];
   const int ta = ltype[i];
   const float hx = (float)xa, hy = (float)ya, hz = (float)za, hq = (float)qa;
@@ -1190,9 +1205,12 @@ int list_build() {
 }
 
 void list_pos_records(bool sorted) {
+  const bool f64 = g.precision == GB_FP64;
+  const ForceZero Z = {g.natms, g.mxatms, f64 ? g.fx : nullptr, g.fy, g.fz, !f64 || sorted ? g.fixp : nullptr,
+                       sorted ? g.fixs : nullptr};
   k_pos_records<<<nblocks(g.mxatms, 256), 256, 0, g.stream>>>(
-      g.sc, g.sorted_pos, g.x, g.y, g.z, g.chge, g.ltype, g.pos_scale, g.xf, g.xlo, g.precision == GB_FP64 ? g.qdf : nullptr,
-      sorted ? g.xhs : nullptr, g.rec, g.precision == GB_MIXED ? g.xlh : nullptr);
+      g.sc, g.sorted_pos, g.x, g.y, g.z, g.chge, g.ltype, g.pos_scale, g.xf, g.xlo, f64 ? g.qdf : nullptr,
+      sorted ? g.xhs : nullptr, g.rec, f64 ? nullptr : g.xlh, Z);
   GB_LAUNCHED();
 }
 

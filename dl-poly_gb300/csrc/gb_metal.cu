@@ -224,7 +224,7 @@ __global__ void __launch_bounds__(256) k_metal_density(int natms, const DevScala
 }
 
 // embedding energy and F'(rho) (metal_ld_compute, tab > 0, rho grid)
-__global__ void k_metal_embed(int natms, const int* ltype, MetArgs A, double* rho, double* blk, int* status) {
+__global__ void k_metal_embed(int natms, const int* ltype, MetArgs A, double* rho, double* blk, int* status, GridSum gs) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   double e[1] = {0.0};
   int st = 0;
@@ -250,6 +250,7 @@ __global__ void k_metal_embed(int natms, const int* ltype, MetArgs A, double* rh
   }
   if (st) atomicOr(status, st);
   block_reduce_store<1>(e, blk);
+  grid_finish<1>(blk, gs);
 }
 
 // metal_ld_set_halo: images carry F'(rho) of their source atom
@@ -390,7 +391,7 @@ struct MetSorted {
   const float2* fp;                // F'(rho) per sorted position
   float f_pre, f_rc_lo, f_rc_hi;
   double *s0, *s1, *s2;            // sums per sorted position
-  double* blk;
+  double* blk; GridSum gs;
   int* status;
   unsigned long long* cnt;
 };
@@ -772,6 +773,7 @@ __global__ void __launch_bounds__(MET_NT, 3) k_metal_forces_sorted(MetSorted S, 
   }
   dfr out[2] = {to_dfr(two_sum(e_eng.s, e_eng.c)), to_dfr(two_sum(e_vir.s, e_vir.c))};
   block_reduce_store<2>(out, S.blk);
+  grid_finish<2>(S.blk, S.gs);
 }
 
 // stress (sum over slots of x (x) F, every halo image at its own position) and each slot's
@@ -780,7 +782,7 @@ __global__ void k_metal_force_fold(int natms, const DevScalars* sc, const int* _
                                    const int* __restrict__ src, const double* __restrict__ x,
                                    const double* __restrict__ y, const double* __restrict__ z,
                                    const double* __restrict__ s0, const double* __restrict__ s1,
-                                   const double* __restrict__ s2, double* fx, double* fy, double* fz, double* blk) {
+                                   const double* __restrict__ s2, double* fx, double* fy, double* fz, double* blk, GridSum gs) {
   const int nlast = sc->nlast;
   double st[6] = {0, 0, 0, 0, 0, 0};
   for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < nlast; p += gridDim.x * blockDim.x) {
@@ -796,6 +798,7 @@ __global__ void k_metal_force_fold(int natms, const DevScalars* sc, const int* _
     atomicAdd(&fz[tgt], fc);
   }
   block_reduce_store<6>(st, blk);
+  grid_finish<6>(blk, gs);
 }
 
 // ------------------------------------------------------------------- host state
@@ -1049,6 +1052,8 @@ static void metal_forces_sorted(const MetArgs& A, unsigned long long* cnt) {
   double* blk = gb_blkacc(nbe + 2 * nbf + 6 * nbs);
   double *blk2 = blk + nbe, *blk3 = blk2 + 2 * (size_t)nbf;
   S.blk = blk2;
+  S.gs = gb_grid_sum(nbf, MET_NT, 2, &g.sc->acc[A_METAL]);
+  const GridSum gss = gb_grid_sum(nbs, T, 6, &g.sc->acc[A_METAL + 2]);
   S.cnt = cnt;
   prof_begin(P_METAL_DENSITY);
   GB_CUDA(cudaMemsetAsync(d_slot, 0, sizeof(double) * (size_t)mx, st));
@@ -1058,9 +1063,10 @@ static void metal_forces_sorted(const MetArgs& A, unsigned long long* cnt) {
   GB_LAUNCHED();
   k_metal_rho_fold<<<nbm, T, 0, st>>>(g.natms, g.sc, g.at_list, g.src, d_slot, d_rho);
   GB_LAUNCHED();
-  k_metal_embed<<<nbe, T, 0, st>>>(g.natms, g.ltype, A, d_rho, blk, &g.sc->status);
+  const GridSum gse = gb_grid_sum(nbe, T, 1, &g.sc->acc[A_METAL + 8]);
+  k_metal_embed<<<nbe, T, 0, st>>>(g.natms, g.ltype, A, d_rho, blk, &g.sc->status, gse);
   GB_LAUNCHED();
-  gb_reduce_blocks(blk, nbe, 1, &g.sc->acc[A_METAL + 8]);
+  gb_grid_sum_done(gse, blk, nbe, 1);
   k_metal_fp<<<nbm, T, 0, st>>>(g.sc, g.src, g.sorted_pos, d_rho, d_fp);
   GB_LAUNCHED();
   prof_end(P_METAL_DENSITY);
@@ -1070,10 +1076,10 @@ static void metal_forces_sorted(const MetArgs& A, unsigned long long* cnt) {
   k_metal_forces_sorted<<<nbf, MET_NT, 0, st>>>(S, A);
   GB_LAUNCHED();
   k_metal_force_fold<<<nbs, T, 0, st>>>(g.natms, g.sc, g.at_list, g.src, g.x, g.y, g.z, S.s0, S.s1, S.s2, g.fx, g.fy,
-                                        g.fz, blk3);
+                                        g.fz, blk3, gss);
   GB_LAUNCHED();
-  gb_reduce_blocks(blk2, nbf, 2, &g.sc->acc[A_METAL]);
-  gb_reduce_blocks(blk3, nbs, 6, &g.sc->acc[A_METAL + 2]);
+  gb_grid_sum_done(S.gs, blk2, nbf, 2);
+  gb_grid_sum_done(gss, blk3, nbs, 6);
   prof_end(P_METAL_FORCES);
 }
 
@@ -1088,9 +1094,10 @@ static void metal_forces_fp64(const MetArgs& A, unsigned long long* cnt) {
   GB_LAUNCHED();
   const int nbe = nblocks(g.natms, T);
   double* blk = gb_blkacc(std::max(nbe, 1) + MACC * std::max(1, occ_force * g.nsm));
-  k_metal_embed<<<nbe, T, 0, st>>>(g.natms, g.ltype, A, d_rho, blk, &g.sc->status);
+  const GridSum gse = gb_grid_sum(nbe, T, 1, &g.sc->acc[A_METAL + 8]);
+  k_metal_embed<<<nbe, T, 0, st>>>(g.natms, g.ltype, A, d_rho, blk, &g.sc->status, gse);
   GB_LAUNCHED();
-  gb_reduce_blocks(blk, nbe, 1, &g.sc->acc[A_METAL + 8]);
+  gb_grid_sum_done(gse, blk, nbe, 1);
   k_metal_halo<<<nblocks(std::max(g.mxatms - g.natms, 1), T), T, 0, st>>>(g.natms, g.sc, g.src, d_rho);
   GB_LAUNCHED();
   prof_end(P_METAL_DENSITY);

@@ -19,7 +19,7 @@ constexpr int KIN_SLOTS = 4096;    // of 6 doubles: 196,608 B per device
 constexpr int KIN_BLOCKS = 304;    // two per SM: the partial sums of at most so many blocks are kept
 constexpr int KIN_MAX_DEVICES = 64;
 
-// The blocks' partial sums in its first KIN_BLOCKS slots; its last word counts the blocks
+// The blocks' partial sums in its first KIN_BLOCKS slots, the sums in the next; its last word counts the blocks
 // that are done (0 between calls).
 static __device__ __align__(256) double g_kin_scratch[KIN_SLOTS * 6];
 
@@ -46,11 +46,14 @@ __global__ void __launch_bounds__(KIN_THREADS) k_kin_sum(int n, const double* __
     a[0] = fma(mu, u, a[0]); a[1] = fma(mu, v, a[1]); a[2] = fma(mu, t, a[2]);
     a[3] = fma(mv, v, a[3]); a[4] = fma(mv, t, a[4]); a[5] = fma(m * t, t, a[5]);
   }
-  grid_sum<6>(a, part, reinterpret_cast<unsigned*>(part + KIN_SLOTS * 6) - 1, [&](int k, double s) {
+  block_reduce_store<6>(a, part);
+  double* sum = part + KIN_BLOCKS * 6;
+  const GridSum gs = {reinterpret_cast<unsigned*>(part + KIN_SLOTS * 6) - 1, sum};
+  if (grid_finish<6>(part, gs) && threadIdx.x < 6) {
     const int at[6] = {0, 1, 2, 4, 5, 8}, mirror[6] = {0, 3, 6, 4, 7, 8};
-    out[at[k]] = s;
-    out[mirror[k]] = s;
-  });
+    out[at[threadIdx.x]] = sum[threadIdx.x];
+    out[mirror[threadIdx.x]] = sum[threadIdx.x];
+  }
 }
 
 }  // namespace

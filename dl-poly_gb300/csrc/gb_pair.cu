@@ -215,7 +215,7 @@ __global__ void __launch_bounds__(256, 3) k_pair_fp64(int natms, const DevScalar
 __global__ void k_excl_fp64(int natms, const int* list, int ld, const double* x, const double* y, const double* z,
                             const double* q, const int* ltg, const int* src, double alpha, double scaling,
                             double rcut, double* fx, double* fy, double* fz, double* blk,
-                            unsigned long long* fixp) {
+                            unsigned long long* fixp, GridSum gs) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
   if (i < natms) {
@@ -277,6 +277,7 @@ __global__ void k_excl_fp64(int natms, const int* list, int ld, const double* x,
     }
   }
   block_reduce_store<8>(acc, blk);
+  grid_finish<8>(blk, gs);
 }
 
 // -------------------------------------------------------------- mixed form
@@ -1123,7 +1124,7 @@ __global__ void k_slot_stress_fold(int natms, const DevScalars* sc, const int* _
                                    const double* __restrict__ y, const double* __restrict__ z,
                                    const long long* __restrict__ s0, const long long* __restrict__ s1,
                                    const long long* __restrict__ s2, const float2* __restrict__ eat,
-                                   unsigned long long* fixp, double* blk) {
+                                   unsigned long long* fixp, double* blk, GridSum gs) {
   const int nlast = sc->nlast;
   const double s = 1.0 / 1099511627776.0;
   double st[6] = {0, 0, 0, 0, 0, 0};
@@ -1156,6 +1157,7 @@ __global__ void k_slot_stress_fold(int natms, const DevScalars* sc, const int* _
 #pragma unroll
   for (int k = 0; k < 6; ++k) out[NACC_DF + k] = dfr(st[k]);
   block_reduce_store<NACC_DF + 6>(out, blk);
+  grid_finish<NACC_DF + 6>(blk, gs);
 }
 
 // Pair stress of the double-float kernel from its per-slot forces: with every image's
@@ -1286,10 +1288,10 @@ void pair_forces_sorted(PairGeom& pg, int nb2) {
   const int nbs = std::max(1, std::min(nblocks(g.mxatms, 256), 4 * g.nsm));  // stress blocks
   double* blks = gb_blkacc(nbs * NACC + nb2 * 8);
   double* blk2 = blks + (size_t)nbs * NACC;
+  const GridSum gss = gb_grid_sum(nbs, 256, NACC, &g.sc->acc[A_PAIR]);
   A.eat = g.eat;
   A.pool = apw > 0 ? nullptr : A.f2 + g.mxatms;
-  GB_CUDA(cudaMemsetAsync(g.fixs, 0, sizeof(long long) * (3 * (size_t)g.mxatms + 1), st));
-  if (!mixed) GB_CUDA(cudaMemsetAsync(g.fixp, 0, sizeof(long long) * 3 * (size_t)g.mxatms, st));
+  // (list_pos_records has cleared the sums)
   prof_begin(P_PAIR);
   kern<<<nb, nt, dsm, st>>>(A, pg);
   GB_LAUNCHED();
@@ -1297,22 +1299,23 @@ void pair_forces_sorted(PairGeom& pg, int nb2) {
   side_join();  // the reciprocal-space forces are in place before the pair forces join them
   k_slot_stress_fold<<<nbs, 256, 0, st>>>(g.natms, g.sc, g.at_list, g.src, g.x, g.y, g.z, (const long long*)A.f0,
                                           (const long long*)A.f1, (const long long*)A.f2, g.eat,
-                                          (unsigned long long*)g.fixp, blks);
+                                          (unsigned long long*)g.fixp, blks, gss);
   GB_LAUNCHED();
+  gb_grid_sum_done(gss, blks, nbs, NACC);
   if (!mixed) {
     k_fix_add_fp64<<<nblocks(g.natms, 256), 256, 0, st>>>(g.natms, g.fixp, g.fx, g.fy, g.fz);
     GB_LAUNCHED();
   }
   prof_end(P_PAIR);
-  gb_reduce_blocks(blks, nbs, NACC, &g.sc->acc[A_PAIR]);
   if (g.lbook) {
     prof_begin(P_EXCL);
+    const GridSum gse = gb_grid_sum(nb2, 128, 8, &g.sc->acc[A_EXCL]);
     k_excl_fp64<<<nb2, 128, 0, st>>>(g.natms, g.list, g.ld, g.x, g.y, g.z, g.chge, g.ltg, g.src, g.p.alpha,
                                      g.scaling, g.p.rcut, g.fx, g.fy, g.fz, blk2,
-                                     mixed ? (unsigned long long*)g.fixp : nullptr);
+                                     mixed ? (unsigned long long*)g.fixp : nullptr, gse);
     GB_LAUNCHED();
     prof_end(P_EXCL);
-    gb_reduce_blocks(blk2, nb2, 8, &g.sc->acc[A_EXCL]);
+    gb_grid_sum_done(gse, blk2, nb2, 8);
   }
 }
 
@@ -1407,11 +1410,12 @@ void pair_forces(double* eng6, double* stress9) {
     if (g.lbook) {
       double* blk2 = blk + (size_t)nb * NACC;
       prof_begin(P_EXCL);
+      const GridSum gse = gb_grid_sum(nb2, 128, 8, &g.sc->acc[A_EXCL]);
       k_excl_fp64<<<nb2, 128, 0, st>>>(g.natms, g.list, g.ld, g.x, g.y, g.z, g.chge, g.ltg, g.src, g.p.alpha,
-                                       g.scaling, g.p.rcut, g.fx, g.fy, g.fz, blk2, nullptr);
+                                       g.scaling, g.p.rcut, g.fx, g.fy, g.fz, blk2, nullptr, gse);
       GB_LAUNCHED();
       prof_end(P_EXCL);
-      gb_reduce_blocks(blk2, nb2, 8, &g.sc->acc[A_EXCL]);
+      gb_grid_sum_done(gse, blk2, nb2, 8);
     }
   } else if (g.precision == GB_FP64) {
     static int occ64 = 0;
@@ -1428,11 +1432,12 @@ void pair_forces(double* eng6, double* stress9) {
     if (g.lbook) {
       double* blk2 = blk + (size_t)nb * NACC;
       prof_begin(P_EXCL);
+      const GridSum gse = gb_grid_sum(nb2, 128, 8, &g.sc->acc[A_EXCL]);
       k_excl_fp64<<<nb2, 128, 0, st>>>(g.natms, g.list, g.ld, g.x, g.y, g.z, g.chge, g.ltg, g.src, g.p.alpha,
-                                       g.scaling, g.p.rcut, g.fx, g.fy, g.fz, blk2, nullptr);
+                                       g.scaling, g.p.rcut, g.fx, g.fy, g.fz, blk2, nullptr, gse);
       GB_LAUNCHED();
       prof_end(P_EXCL);
-      gb_reduce_blocks(blk2, nb2, 8, &g.sc->acc[A_EXCL]);
+      gb_grid_sum_done(gse, blk2, nb2, 8);
     }
   } else {
     static int occ32 = 0;
@@ -1450,11 +1455,12 @@ void pair_forces(double* eng6, double* stress9) {
     if (g.lbook) {
       double* blk2 = blk + (size_t)nb * NACC;
       prof_begin(P_EXCL);
+      const GridSum gse = gb_grid_sum(nb2, 128, 8, &g.sc->acc[A_EXCL]);
       k_excl_fp64<<<nb2, 128, 0, st>>>(g.natms, g.list, g.ld, g.x, g.y, g.z, g.chge, g.ltg, g.src, g.p.alpha,
-                                       g.scaling, g.p.rcut, g.fx, g.fy, g.fz, blk2, (unsigned long long*)g.fixp);
+                                       g.scaling, g.p.rcut, g.fx, g.fy, g.fz, blk2, (unsigned long long*)g.fixp, gse);
       GB_LAUNCHED();
       prof_end(P_EXCL);
-      gb_reduce_blocks(blk2, nb2, 8, &g.sc->acc[A_EXCL]);
+      gb_grid_sum_done(gse, blk2, nb2, 8);
     }
   }
   if (g.defer_scalars) return;  // the MD loop reads the sums after its last step

@@ -496,7 +496,7 @@ template <typename T, int P>
 __global__ void k_spme_gather(int natms, const double* __restrict__ x, const double* __restrict__ y,
                               const double* __restrict__ z, const double* __restrict__ q, SpmeGeom sg,
                               const T* __restrict__ phi, double rk0, double rk1, double rk2, double* fout,
-                              double* blk) {
+                              double* blk, GridSum gs) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   double acc[4] = {0, 0, 0, 0};
   if (i < natms && fabs(q[i]) > DBL_MIN) {
@@ -553,6 +553,7 @@ __global__ void k_spme_gather(int natms, const double* __restrict__ x, const dou
     fout[3 * i] = 0; fout[3 * i + 1] = 0; fout[3 * i + 2] = 0;
   }
   block_reduce_store<4>(acc, blk);
+  grid_finish<4>(blk, gs);
 }
 
 // FP32 gather, one warp per atom: lane pr = (j, k) of the p x p (x, y) rows sums its z
@@ -565,7 +566,7 @@ template <int P>
 __global__ void __launch_bounds__(256, 4) k_spme_gather_f32(int natms, int ab, const float* __restrict__ q4, SpmeGeom sg,
                                                          const int* __restrict__ gidx, const float* __restrict__ gw,
                                                          const float* __restrict__ phi, float rk0, float rk1,
-                                                         float rk2, float* __restrict__ fout, double* blk) {
+                                                         float rk2, float* __restrict__ fout, double* blk, GridSum gs) {
   __shared__ float sp[8][GATHER_AB][2][3][P];  // per warp and atom: value/derivative, dimension, point
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int nwarps = (gridDim.x * blockDim.x) >> 5;
@@ -641,6 +642,7 @@ __global__ void __launch_bounds__(256, 4) k_spme_gather_f32(int natms, int ab, c
     __syncwarp();  // the batch's splines are read before the next batch writes them
   }
   block_reduce_store<4>(acc, blk);
+  grid_finish<4>(blk, gs);
 }
 
 // a * b as an unnormalised compensated pair: the exact product's high part and, in the
@@ -694,7 +696,7 @@ __global__ void __launch_bounds__(256, 6) k_spme_gather_wdf(int natms, int ab, S
                                                          const float2* __restrict__ gq, const dfr* __restrict__ phi,
                                                          float2 rk0, float2 rk1, float2 rk2, float qmax,
                                                          const unsigned* __restrict__ vmax,
-                                                         float2* __restrict__ fout, double* blk) {
+                                                         float2* __restrict__ fout, double* blk, GridSum gs) {
   // C of off_add_prod: a power of two, at least twice the largest |charge x potential|, which
   // bounds every sum over a stencil (the spline values of a dimension are positive and add
   // up to 1, the derivatives' magnitudes to about 1)
@@ -830,6 +832,7 @@ __global__ void __launch_bounds__(256, 6) k_spme_gather_wdf(int natms, int ab, S
 #pragma unroll
   for (int c = 0; c < 4; ++c) out[c] = to_dfr(two_sum(acc[c].s, acc[c].c));
   block_reduce_store<4>(out, blk);
+  grid_finish<4>(blk, gs);
 }
 
 // FP64 form with the double-float gather: forces += (F - Fnet/N) * 2 * scale
@@ -1338,10 +1341,12 @@ void grid_run(SpmeGrid& S, bool coarse, float* rec, double* eng_rc, double* vir_
   prof_end(pid(P_FFT_Y));
   const int nbz = ntx * K2;
   double* blkz = gb_blkacc(nbz * 6 + nblocks((long long)n * 32, 128) * 4);
+  const GridSum gsz = gb_grid_sum(nbz, thz, 6, &g.sc->acc[A_SPME_STR]);
   prof_begin(pid(P_FFT_Z));
   fk.z_conv<<<nbz, thz, fft_smem(K3, TX, sizeof(T2)) + K3 * sizeof(T), st>>>(G, K1, K2, K3, S.plan[2], tw3,
-                                                                                       th, ps, S.sg, blkz);
+                                                                                       th, ps, S.sg, blkz, gsz);
   GB_LAUNCHED();
+  gb_grid_sum_done(gsz, blkz, nbz, 6);
   prof_end(pid(P_FFT_Z));
   prof_begin(pid(P_FFT_Y));
   fk.y_inv<<<ntx * K3, thy, fft_smem(K2, TX, sizeof(T2)), st>>>(G, Kx, K2, S.plan[1], tw2);
@@ -1369,6 +1374,7 @@ void grid_run(SpmeGrid& S, bool coarse, float* rec, double* eng_rc, double* vir_
   const int ab = std::max(1, std::min(GATHER_AB, n / (8 * std::max(1, slots))));
   const int nbg = warp_gather ? std::max(1, std::min(slots, nblocks((long long)nblocks(n, ab) * 32, 256))) : nblocks(n, 128);
   double* blkg = blkz + (size_t)nbz * 6;
+  const GridSum gsg = gb_grid_sum(nbg, warp_gather ? 256 : 128, 4, &g.sc->acc[A_GATHER]);
   prof_begin(pid(P_SPME_GATHER));
   if (warp_gather && DF) {
     auto kern = p == 8 ? k_spme_gather_wdf<8> : k_spme_gather_wdf<6>;
@@ -1376,20 +1382,19 @@ void grid_run(SpmeGrid& S, bool coarse, float* rec, double* eng_rc, double* vir_
     for (int a = 0; a < 3; ++a) df_split(rk[a], &rkd[a].x, &rkd[a].y);
     kern<<<nbg, 256, 0, st>>>(n, ab, S.sg, S.gidx, reinterpret_cast<const dfr*>(S.gsp),
                               reinterpret_cast<const float2*>(S.gw + 6 * (size_t)n), reinterpret_cast<const dfr*>(Q),
-                              rkd[0], rkd[1], rkd[2], S.qmax, vmax, reinterpret_cast<float2*>(S.fspme), blkg);
+                              rkd[0], rkd[1], rkd[2], S.qmax, vmax, reinterpret_cast<float2*>(S.fspme), blkg, gsg);
   } else if (warp_gather) {
     auto kern = p == 8 ? k_spme_gather_f32<8> : k_spme_gather_f32<6>;
     kern<<<nbg, 256, 0, st>>>(n, ab, reinterpret_cast<const float*>(g.xf), S.sg, S.gidx, S.gw,
                               reinterpret_cast<const float*>(Q), (float)rk[0], (float)rk[1], (float)rk[2], S.fout_f,
-                              blkg);
+                              blkg, gsg);
   } else {
     auto gather = p == 8 ? k_spme_gather<T, 8> : k_spme_gather<T, 0>;
-    gather<<<nbg, 128, 0, st>>>(n, g.x, g.y, g.z, g.chge, S.sg, Q, rk[0], rk[1], rk[2], S.fspme, blkg);
+    gather<<<nbg, 128, 0, st>>>(n, g.x, g.y, g.z, g.chge, S.sg, Q, rk[0], rk[1], rk[2], S.fspme, blkg, gsg);
   }
   GB_LAUNCHED();
   prof_end(pid(P_SPME_GATHER));
-  gb_reduce_blocks(blkz, nbz, 6, &g.sc->acc[A_SPME_STR]);
-  gb_reduce_blocks(blkg, nbg, 4, &g.sc->acc[A_GATHER]);
+  gb_grid_sum_done(gsg, blkg, nbg, 4);
   const double pi = 3.14159265358979323846264338327950288;
   const double scale = pi * std::sqrt(pi) * std::pow(g.p.alpha, 1 - 3) * (0.5 / g.volm) * g.scaling;
   unsigned long long* fixp = coarse ? nullptr : (unsigned long long*)g.fixp;
