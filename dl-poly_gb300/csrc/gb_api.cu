@@ -341,10 +341,7 @@ int compute_forces(double* eng8, double* stress9, bool do_spme, bool do_real, bo
   double e6[6] = {0, 0, 0, 0, 0, 0};
   // FP32 hi + lo positions by atom index and, for the sorted-position pair kernels, the same
   // per sorted position, and cleared force sums (one pass)
-  if (g.precision == GB_MIXED || !g.fp64_native)
-    list_pos_records(do_real && g.spos_valid && g.use_sorted);
-  else
-    integ_zero_forces();
+  list_pos_records(do_real && g.spos_valid && g.use_sorted && !(g.precision == GB_FP64 && g.fp64_native));
   const bool mts = md_step && do_spme && mts_active();
   const bool full = mts ? mts_step_needs_spme() : (do_spme && g.has_coul);
   // a learned-MTS inner step: the coarse grid, the network's inputs and inference go to the

@@ -502,7 +502,6 @@ int integ_vnl_check();
 void integ_vnl_launch();          // the displacement check
 void integ_stage1_check();        // NVE stage 1 and the displacement check in one kernel
 int integ_vnl_result();           // its decision from the copied scalars (after a wait)
-void integ_zero_forces();         // of the FP64 form by instructions; list_pos_records clears the others'
 void integ_forces_to_fp64();      // mixed: fixed point -> FP64 forces
 void integ_setup_constraints(const int32_t* listcon, const double* prmcon);
 // thermostats (gb_thermostat.cu)

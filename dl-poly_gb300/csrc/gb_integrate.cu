@@ -145,11 +145,6 @@ __global__ void k_maxdisp(int n, const double* __restrict__ hdw, double tstep, c
   if ((threadIdx.x & 31) == 0) atomicMax(out, (unsigned long long)__double_as_longlong(r2));
 }
 
-__global__ void k_zero3(int n, double* a, double* b, double* c) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) { a[i] = 0.0; b[i] = 0.0; c[i] = 0.0; }
-}
-
 __global__ void k_fix_to_fp64(int n, const long long* fixp, double* fx, double* fy, double* fz) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= n) return;
@@ -1141,11 +1136,6 @@ void integ_setup_constraints(const int32_t* listcon, const double* prmcon) {
       coop_blocks_cl = std::max(1, std::min(bps * g.nsm, nblocks(n_clusters, CL_THREADS)));
     }
   }
-}
-
-void integ_zero_forces() {
-  k_zero3<<<nblocks(g.natms, 256), 256, 0, g.stream>>>(g.natms, g.fx, g.fy, g.fz);
-  GB_LAUNCHED();
 }
 
 void integ_forces_to_fp64() {
