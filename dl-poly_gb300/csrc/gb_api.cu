@@ -196,7 +196,7 @@ void free_all() {
                   g.cell_count, g.cell_start, g.cell_lstart, g.at_list, g.sorted_pos, g.xs, g.xsf, g.list, g.blk,
                   g.list_excl, g.erfc_coef, g.erfc_coef_f, g.vdw_coef, g.vdw_coef_f,
                   g.vdw_kind, g.vdw_eps, g.vdw_sig, g.erfc_df, g.vdw_df, g.qdf, g.spos, g.xhs, g.rec, g.xlh, g.fixs, g.eat, g.loc_sp,
-                  g.tile_rows, g.tile_info, g.tile_over, g.blkacc, g.con_i, g.con_j, g.con_d0, g.dxx, g.dyy,
+                  g.tile_rows, g.tile_info, g.blkacc, g.con_i, g.con_j, g.con_d0, g.dxx, g.dyy,
                   g.dzz, g.dxt, g.dyt, g.dzt, g.dt2, g.gam, g.listot, g.acon_start, g.acon_list, g.sc, d_scratch,
                   d_scratch_s, g.blkacc_s};
   for (void* p : ptrs)
@@ -683,7 +683,7 @@ int gb_init(const gb_params* prm, int natms, const int32_t* ltype, const double*
     dalloc(&g.xbg, natms); dalloc(&g.ybg, natms); dalloc(&g.zbg, natms);
     dalloc(&g.ox, natms); dalloc(&g.oy, natms); dalloc(&g.oz, natms);
     dalloc(&g.which_cell, mx); dalloc(&g.at_list, mx); dalloc(&g.sorted_pos, mx);
-    dalloc(&g.xs, mx); dalloc(&g.xsf, mx);
+    dalloc(&g.xs, mx); dalloc(&g.xsf, mx + 8);
     g.ld = prm->max_list + 4;
     dalloc(&g.list, (size_t)g.ld * natms);
     g.ldt = ((prm->max_list + 1 + 3) / 4) * 4;  // spos(k, i), k = 1..max_list, rows 16-byte aligned

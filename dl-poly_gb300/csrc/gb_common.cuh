@@ -41,8 +41,7 @@ struct DevScalars {
   int rattle_iters;
   int converged;    // constraint iteration flag
   int ncand_fp64;   // list-build candidates resolved in FP64
-  int tile_over;    // cell tiles whose staged atoms exceed the first launch's capacity
-  int tile_max;     // most staged atoms of any cell tile
+  int tile_over;    // cell tiles whose staged atoms exceed the capacity
   int halo_fwd;     // list entries with a halo image found in the forward half shell (evaluated)
   int halo_bwd;     // list entries with a halo image found in the backward halo pass (skipped)
   unsigned count_s; // the same on the side stream
@@ -70,7 +69,7 @@ enum {
 // shell of its cells reaches, as one contiguous run of sorted positions per row
 // (dy, dz) of that shell.
 constexpr int TILE_MAX_ROWS = 32;
-constexpr int TILE_CAP_TARGET = 1600;  // staged atoms per tile of the list build's first launch
+constexpr int TILE_CAP_TARGET = 1600;  // staged atoms per tile of the list build
 constexpr int TILE_CAP_MAX = 8192;     // largest staged set a list CTA holds (20 B per atom)
 struct TilePlan {
   int m;                    // local cells per tile along x
@@ -167,12 +166,12 @@ struct Dev {
   TilePlan tp{};
   int* tile_rows = nullptr;    // ntiles x nrows x (first sorted position, slot base)
   int* tile_info = nullptr;    // ntiles x 4: staged atoms, first and end sorted position of the i atoms
-  int* tile_over = nullptr;    // ids of the tiles above the first launch's capacity
   int tiles_alloc = 0;
   int* spos = nullptr;         // natms x ldt: per list entry the partner's sorted position (-1: backward copy)
   int ldt = 0;
-  int tile_cap_list = 0;       // staged atoms per tile of the list build's first launch
-  int n_tile_over = 0, tile_max_staged = 0;   // from the last list build
+  int tile_cap_list = 0;       // staged atoms per tile of the list build
+  bool tiles_any = false;      // the tile kernel at any size (GB_TILE_CAP)
+  int n_tile_over = 0;         // not 0: tiles above it were met, the list comes from k_list_lanes
   bool spos_valid = false;     // the last list pairs every halo entry with its backward copy
   bool use_sorted = true;      // sorted-position pair kernels (GB_PAIR_SORTED=0: the atom-index kernels)
   // MD loop without learned MTS: the energy, virial and stress sums of each step are copied

@@ -24,9 +24,6 @@ namespace {
 
 constexpr int MAX_SBC = 1024;  // semi-ball offsets capacity
 
-__constant__ int c_off[MAX_SBC];   // linear cell offset of each semi-ball cell
-__constant__ int c_nix[MAX_SBC], c_niy[MAX_SBC], c_niz[MAX_SBC];
-__constant__ unsigned char c_nir[MAX_SBC];
 // for k_list_tiles, read a lane each: per semi-ball cell its linear offset and
 // (nix + 64) | (niy + 64) << 8 | (niz + 64) << 16 | nir << 24; and, as the semi-ball cells in
 // the reference order form, tile row (dy, dz) by tile row, runs of consecutive cells along x
@@ -242,7 +239,7 @@ __global__ void __launch_bounds__(1024) k_cell_scan(int n, CellGeom cg, const in
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     sc->ibig = 0;
-    sc->tile_over = sc->tile_max = sc->halo_fwd = sc->halo_bwd = 0;
+    sc->tile_over = sc->halo_fwd = sc->halo_bwd = 0;
   }
   const bool local = blockIdx.x == 1;
   const int per = ((n + 1023) / 1024) * 32, lo = min(n, wid * per), hi = min(n, lo + per);
@@ -366,7 +363,7 @@ __global__ void k_cell_scatter(const DevScalars* sc, const int* which_cell, cons
 
 __device__ __forceinline__ void tile_row(int t, const TilePlan& tp, const CellGeom& cg, const int* __restrict__ start,
                                          int* __restrict__ tile_rows, int* __restrict__ tile_info, int cap,
-                                         int* __restrict__ tile_over, DevScalars* sc);
+                                         DevScalars* sc);
 
 // Stable order inside each cell (ascending atom index, as the reference's
 // counting sort over i = 1..nlast): rank of each member by counting.  A local atom's
@@ -378,13 +375,12 @@ __global__ void __launch_bounds__(SORT_NT) k_cell_sort(int ncells_p1, int natms,
                                                        const int* tmp, int* at_list, int* sorted_pos, int* loc_sp,
                                                        const double* x, const double* y, const double* z,
                                                        double4_32a* xs, float4* xsf, TilePlan tp, CellGeom cg,
-                                                       int* tile_rows, int* tile_info, int cap, int* tile_over,
-                                                       DevScalars* sc) {
+                                                       int* tile_rows, int* tile_info, int cap, DevScalars* sc) {
   const int ncb = (ncells_p1 + SORT_NT / 32 - 1) / (SORT_NT / 32);
   if ((int)blockIdx.x >= ncb) {
     const int rb = blockIdx.x - ncb;
     if (rb >= RESID_BLOCKS) {
-      tile_row((rb - RESID_BLOCKS) * SORT_NT + threadIdx.x, tp, cg, start, tile_rows, tile_info, cap, tile_over, sc);
+      tile_row((rb - RESID_BLOCKS) * SORT_NT + threadIdx.x, tp, cg, start, tile_rows, tile_info, cap, sc);
       return;
     }
     // residual halo cell: never a neighbour cell, order irrelevant
@@ -395,7 +391,7 @@ __global__ void __launch_bounds__(SORT_NT) k_cell_sort(int ncells_p1, int natms,
       sorted_pos[v] = a;
       const double xv = x[v], yv = y[v], zv = z[v];
       xs[a] = make_double4_32a(xv, yv, zv, 0.0);
-      xsf[a] = make_float4((float)xv, (float)yv, (float)zv, 0.0f);
+      xsf[a] = make_float4((float)xv, (float)yv, (float)zv, __int_as_float(v));
     }
     return;
   }
@@ -412,126 +408,17 @@ __global__ void __launch_bounds__(SORT_NT) k_cell_sort(int ncells_p1, int natms,
     if (v < natms) loc_sp[ls + r] = pos;
     double xv = x[v], yv = y[v], zv = z[v];
     xs[pos] = make_double4_32a(xv, yv, zv, 0.0);
-    xsf[pos] = make_float4((float)xv, (float)yv, (float)zv, 0.0f);
-  }
-}
-
-// Half-shell Verlet list (neighbours.F90:876-1184): one warp per local atom.
-// Entries are appended in the reference order (semi-ball cell by cell, each
-// cell's members in ascending order), with ballot-based compaction.
-__global__ void __launch_bounds__(256) k_list_pairs(int natms, const DevScalars* sc_c, CellGeom cg, int nsbcll,
-                                                    const int* at_list, const int* which_cell, const int* start,
-                                                    const double4_32a* xs, const float4* xsf, int* list, int ld,
-                                                    int* spos, int ldt, int max_list, DevScalars* sc) {
-  const int warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const int lane = threadIdx.x & 31;
-  const int nlast = sc_c->nlast;
-  if (warp >= nlast) return;
-  const int p = warp;  // sorted position
-  const int i = at_list[p];
-  if (i >= natms) return;
-  const int ic = which_cell[i];
-  const int icm = ic - 1;
-  const int ix = icm % cg.NX;
-  const int iz = icm / (cg.NX * cg.NY);
-  const int iy = icm / cg.NX - cg.NY * iz;
-  const double4_32a xi = xs[p];
-  const float4 xif = xsf[p];
-  const int nlp = cg.nlp;
-  const int nlx0e = nlp - 1, nly0e = nlp - 1, nlz0e = nlp - 1;
-  const int nlx1s = cg.nlx + nlp, nly1s = cg.nly + nlp, nlz1s = cg.nlz + nlp;
-  int* li = list + (size_t)i * ld + 3;  // li[k] == list(k, i)
-  int* si = spos + (size_t)i * ldt;
-  int count = 0;
-  int ncand64 = 0, nfwd = 0, nbwd = 0;
-  const unsigned lt = (1u << lane) - 1u;
-  for (int pass = 1; pass <= 2; ++pass) {
-    if (pass == 2) {
-      const int ix1 = ix - nlx0e, ix2 = ix - nlx1s, iy1 = iy - nly0e, iy2 = iy - nly1s, iz1 = iz - nlz0e,
-                iz2 = iz - nlz1s;
-      bool border = (ix1 >= 1 && ix1 <= nlp) || (ix2 <= -1 && ix2 >= -nlp) || (iy1 >= 1 && iy1 <= nlp) ||
-                    (iy2 <= -1 && iy2 >= -nlp) || (iz1 >= 1 && iz1 <= nlp) || (iz2 <= -1 && iz2 >= -nlp);
-      if (!border) break;
-    }
-    for (int kk = (pass == 1 ? 0 : 1); kk < nsbcll; ++kk) {
-      int jc, s;
-      if (pass == 1) {
-        jc = ic + c_off[kk];
-        s = (jc != ic) ? start[jc] : p + 1;
-      } else {
-        int jx = ix - c_nix[kk], jy = iy - c_niy[kk], jz = iz - c_niz[kk];
-        if (!(jx <= nlx0e || jx >= nlx1s || jy <= nly0e || jy >= nly1s || jz <= nlz0e || jz >= nlz1s)) continue;
-        jc = ic - c_off[kk];
-        s = start[jc];
-      }
-      const int e = start[jc + 1];
-      const bool nir = c_nir[kk] != 0;
-      for (int b = s; b < e; b += 32) {
-        const int jj = b + lane;
-        bool acc = false;
-        if (jj < e) {
-          if (nir) {
-            acc = true;
-          } else {
-            float4 xj = xsf[jj];
-            float dx = xj.x - xif.x, dy = xj.y - xif.y, dz = xj.z - xif.z;
-            float r2 = dx * dx + dy * dy + dz * dz;
-            if (r2 < cg.rcsq_lo) {
-              acc = true;
-            } else if (r2 <= cg.rcsq_hi) {
-              double4_32a xd = xs[jj];
-              double ddx = sub_rn(xd.x, xi.x), ddy = sub_rn(xd.y, xi.y), ddz = sub_rn(xd.z, xi.z);
-              double rsq = add_rn(add_rn(mul_rn(ddx, ddx), mul_rn(ddy, ddy)), mul_rn(ddz, ddz));
-              acc = rsq <= cg.rcsq;
-              ++ncand64;
-            }
-          }
-        }
-        const unsigned m = __ballot_sync(0xffffffffu, acc);
-        if (acc) {
-          const int k = count + __popc(m & lt) + 1;
-          const int a = at_list[jj];
-          if (pass == 1) nfwd += a >= natms;
-          else ++nbwd;
-          if (k <= max_list) {
-            li[k] = a + 1;
-            si[k] = pass == 1 ? jj : -1;
-          }
-        }
-        count += __popc(m);
-      }
-    }
-  }
-  ncand64 = warp_sumi(ncand64);
-  nfwd = warp_sumi(nfwd);
-  nbwd = warp_sumi(nbwd);
-  if (lane == 0) {
-    if (nfwd) atomicAdd(&sc->halo_fwd, nfwd);
-    if (nbwd) atomicAdd(&sc->halo_bwd, nbwd);
-  }
-  if (lane == 0) {
-    // the stored length never exceeds max_list, so no later kernel can read
-    // past the column even when the overflow status is ignored
-    const int stored = min(count, max_list);
-    li[0] = stored;
-    li[-1] = stored;
-    li[-2] = stored;
-    li[-3] = stored;
-    if (count > max_list) {
-      atomicOr(&sc->status, ST_LIST_OVERFLOW);
-      atomicMax(&sc->ibig, count);
-    }
-    if (ncand64) atomicAdd(&sc->ncand_fp64, ncand64);
+    xsf[pos] = make_float4((float)xv, (float)yv, (float)zv, __int_as_float(v));
   }
 }
 
 // Row tables of the cell tiles: per row (dy, dz) the first sorted position of its x run
 // of cells and its slot base in the tile's staged set; per tile the staged total and the
-// sorted-position range of its own (i) atoms.  Tiles above the capacity of the first
-// launches go to tile_over for a second launch with more shared memory.
+// sorted-position range of its own (i) atoms.  Tiles above the capacity are counted: the
+// list then comes from k_list_lanes.
 __device__ __forceinline__ void tile_row(int t, const TilePlan& tp, const CellGeom& cg, const int* __restrict__ start,
                                          int* __restrict__ tile_rows, int* __restrict__ tile_info, int cap,
-                                         int* __restrict__ tile_over, DevScalars* sc) {
+                                         DevScalars* sc) {
   if (t >= tp.ntiles) return;
   const int tx = t % tp.ntx, ty = (t / tp.ntx) % tp.nty, tz = t / (tp.ntx * tp.nty);
   const int nlp = cg.nlp;
@@ -551,16 +438,10 @@ __device__ __forceinline__ void tile_row(int t, const TilePlan& tp, const CellGe
   tile_info[4 * t + 1] = start[1 + x0 + plane];
   tile_info[4 * t + 2] = start[1 + (x1 - 1) + plane + 1];
   tile_info[4 * t + 3] = 0;
-  if (base > cap) tile_over[atomicAdd(&sc->tile_over, 1)] = t;
-  atomicMax(&sc->tile_max, base);
+  if (base > cap) atomicAdd(&sc->tile_over, 1);
 }
 
-__global__ void k_tile_rows(TilePlan tp, CellGeom cg, const int* __restrict__ start, int* __restrict__ tile_rows,
-                            int* __restrict__ tile_info, int cap, int* __restrict__ tile_over, DevScalars* sc) {
-  tile_row(blockIdx.x * blockDim.x + threadIdx.x, tp, cg, start, tile_rows, tile_info, cap, tile_over, sc);
-}
-
-// Half-shell Verlet list (neighbours.F90:876-1184), one CTA per cell tile: the tile's
+// Half-shell Verlet list (neighbours.F90:876-1184) of a small system, several CTAs per cell tile: the tile's
 // forward half shell (FP32 positions and atom ids) is staged in shared memory and one
 // warp per local atom walks it in the reference order (semi-ball cell by cell, each
 // cell's members in ascending order), one run of consecutive cells at a time, with
@@ -568,12 +449,11 @@ __global__ void k_tile_rows(TilePlan tp, CellGeom cg, const int* __restrict__ st
 // sorted position, or -1 for the entries of the backward halo pass (pass 2), whose
 // pairs the partner atom's forward pass also lists, so that the pair kernels evaluate
 // each pair once, from its forward copy.  Bound by issue in pass 1 and by the latency of
-// its loads in pass 2, whose cells are read from global memory: with the bounds of 32 cells
-// or runs loaded at once and pass 2's members taken as one sequence, a build takes 0.37
-// instead of 0.54 ms (98,304-atom water), 0.48 instead of 0.81 ms (175,616 ions) and 0.047
-// instead of 0.145 ms (1,536 atoms, where seven CTAs share a tile).
+// its loads in pass 2, whose cells are read from global memory: 32 cells' bounds are loaded
+// at once and their members taken as one sequence (0.048 ms for 1,536 atoms, where seven CTAs
+// share a tile; k_list_lanes takes 0.061 there and 0.059 instead of 0.062 at 4,096).
 __global__ void __launch_bounds__(256) k_list_tiles(int natms, CellGeom cg, TilePlan tp, int nsbcll, int nseg,
-                                                    const int* __restrict__ tile_ids, int cap,
+                                                    int cap,
                                                     const int* __restrict__ tile_rows, const int* __restrict__ tile_info,
                                                     const int* __restrict__ at_list, const int* __restrict__ which_cell,
                                                     const int* __restrict__ start, const double4_32a* __restrict__ xs,
@@ -582,9 +462,9 @@ __global__ void __launch_bounds__(256) k_list_tiles(int natms, CellGeom cg, Tile
   extern __shared__ float4 s_x[];  // cap staged FP32 positions, then cap atom ids
   int* s_at = reinterpret_cast<int*>(s_x + cap);
   __shared__ int s_first[TILE_MAX_ROWS], s_base[TILE_MAX_ROWS + 1];
-  const int t = tile_ids ? tile_ids[blockIdx.x] : blockIdx.x;
+  const int t = blockIdx.x;
   const int nst = tile_info[4 * t];
-  if (nst > cap) return;  // the overflow launch builds this tile (uniform over the CTA)
+  if (nst > cap) return;  // k_list_lanes then builds the list (uniform over the CTA)
   const int nrows = tp.nrows;
   if (threadIdx.x < nrows) {
     s_first[threadIdx.x] = tile_rows[2 * (t * nrows + threadIdx.x)];
@@ -759,6 +639,220 @@ __global__ void __launch_bounds__(256) k_list_tiles(int natms, CellGeom cg, Tile
         atomicOr(&sc->status, ST_LIST_OVERFLOW);
         atomicMax(&sc->ibig, count);
       }
+    }
+  }
+  ncand64 = warp_sumi(ncand64);
+  nfwd = warp_sumi(nfwd);
+  nbwd = warp_sumi(nbwd);
+  if (lane == 0) {
+    if (ncand64) atomicAdd(&sc->ncand_fp64, ncand64);
+    if (nfwd) atomicAdd(&sc->halo_fwd, nfwd);
+    if (nbwd) atomicAdd(&sc->halo_bwd, nbwd);
+  }
+}
+
+// Half-shell Verlet list (neighbours.F90:876-1184), G lanes per local atom: the 32 / G
+// consecutive local atoms of a warp (in sorted order: one or two cells) walk the reference's
+// order of their own shells together, pass 1 run by run of consecutive cells, pass 2 (the backward
+// cells that are halo cells) cell by cell.  The atoms of a cell read the same candidates, LANE_U
+// consecutive ones per lane and step; an atom's lanes add up their accepted ones, which go to the
+// atom's column in shared memory, and the warp writes the columns as rows of list(k, i) and
+// spos(k, i) when one is nearly full.  A step with a candidate that FP32 cannot decide takes
+// FP64 for that one.
+// Beside list(k, i) the kernel writes spos(k, i): the partner's sorted position, or -1 for
+// the entries of pass 2, whose pairs the partner atom's forward pass also lists, so that
+// the pair kernels evaluate each pair once, from its forward copy.
+// A warp per atom, its lanes over the candidates of a staged cell tile (k_list_tiles), spends 76
+// instructions on 32 candidates, most of them on the compaction.  In ms, that kernel and this
+// one (with G lanes per atom and U candidates per lane and step):
+//                            tiles   2, 4    4, 4    8, 2    16, 2
+//   4,096 ions               0.062   0.117   0.079   0.073   0.059
+//   6,591-atom water         0.106   0.130   0.087   0.080   0.065
+//   13,824 ions              0.105   0.110   0.079   0.077   0.091
+//   46,656 ions              0.189   0.127   0.136   0.160   0.215
+//   98,304-atom water        0.370   0.274   0.283   0.336   0.434
+//   262,144 ions             0.697   0.445   0.509   0.632   0.891
+// More lanes per atom shorten a warp's walk, which is what few warps wait for; fewer lanes
+// waste fewer candidates at the ends of runs and cells.  Bound by issue and L1 reads at 262,144.
+constexpr int LANE_NT = 64, LANE_CAP = 64, LANE_LD = LANE_CAP + 1;
+template <int G, int LANE_U>
+__global__ void __launch_bounds__(LANE_NT) k_list_lanes(int natms, CellGeom cg, int nsbcll, int nseg,
+                                                        const int* __restrict__ loc_sp, const int* __restrict__ at_list,
+                                                        const int* __restrict__ which_cell,
+                                                        const int* __restrict__ start,
+                                                        const double4_32a* __restrict__ xs,
+                                                        const float4* __restrict__ xsf, int* __restrict__ list, int ld,
+                                                        int* __restrict__ spos, int ldt, int max_list, DevScalars* sc) {
+  constexpr int NA = 32 / G, STEP = G * LANE_U;  // atoms per warp, candidates per step
+  static_assert(STEP <= LANE_CAP / 2, "a step fits the column");
+  __shared__ int2 s_buf[LANE_NT / 32][NA * LANE_LD];
+  const int lane = threadIdx.x & 31, r = lane % G, w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (w * NA >= natms) return;
+  int2* buf = s_buf[threadIdx.x >> 5];
+  int2* const col = buf + (lane / G) * LANE_LD;
+  const bool on = w * NA + lane / G < natms;
+  const int p = loc_sp[min(w * NA + lane / G, natms - 1)];
+  const int i = at_list[p], ic = which_cell[i];
+  const float4 xif = xsf[p];
+  int cnt = 0, pend = 0;  // entries written, entries in the column
+  int ncand64 = 0, nfwd = 0, nbwd = 0;
+
+  auto flush = [&]() {
+    __syncwarp();
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+      const int n = __shfl_sync(0xffffffffu, pend, a * G), il = __shfl_sync(0xffffffffu, i, a * G),
+                k0 = __shfl_sync(0xffffffffu, cnt, a * G) + 1;
+      for (int e = lane; e < n; e += 32) {
+        const int2 v = buf[a * LANE_LD + e];
+        const int k = k0 + e;
+        if (v.y < 0) ++nbwd;
+        else if (v.x >= natms) ++nfwd;
+        if (k <= max_list) {
+          list[(size_t)il * ld + 3 + k] = v.x + 1;
+          spos[(size_t)il * ldt + k] = v.y;
+        }
+      }
+    }
+    __syncwarp();
+    cnt += pend;
+    pend = 0;
+  };
+  // the lines of the next candidates, a lane each, into L1
+  auto touch = [&](int s0, int e) {
+    const int jj = s0 + 8 * (lane & 7);
+    float v;
+    if (jj < e) asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(&xsf[jj].x));
+  };
+  // the candidates [s0, e) of each atom, in step; back: pass 2, whose entries carry -1.  (Up
+  // to LANE_U - 1 records beyond e are read, and not used: xsf has room for them.)
+  const float mid = 0.5f * (cg.rcsq_lo + cg.rcsq_hi), half = 0.5f * (cg.rcsq_hi - cg.rcsq_lo);
+  auto walk = [&](int s0, int e, bool nir, bool back) {
+    const int len = __reduce_max_sync(0xffffffffu, e - s0);
+    const float cut = nir ? 3.0e38f : mid, undecided = nir ? -1.f : 1.01f * half;
+    float4 xn[LANE_U];
+    auto load = [&](int jj) {
+      const float4* q = xsf + (jj < e ? jj : p);
+#pragma unroll
+      for (int u = 0; u < LANE_U; ++u) xn[u] = q[u];
+    };
+    if (len > 0) load(s0 + r * LANE_U);
+    for (int t = 0; t < len; t += STEP) {
+      const int jj = s0 + t + r * LANE_U, rem = e - jj;
+      float r2[LANE_U], b = 3.0e38f;
+      int id[LANE_U];
+#pragma unroll
+      for (int u = 0; u < LANE_U; ++u) {
+        const float dx = xn[u].x - xif.x, dy = xn[u].y - xif.y, dz = xn[u].z - xif.z;
+        r2[u] = dx * dx + dy * dy + dz * dz;
+        b = fminf(b, fabsf(r2[u] - cut));
+        id[u] = __float_as_int(xn[u].w);
+      }
+      if (t + STEP < len) load(jj + STEP);
+      unsigned m = 0;
+#pragma unroll
+      for (int u = 0; u < LANE_U; ++u)
+        if (u < rem && r2[u] < cut) m |= 1u << u;
+      if (__any_sync(0xffffffffu, b <= undecided)) {
+#pragma unroll
+        for (int u = 0; u < LANE_U; ++u)
+          if (u < rem && r2[u] >= cg.rcsq_lo && r2[u] <= cg.rcsq_hi) {
+            const double4_32a xi = xs[p], xd = xs[jj + u];
+            const double ddx = sub_rn(xd.x, xi.x), ddy = sub_rn(xd.y, xi.y), ddz = sub_rn(xd.z, xi.z);
+            const bool ok = add_rn(add_rn(mul_rn(ddx, ddx), mul_rn(ddy, ddy)), mul_rn(ddz, ddz)) <= cg.rcsq;
+            m = (m & ~(1u << u)) | (nir || ok ? 1u << u : 0u);
+            ++ncand64;
+          }
+        __syncwarp();
+      }
+      const int c = __popc(m);
+      int inc = c;
+#pragma unroll
+      for (int o = 1; o < G; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, inc, o, G);
+        if (r >= o) inc += v;
+      }
+      int2* at = col + (pend + inc - c);
+#pragma unroll
+      for (int u = 0; u < LANE_U; ++u)
+        if ((m >> u) & 1u) *at++ = make_int2(id[u], back ? -1 : jj + u);
+      pend += __shfl_sync(0xffffffffu, inc, G - 1, G);
+      if (__any_sync(0xffffffffu, pend > LANE_CAP - STEP)) flush();
+    }
+  };
+
+  // pass 1 (the bounds of the run after the next and the lines of the next are on their way
+  // while this one is walked)
+  {
+    int s0 = p + 1, e = start[ic + d_seg[0].y + 1], s1 = 0, e1 = 0;  // segment 0 starts with the own cell
+    if (nseg > 1) {
+      s1 = start[ic + d_seg[1].x];
+      e1 = start[ic + d_seg[1].y + 1];
+    }
+    touch(s0, e);
+    for (int q = 0; q < nseg; ++q) {
+      int s2 = 0, e2 = 0;
+      if (q + 2 < nseg) {
+        const int4 d = d_seg[q + 2];
+        s2 = start[ic + d.x];
+        e2 = start[ic + d.y + 1];
+      }
+      touch(s1, e1);
+      walk(s0, on ? e : s0, d_seg[q].w != 0, false);
+      s0 = s1; e = e1;
+      s1 = s2; e1 = e2;
+    }
+  }
+  // pass 2: backward cells that are halo cells (border atoms only)
+  {
+    const int icm = ic - 1, ix = icm % cg.NX, iz = icm / (cg.NX * cg.NY), iy = icm / cg.NX - cg.NY * iz;
+    const int nlp = cg.nlp, nl0e = nlp - 1;
+    const int nlx1s = cg.nlx + nlp, nly1s = cg.nly + nlp, nlz1s = cg.nlz + nlp;
+    const int ix1 = ix - nl0e, ix2 = ix - nlx1s, iy1 = iy - nl0e, iy2 = iy - nly1s, iz1 = iz - nl0e, iz2 = iz - nlz1s;
+    const bool border = on && ((ix1 >= 1 && ix1 <= nlp) || (ix2 <= -1 && ix2 >= -nlp) || (iy1 >= 1 && iy1 <= nlp) ||
+                               (iy2 <= -1 && iy2 >= -nlp) || (iz1 >= 1 && iz1 <= nlp) || (iz2 <= -1 && iz2 >= -nlp));
+    auto bounds = [&](int k, int& s0, int& e) {
+      s0 = e = 0;
+      if (!border || k >= nsbcll) return;
+      const int2 d = d_sbc[k];
+      const int jx = ix - ((d.y & 255) - 64), jy = iy - (((d.y >> 8) & 255) - 64), jz = iz - (((d.y >> 16) & 255) - 64);
+      if (jx <= nl0e || jx >= nlx1s || jy <= nl0e || jy >= nly1s || jz <= nl0e || jz >= nlz1s) {
+        s0 = start[ic - d.x];
+        e = start[ic - d.x + 1];
+      }
+    };
+    if (__any_sync(0xffffffffu, border)) {
+      int s0, e, s1, e1, s2, e2, s3, e3, s4, e4;
+      bounds(1, s0, e);
+      bounds(2, s1, e1);
+      bounds(3, s2, e2);
+      bounds(4, s3, e3);
+      touch(s0, e);
+      touch(s1, e1);
+      for (int k = 1; k < nsbcll; ++k) {
+        bounds(k + 4, s4, e4);
+        touch(s2, e2);
+        walk(s0, e, d_sbc[k].y >> 24 != 0, true);
+        s0 = s1; e = e1;
+        s1 = s2; e1 = e2;
+        s2 = s3; e2 = e3;
+        s3 = s4; e3 = e4;
+      }
+    }
+  }
+  flush();
+  if (on && r == 0) {
+    // the stored length never exceeds max_list, so no later kernel can read
+    // past the column even when the overflow status is ignored
+    int* li = list + (size_t)i * ld + 3;
+    const int stored = min(cnt, max_list);
+    li[0] = stored;
+    li[-1] = stored;
+    li[-2] = stored;
+    li[-3] = stored;
+    if (cnt > max_list) {
+      atomicOr(&sc->status, ST_LIST_OVERFLOW);
+      atomicMax(&sc->ibig, cnt);
     }
   }
   ncand64 = warp_sumi(ncand64);
@@ -1030,22 +1124,19 @@ void list_setup() {
     tp.ntx = (nlx + m - 1) / m; tp.nty = nly; tp.ntz = nlz;
     tp.ntiles = tp.ntx * tp.nty * tp.ntz;
     int cap = (int)(1.3 * cells_of(m) * apc) + 64;
-    const char* ec = getenv("GB_TILE_CAP");  // a smaller first-launch capacity sends more tiles to the second launch
-    if (ec && atoi(ec) > 0) cap = atoi(ec);
+    const char* ec = getenv("GB_TILE_CAP");  // this capacity, and the tile kernel at any size
+    g.tiles_any = ec && atoi(ec) > 0;
+    if (g.tiles_any) cap = atoi(ec);
     g.tile_cap_list = std::min(((cap + 31) / 32) * 32, (int)TILE_CAP_MAX);
+    g.n_tile_over = 0;
+    GB_CUDA(cudaFuncSetAttribute(k_list_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, 20 * TILE_CAP_MAX));
     if (g.tiles_alloc < tp.ntiles) {
-      cudaFree(g.tile_rows); cudaFree(g.tile_info); cudaFree(g.tile_over);
+      cudaFree(g.tile_rows); cudaFree(g.tile_info);
       GB_CUDA(cudaMalloc(&g.tile_rows, sizeof(int) * 2 * (size_t)tp.ntiles * TILE_MAX_ROWS));
       GB_CUDA(cudaMalloc(&g.tile_info, sizeof(int) * 4 * (size_t)tp.ntiles));
-      GB_CUDA(cudaMalloc(&g.tile_over, sizeof(int) * (size_t)tp.ntiles));
       g.tiles_alloc = tp.ntiles;
     }
   }
-  GB_CUDA(cudaMemcpyToSymbol(c_off, off.data(), sizeof(int) * off.size()));
-  GB_CUDA(cudaMemcpyToSymbol(c_nix, nix.data(), sizeof(int) * nix.size()));
-  GB_CUDA(cudaMemcpyToSymbol(c_niy, niy.data(), sizeof(int) * niy.size()));
-  GB_CUDA(cudaMemcpyToSymbol(c_niz, niz.data(), sizeof(int) * niz.size()));
-  GB_CUDA(cudaMemcpyToSymbol(c_nir, nir.data(), nir.size()));
   for (int k = 0; k < 9; ++k) h_cg.rc[k] = h_halo.rc[k];
   h_cg.xdc = (double)(nlx * 1); h_cg.ydc = (double)(nly * 1); h_cg.zdc = (double)(nlz * 1);
   h_cg.nlp = nlp; h_cg.nlx = nlx; h_cg.nly = nly; h_cg.nlz = nlz;
@@ -1126,6 +1217,7 @@ int list_build() {
   const int mx = g.mxatms;
   const TilePlan& tp = g.tp;
   const int cap = g.tile_cap_list;
+  bool tiles = (g.natms / 2 < 12 * g.nsm || g.tiles_any) && g.n_tile_over == 0;
   prof_begin(P_BIN);
   k_bin<<<nblocks(mx, T), T, 0, st>>>(g.natms, g.sc, g.x, g.y, g.z, h_cg, g.which_cell, g.cell_count);
   GB_LAUNCHED();
@@ -1134,64 +1226,44 @@ int list_build() {
   int* tmp = gb_scan_scratch(mx + 1);
   k_cell_scatter<<<nblocks(mx, T), T, 0, st>>>(g.sc, g.which_cell, g.cell_start, g.cell_count, tmp);
   GB_LAUNCHED();
-  k_cell_sort<<<nblocks(g.ncells + 1, SORT_NT / 32) + RESID_BLOCKS + nblocks(tp.ntiles, SORT_NT), SORT_NT, 0, st>>>(
+  k_cell_sort<<<nblocks(g.ncells + 1, SORT_NT / 32) + RESID_BLOCKS + (tiles ? nblocks(tp.ntiles, SORT_NT) : 0), SORT_NT,
+                0, st>>>(
       g.ncells + 1, g.natms, g.cell_start, g.cell_lstart, tmp, g.at_list, g.sorted_pos, g.loc_sp, g.x, g.y, g.z, g.xs,
-      g.xsf, tp, h_cg, g.tile_rows, g.tile_info, cap, g.tile_over, g.sc);
+      g.xsf, tp, h_cg, g.tile_rows, g.tile_info, cap, g.sc);
   GB_LAUNCHED();
   prof_end(P_BIN);
   prof_begin(P_LIST);
-  // few tiles: several CTAs share a tile's atoms (each stages its whole shell), so that
-  // the device has about three CTAs per SM
-  const int split = std::max(1, std::min(8, 3 * g.nsm / std::max(tp.ntiles, 1)));
-  GB_CUDA(cudaFuncSetAttribute(k_list_tiles, cudaFuncAttributeMaxDynamicSharedMemorySize, 20 * TILE_CAP_MAX));
-  // The host waits once, after the last kernel, unless the previous build had tiles above
-  // the first launch's capacity: then it looks before the second launch.  The first build
-  // that meets such tiles runs its kernels again with that launch.
-  for (bool again = false;; again = true) {
-    if (again) {
-      GB_CUDA(cudaMemsetAsync(&g.sc->ibig, 0, sizeof(int), st));
-      GB_CUDA(cudaMemsetAsync(&g.sc->tile_over, 0, 4 * sizeof(int), st));  // tile_over, tile_max, halo_fwd, halo_bwd
-      k_tile_rows<<<nblocks(tp.ntiles, 128), 128, 0, st>>>(tp, h_cg, g.cell_start, g.tile_rows, g.tile_info, cap,
-                                                            g.tile_over, g.sc);
-      GB_LAUNCHED();
+  // The lanes per atom by the warps per SM that they give (the table at k_list_lanes); below
+  // 12 with the most lanes the tiles' CTAs, which share a tile's atoms, are faster.
+  const int n = g.natms, nsm = g.nsm;
+  const int G = n / 16 >= 10 * nsm ? 2 : n / 4 >= 16 * nsm ? 8 : 16;
+  auto lanes = G == 2 ? k_list_lanes<2, 4> : G == 8 ? k_list_lanes<8, 2> : k_list_lanes<16, 2>;
+  for (;;) {
+    if (tiles) {
+      // several CTAs share a tile's atoms (each stages its whole shell), so that the device has
+      // about three CTAs per SM
+      const int split = std::max(1, std::min(8, 3 * nsm / std::max(tp.ntiles, 1)));
+      k_list_tiles<<<dim3(tp.ntiles, split), 256, (size_t)cap * 20, st>>>(
+          n, h_cg, tp, g.nsbcll, g.nseg, cap, g.tile_rows, g.tile_info, g.at_list, g.which_cell, g.cell_start, g.xs,
+          g.xsf, g.list, g.ld, g.spos, g.ldt, g.p.max_list, g.sc);
+    } else {
+      lanes<<<nblocks((long long)n * G, LANE_NT), LANE_NT, 0, st>>>(
+          n, h_cg, g.nsbcll, g.nseg, g.loc_sp, g.at_list, g.which_cell, g.cell_start, g.xs, g.xsf, g.list, g.ld, g.spos,
+          g.ldt, g.p.max_list, g.sc);
     }
-    k_list_tiles<<<dim3(tp.ntiles, split), 256, (size_t)cap * 20, st>>>(
-        g.natms, h_cg, tp, g.nsbcll, g.nseg, nullptr, cap, g.tile_rows, g.tile_info, g.at_list, g.which_cell,
-        g.cell_start, g.xs, g.xsf, g.list, g.ld, g.spos, g.ldt, g.p.max_list, g.sc);
     GB_LAUNCHED();
-    const bool looked = g.n_tile_over > 0;
-    if (looked) {
-      gb_sync_scalars();
-      g.n_tile_over = g.hsc->tile_over;
-      g.tile_max_staged = g.hsc->tile_max;
-      if (g.n_tile_over > 0 && g.tile_max_staged <= TILE_CAP_MAX) {
-        // the tiles above the capacity, with shared memory for the largest of them
-        k_list_tiles<<<g.n_tile_over, 256, (size_t)g.tile_max_staged * 20, st>>>(
-            g.natms, h_cg, tp, g.nsbcll, g.nseg, g.tile_over, g.tile_max_staged, g.tile_rows, g.tile_info, g.at_list,
-            g.which_cell, g.cell_start, g.xs, g.xsf, g.list, g.ld, g.spos, g.ldt, g.p.max_list, g.sc);
-        GB_LAUNCHED();
-      } else if (g.n_tile_over > 0) {
-        // a tile too dense for one CTA's shared memory: the whole list from the per-atom kernel
-        GB_CUDA(cudaMemsetAsync(&g.sc->halo_fwd, 0, 2 * sizeof(int), st));
-        k_list_pairs<<<nblocks((long long)mx * 32, T), T, 0, st>>>(g.natms, g.sc, h_cg, g.nsbcll, g.at_list,
-                                                                   g.which_cell, g.cell_start, g.xs, g.xsf, g.list,
-                                                                   g.ld, g.spos, g.ldt, g.p.max_list, g.sc);
-        GB_LAUNCHED();
-      }
-    }
-    if (g.lbook || g.megfrz > 1) {  // (lists of tiles not built yet hold valid older entries, or none)
-      k_list_reorder<<<nblocks((long long)g.natms * 32, 256), 256, 0, st>>>(g.natms, g.list, g.ld, g.spos, g.ldt,
-                                                                            g.lfrzn, g.ltg, g.list_excl,
-                                                                            g.p.max_exclude + 1, g.megfrz,
-                                                                            g.lbook ? 1 : 0);
+    if (g.lbook || g.megfrz > 1) {  // (lists of tiles left out hold valid older entries, or none)
+      k_list_reorder<<<nblocks((long long)n * 32, 256), 256, 0, st>>>(n, g.list, g.ld, g.spos, g.ldt, g.lfrzn, g.ltg,
+                                                                      g.list_excl, g.p.max_exclude + 1, g.megfrz,
+                                                                      g.lbook ? 1 : 0);
       GB_LAUNCHED();
     }
     gb_sync_scalars();
-    if (looked || g.hsc->tile_over == 0) {
-      g.tile_max_staged = g.hsc->tile_max;
-      break;
-    }
-    g.n_tile_over = g.hsc->tile_over;
+    if (!tiles || g.hsc->tile_over == 0) break;
+    g.n_tile_over = g.hsc->tile_over;  // denser tiles than planned: this list and the later ones from the other kernel
+    tiles = false;
+    GB_CUDA(cudaMemsetAsync(&g.sc->ibig, 0, sizeof(int), st));
+    GB_CUDA(cudaMemsetAsync(&g.sc->halo_fwd, 0, 2 * sizeof(int), st));  // halo_fwd, halo_bwd
   }
   prof_end(P_LIST);
   if (g.hsc->status & ST_HALO_OVERFLOW) return GB_ERR_HALO;  // (list_relocate_and_halo without its wait)

@@ -332,7 +332,7 @@ int gb_set_overlap(int enable);
  * [3] list entries with a halo image from the forward half shell, [4] from the
  * backward halo pass (equal when every such pair is listed from both atoms),
  * [5] 1 when the pair kernels walked the sorted-position list, [6] list-build
- * tiles of the second (larger shared memory) launch, [7] link cells per tile along x. */
+ * tiles above the planned capacity (small systems), [7] link cells per tile along x. */
 int gb_pair_counts(int64_t* out, int n);
 
 /* FP64 FMA throughput of this device in TFLOP/s, measured by a register-

@@ -47,3 +47,16 @@ def test_halo_runs_longer_than_a_pass(gpu_lib, oracle_lib, monkeypatch, blocks):
                                   lambda: systems.nacl_melt(22, kmax=64)])
 def test_small_and_ragged_boxes(gpu_lib, oracle_lib, make):
     _same(*_lists(gpu_lib, oracle_lib, make()))
+
+
+@pytest.mark.parametrize("molecules", [11, 15, 21])
+def test_lanes_per_atom(gpu_lib, oracle_lib, molecules):
+    """3,993, 10,125 and 27,783 atoms: each number of lanes per atom, with a last warp that has
+    fewer atoms than the others."""
+    _same(*_lists(gpu_lib, oracle_lib, systems.spce_water(molecules, kmax=64)))
+
+
+def test_tiles_above_their_capacity(gpu_lib, oracle_lib, monkeypatch):
+    monkeypatch.setenv("GB_TILE_CAP", "64")
+    _same(*_lists(gpu_lib, oracle_lib, systems.spce_water(8)))
+    monkeypatch.delenv("GB_TILE_CAP")
