@@ -18,7 +18,8 @@
 
 namespace gbspme {
 
-constexpr int TX = 4;  // columns per tile in the strided passes
+constexpr int TX = 4;      // columns per tile in the strided passes
+constexpr int XLINES = 8;  // rows per block in the x passes
 
 struct FftPlan {
   int N;
@@ -36,8 +37,8 @@ struct SpmeGeom {
 // the five FFT kernels one grid launches, for working type T (complex T2)
 template <typename T, typename T2>
 struct FftKernels {
-  void (*x_fwd)(const T*, T2*, FftPlan, const T2*, const T2*, int, int);
-  void (*x_inv)(const T2*, T*, FftPlan, const T2*, const T2*, int, int, unsigned*);
+  void (*x_fwd)(const T*, T2*, FftPlan, const T2*, const T2*, int);
+  void (*x_inv)(const T2*, T*, FftPlan, const T2*, const T2*, int, unsigned*);
   void (*y_fwd)(T2*, int, int, FftPlan, const T2*);
   void (*y_inv)(T2*, int, int, FftPlan, const T2*);
   void (*z_conv)(T2*, int, int, int, FftPlan, const T2*, const T*, const T*, SpmeGeom, double*, GridSum);
@@ -147,19 +148,33 @@ __device__ __forceinline__ void bfly(const T2 (&v)[5], T2 (&o)[5]) {
   }
 }
 
+// Elements between the lines in shared memory.  The lanes of a warp take the lines in turn
+// (lane % LN), so that LN lanes share a butterfly's place in the line and its twiddles, and no
+// index needs a division by the line's length.  With ld = 3 mod 8 (16-byte elements) or 5 mod
+// 16 the strided stores of the first stage reach all banks, and its loads and the
+// transposed fill of the y and z passes nearly all.  With line after line, 32 places and twiddles
+// per warp, the passes were bound by shared memory and L1: the
+// y pass of a 160^3 double-float grid took 0.050 ms, now 0.044; ten MD steps on a 192^3 grid 24.0
+// and now 23.6 ms; the double-precision z pass of a 72^3 grid 0.062 and now 0.047 ms.
+// Lines above 1024 stay unpadded, for the shared memory.
+template <typename T2>
+__host__ __device__ constexpr int fft_ld(int n) {
+  return n > 1024 ? n : sizeof(T2) == 16 ? n + ((3 - n) & 7) : n + ((5 - n) & 15);
+}
+
 // one Stockham stage over nlines lines of length N held in shared memory.
 // The twiddle index r*k*step stays below N (k < Ns, r < R, step = N/(Ns R)).
-template <typename T, typename T2, int ISIGN>
+template <typename T, typename T2, int ISIGN, int LN>
 __device__ void fft_stage(const T2* __restrict__ in, T2* __restrict__ out, int N, int nlines, int R, int Ns,
                           const T2* __restrict__ tw) {
   const int T_ = N / R;
-  const int total = nlines * T_;
+  const int total = LN * T_, LD = fft_ld<T2>(N);
   for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-    const int line = idx / T_;
-    const int j = idx - line * T_;
+    const int line = idx % LN, j = idx / LN;
+    if (line >= nlines) continue;
     const int k = j % Ns;
-    const T2* src = in + line * N;
-    T2* dst = out + line * N;
+    const T2* src = in + line * LD;
+    T2* dst = out + line * LD;
     T2 v[5];
 #pragma unroll 5
     for (int r = 0; r < 5; ++r)
@@ -180,7 +195,7 @@ __device__ void fft_stage(const T2* __restrict__ in, T2* __restrict__ out, int N
     else if (R == 2) bfly<T, T2, ISIGN, 2>(v, o);
     else if (R == 3) bfly<T, T2, ISIGN, 3>(v, o);
     else bfly<T, T2, ISIGN, 5>(v, o);
-    const int base = (j / Ns) * Ns * R + k;
+    const int base = (j - k) * R + k;  // (j / Ns) Ns R + k
 #pragma unroll 5
     for (int r = 0; r < 5; ++r)
       if (r < R) dst[base + r * Ns] = o[r];
@@ -188,12 +203,12 @@ __device__ void fft_stage(const T2* __restrict__ in, T2* __restrict__ out, int N
 }
 
 // full transform of nlines lines; returns the buffer holding the result
-template <typename T, typename T2, int ISIGN>
+template <typename T, typename T2, int ISIGN, int LN>
 __device__ T2* fft_lines(T2* a, T2* b, const FftPlan& pl, int nlines, const T2* tw) {
   int Ns = 1;
   for (int s = 0; s < pl.nrad; ++s) {
     __syncthreads();
-    fft_stage<T, T2, ISIGN>(a, b, pl.N, nlines, pl.rad[s], Ns, tw);
+    fft_stage<T, T2, ISIGN, LN>(a, b, pl.N, nlines, pl.rad[s], Ns, tw);
     Ns *= pl.rad[s];
     T2* t = a; a = b; b = t;
   }
@@ -208,18 +223,18 @@ __device__ T2* fft_lines(T2* a, T2* b, const FftPlan& pl, int nlines, const T2* 
 template <int M>
 constexpr int next_radix() { return M % 4 == 0 ? 4 : (M % 3 == 0 ? 3 : (M % 5 == 0 ? 5 : 2)); }
 
-template <typename T, typename T2, int ISIGN, int N, int R, int Ns>
+template <typename T, typename T2, int ISIGN, int N, int R, int Ns, int LN>
 __device__ __forceinline__ void fft_stage_ct(const T2* __restrict__ in, T2* __restrict__ out, int nlines,
                                              const T2* __restrict__ tw) {
   constexpr int T_ = N / R;
-  constexpr int step = N / (Ns * R);
-  const int total = nlines * T_;
+  constexpr int step = N / (Ns * R), LD = fft_ld<T2>(N);
+  const int total = LN * T_;
   for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-    const int line = idx / T_;
-    const int j = idx - line * T_;
+    const int line = idx % LN, j = idx / LN;
+    if (line >= nlines) continue;
     const int k = j % Ns;
-    const T2* src = in + line * N;
-    T2* dst = out + line * N;
+    const T2* src = in + line * LD;
+    T2* dst = out + line * LD;
     T2 v[5];
 #pragma unroll
     for (int r = 0; r < R; ++r) v[r] = src[j + r * T_];
@@ -239,7 +254,7 @@ __device__ __forceinline__ void fft_stage_ct(const T2* __restrict__ in, T2* __re
   }
 }
 
-template <typename T, typename T2, int ISIGN, int N, int Ns>
+template <typename T, typename T2, int ISIGN, int N, int Ns, int LN>
 __device__ __forceinline__ T2* fft_ct(T2* a, T2* b, int nlines, const T2* tw) {
   if constexpr (Ns == N) {
     __syncthreads();
@@ -248,16 +263,16 @@ __device__ __forceinline__ T2* fft_ct(T2* a, T2* b, int nlines, const T2* tw) {
     constexpr int R = next_radix<N / Ns>();
     static_assert((N / Ns) % R == 0, "FFT lengths are 2^a 3^b 5^c");
     __syncthreads();
-    fft_stage_ct<T, T2, ISIGN, N, R, Ns>(a, b, nlines, tw);
-    return fft_ct<T, T2, ISIGN, N, Ns * R>(b, a, nlines, tw);
+    fft_stage_ct<T, T2, ISIGN, N, R, Ns, LN>(a, b, nlines, tw);
+    return fft_ct<T, T2, ISIGN, N, Ns * R, LN>(b, a, nlines, tw);
   }
 }
 
 // NC > 0: the compile-time transform of length NC (== pl.N); NC == 0: any length
-template <typename T, typename T2, int ISIGN, int NC>
+template <typename T, typename T2, int ISIGN, int NC, int LN>
 __device__ __forceinline__ T2* fft_run(T2* a, T2* b, const FftPlan& pl, int nlines, const T2* tw) {
-  if constexpr (NC == 0) return fft_lines<T, T2, ISIGN>(a, b, pl, nlines, tw);
-  else return fft_ct<T, T2, ISIGN, NC, 1>(a, b, nlines, tw);
+  if constexpr (NC == 0) return fft_lines<T, T2, ISIGN, LN>(a, b, pl, nlines, tw);
+  else return fft_ct<T, T2, ISIGN, NC, 1, LN>(a, b, nlines, tw);
 }
 
 
@@ -280,20 +295,24 @@ __device__ __forceinline__ dfr rc_at<dfr>(const SpmeGeom& sg, int k) { return df
 // real part of the full inverse transform, as before.
 template <typename T, typename T2, int NC>
 __global__ void k_fft_x_fwd(const T* __restrict__ Q, T2* __restrict__ G, FftPlan pl, const T2* __restrict__ tw,
-                            const T2* __restrict__ twN, int nrows, int lines) {
+                            const T2* __restrict__ twN, int nrows) {
   extern __shared__ unsigned char smem_raw[];
-  const int M = NC ? NC : pl.N, Kx = M + 1;
+  const int M = NC ? NC : pl.N, Kx = M + 1, LD = fft_ld<T2>(M);
   T2* a = reinterpret_cast<T2*>(smem_raw);
-  T2* b = a + lines * M;
-  const size_t row0 = (size_t)blockIdx.x * lines;
-  const int nl = (int)min((size_t)lines, (size_t)nrows - row0);
+  T2* b = a + XLINES * LD;
+  const size_t row0 = (size_t)blockIdx.x * XLINES;
+  const int nl = (int)min((size_t)XLINES, (size_t)nrows - row0);
   const T2* Qc = reinterpret_cast<const T2*>(Q);
-  for (int e = threadIdx.x; e < nl * M; e += blockDim.x) a[e] = Qc[row0 * M + e];
-  T2* r = fft_run<T, T2, +1, NC>(a, b, pl, nl, tw);
+  for (int e = threadIdx.x; e < nl * M; e += blockDim.x) {
+    const int line = e / M, k = e - line * M;
+    a[line * LD + k] = Qc[row0 * M + e];
+  }
+  T2* r = fft_run<T, T2, +1, NC, XLINES>(a, b, pl, nl, tw);
   for (int e = threadIdx.x; e < nl * Kx; e += blockDim.x) {
     const int line = e / Kx, k = e - line * Kx;
-    const T2 zk = r[line * M + (k == M ? 0 : k)];
-    const T2 zc = r[line * M + (k == 0 ? 0 : M - k)];  // Z_{M-k}, conjugated below
+    const int k1 = k == M ? 0 : k, k2 = k == 0 ? 0 : M - k;
+    const T2 zk = r[line * LD + k1];
+    const T2 zc = r[line * LD + k2];  // Z_{M-k}, conjugated below
     const T ex = (T)0.5 * (zk.x + zc.x), ey = (T)0.5 * (zk.y - zc.y);
     const T ox = (T)0.5 * (zk.y + zc.y), oy = (T)0.5 * (zc.x - zk.x);
     const T2 w = twN[k];
@@ -306,13 +325,13 @@ __global__ void k_fft_x_fwd(const T* __restrict__ Q, T2* __restrict__ G, FftPlan
 
 template <typename T, typename T2, int NC>
 __global__ void k_fft_x_inv(const T2* __restrict__ G, T* __restrict__ Q, FftPlan pl, const T2* __restrict__ tw,
-                            const T2* __restrict__ twN, int nrows, int lines, unsigned* vmax) {
+                            const T2* __restrict__ twN, int nrows, unsigned* vmax) {
   extern __shared__ unsigned char smem_raw[];
-  const int M = NC ? NC : pl.N, Kx = M + 1;
+  const int M = NC ? NC : pl.N, Kx = M + 1, LD = fft_ld<T2>(M);
   T2* a = reinterpret_cast<T2*>(smem_raw);
-  T2* b = a + lines * M;
-  const size_t row0 = (size_t)blockIdx.x * lines;
-  const int nl = (int)min((size_t)lines, (size_t)nrows - row0);
+  T2* b = a + XLINES * LD;
+  const size_t row0 = (size_t)blockIdx.x * XLINES;
+  const int nl = (int)min((size_t)XLINES, (size_t)nrows - row0);
   for (int e = threadIdx.x; e < nl * M; e += blockDim.x) {
     const int line = e / M, k = e - line * M;
     const T2 xk = G[(row0 + line) * Kx + k];
@@ -324,16 +343,19 @@ __global__ void k_fft_x_inv(const T2* __restrict__ G, T* __restrict__ Q, FftPlan
     T2 v;
     v.x = ax - by;
     v.y = ay + bx;
-    a[e] = v;
+    a[line * LD + k] = v;
   }
-  T2* r = fft_run<T, T2, -1, NC>(a, b, pl, nl, tw);
+  T2* r = fft_run<T, T2, -1, NC, XLINES>(a, b, pl, nl, tw);
   T2* Qc = reinterpret_cast<T2*>(Q);
-  for (int e = threadIdx.x; e < nl * M; e += blockDim.x) Qc[row0 * M + e] = r[e];
+  unsigned m = 0;  // the bits of the largest |potential| of the grid, for the double-float gather
+  for (int e = threadIdx.x; e < nl * M; e += blockDim.x) {
+    const int line = e / M, k = e - line * M;
+    const T2 v = r[line * LD + k];
+    Qc[row0 * M + e] = v;
+    if constexpr (std::is_same<T, dfr>::value)
+      m = max(m, max(__float_as_uint(v.x.hi) & 0x7fffffffu, __float_as_uint(v.y.hi) & 0x7fffffffu));
+  }
   if constexpr (std::is_same<T, dfr>::value) {
-    // the bits of the largest |potential| of the grid, for the gather
-    unsigned m = 0;
-    for (int e = threadIdx.x; e < nl * M; e += blockDim.x)
-      m = max(m, max(__float_as_uint(r[e].x.hi) & 0x7fffffffu, __float_as_uint(r[e].y.hi) & 0x7fffffffu));
     m = __reduce_max_sync(0xffffffffu, m);
     if ((threadIdx.x & 31) == 0 && m > *reinterpret_cast<volatile unsigned*>(vmax)) atomicMax(vmax, m);
   }
@@ -343,9 +365,9 @@ __global__ void k_fft_x_inv(const T2* __restrict__ G, T* __restrict__ Q, FftPlan
 template <typename T, typename T2, int ISIGN, int NC>
 __global__ void k_fft_y(T2* __restrict__ G, int Kx, int K2_, FftPlan pl, const T2* __restrict__ tw) {
   extern __shared__ unsigned char smem_raw[];
-  const int K2 = NC ? NC : K2_;
+  const int K2 = NC ? NC : K2_, LD = fft_ld<T2>(K2);
   T2* a = reinterpret_cast<T2*>(smem_raw);
-  T2* b = a + TX * K2;
+  T2* b = a + TX * LD;
   const int ntx = (Kx + TX - 1) / TX;
   const int x0 = (blockIdx.x % ntx) * TX;
   const int zz = blockIdx.x / ntx;
@@ -355,12 +377,12 @@ __global__ void k_fft_y(T2* __restrict__ G, int Kx, int K2_, FftPlan pl, const T
     int yy = e / TX, t = e - yy * TX;
     T2 v; v.x = (T)0; v.y = (T)0;
     if (t < nt) v = base[(size_t)yy * Kx + t];
-    a[t * K2 + yy] = v;
+    a[t * LD + yy] = v;
   }
-  T2* r = fft_run<T, T2, ISIGN, NC>(a, b, pl, TX, tw);
+  T2* r = fft_run<T, T2, ISIGN, NC, TX>(a, b, pl, TX, tw);
   for (int e = threadIdx.x; e < TX * K2; e += blockDim.x) {
     int yy = e / TX, t = e - yy * TX;
-    if (t < nt) base[(size_t)yy * Kx + t] = r[t * K2 + yy];
+    if (t < nt) base[(size_t)yy * Kx + t] = r[t * LD + yy];
   }
 }
 
@@ -372,9 +394,9 @@ __global__ void k_fft_z_conv(T2* __restrict__ G, int K1, int K2, int K3_, FftPla
                              const T* __restrict__ theta, const T* __restrict__ psi, SpmeGeom sg, double* blk,
                              GridSum gs) {
   extern __shared__ unsigned char smem_raw[];
-  const int K3 = NC ? NC : K3_;
+  const int K3 = NC ? NC : K3_, LD = fft_ld<T2>(K3);
   T2* a = reinterpret_cast<T2*>(smem_raw);
-  T2* b = a + TX * K3;
+  T2* b = a + TX * LD;
   const int Kx = K1 / 2 + 1;
   const int ntx = (Kx + TX - 1) / TX;
   const int x0 = (blockIdx.x % ntx) * TX;
@@ -386,15 +408,15 @@ __global__ void k_fft_z_conv(T2* __restrict__ G, int K1, int K2, int K3_, FftPla
     int zz = e / TX, t = e - zz * TX;
     T2 v; v.x = (T)0; v.y = (T)0;
     if (t < nt) v = base[(size_t)zz * plane + t];
-    a[t * K3 + zz] = v;
+    a[t * LD + zz] = v;
   }
   // m_z = ll * rcell(9) for the cubic cell (gb_init accepts cubic cells only)
-  T* rzt = reinterpret_cast<T*>(b + TX * K3);
+  T* rzt = reinterpret_cast<T*>(b + TX * LD);
   for (int zz = threadIdx.x; zz < K3; zz += blockDim.x) {
     int ll = zz; if (2 * ll > K3) ll -= K3;
     rzt[zz] = (T)ll * rc_at<T>(sg, 8);
   }
-  T2* r = fft_run<T, T2, +1, NC>(a, b, pl, TX, tw);
+  T2* r = fft_run<T, T2, +1, NC, TX>(a, b, pl, TX, tw);
   // Reciprocal stress sum_m m_a m_b psi |Q(m)|^2 (ewald_spole.F90:1362-1371): with
   // m = (mx, my, mz) and mx, my fixed along a z line, each line needs only
   // A = sum psi|Q|^2, B = sum mz psi|Q|^2, C = sum mz^2 psi|Q|^2.
@@ -404,11 +426,12 @@ __global__ void k_fft_z_conv(T2* __restrict__ G, int K1, int K2, int K3_, FftPla
   T A = 0, B = 0, Bn = 0, C = 0;
   if (t < nt) {
     const size_t line0 = (size_t)yy * Kx + x0 + t;
-    T2* rl = r + t * K3;
+    T2* rl = r + t * LD;
     for (int zz = threadIdx.x - t * tpl; zz < K3; zz += tpl) {
       const size_t gi = line0 * K3 + zz;  // theta/psi are stored z-contiguous per (x,y) line
       const T th = theta[gi];
-      T2 v = rl[zz];
+      T2& at = rl[zz];
+      T2 v = at;
       if (nonzero_bits(th)) {
         const T pv = psi[gi] * (v.x * v.x + v.y * v.y);
         const T u = pv * rzt[zz];
@@ -420,7 +443,7 @@ __global__ void k_fft_z_conv(T2* __restrict__ G, int K1, int K2, int K3_, FftPla
       } else {
         v.x = (T)0; v.y = (T)0;
       }
-      rl[zz] = v;
+      at = v;
     }
   }
   // in the working precision T: the FP32 form issues no FP64 instruction here
@@ -450,10 +473,10 @@ __global__ void k_fft_z_conv(T2* __restrict__ G, int K1, int K2, int K3_, FftPla
     }
   }
   T2* o = (r == a) ? b : a;
-  T2* r2 = fft_run<T, T2, -1, NC>(r, o, pl, TX, tw);
+  T2* r2 = fft_run<T, T2, -1, NC, TX>(r, o, pl, TX, tw);
   for (int e = threadIdx.x; e < TX * K3; e += blockDim.x) {
     int zz = e / TX, t = e - zz * TX;
-    if (t < nt) base[(size_t)zz * plane + t] = r2[t * K3 + zz];
+    if (t < nt) base[(size_t)zz * plane + t] = r2[t * LD + zz];
   }
   block_reduce_store<6>(st, blk);
   grid_finish<6>(blk, gs);

@@ -1005,7 +1005,9 @@ int choose_brick(int K, int p, bool coarse) {
   return -1;
 }
 
-size_t fft_smem(int N, int lines, size_t esz) { return (size_t)2 * lines * N * esz; }
+size_t fft_smem(int N, int lines, size_t esz) {
+  return (size_t)2 * lines * (esz == 16 ? fft_ld<double2>(N) : fft_ld<float2>(N)) * esz;
+}
 
 }  // namespace
 
@@ -1251,8 +1253,10 @@ void grid_setup(SpmeGrid& S, const int* Kin, int p, bool fp64) {
   }
   // dynamic shared memory limits
   const int maxN = std::max(S.K[0], std::max(S.K[1], S.K[2]));
-  int smem = (int)std::max(fft_smem(maxN, TX, sizeof(double2)), fft_smem(S.K[0], 8, sizeof(double2)));
-  smem = std::max(smem, 48 * 1024);
+  int smem = std::max(48 * 1024, (int)sizeof(double2) * 2 * std::max(TX * maxN, 8 * S.K[0]));
+  if (maxN <= 1024)  // with the lines' padding, and the z pass's table behind its lines
+    smem = std::max(smem, (int)std::max(fft_smem(maxN, TX, sizeof(double2)) + sizeof(double) * maxN,
+                                        fft_smem(S.K[0] / 2, 8, sizeof(double2))));
   raise_fft<double, double2>(S, smem);
   raise_fft<float, float2>(S, smem);
   if (S.fp64) raise_fft<dfr, dfc>(S, smem);
@@ -1351,7 +1355,6 @@ void grid_run(SpmeGrid& S, bool coarse, float* rec, double* eng_rc, double* vir_
     prof_end(pid(P_SPME_SPREAD));
   }
   // FFT + convolution: real-to-complex x pass, y and z passes on the Kx = K1/2+1 columns
-  const int lines = 8;
   const int rows = K2 * K3;
   const int Kx = S.Kx, M = K1 / 2;
   const T2* twh = DF ? reinterpret_cast<const T2*>(S.twh_d)
@@ -1359,9 +1362,8 @@ void grid_run(SpmeGrid& S, bool coarse, float* rec, double* eng_rc, double* vir_
   const int ntx = (Kx + TX - 1) / TX;
   prof_begin(pid(P_FFT_XF));
   const FftKernels<T, T2> fk = fft_kernels<T, T2>(M, K2, K3);
-  const int thx = fft_threads(S.planh, lines), thy = fft_threads(S.plan[1], TX), thz = fft_threads(S.plan[2], TX);
-  fk.x_fwd<<<nblocks(rows, lines), thx, fft_smem(M, lines, sizeof(T2)), st>>>(Q, G, S.planh, twh, tw1,
-                                                                                            rows, lines);
+  const int thx = fft_threads(S.planh, XLINES), thy = fft_threads(S.plan[1], TX), thz = fft_threads(S.plan[2], TX);
+  fk.x_fwd<<<nblocks(rows, XLINES), thx, fft_smem(M, XLINES, sizeof(T2)), st>>>(Q, G, S.planh, twh, tw1, rows);
   GB_LAUNCHED();
   prof_end(pid(P_FFT_XF));
   prof_begin(pid(P_FFT_Y));
@@ -1384,8 +1386,7 @@ void grid_run(SpmeGrid& S, bool coarse, float* rec, double* eng_rc, double* vir_
   prof_begin(pid(P_FFT_XI));
   // (the largest |potential| goes to the zeroed entry after the brick counts)
   unsigned* vmax = reinterpret_cast<unsigned*>(S.brick_count + S.nbricks + 1);
-  fk.x_inv<<<nblocks(rows, lines), thx, fft_smem(M, lines, sizeof(T2)), st>>>(G, Q, S.planh, twh, tw1,
-                                                                                            rows, lines, vmax);
+  fk.x_inv<<<nblocks(rows, XLINES), thx, fft_smem(M, XLINES, sizeof(T2)), st>>>(G, Q, S.planh, twh, tw1, rows, vmax);
   GB_LAUNCHED();
   prof_end(pid(P_FFT_XI));
   // gather
