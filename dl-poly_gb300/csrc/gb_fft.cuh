@@ -19,7 +19,8 @@
 namespace gbspme {
 
 constexpr int TX = 4;      // columns per tile in the strided passes
-constexpr int XLINES = 8;  // rows per block in the x passes
+constexpr int XLINES = 8;  // rows per block in the x passes (a kernel argument too: with the constant
+                           // alone the FP32 x pass of a 192^3 grid took 0.029 ms, not 0.023)
 
 struct FftPlan {
   int N;
@@ -37,8 +38,8 @@ struct SpmeGeom {
 // the five FFT kernels one grid launches, for working type T (complex T2)
 template <typename T, typename T2>
 struct FftKernels {
-  void (*x_fwd)(const T*, T2*, FftPlan, const T2*, const T2*, int);
-  void (*x_inv)(const T2*, T*, FftPlan, const T2*, const T2*, int, unsigned*);
+  void (*x_fwd)(const T*, T2*, FftPlan, const T2*, const T2*, int, int);
+  void (*x_inv)(const T2*, T*, FftPlan, const T2*, const T2*, int, int, unsigned*);
   void (*y_fwd)(T2*, int, int, FftPlan, const T2*);
   void (*y_inv)(T2*, int, int, FftPlan, const T2*);
   void (*z_conv)(T2*, int, int, int, FftPlan, const T2*, const T*, const T*, SpmeGeom, double*, GridSum);
@@ -148,18 +149,21 @@ __device__ __forceinline__ void bfly(const T2 (&v)[5], T2 (&o)[5]) {
   }
 }
 
-// Elements between the lines in shared memory.  The lanes of a warp take the lines in turn
-// (lane % LN), so that LN lanes share a butterfly's place in the line and its twiddles, and no
-// index needs a division by the line's length.  With ld = 3 mod 8 (16-byte elements) or 5 mod
-// 16 the strided stores of the first stage reach all banks, and its loads and the
-// transposed fill of the y and z passes nearly all.  With line after line, 32 places and twiddles
-// per warp, the passes were bound by shared memory and L1: the
-// y pass of a 160^3 double-float grid took 0.050 ms, now 0.044; ten MD steps on a 192^3 grid 24.0
-// and now 23.6 ms; the double-precision z pass of a 72^3 grid 0.062 and now 0.047 ms.
+// With 16-byte elements the lanes of a warp take the lines in turn (lane % LN), so that LN
+// lanes share a butterfly's place in the line and its twiddles, and no index needs a
+// division by the line's length.  Lines ld apart, ld = 3 mod 8: the strided stores of the first
+// stage reach all banks, its loads and the transposed fill of the y and z passes nearly
+// all.  With line after line, 32 places and twiddles per warp, the passes were bound by shared
+// memory and L1: the y pass of a 160^3 double-float grid took 0.050 ms, now 0.044; ten MD steps on
+// a 192^3 grid 24.0 and now 23.6 ms; the double-precision z pass of a 72^3 grid 0.062 and now
+// 0.047 ms.  8-byte elements (FP32) keep line after line: in turns the z pass of a 192^3
+// grid took 0.068 ms instead of 0.062.
 // Lines above 1024 stay unpadded, for the shared memory.
 template <typename T2>
+__host__ __device__ constexpr bool fft_turns() { return sizeof(T2) == 16; }
+template <typename T2>
 __host__ __device__ constexpr int fft_ld(int n) {
-  return n > 1024 ? n : sizeof(T2) == 16 ? n + ((3 - n) & 7) : n + ((5 - n) & 15);
+  return n > 1024 || !fft_turns<T2>() ? n : n + ((3 - n) & 7);
 }
 
 // one Stockham stage over nlines lines of length N held in shared memory.
@@ -168,10 +172,10 @@ template <typename T, typename T2, int ISIGN, int LN>
 __device__ void fft_stage(const T2* __restrict__ in, T2* __restrict__ out, int N, int nlines, int R, int Ns,
                           const T2* __restrict__ tw) {
   const int T_ = N / R;
-  const int total = LN * T_, LD = fft_ld<T2>(N);
+  const int total = (fft_turns<T2>() ? LN : nlines) * T_, LD = fft_ld<T2>(N);
   for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-    const int line = idx % LN, j = idx / LN;
-    if (line >= nlines) continue;
+    const int line = fft_turns<T2>() ? idx % LN : idx / T_, j = fft_turns<T2>() ? idx / LN : idx - line * T_;
+    if (fft_turns<T2>() && line >= nlines) continue;
     const int k = j % Ns;
     const T2* src = in + line * LD;
     T2* dst = out + line * LD;
@@ -228,10 +232,10 @@ __device__ __forceinline__ void fft_stage_ct(const T2* __restrict__ in, T2* __re
                                              const T2* __restrict__ tw) {
   constexpr int T_ = N / R;
   constexpr int step = N / (Ns * R), LD = fft_ld<T2>(N);
-  const int total = LN * T_;
+  const int total = (fft_turns<T2>() ? LN : nlines) * T_;
   for (int idx = threadIdx.x; idx < total; idx += blockDim.x) {
-    const int line = idx % LN, j = idx / LN;
-    if (line >= nlines) continue;
+    const int line = fft_turns<T2>() ? idx % LN : idx / T_, j = fft_turns<T2>() ? idx / LN : idx - line * T_;
+    if (fft_turns<T2>() && line >= nlines) continue;
     const int k = j % Ns;
     const T2* src = in + line * LD;
     T2* dst = out + line * LD;
@@ -295,17 +299,16 @@ __device__ __forceinline__ dfr rc_at<dfr>(const SpmeGeom& sg, int k) { return df
 // real part of the full inverse transform, as before.
 template <typename T, typename T2, int NC>
 __global__ void k_fft_x_fwd(const T* __restrict__ Q, T2* __restrict__ G, FftPlan pl, const T2* __restrict__ tw,
-                            const T2* __restrict__ twN, int nrows) {
+                            const T2* __restrict__ twN, int nrows, int lines) {
   extern __shared__ unsigned char smem_raw[];
-  const int M = NC ? NC : pl.N, Kx = M + 1, LD = fft_ld<T2>(M);
+  const int M = NC ? NC : pl.N, Kx = M + 1, LD = fft_turns<T2>() ? fft_ld<T2>(M) : M;
   T2* a = reinterpret_cast<T2*>(smem_raw);
-  T2* b = a + XLINES * LD;
-  const size_t row0 = (size_t)blockIdx.x * XLINES;
-  const int nl = (int)min((size_t)XLINES, (size_t)nrows - row0);
+  T2* b = a + lines * LD;
+  const size_t row0 = (size_t)blockIdx.x * lines;
+  const int nl = (int)min((size_t)lines, (size_t)nrows - row0);
   const T2* Qc = reinterpret_cast<const T2*>(Q);
   for (int e = threadIdx.x; e < nl * M; e += blockDim.x) {
-    const int line = e / M, k = e - line * M;
-    a[line * LD + k] = Qc[row0 * M + e];
+    a[fft_turns<T2>() ? e + (e / M) * (LD - M) : e] = Qc[row0 * M + e];
   }
   T2* r = fft_run<T, T2, +1, NC, XLINES>(a, b, pl, nl, tw);
   for (int e = threadIdx.x; e < nl * Kx; e += blockDim.x) {
@@ -325,13 +328,13 @@ __global__ void k_fft_x_fwd(const T* __restrict__ Q, T2* __restrict__ G, FftPlan
 
 template <typename T, typename T2, int NC>
 __global__ void k_fft_x_inv(const T2* __restrict__ G, T* __restrict__ Q, FftPlan pl, const T2* __restrict__ tw,
-                            const T2* __restrict__ twN, int nrows, unsigned* vmax) {
+                            const T2* __restrict__ twN, int nrows, int lines, unsigned* vmax) {
   extern __shared__ unsigned char smem_raw[];
-  const int M = NC ? NC : pl.N, Kx = M + 1, LD = fft_ld<T2>(M);
+  const int M = NC ? NC : pl.N, Kx = M + 1, LD = fft_turns<T2>() ? fft_ld<T2>(M) : M;
   T2* a = reinterpret_cast<T2*>(smem_raw);
-  T2* b = a + XLINES * LD;
-  const size_t row0 = (size_t)blockIdx.x * XLINES;
-  const int nl = (int)min((size_t)XLINES, (size_t)nrows - row0);
+  T2* b = a + lines * LD;
+  const size_t row0 = (size_t)blockIdx.x * lines;
+  const int nl = (int)min((size_t)lines, (size_t)nrows - row0);
   for (int e = threadIdx.x; e < nl * M; e += blockDim.x) {
     const int line = e / M, k = e - line * M;
     const T2 xk = G[(row0 + line) * Kx + k];
@@ -343,14 +346,13 @@ __global__ void k_fft_x_inv(const T2* __restrict__ G, T* __restrict__ Q, FftPlan
     T2 v;
     v.x = ax - by;
     v.y = ay + bx;
-    a[line * LD + k] = v;
+    a[e + line * (LD - M)] = v;
   }
   T2* r = fft_run<T, T2, -1, NC, XLINES>(a, b, pl, nl, tw);
   T2* Qc = reinterpret_cast<T2*>(Q);
   unsigned m = 0;  // the bits of the largest |potential| of the grid, for the double-float gather
   for (int e = threadIdx.x; e < nl * M; e += blockDim.x) {
-    const int line = e / M, k = e - line * M;
-    const T2 v = r[line * LD + k];
+    const T2 v = r[fft_turns<T2>() ? e + (e / M) * (LD - M) : e];
     Qc[row0 * M + e] = v;
     if constexpr (std::is_same<T, dfr>::value)
       m = max(m, max(__float_as_uint(v.x.hi) & 0x7fffffffu, __float_as_uint(v.y.hi) & 0x7fffffffu));

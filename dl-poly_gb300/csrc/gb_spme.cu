@@ -14,9 +14,9 @@
 // (n = Int(u), w = u - Aint(u)) and periodic grid reads, so atoms that drifted
 // out of the cell between relocations get the same spline values.
 //
-// Spreading is atomic free: atoms are sorted by grid brick (B >= p-1 points
-// per side); one CTA owns a brick and gathers from the 2x2x2 source bricks
-// whose atoms can reach it, one thread per grid row along x.
+// Spreading is atomic free: the preparation kernel puts each atom into its grid brick's slot
+// list, one CTA per brick sorts its atoms and scatters them into a shared tile of the brick and
+// the p - 1 planes beyond it, and a second kernel sums the tiles in a fixed order.
 //
 // The 3-D FFT is an in-shared-memory Stockham transform (radix 4, 3, 5, 2)
 // along x, y and z; the z pass applies the influence function theta(m)
@@ -1363,7 +1363,8 @@ void grid_run(SpmeGrid& S, bool coarse, float* rec, double* eng_rc, double* vir_
   prof_begin(pid(P_FFT_XF));
   const FftKernels<T, T2> fk = fft_kernels<T, T2>(M, K2, K3);
   const int thx = fft_threads(S.planh, XLINES), thy = fft_threads(S.plan[1], TX), thz = fft_threads(S.plan[2], TX);
-  fk.x_fwd<<<nblocks(rows, XLINES), thx, fft_smem(M, XLINES, sizeof(T2)), st>>>(Q, G, S.planh, twh, tw1, rows);
+  fk.x_fwd<<<nblocks(rows, XLINES), thx, fft_smem(M, XLINES, sizeof(T2)), st>>>(Q, G, S.planh, twh, tw1, rows,
+                                                                              XLINES);
   GB_LAUNCHED();
   prof_end(pid(P_FFT_XF));
   prof_begin(pid(P_FFT_Y));
@@ -1386,7 +1387,8 @@ void grid_run(SpmeGrid& S, bool coarse, float* rec, double* eng_rc, double* vir_
   prof_begin(pid(P_FFT_XI));
   // (the largest |potential| goes to the zeroed entry after the brick counts)
   unsigned* vmax = reinterpret_cast<unsigned*>(S.brick_count + S.nbricks + 1);
-  fk.x_inv<<<nblocks(rows, XLINES), thx, fft_smem(M, XLINES, sizeof(T2)), st>>>(G, Q, S.planh, twh, tw1, rows, vmax);
+  fk.x_inv<<<nblocks(rows, XLINES), thx, fft_smem(M, XLINES, sizeof(T2)), st>>>(G, Q, S.planh, twh, tw1, rows,
+                                                                              XLINES, vmax);
   GB_LAUNCHED();
   prof_end(pid(P_FFT_XI));
   // gather
