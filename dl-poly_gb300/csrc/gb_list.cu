@@ -1232,13 +1232,13 @@ int list_build() {
       g.xsf, tp, h_cg, g.tile_rows, g.tile_info, cap, g.sc);
   GB_LAUNCHED();
   prof_end(P_BIN);
-  prof_begin(P_LIST);
   // The lanes per atom by the warps per SM that they give (the table at k_list_lanes); below
   // 12 with the most lanes the tiles' CTAs, which share a tile's atoms, are faster.
   const int n = g.natms, nsm = g.nsm;
   const int G = n / 16 >= 10 * nsm ? 2 : n / 4 >= 16 * nsm ? 8 : 16;
   auto lanes = G == 2 ? k_list_lanes<2, 4> : G == 8 ? k_list_lanes<8, 2> : k_list_lanes<16, 2>;
   for (;;) {
+    prof_begin(P_LIST);
     if (tiles) {
       // several CTAs share a tile's atoms (each stages its whole shell), so that the device has
       // about three CTAs per SM
@@ -1258,14 +1258,14 @@ int list_build() {
                                                                       g.lbook ? 1 : 0);
       GB_LAUNCHED();
     }
-    gb_sync_scalars();
+    prof_end(P_LIST);
+    gb_sync_scalars();  // (resolves the timings)
     if (!tiles || g.hsc->tile_over == 0) break;
     g.n_tile_over = g.hsc->tile_over;  // denser tiles than planned: this list and the later ones from the other kernel
     tiles = false;
     GB_CUDA(cudaMemsetAsync(&g.sc->ibig, 0, sizeof(int), st));
     GB_CUDA(cudaMemsetAsync(&g.sc->halo_fwd, 0, 2 * sizeof(int), st));  // halo_fwd, halo_bwd
   }
-  prof_end(P_LIST);
   if (g.hsc->status & ST_HALO_OVERFLOW) return GB_ERR_HALO;  // (list_relocate_and_halo without its wait)
   if (g.hsc->status & ST_LIST_OVERFLOW) return GB_ERR_LIST_OVERFLOW;
   // every pair across the periodic boundary is listed from both of its atoms, once in a

@@ -1,5 +1,7 @@
 """Verlet list, bit for bit, where its kernels take other branches: frozen and excluded
 atoms moved to the end of the lists, and halo exports longer than a block's registers hold."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -60,3 +62,21 @@ def test_tiles_above_their_capacity(gpu_lib, oracle_lib, monkeypatch):
     monkeypatch.setenv("GB_TILE_CAP", "64")
     _same(*_lists(gpu_lib, oracle_lib, systems.spce_water(8)))
     monkeypatch.delenv("GB_TILE_CAP")
+
+
+def test_phase_timings_of_a_rebuild(gpu_lib):
+    """Every phase's event pair is complete when the build's wait resolves the timings."""
+    gpu_lib.init(systems.nacl_melt(16))
+    L = gpu_lib._opt("profile", ctypes.c_int, [ctypes.c_int])
+    read = gpu_lib._opt("profile_read", ctypes.c_int, [ctypes.c_char_p, ctypes.POINTER(ctypes.c_double),
+                                                      ctypes.POINTER(ctypes.c_int64), ctypes.c_int])
+    L(1)
+    for _ in range(2):
+        gpu_lib.relocate()
+        gpu_lib.link_cell_pairs()
+    names, ms, n = ctypes.create_string_buffer(32 * 32), (ctypes.c_double * 32)(), (ctypes.c_int64 * 32)()
+    k = read(names, ms, n, 32)
+    L(0)
+    got = {names.raw[32 * i:32 * i + 32].split(b"\0")[0].decode(): (ms[i], n[i]) for i in range(k)}
+    for phase in ("halo", "bin_sort", "list_pairs"):
+        assert got[phase][1] == 2 and got[phase][0] > 0.0, phase
