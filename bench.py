@@ -179,29 +179,32 @@ def kernel_work(name, s, cnt, form):
 # for a full-section capture); traffic grows with the list, so the bench scales
 # it by this launch's list entries.
 MEASURED_TRAFFIC = {
-    ("pair_forces", "fp64"): ((223.553536e6 + 4.797952e6) / 40368337,
+    ("pair_forces", "fp64"): ((228.130048e6 + 8.109824e6) / 40368337,
                               "ncu dram__bytes_read.sum + dram__bytes_write.sum of k_pair_sorted<0, 4, 1024> on nacl_175616 "
                               "(profiles/pair_sorted_df64_nacl175616.md), scaled by half-list entries"),
-    ("pair_forces", "fp64_native"): ((200.795648e6 + 3.779072e6) / 40368337,
+    ("pair_forces", "fp64_native"): ((205.167104e6 + 4.668672e6) / 40368337,
                                      "ncu dram__bytes_read.sum + dram__bytes_write.sum of k_pair_fp64 on nacl_175616 "
                                      "(profiles/pair_fp64_nacl175616.md), scaled by half-list entries"),
-    ("pair_forces", "mixed"): ((219.659264e6 + 6.057216e6) / 40368337,
+    ("pair_forces", "mixed"): ((222.353152e6 + 7.757312e6) / 40368337,
                                "ncu dram__bytes_read.sum + dram__bytes_write.sum of k_pair_sorted<1, 4, 256> on nacl_175616 "
                                "(profiles/pair_sorted_mixed_nacl175616.md), scaled by half-list entries"),
-    ("metal_forces", "fp64"): ((131.494144e6 + 4.494848e6) / 19246179,
-                               "ncu dram__bytes_read.sum + dram__bytes_write.sum of k_metal_forces on eam_256000 "
+    ("metal_forces", "fp64"): ((167.879168e6 + 10.868992e6) / 19246179,
+                               "ncu dram__bytes_read.sum + dram__bytes_write.sum of k_metal_forces_sorted on eam_256000 "
                                "(profiles/metal_kernels_eam256000.md), scaled by half-list entries"),
 }
 
 
-# Warp instructions executed per half-list entry by the double-float pair kernel (ncu
+# Warp instructions executed per half-list entry by the double-float pair kernels (ncu
 # smsp__inst_executed.sum of one launch on the 175,616-ion melt over its list
 # entries).  That kernel runs on the FP32/ALU pipes and is bound by instruction
 # issue, so its roofline is issue slots: 4 warp instructions per clock per SM.
 MEASURED_INST = {
-    ("pair_forces", "fp64"): (601732163 / 40368337,
+    ("pair_forces", "fp64"): (560096967 / 40368337,
                               "ncu smsp__inst_executed.sum of k_pair_sorted<0, 4, 1024> on nacl_175616 "
                               "(profiles/pair_sorted_df64_nacl175616.md), scaled by half-list entries"),
+    ("metal_forces", "fp64"): (498557038 / 19246179,
+                               "ncu smsp__inst_executed.sum of k_metal_forces_sorted on eam_256000 "
+                               "(profiles/metal_kernels_eam256000.md), scaled by half-list entries"),
 }
 
 

@@ -115,7 +115,7 @@ struct Dev {
   cudaStream_t main_stream = nullptr, side_stream = nullptr;
   cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
   bool side = false, join_pending = false, use_overlap = true;
-  int pair_apw = -1;  // atoms per warp of the sorted pair kernels' CTAs (GB_PAIR_APW; 0: resident CTAs, -1: by form)
+  int pair_apw = -1;  // atoms per warp of the sorted pair kernels' CTAs (GB_PAIR_APW; 0 or -1: resident CTAs)
   // work to put on the side stream once the pair kernel is launched (run by pair_forces
   // before it joins the side stream)
   void (*side_hook)(void*) = nullptr;
