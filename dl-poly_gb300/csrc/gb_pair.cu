@@ -235,72 +235,98 @@ __global__ void __launch_bounds__(256, 3) k_pair_fp64(int natms, const DevScalar
   block_reduce_store<NACC>(acc, blk);
 }
 
-// exclusion correction (FP64), one thread per atom over its excluded section
-// In the mixed form the same FP64 kernel writes fixed-point forces (fixp != 0):
-// the intramolecular exclusion terms cancel against the reciprocal energy
-// (tens of millions of internal units for water), so they stay in FP64.
+// Exclusion correction (FP64) over the atoms' excluded sections: a warp takes the pairs of 32
+// atoms as one sequence, a lane each (a water's atoms have two, one and none, so that a thread
+// per atom left half of its FP64 issue slots idle: 0.058 ms for 98,304 atoms of water, now 0.034).
+// Forces go to the pairs' int64 fixed-point sums (fixp; in the FP64 form they join the others'
+// with k_fix_add_fp64), whose sum does not depend on the order; the FP64 form by instructions
+// (fixp = 0) adds them in FP64.  The force of an excluded pair is bounded (it vanishes with
+// r), below 2e4 q^2 internal units.  In the mixed form too this kernel stays in FP64: the
+// intramolecular exclusion terms cancel against the reciprocal energy (tens of millions of
+// internal units for water).
 __global__ void k_excl_fp64(int natms, const int* list, int ld, const double* x, const double* y, const double* z,
                             const double* q, const int* ltg, const int* src, double alpha, double scaling,
                             double rcut, double* fx, double* fy, double* fz, double* blk,
                             unsigned long long* fixp, GridSum gs) {
-  int i = blockIdx.x * blockDim.x + threadIdx.x;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
   double acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  int first = 0, lim = 0, gi = 0;
+  double xi = 0.0, yi = 0.0, zi = 0.0, qi = 0.0;
   if (i < natms) {
     const int* li = list + (size_t)i * ld + 3;
-    int lim = li[-1] - li[0];
-    double chgea = q[i];
-    if (lim > 0 && fabs(chgea) > DBL_MIN) {
-      chgea *= scaling;
-      const double a1 = 0.254829592, a2 = -0.284496736, a3 = 1.421413741, a4 = -1.453152027,
-                   a5 = 1.061405429, pp = 0.3275911, r10 = 0.1, r216 = 1.0 / 216.0, r42 = 1.0 / 42.0,
-                   rr3 = 1.0 / 3.0, sqrpi = 1.7724538509055160273;
-      double fix = 0, fiy = 0, fiz = 0;
-      for (int m = 1; m <= lim; ++m) {
-        int j = li[li[0] + m] - 1;
-        double xx = x[i] - x[j], yy = y[i] - y[j], zz = z[i] - z[j];
-        double rrr = sqrt(xx * xx + yy * yy + zz * zz);
-        double chgprd = q[j];
-        if (fabs(chgprd) > DBL_MIN && rrr < rcut) {
-          chgprd *= chgea;
-          double rsq = rrr * rrr, alpr = rrr * alpha, alpr2 = alpr * alpr, erfr, egamma;
-          if (alpr < 1.0e-2) {
-            erfr = 2.0 * chgprd * (alpha / sqrpi) * (1.0 + alpr2 * (-rr3 + alpr2 * (r10 + alpr2 * (-r42 + alpr2 * r216))));
-            egamma = -4.0 * chgprd * (alpha * alpha * alpha / sqrpi) *
-                     (rr3 + alpr2 * (-2.0 * r10 + alpr2 * (3.0 * r42 - 4.0 * alpr2 * r216)));
-          } else {
-            double exp1 = exp(-(alpha * rrr) * (alpha * rrr));
-            double tt = 1.0 / (1.0 + pp * alpha * rrr);
-            erfr = chgprd * (1.0 - tt * (a1 + tt * (a2 + tt * (a3 + tt * (a4 + tt * a5)))) * exp1) / rrr;
-            egamma = -(erfr - 2.0 * chgprd * (alpha / sqrpi) * exp1) / rsq;
-          }
-          double fx_ = egamma * xx, fy_ = egamma * yy, fz_ = egamma * zz;
-          fix += fx_; fiy += fy_; fiz += fz_;
-          if (j < natms) {
-            if (fixp) {
-              const double sc = 1099511627776.0;
-              atomicAdd(&fixp[3 * j + 0], (unsigned long long)(-__double2ll_rn(fx_ * sc)));
-              atomicAdd(&fixp[3 * j + 1], (unsigned long long)(-__double2ll_rn(fy_ * sc)));
-              atomicAdd(&fixp[3 * j + 2], (unsigned long long)(-__double2ll_rn(fz_ * sc)));
-            } else {
-              atomicAdd(&fx[j], -fx_); atomicAdd(&fy[j], -fy_); atomicAdd(&fz[j], -fz_);
-            }
-          }
-          if (j < natms || ltg[i] < ltg[j]) {
-            acc[0] -= erfr;
-            acc[1] -= egamma * rsq;
-            acc[2] += xx * fx_; acc[3] += xx * fy_; acc[4] += xx * fz_;
-            acc[5] += yy * fy_; acc[6] += yy * fz_; acc[7] += zz * fz_;
-          }
-        }
+    first = li[0];
+    qi = q[i];
+    lim = fabs(qi) > DBL_MIN ? max(li[-1] - first, 0) : 0;
+    if (lim > 0) {
+      qi *= scaling;
+      xi = x[i]; yi = y[i]; zi = z[i];
+      gi = ltg[i];
+    }
+  }
+  int inc = lim;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int v = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += v;
+  }
+  const int tot = __shfl_sync(0xffffffffu, inc, 31);
+  const double a1 = 0.254829592, a2 = -0.284496736, a3 = 1.421413741, a4 = -1.453152027, a5 = 1.061405429,
+               pp = 0.3275911, r10 = 0.1, r216 = 1.0 / 216.0, r42 = 1.0 / 42.0, rr3 = 1.0 / 3.0,
+               sqrpi = 1.7724538509055160273;
+  for (int b = 0; b < tot; b += 32) {
+    const int s = b + lane;
+    int L = 0;  // lanes whose pairs all precede s
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1)
+      if (__shfl_sync(0xffffffffu, inc, L + o - 1) <= s) L += o;
+    L &= 31;
+    const int m = s - __shfl_sync(0xffffffffu, inc - lim, L) + 1 + __shfl_sync(0xffffffffu, first, L);
+    const int a = __shfl_sync(0xffffffffu, i, L), ga = __shfl_sync(0xffffffffu, gi, L);
+    const double xa = __shfl_sync(0xffffffffu, xi, L), ya = __shfl_sync(0xffffffffu, yi, L),
+                 za = __shfl_sync(0xffffffffu, zi, L), qa = __shfl_sync(0xffffffffu, qi, L);
+    if (s >= tot) continue;
+    const int j = list[(size_t)a * ld + 3 + m] - 1;
+    const double xx = xa - x[j], yy = ya - y[j], zz = za - z[j];
+    const double rsq = xx * xx + yy * yy + zz * zz, rrr = sqrt(rsq);
+    double chgprd = q[j];
+    if (!(fabs(chgprd) > DBL_MIN) || !(rrr < rcut)) continue;
+    chgprd *= qa;
+    const double alpr = rrr * alpha, alpr2 = alpr * alpr;
+    double erfr, egamma;
+    if (alpr < 1.0e-2) {
+      erfr = 2.0 * chgprd * (alpha / sqrpi) * (1.0 + alpr2 * (-rr3 + alpr2 * (r10 + alpr2 * (-r42 + alpr2 * r216))));
+      egamma = -4.0 * chgprd * (alpha * alpha * alpha / sqrpi) *
+               (rr3 + alpr2 * (-2.0 * r10 + alpr2 * (3.0 * r42 - 4.0 * alpr2 * r216)));
+    } else {
+      const double exp1 = exp(-alpr2), tt = 1.0 / (1.0 + pp * alpha * rrr), ri = 1.0 / rrr;
+      erfr = chgprd * (1.0 - tt * (a1 + tt * (a2 + tt * (a3 + tt * (a4 + tt * a5)))) * exp1) * ri;
+      egamma = -(erfr - 2.0 * chgprd * (alpha / sqrpi) * exp1) * (ri * ri);
+    }
+    const double fx_ = egamma * xx, fy_ = egamma * yy, fz_ = egamma * zz;
+    if (fixp) {
+      const double sc = 1099511627776.0;
+      const unsigned long long ux = (unsigned long long)__double2ll_rn(fx_ * sc),
+                               uy = (unsigned long long)__double2ll_rn(fy_ * sc),
+                               uz = (unsigned long long)__double2ll_rn(fz_ * sc);
+      atomicAdd(&fixp[3 * a + 0], ux);
+      atomicAdd(&fixp[3 * a + 1], uy);
+      atomicAdd(&fixp[3 * a + 2], uz);
+      if (j < natms) {
+        atomicAdd(&fixp[3 * j + 0], 0ull - ux);
+        atomicAdd(&fixp[3 * j + 1], 0ull - uy);
+        atomicAdd(&fixp[3 * j + 2], 0ull - uz);
       }
-      if (fixp) {
-        const double sc = 1099511627776.0;
-        atomicAdd(&fixp[3 * i + 0], (unsigned long long)__double2ll_rn(fix * sc));
-        atomicAdd(&fixp[3 * i + 1], (unsigned long long)__double2ll_rn(fiy * sc));
-        atomicAdd(&fixp[3 * i + 2], (unsigned long long)__double2ll_rn(fiz * sc));
-      } else {
-        atomicAdd(&fx[i], fix); atomicAdd(&fy[i], fiy); atomicAdd(&fz[i], fiz);
+    } else {
+      atomicAdd(&fx[a], fx_); atomicAdd(&fy[a], fy_); atomicAdd(&fz[a], fz_);
+      if (j < natms) {
+        atomicAdd(&fx[j], -fx_); atomicAdd(&fy[j], -fy_); atomicAdd(&fz[j], -fz_);
       }
+    }
+    if (j < natms || ga < ltg[j]) {
+      acc[0] -= erfr;
+      acc[1] -= egamma * rsq;
+      acc[2] += xx * fx_; acc[3] += xx * fy_; acc[4] += xx * fz_;
+      acc[5] += yy * fy_; acc[6] += yy * fz_; acc[7] += zz * fz_;
     }
   }
   block_reduce_store<8>(acc, blk);
@@ -1329,18 +1355,20 @@ void pair_forces_sorted(PairGeom& pg, int nb2) {
                                           (unsigned long long*)g.fixp, blks, gss);
   GB_LAUNCHED();
   gb_grid_sum_done(gss, blks, nbs, NACC);
-  if (!mixed) {
+  auto add = [&]() {
+    if (mixed) return;
     k_fix_add_fp64<<<nblocks(g.natms, 256), 256, 0, st>>>(g.natms, g.fixp, g.fx, g.fy, g.fz);
     GB_LAUNCHED();
-  }
+  };
+  if (!g.lbook) add();
   prof_end(P_PAIR);
   if (g.lbook) {
     prof_begin(P_EXCL);
     const GridSum gse = gb_grid_sum(nb2, 128, 8, &g.sc->acc[A_EXCL]);
     k_excl_fp64<<<nb2, 128, 0, st>>>(g.natms, g.list, g.ld, g.x, g.y, g.z, g.chge, g.ltg, g.src, g.p.alpha,
-                                     g.scaling, g.p.rcut, g.fx, g.fy, g.fz, blk2,
-                                     mixed ? (unsigned long long*)g.fixp : nullptr, gse);
+                                     g.scaling, g.p.rcut, g.fx, g.fy, g.fz, blk2, (unsigned long long*)g.fixp, gse);
     GB_LAUNCHED();
+    add();
     prof_end(P_EXCL);
     gb_grid_sum_done(gse, blk2, nb2, 8);
   }
@@ -1429,8 +1457,6 @@ void pair_forces(double* eng6, double* stress9) {
     k_fold_images<<<std::max(1, nblocks(g.mxatms - g.natms, 256)), 256, 0, st>>>(g.natms, g.sc, g.src,
                                                                     (unsigned long long*)g.fixp);
     GB_LAUNCHED();
-    k_fix_add_fp64<<<nblocks(g.natms, 256), 256, 0, st>>>(g.natms, g.fixp, g.fx, g.fy, g.fz);
-    GB_LAUNCHED();
     prof_end(P_PAIR);
     gb_reduce_blocks(blk, nb, NACC_DF, &g.sc->acc[A_PAIR]);
     gb_reduce_blocks(blks, nbs, 6, &g.sc->acc[A_PAIR + NACC_DF]);
@@ -1439,11 +1465,13 @@ void pair_forces(double* eng6, double* stress9) {
       prof_begin(P_EXCL);
       const GridSum gse = gb_grid_sum(nb2, 128, 8, &g.sc->acc[A_EXCL]);
       k_excl_fp64<<<nb2, 128, 0, st>>>(g.natms, g.list, g.ld, g.x, g.y, g.z, g.chge, g.ltg, g.src, g.p.alpha,
-                                       g.scaling, g.p.rcut, g.fx, g.fy, g.fz, blk2, nullptr, gse);
+                                       g.scaling, g.p.rcut, g.fx, g.fy, g.fz, blk2, (unsigned long long*)g.fixp, gse);
       GB_LAUNCHED();
       prof_end(P_EXCL);
       gb_grid_sum_done(gse, blk2, nb2, 8);
     }
+    k_fix_add_fp64<<<nblocks(g.natms, 256), 256, 0, st>>>(g.natms, g.fixp, g.fx, g.fy, g.fz);
+    GB_LAUNCHED();
   } else if (g.precision == GB_FP64) {
     static int occ64 = 0;
     if (!occ64) GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ64, k_pair_fp64, T, 0));
