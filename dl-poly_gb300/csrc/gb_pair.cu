@@ -838,17 +838,19 @@ __device__ __forceinline__ df prod_pair(df a, df b) {
   return df_make(p.hi, __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.lo, b.hi, p.lo)));
 }
 
-// r (relative error about 1e-14: an FP32 root and the first-order remainder) and 1/r^2
-// (3e-14) of a double-float r^2
+// r (an FP32 root and its remainder to second order) and 1/r^2 (an FP32 reciprocal to the last
+// bit and its remainder) of a double-float r^2, both with relative errors below 1e-14
 __device__ __forceinline__ df dist_inv2(df r2, df* inv) {
   const float rs = rsqrtf(r2.hi);
   const float s = __fmul_rn(r2.hi, rs);
   const df ss = two_prod(s, s);
   const float e = __fadd_rn(__fsub_rn(__fsub_rn(r2.hi, ss.hi), ss.lo), r2.lo);
-  const float q = __fmul_rn(rs, rs);
-  const float g = __fmaf_rn(-r2.lo, q, __fmaf_rn(-r2.hi, q, 1.f));  // 1 - r2 q
-  *inv = df_make(q, __fmul_rn(q, __fmaf_rn(g, g, g)));
-  return quick_two_sum(s, __fmul_rn(__fmul_rn(0.5f, rs), e));
+  const float q0 = __fmul_rn(rs, rs);
+  const float g0 = __fmaf_rn(-r2.hi, q0, 1.f);  // 1 - r2 q0
+  const float q = __fmaf_rn(q0, g0, q0);
+  *inv = df_make(q, __fmul_rn(q, __fmaf_rn(-r2.lo, q, __fmaf_rn(-r2.hi, q, 1.f))));
+  const float rc = __fmaf_rn(rs, __fmul_rn(0.5f, g0), rs);  // 1/r to the last bit
+  return quick_two_sum(s, __fmul_rn(__fmul_rn(0.5f, rc), e));
 }
 
 // The FP64 form's terms of one pair (the formulas of pair_terms_df64, partner data
