@@ -14,17 +14,13 @@
 #include <cmath>
 #include <cstring>
 
-#include <cooperative_groups.h>
-
 #include "gb_common.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace {
 
 constexpr int MAX_SBC = 1024;  // semi-ball offsets capacity
 
-// for k_list_tiles, read a lane each: per semi-ball cell its linear offset and
+// for the list kernels: per semi-ball cell its linear offset and
 // (nix + 64) | (niy + 64) << 8 | (niz + 64) << 16 | nir << 24; and, as the semi-ball cells in
 // the reference order form, tile row (dy, dz) by tile row, runs of consecutive cells along x
 // (contiguous sorted positions), per run with one nir flag the linear offsets of its first
