@@ -370,8 +370,8 @@ __global__ void __launch_bounds__(256, 3) k_metal_forces(int natms, const DevSca
 //               against 64 bits 1.2e-13, the FP64 kernels 0.8e-13: both from r, on which
 //               the difference of a pair's terms depends forty times over; energies and
 //               stress are nearer than the FP64 kernels')
-// A pair near a cutoff, at an end of its table, with a negative density or outside the
-// FP32 range takes the FP64 formulas of the kernels above (metal_density_slow,
+// A pair near a cutoff, at an end of its table, next to the middle of two points, with a
+// negative density or outside the FP32 range takes the FP64 formulas of the kernels above (metal_density_slow,
 // metal_force_slow).  Densities and forces are summed in FP64 per sorted position and
 // folded onto the atoms (a halo image's onto its source) afterwards.
 struct __align__(16) CoefF {
@@ -426,7 +426,9 @@ __device__ __forceinline__ df met_dist(df r2, df* inv) {
   return quick_two_sum(s, __fmul_rn(__fmul_rn(0.5f, y), e));
 }
 
-// table point l and fraction p in [-0.5, 0.5] of a double-float r; false at a table's ends.
+// table point l and fraction p in [-0.5, 0.5] of a double-float r; false at a table's ends and
+// next to the middle of two points (|p| = 0.5 to FP32, one lookup in 10^7), where the
+// interpolant jumps by an eighth of the third difference and FP64 decides which point is nearer.
 // p = (r - r_l) / dr from the point's own r: the product r / dr would be rounded at 2^-48 of
 // a coordinate of some thousand.
 __device__ __forceinline__ bool met_coord(const MetTab& t, const CoefF* __restrict__ c, df r, int* l, df* p) {
@@ -446,7 +448,7 @@ __device__ __forceinline__ bool met_coord(const MetTab& t, const CoefF* __restri
   }
   *l = i;
   *p = d;
-  return i > 5 && i < t.n - 1;
+  return i > 5 && i < t.n - 1 && fabsf(d.hi) != 0.5f;
 }
 
 __device__ __forceinline__ df met_poly(const CoefF* __restrict__ c, int l, df p) {

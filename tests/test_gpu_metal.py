@@ -64,3 +64,27 @@ def test_eam_error_statuses_on_gpu(gpu_lib):
     with pytest.raises(Exception, match="507"):
         gpu_lib.start()
     kat_check(gpu_lib)             # the context is still usable
+
+
+@pytest.mark.parametrize("side", [-1, 1])
+@pytest.mark.parametrize("off", [2e-9, 1e-8, 2.5e-8, 1e-6])
+def test_eam_pairs_next_to_a_midpoint(gpu_lib, oracle_lib, side, off):
+    """Separations a small fraction of an interval from the middle of two table points, where
+    the three-point interpolant jumps (here by 1e-5 of the force): the nearer point is taken."""
+    ng = 100
+    r = np.linspace(1.0, 6.0, ng)
+    rho = np.linspace(0.0, 10.0, ng)
+    dr = 5.0 / (ng - 1)
+    for k in (23, 40, 61):
+        s = two_atoms(1.0 + (k + 0.5 + side * off) * dr)
+        s.eam = [{"kind": "pair", "types": (1, 1), "start": 1.0, "finish": 6.0, "values": r ** -3},
+                 {"kind": "dens", "types": (1, 1), "start": 1.0, "finish": 6.0, "values": r ** -2},
+                 {"kind": "embe", "types": (1, 1), "start": 0.0, "finish": 10.0, "values": 0.01 * rho ** 2}]
+        out = []
+        for lib in (gpu_lib, oracle_lib):
+            lib.init(s)
+            lib.start()
+            out.append((lib.download()["fx"], lib.metal_rho()))
+        (fa, ra), (fb, rb) = out
+        assert np.abs(fa - fb).max() <= 1e-10 * np.abs(fb).max()
+        np.testing.assert_allclose(ra, rb, rtol=1e-10)
