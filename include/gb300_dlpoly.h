@@ -44,7 +44,7 @@ extern "C" {
 #define GB_ERR_ARG (-3)
 #define GB_ERR_NO_DEVICE (-4)
 #define GB_ERR_NONFINITE (-5)
-#define GB_ERR_TOO_LARGE (-6)  /* size beyond a fixed scratch limit (gb_kinstress_noalloc) */
+#define GB_ERR_TOO_LARGE (-6)  /* more atoms than gb_kinstress_noalloc takes */
 #define GB_ERR_RNG (-7)        /* a Gaussian deviate's rejection loop hit its iteration cap */
 #define GB_ERR_MULTI_RANK (-8) /* gb_params.mxnode > 1: a multi-rank run cannot use the device path */
 #define GB_ERR_DEVICE_WAIT (-9) /* a kernel's wait on its tensor-core completion hit its iteration limit */
@@ -348,14 +348,14 @@ double gb_fp64_peak_tflops(void);
  *   (9 doubles, the symmetric 3x3 tensor) are DEVICE pointers; stream may be
  *   NULL (the default stream).  The call only enqueues work: synchronise the
  *   stream before reading strkin_out.  It needs no gb_init.
- * It allocates nothing.  Its scratch is a fixed array of 4096 x 6 doubles
- * (196,608 bytes) in the library's device memory, held on every GPU that loads
- * the library until the process exits, so n is limited to 1,048,576 atoms;
- * larger n returns GB_ERR_TOO_LARGE and launches nothing.  The first call on
- * each device looks up the address of that array; make that first call before
- * any stream capture.  All calls share the one array: calls that overlap on
- * the GPU (concurrent streams, or another host thread) race and give wrong
- * results, so serialise them.
+ * It allocates nothing.  Its scratch is a fixed array of 14,648 bytes in the
+ * library's device memory, held on every GPU that loads the library until the
+ * process exits.  n is limited to 1,048,576 atoms; larger n returns
+ * GB_ERR_TOO_LARGE and launches nothing.  The first call on each device looks
+ * up the address of that array; make that first call before any stream
+ * capture.  All calls share the one array: calls that overlap on the GPU
+ * (concurrent streams, or another host thread) race and give wrong results,
+ * so serialise them.  Later calls are not affected.
  */
 int gb_kinstress_noalloc(const double* vx, const double* vy, const double* vz, const double* weight,
                          const int32_t* lfrzn, int n, double* strkin_out, void* stream);

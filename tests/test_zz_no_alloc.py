@@ -115,3 +115,58 @@ def test_kinstress_noalloc_rejects_too_many_atoms(gpu_lib):
     dummy = ctypes.c_void_p(16)
     rc = f(dummy, dummy, dummy, dummy, None, 1 << 21, dummy, None)
     assert rc == -6
+
+
+class _MemsetParams(ctypes.Structure):  # CUDA_MEMSET_NODE_PARAMS
+    _fields_ = [("dst", ctypes.c_uint64), ("pitch", ctypes.c_size_t), ("value", ctypes.c_uint),
+                ("elementSize", ctypes.c_uint), ("width", ctypes.c_size_t), ("height", ctypes.c_size_t)]
+
+
+def test_kinstress_noalloc_recovers_from_a_stale_block_count(gpu_lib):
+    """A count of finished blocks left over from calls that overlapped does not reach the next
+    call, which clears it on its stream: its place is read from a captured call, and garbage put there."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device visible to torch")
+    f = _bind(gpu_lib.lib)
+    cu = ctypes.CDLL("libcuda.so.1")
+    dev = torch.device("cuda", 0)
+    n = 5000
+    rng = np.random.default_rng(3)
+    h = [rng.standard_normal(n) for _ in range(3)] + [rng.uniform(1.0, 60.0, n)]
+    vx, vy, vz, w = (torch.tensor(v, dtype=torch.float64, device=dev) for v in h)
+    expect = _kin_numpy(dict(vx=h[0], vy=h[1], vz=h[2]), h[3])
+    out = torch.full((9,), float("nan"), dtype=torch.float64, device=dev)
+    torch.cuda.synchronize()
+    stream = torch.cuda.Stream(dev)
+    sp = ctypes.c_void_p(stream.cuda_stream)
+    args = (vx.data_ptr(), vy.data_ptr(), vz.data_ptr(), w.data_ptr(), None, n, out.data_ptr(), sp)
+    assert f(*args) == 0  # (looks the scratch up)
+    stream.synchronize()
+    graph = ctypes.c_void_p()
+    assert cu.cuStreamBeginCapture_v2(sp, ctypes.c_int(2)) == 0  # relaxed
+    assert f(*args) == 0
+    assert cu.cuStreamEndCapture(sp, ctypes.byref(graph)) == 0
+    num = ctypes.c_size_t(16)
+    nodes = (ctypes.c_void_p * 16)()
+    assert cu.cuGraphGetNodes(graph, nodes, ctypes.byref(num)) == 0
+    cleared = []
+    for k in range(num.value):
+        kind = ctypes.c_int()
+        assert cu.cuGraphNodeGetType(ctypes.c_void_p(nodes[k]), ctypes.byref(kind)) == 0
+        if kind.value == 2:  # a memset
+            p = _MemsetParams()
+            assert cu.cuGraphMemsetNodeGetParams(ctypes.c_void_p(nodes[k]), ctypes.byref(p)) == 0
+            assert (p.value, p.elementSize * p.width, p.height) == (0, 4, 1)
+            cleared.append(p.dst)
+    cu.cuGraphDestroy(graph)
+    assert len(cleared) == 1
+    for stale in (1, 19, 1 << 20):
+        assert cu.cuMemsetD32_v2(ctypes.c_uint64(cleared[0]), ctypes.c_uint(stale), ctypes.c_size_t(1)) == 0
+        torch.cuda.synchronize()
+        out.fill_(float("nan"))
+        torch.cuda.synchronize()
+        assert f(*args) == 0
+        stream.synchronize()
+        got = out.cpu().numpy()
+        assert np.abs(got - expect).max() <= REL * np.abs(expect).max()
