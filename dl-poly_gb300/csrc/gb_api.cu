@@ -596,6 +596,8 @@ GridSum gb_grid_sum(int nb, int nt, int nv, double* out_dev) {
   return {nb <= 20 * std::max(rows, 1) ? (g.side ? &g.sc->count_s : &g.sc->count) : nullptr, out_dev};
 }
 
+StopIf stop_if(int mask) { return {&g.sc->status, g.defer_scalars ? mask : 0}; }
+
 void gb_grid_sum_done(const GridSum& gs, const double* blk, int nb, int nv) {
   if (!gs.count) gb_reduce_blocks(blk, nb, nv, gs.out);
 }
@@ -1087,9 +1089,10 @@ static void md_step_stats(const DevScalars* h, int32_t rebuilt, gb_step_stats& S
 }
 
 // The loop without learned MTS: the host waits only for the Verlet-list decision of each
-// step (vnl_check), where it also sees the status bits set since the last one (a RATTLE
-// or metal table failure of a step thus ends the call at the next step's decision, after
-// that step's stage 1, with the same code); each step's energy, virial and stress sums are
+// step (vnl_check), where it also sees the status bits set since the last one.  A RATTLE or
+// metal failure of a step thus ends the call at the next step's decision; the work behind it
+// has left the state alone (StopIf), and the step counter goes back to the failing step.  Each
+// step's energy, virial and stress sums are
 // copied to a pinned ring with the step's other work and turned into gb_step_stats after
 // the last step.  With 3 or more steps the steps run as two CUDA graphs: stage 1 with the
 // displacement check (its sums copied to the pinned scalars), then, after the host's
@@ -1131,16 +1134,20 @@ static int md_run_deferred(int nsteps, gb_step_stats* stats) {
   const bool graph1 = graphs && g.ens != GB_NVT_LANGEVIN && capture_graph(&g.gx_vv1, &g.gl_vv1, stage1);
   if (graphs && g.ens != GB_NVT_LANGEVIN && !graph1) graphs = false;
   bool step_ok = false, step_spos = false;  // gx_step holds the step's rest for this kind of list
-  int code = GB_OK, done = 0;
+  int code = GB_OK, done = 0, last = -1;  // steps to report; last step with sums in the ring
   for (int s = 0; s < nsteps && code == GB_OK; ++s) {
     ++g.nstep;
     if (graph1) launch_graph(g.gx_vv1, g.gl_vv1);
     else stage1();
     GB_CUDA(cudaStreamSynchronize(g.stream));
     if (g.prof_on) gb_sync_scalars();  // resolves the pending profile events
-    code = md_status(g.hsc->status);
+    code = md_status(g.hsc->status & ~ST_RNG);
     if (code != GB_OK) {
-      done = (g.hsc->status & ST_SHAKE_FAIL) ? s : std::max(0, s - 1);
+      done = s;
+      if (!(g.hsc->status & ST_SHAKE_FAIL)) {  // of the step before
+        done = std::max(0, s - 1);
+        --g.nstep;
+      }
       break;
     }
     done = s;
@@ -1160,14 +1167,16 @@ static int md_run_deferred(int nsteps, gb_step_stats* stats) {
     if (graphs && step_ok) launch_graph(g.gx_step, g.gl_step);
     else step_rest();
     GB_CUDA(cudaMemcpyAsync(&g.ring[s], g.sc, sizeof(DevScalars), cudaMemcpyDeviceToHost, g.stream));
+    last = s;
     done = s + 1;
+    if (g.hsc->status & ST_RNG) break;  // Langevin's noise (stage 1) ends the call after the step
   }
   g.defer_scalars = false;
   GB_CUDA(cudaEventRecord(g.ev[6], g.stream));
   GB_CUDA(cudaEventSynchronize(g.ev[6]));
-  if (code == GB_OK && nsteps > 0) {
-    code = md_status(g.ring[nsteps - 1].status);
-    if (code != GB_OK) done = nsteps - 1;
+  if (code == GB_OK && last >= 0) {
+    code = md_status(g.ring[last].status);
+    if (code != GB_OK) done = last;
   }
   float span = 0.f;
   cudaEventElapsedTime(&span, g.ev[5], g.ev[6]);
@@ -1176,10 +1185,10 @@ static int md_run_deferred(int nsteps, gb_step_stats* stats) {
   g.last_ms[5] = span;
   if (stats)
     for (int s = 0; s < done; ++s) md_step_stats(&g.ring[s], rebuilt[s], stats[s]);
-  for (int k = 0; k < 4; ++k) g.metal_e4[k] = 0.0;
-  if (g.has_metal && done > 0) {
+  if (last >= 0) {  // the sums of the last evaluation (none of a failed one)
     double st[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
-    metal_scalars(&g.ring[done - 1], g.metal_e4, st);
+    for (int k = 0; k < 4; ++k) g.metal_e4[k] = 0.0;
+    if (g.has_metal && !(g.ring[last].status & ST_STOP2)) metal_scalars(&g.ring[last], g.metal_e4, st);
   }
   return code;
 }

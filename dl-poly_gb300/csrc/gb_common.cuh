@@ -26,6 +26,18 @@ enum : int {
   ST_METAL_TABLE = 256,  // a metal table read below its first point (error 506)
   ST_METAL_DENSITY = 512,  // a local density outside its embedding table (error 507)
   ST_DEVICE_WAIT = 1024,   // a kernel's wait on an mbarrier hit its iteration limit
+  // The MD loop that reads the status once per step enqueues work behind a failure that it has
+  // not seen yet: stage 2 does nothing after a failed force evaluation, and the next stage 1
+  // nothing after a failed step, so that the state is that of the failing step.
+  ST_STOP2 = ST_METAL_TABLE | ST_METAL_DENSITY,
+  ST_STOP1 = ST_STOP2 | ST_RATTLE_FAIL,
+};
+
+// For the kernels of the VV stages: nothing to do once one of these bits is set (0: never).
+struct StopIf {
+  const int* status;
+  int mask;
+  __device__ __forceinline__ bool set() const { return mask && (*status & mask); }
 };
 
 // Device-resident scalars: one small block so a single copy returns them all.
@@ -466,6 +478,8 @@ GridSum gb_grid_sum(int nb, int nt, int nv, double* out_dev);
 void gb_grid_sum_done(const GridSum& gs, const double* blk, int nb, int nv);
 void side_join();                 // the first stream waits for the side stream (no-op without a fork)
 void run_side_hook();             // enqueue the pending side-stream work (g.side_hook), if any
+
+StopIf stop_if(int mask);         // in the MD loop that reads the status once per step; never elsewhere
 
 // module entry points (host)
 // pbcshift + halo + vnl_set_check (gb_list.cu); wait = false leaves the halo's status to the

@@ -53,9 +53,9 @@ __device__ __forceinline__ double image_short(double d, long long quarter_bits, 
 // instead of dividing on the FP64 unit.
 __global__ void k_vv1(int n, const double* __restrict__ hdw, double tstep, const double* __restrict__ fx,
                       const double* __restrict__ fy, const double* __restrict__ fz, double* vx, double* vy, double* vz,
-                      double* x, double* y, double* z) {
+                      double* x, double* y, double* z, StopIf stop) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  if (i >= n || stop.set()) return;
   const double tmp = hdw[i];
   if (tmp > 0.0) {
     vx[i] = vx[i] + tmp * fx[i];
@@ -69,9 +69,9 @@ __global__ void k_vv1(int n, const double* __restrict__ hdw, double tstep, const
 
 __global__ void k_vv2(int n, const double* __restrict__ hdw, const double* __restrict__ fx,
                       const double* __restrict__ fy, const double* __restrict__ fz, double* vx, double* vy,
-                      double* vz) {
+                      double* vz, StopIf stop) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  if (i >= n || stop.set()) return;
   const double tmp = hdw[i];
   if (tmp > 0.0) {
     vx[i] = vx[i] + tmp * fx[i];
@@ -91,8 +91,9 @@ __global__ void __launch_bounds__(KIN_NT) k_kinstress(int n, const double* __res
                                                       const double* __restrict__ fx, const double* __restrict__ fy,
                                                       const double* __restrict__ fz, double* __restrict__ vx,
                                                       double* __restrict__ vy, double* __restrict__ vz, double* part,
-                                                      GridSum gs) {
+                                                      GridSum gs, StopIf stop) {
   double a[6] = {0, 0, 0, 0, 0, 0};
+  if (stop.set()) hdw = nullptr;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double m = w[i];
     double u = vx[i], v = vy[i], t = vz[i];
@@ -121,8 +122,9 @@ __global__ void k_maxdisp(int n, const double* __restrict__ hdw, double tstep, c
                           double* __restrict__ vy, double* __restrict__ vz, double* __restrict__ x,
                           double* __restrict__ y, double* __restrict__ z, const double* __restrict__ xb,
                           const double* __restrict__ yb, const double* __restrict__ zb, double c0, double a0,
-                          unsigned long long* out) {
+                          unsigned long long* out, StopIf stop) {
   double r2 = 0.0;
+  if (stop.set()) hdw = nullptr;
   const long long quarter = __double_as_longlong(0.25 * c0);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     double px = x[i], py = y[i], pz = z[i];
@@ -178,10 +180,12 @@ struct ConArgs {
   bool tags;       // RATTLE of k_constrain_small: form the bond vectors from the positions (and store them)
   DevScalars* sc;
   double* blk;     // per-block stress partials (6)
+  StopIf stop;
 };
 
 // constraints_shake_vv: Jacobi sweeps until every |d^2 - d0^2|/2 < tol*d0
 __global__ void k_shake(ConArgs A) {
+  if (A.stop.set()) return;
   cg::grid_group grid = cg::this_grid();
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int nth = gridDim.x * blockDim.x;
@@ -246,6 +250,7 @@ __global__ void k_shake(ConArgs A) {
 
 // constraints_rattle: normalise the bond vectors, then Jacobi sweeps on v
 __global__ void k_rattle(ConArgs A) {
+  if (A.stop.set()) return;
   cg::grid_group grid = cg::this_grid();
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
   const int nth = gridDim.x * blockDim.x;
@@ -463,6 +468,7 @@ template <int MA, int MC>
 __global__ void __launch_bounds__(128) k_constrain_cl(ConArgs A, const ClusterTab* __restrict__ tabs, int ncl,
                                                       double* __restrict__ ring, double* __restrict__ gsum,
                                                       int rattle_i) {
+  if (A.stop.set()) return;
   cg::grid_group grid = cg::this_grid();
   const bool rattle = rattle_i != 0;
   const int tid = blockIdx.x * blockDim.x + threadIdx.x;
@@ -756,6 +762,7 @@ __global__ void __launch_bounds__(CS_THREADS) k_constrain_small(ConArgs A, const
                                                                float2* __restrict__ pbuf, double rstep, double* fx,
                                                                double* fy, double* fz) {
   extern __shared__ float2 cs_hist[];  // [CS_CHUNK][blockDim.x]: the scalar before each sweep of the chunk
+  if (A.stop.set()) return;
   cg::grid_group grid = cg::this_grid();
   const int lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const int wstep = ((gridDim.x * blockDim.x) >> 5) * CS_PERWARP;
@@ -905,9 +912,9 @@ __global__ void __launch_bounds__(CS_THREADS) k_constrain_small(ConArgs A, const
 __global__ void k_shake_post(int n, const int* astart, const int* lfrzn, double rstep, double hstep, const double* w,
                              const double* x, const double* y, const double* z, const double* ox, const double* oy,
                              const double* oz, double* vx, double* vy, double* vz, double* fx, double* fy,
-                             double* fz) {
+                             double* fz, StopIf stop) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  if (i >= n || stop.set()) return;
   if (astart[i + 1] == astart[i] || lfrzn[i] != 0) return;
   double xt = (x[i] - ox[i]) * rstep, yt = (y[i] - oy[i]) * rstep, zt = (z[i] - oz[i]) * rstep;
   vx[i] += xt; vy[i] += yt; vz[i] += zt;
@@ -1148,7 +1155,7 @@ void integ_forces_to_fp64() {
 static void launch_maxdisp(bool stage1) {
   k_maxdisp<<<std::min(nblocks(g.natms, 128), 4 * g.nsm), 128, 0, g.stream>>>(
       g.natms, stage1 ? g.hdw : nullptr, g.p.tstep, g.fx, g.fy, g.fz, g.vx, g.vy, g.vz, g.x, g.y, g.z, g.xbg, g.ybg,
-      g.zbg, g.cell[0], 1.0 / g.cell[0], (unsigned long long*)&g.sc->maxdisp);
+      g.zbg, g.cell[0], 1.0 / g.cell[0], (unsigned long long*)&g.sc->maxdisp, stop_if(ST_STOP1));
   GB_LAUNCHED();
 }
 
@@ -1173,7 +1180,7 @@ int integ_vnl_check() {
   return integ_vnl_result();
 }
 
-static void con_args(ConArgs& A) {
+static void con_args(ConArgs& A, int stop) {
   A.nc = g.ntcons; A.natms = g.natms; A.maxit = g.p.shake_maxit;
   A.ci = g.con_i; A.cj = g.con_j; A.listot = g.listot; A.astart = g.acon_start; A.alist = g.acon_list;
   A.lfrzn = g.lfrzn; A.d0 = g.con_d0;
@@ -1182,6 +1189,7 @@ static void con_args(ConArgs& A) {
   A.x = g.x; A.y = g.y; A.z = g.z; A.vx = g.vx; A.vy = g.vy; A.vz = g.vz; A.w = g.weight;
   A.tstep = g.p.tstep; A.tol = g.p.shake_tol; A.c0 = g.cell[0]; A.a0 = 1.0 / g.cell[0];
   A.flags = d_flags; A.sc = g.sc; A.blk = nullptr; A.gs = {nullptr, nullptr}; A.tags = false;
+  A.stop = stop_if(stop);
 }
 
 template <bool RATTLE>
@@ -1220,7 +1228,7 @@ void integ_shake(int* iters, double* vircon, double* strcon) {
   }
   GB_CUDA(cudaMemsetAsync(d_flags, 0, sizeof(int) * (g.p.shake_maxit + CL_CHUNK + 2), st));
   ConArgs A;
-  con_args(A);
+  con_args(A, ST_STOP1);
   const int nbs = cl_small ? coop_blocks_small : n_clusters ? coop_blocks_cl : coop_blocks_shake;
   A.blk = gb_blkacc(nbs * 6);
   if (cl_small) A.gs = gb_grid_sum(nbs, cs_threads, 6, &g.sc->acc[A_STRCON]);
@@ -1243,7 +1251,8 @@ void integ_shake(int* iters, double* vircon, double* strcon) {
   if (!A.gs.count) gb_reduce_blocks(A.blk, nbs, 6, &g.sc->acc[A_STRCON]);
   if (!cl_small) {
     k_shake_post<<<nblocks(n, 256), 256, 0, st>>>(n, g.acon_start, g.lfrzn, rstep, hstep, g.weight, g.x, g.y, g.z,
-                                                   g.ox, g.oy, g.oz, g.vx, g.vy, g.vz, g.fx, g.fy, g.fz);
+                                                   g.ox, g.oy, g.oz, g.vx, g.vy, g.vz, g.fx, g.fy, g.fz,
+                                                   stop_if(ST_STOP1));
     GB_LAUNCHED();
   }
   if (g.defer_scalars) return;  // the MD loop reads the sums and the status
@@ -1262,7 +1271,7 @@ void integ_rattle_launch(bool tags) {
   cudaStream_t st = g.stream;
   GB_CUDA(cudaMemsetAsync(d_flags, 0, sizeof(int) * (g.p.shake_maxit + CL_CHUNK + 2), st));
   ConArgs A;
-  con_args(A);
+  con_args(A, ST_STOP2);
   if (tags && !cl_small) integ_con_tags();
   A.tags = tags;
   prof_begin(P_RATTLE);
@@ -1288,7 +1297,7 @@ static void launch_kinstress(bool kick) {
   const GridSum gs = gb_grid_sum(nb, KIN_NT, 6, &g.sc->acc[A_STRKIN]);
   double* part = gb_blkacc(nb * 6);
   k_kinstress<<<nb, KIN_NT, 0, g.stream>>>(g.natms, g.weight, g.lfrzn, kick ? g.hdw : nullptr, g.fx, g.fy, g.fz, g.vx,
-                                           g.vy, g.vz, part, gs);
+                                           g.vy, g.vz, part, gs, stop_if(ST_STOP2));
   GB_LAUNCHED();
   gb_grid_sum_done(gs, part, nb, 6);
 }
@@ -1302,7 +1311,8 @@ void integ_vv(int stage, double* strkin, double* engke, int* iters, double* virc
     integ_con_tags();
     prof_begin(P_VV);
     if (!thermo_vv1(hstep, tstep)) {
-      k_vv1<<<nblocks(n, 256), 256, 0, st>>>(n, g.hdw, tstep, g.fx, g.fy, g.fz, g.vx, g.vy, g.vz, g.x, g.y, g.z);
+      k_vv1<<<nblocks(n, 256), 256, 0, st>>>(n, g.hdw, tstep, g.fx, g.fy, g.fz, g.vx, g.vy, g.vz, g.x, g.y, g.z,
+                                             stop_if(ST_STOP1));
       GB_LAUNCHED();
     }
     prof_end(P_VV);
@@ -1311,7 +1321,7 @@ void integ_vv(int stage, double* strkin, double* engke, int* iters, double* virc
     const bool fused = g.ntcons <= 0 && g.ens == GB_NVE;  // the kick and the kinetic stress in one pass
     prof_begin(P_VV);
     if (!fused) {
-      k_vv2<<<nblocks(n, 256), 256, 0, st>>>(n, g.hdw, g.fx, g.fy, g.fz, g.vx, g.vy, g.vz);
+      k_vv2<<<nblocks(n, 256), 256, 0, st>>>(n, g.hdw, g.fx, g.fy, g.fz, g.vx, g.vy, g.vz, stop_if(ST_STOP2));
       GB_LAUNCHED();
     }
     if (fused) launch_kinstress(true);

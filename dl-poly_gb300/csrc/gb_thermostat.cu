@@ -186,7 +186,8 @@ __device__ __forceinline__ void thermo_post(DevScalars* sc, const ThermoPost& t)
 __global__ void __launch_bounds__(256) k_kin_mom(int n, const double* __restrict__ w, const int* __restrict__ lfrzn,
                                                  const double* __restrict__ vx, const double* __restrict__ vy,
                                                  const double* __restrict__ vz, double* part, GridSum gs,
-                                                 DevScalars* sc, ThermoPost post) {
+                                                 DevScalars* sc, ThermoPost post, StopIf stop) {
+  if (stop.set()) return;
   double a[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     if (lfrzn[i] != 0) continue;
@@ -206,7 +207,8 @@ __global__ void __launch_bounds__(256) k_kin_mom(int n, const double* __restrict
 __global__ void __launch_bounds__(256) k_scale_kin(int n, const double* th, int sub_vom, const double* __restrict__ w,
                                                    const int* __restrict__ lfrzn, double* __restrict__ vx,
                                                    double* __restrict__ vy, double* __restrict__ vz, double* part,
-                                                   GridSum gs, DevScalars* sc, ThermoPost post) {
+                                                   GridSum gs, DevScalars* sc, ThermoPost post, StopIf stop) {
+  if (stop.set()) return;
   double a[6] = {0, 0, 0, 0, 0, 0};
   const double s = th[2];
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -225,9 +227,9 @@ __global__ void __launch_bounds__(256) k_scale_kin(int n, const double* th, int 
 // Nose-Hoover stage 1: v <- scale*v (nvt_h0_scl), then the VV half kick and drift
 __global__ void k_vv1_scaled(int n, double hstep, double tstep, const double* th, const double* w, const double* fx,
                              const double* fy, const double* fz, double* vx, double* vy, double* vz, double* x,
-                             double* y, double* z) {
+                             double* y, double* z, StopIf stop) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  if (i >= n || stop.set()) return;
   const double s = th[2];
   double ux = s * vx[i], uy = s * vy[i], uz = s * vz[i];
   if (w[i] > 1.0e-6) {
@@ -252,9 +254,9 @@ struct LangevinArgs {
 // (langevin_forces), drawn here per atom, enter the drift and the velocity
 __global__ void k_vv1_langevin(int n, LangevinArgs L, const double* w, const int* lfrzn, const int* ltg,
                                const double* fx, const double* fy, const double* fz, double* vx, double* vy,
-                               double* vz, double* x, double* y, double* z, int* status) {
+                               double* vz, double* x, double* y, double* z, int* status, StopIf stop) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n || !(w[i] > 1.0e-6)) return;
+  if (i >= n || !(w[i] > 1.0e-6) || stop.set()) return;
   double fr[3] = {0, 0, 0}, fl[3] = {0, 0, 0};
   if (lfrzn[i] == 0) {
     int bad = 0;
@@ -341,11 +343,11 @@ void thermo_state(double* chi_t, double* cint, double* consv) {
 }
 
 // up to two blocks of 256 threads per SM
-static void launch_kin_mom(const ThermoPost& post) {
+static void launch_kin_mom(const ThermoPost& post, int stop) {
   const int nb = std::min(nblocks(g.natms, 256), 2 * g.nsm);
   double* part = gb_blkacc(nb * 9);
   k_kin_mom<<<nb, 256, 0, g.stream>>>(g.natms, g.weight, g.lfrzn, g.vx, g.vy, g.vz, part,
-                                      {&g.sc->count, &g.sc->acc[A_KINMOM]}, g.sc, post);
+                                      {&g.sc->count, &g.sc->acc[A_KINMOM]}, g.sc, post, stop_if(stop));
   GB_LAUNCHED();
 }
 
@@ -354,9 +356,9 @@ static ThermoPost nh_post(double ts) { return {1, 0, ts, g.qmass, g.ceng, 0.0, 0
 bool thermo_vv1(double hstep, double tstep) {
   const int n = g.natms, nb = nblocks(n, 256);
   if (g.ens == GB_NVT_NOSE_HOOVER) {
-    launch_kin_mom(nh_post(hstep));
+    launch_kin_mom(nh_post(hstep), ST_STOP1);
     k_vv1_scaled<<<nb, 256, 0, g.stream>>>(n, hstep, tstep, g.sc->th, g.weight, g.fx, g.fy, g.fz, g.vx, g.vy, g.vz,
-                                           g.x, g.y, g.z);
+                                           g.x, g.y, g.z, stop_if(ST_STOP1));
     GB_LAUNCHED();
     return true;
   }
@@ -368,7 +370,7 @@ bool thermo_vv1(double hstep, double tstep) {
     L.nstep = g.nstep;
     for (int k = 0; k < 3; ++k) L.seed[k] = g.seed[k];
     k_vv1_langevin<<<nb, 256, 0, g.stream>>>(n, L, g.weight, g.lfrzn, g.ltg, g.fx, g.fy, g.fz, g.vx, g.vy, g.vz,
-                                             g.x, g.y, g.z, &g.sc->status);
+                                             g.x, g.y, g.z, &g.sc->status, stop_if(ST_STOP1));
     GB_LAUNCHED();
     return true;
   }
@@ -381,10 +383,11 @@ bool thermo_vv2_finish(double* strkin, double* engke) {
   const bool nh = g.ens == GB_NVT_NOSE_HOOVER, ber = g.ens == GB_NVT_BERENDSEN;
   const ThermoPost vom = {2, ber ? 1 : 0, 0.0, 0.0, 0.0, g.p.tstep, g.tau_t, g.sigma, g.totmas};
   const ThermoPost fin = {ber ? 3 : 0, 0, 0.0, 0.0, 0.0, g.p.tstep, g.tau_t, g.sigma, 0.0};
-  launch_kin_mom(nh ? nh_post(0.5 * g.p.tstep) : vom);
+  launch_kin_mom(nh ? nh_post(0.5 * g.p.tstep) : vom, ST_STOP2);
   double* part = gb_blkacc(nb * 6);
   k_scale_kin<<<nb, 256, 0, g.stream>>>(n, g.sc->th, nh ? 0 : 1, g.weight, g.lfrzn, g.vx, g.vy, g.vz, part,
-                                        {&g.sc->count, &g.sc->acc[A_STRKIN]}, g.sc, fin);
+                                        {&g.sc->count, &g.sc->acc[A_STRKIN]}, g.sc, fin,
+                                        stop_if(ST_STOP2));
   GB_LAUNCHED();
   if (g.defer_scalars) return true;  // the MD loop reads the sums
   gb_sync_scalars();

@@ -212,8 +212,10 @@ int gb_rattle(int32_t* iters);
  * refresh, forces, VV2+RATTLE with no host round trip; stats[nsteps] may be NULL.
  * Each step first advances the step counter (gb_set_step).  Without learned MTS a call
  * of 3 or more steps replays each step as CUDA graphs captured inside the call (same
- * kernels and results), and a step's failure that its forces or stage 2 set ends the call
- * at the next step's list decision, with that step's code. */
+ * kernels and results).  A failing step (SHAKE, RATTLE, metal, noise) ends the call with its
+ * code: the steps before it are in stats, and the state and the step counter are those that the
+ * failure left (after SHAKE: stage 1; after a metal failure: stage 1 and the forces; after
+ * RATTLE or the noise: the whole step). */
 int gb_md_run(int nsteps, gb_step_stats* stats);
 
 /* Ensemble of the VV stages: the dispatch on thermo%ensemble (drivers.F90:1132-1175)

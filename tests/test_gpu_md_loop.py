@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 from dlpoly_gb300 import systems
+from test_metal_oracle import poly_tables, two_atoms
 
 pytestmark = pytest.mark.gpu
 
@@ -64,3 +65,77 @@ def test_failing_step_ends_the_call_with_its_code(gpu_lib):
     gpu_lib.init(s)
     gpu_lib.start()
     assert all(x.shake_iters > 20 for x in gpu_lib.md_vv(5))
+
+
+def _colliding_water():
+    """64 molecules, one of which reaches another's oxygen in two steps: RATTLE of the second
+    step then has velocities that need more sweeps than it is given."""
+    s = systems.spce_water(4, box=24.0, rcut=7.0, kmax=32)
+    s.tstep = 2e-5
+    for v in (s.vx, s.vy, s.vz):
+        v[:] = 0.0
+    s.vx[:3] = (s.x[48] - s.x[0] - 1.8) / (2.0 * s.tstep)
+    for c in (s.y, s.z):
+        c[:3] += c[48] - c[0]
+    return s
+
+
+def _closing_metal():
+    """Two atoms that come closer than their tables' first point in the second step."""
+    s = two_atoms(1.02)
+    s.eam = poly_tables()
+    s.vx[:] = (4.0, -4.0)
+    return s
+
+
+FAILURES = {
+    "rattle_nve": (_colliding_water, dict(shake_maxit=22), "nve", 515, 1),
+    "rattle_langevin": (_colliding_water, dict(shake_maxit=22), "langevin", 515, 1),
+    "metal_nve": (_closing_metal, {}, "nve", 506, 1),
+    "metal_nose_hoover": (_closing_metal, {}, "nose-hoover", 506, 1),
+}
+
+
+@pytest.mark.parametrize("graphs", ["0", "1"])
+@pytest.mark.parametrize("steps", ["last", "more"])
+@pytest.mark.parametrize("name", FAILURES)
+def test_failed_step_leaves_its_own_state(gpu_lib, monkeypatch, name, steps, graphs):
+    """A step that fails in its forces or in stage 2 leaves the state, the thermostat and the
+    step counter (which keys Langevin's noise) of that step, and reports the steps before it."""
+    make, over, ens, code, good = FAILURES[name]
+    n = good + 1 if steps == "last" else good + 4
+    out = []
+    for defer in ("0", "1"):
+        monkeypatch.setenv("GB_MD_DEFER", defer)
+        monkeypatch.setenv("GB_GRAPHS", graphs)
+        s = make()
+        gpu_lib.init(s, **over)
+        if ens != "nve":
+            gpu_lib.set_ensemble(ens, temp=300.0, tau_t=0.5, chi=0.01)
+        gpu_lib.start()
+        arr = (systems.GbStepStats * n)()
+        for x in arr:
+            x.engke = -1.0
+        assert gpu_lib.fn["md_run"](n, arr) == code
+        state = gpu_lib.download()
+        th = gpu_lib.thermostat_state()
+        again = {}
+        if ens == "langevin":
+            s = make()
+            for v in (s.vx, s.vy, s.vz):
+                v[:] = 0.0
+            gpu_lib.upload(s.x, s.y, s.z, s.vx, s.vy, s.vz)
+            gpu_lib.start()
+            gpu_lib.md_vv(1)
+            again = gpu_lib.download()
+        out.append((state, th, [x.engke for x in arr], again))
+    monkeypatch.delenv("GB_MD_DEFER")
+    monkeypatch.delenv("GB_GRAPHS")
+    (a, ta, ka, ga), (b, tb, kb, gb) = out
+    for k in a:
+        assert np.abs(a[k] - b[k]).max() <= 1e-12 * np.abs(a[k]).max(), k
+    for k in ta:
+        assert abs(ta[k] - tb[k]) <= 1e-12 * max(abs(ta[k]), 1e-30), k
+    assert [k == -1.0 for k in ka] == [k == -1.0 for k in kb] == [k >= good for k in range(n)]
+    for k in ga:
+        assert np.abs(ga[k] - gb[k]).max() <= 1e-12 * np.abs(ga[k]).max(), k
