@@ -596,7 +596,11 @@ GridSum gb_grid_sum(int nb, int nt, int nv, double* out_dev) {
   return {nb <= 20 * std::max(rows, 1) ? (g.side ? &g.sc->count_s : &g.sc->count) : nullptr, out_dev};
 }
 
-StopIf stop_if(int mask) { return {&g.sc->status, g.defer_scalars ? mask : 0}; }
+// (a mask of 0, and no load, for bits that this system's kernels never set)
+StopIf stop_if(int mask) {
+  const int can = (g.ntcons > 0 ? ST_RATTLE_FAIL : 0) | (g.has_metal ? ST_STOP2 : 0);
+  return {&g.sc->status, g.defer_scalars ? mask & can : 0};
+}
 
 void gb_grid_sum_done(const GridSum& gs, const double* blk, int nb, int nv) {
   if (!gs.count) gb_reduce_blocks(blk, nb, nv, gs.out);
