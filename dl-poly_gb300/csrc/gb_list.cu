@@ -226,12 +226,17 @@ __global__ void __launch_bounds__(HALO_NT) k_halo_write(HaloArgs A) {
   }
 }
 
+// The list's kernels do nothing after a halo overflow: the last list stays (the MD loop enqueues
+// them behind the halo without waiting for its status).
+__device__ __forceinline__ bool halo_cut(const DevScalars* sc) { return sc->status & ST_HALO_OVERFLOW; }
+
 // Exclusive scan of the cells' counts (block 0: all cells, into start; block 1: the domain's
 // cells, which hold the local atoms, into lstart) and the zeros that the list's kernels
 // count from.  A warp takes 1/32 of the cells, 32 at a time.
 __global__ void __launch_bounds__(1024) k_cell_scan(int n, CellGeom cg, const int* __restrict__ count, int* start,
                                                     int* lstart, DevScalars* sc) {
   __shared__ int s_w[32];
+  if (halo_cut(sc)) return;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
     sc->ibig = 0;
@@ -291,7 +296,7 @@ __global__ void k_bin(int natms, const DevScalars* sc, const double* x, const do
                       CellGeom cg, int* which_cell, int* count) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
   const int nlast = sc->nlast;
-  if (i >= nlast) return;
+  if (i >= nlast || halo_cut(sc)) return;
   const double xx = red_coord(cg.rc, 0, x[i]);
   const double yy = red_coord(cg.rc, 1, y[i]);
   const double zz = red_coord(cg.rc, 2, z[i]);
@@ -351,7 +356,7 @@ __global__ void k_bin(int natms, const DevScalars* sc, const double* x, const do
 __global__ void k_cell_scatter(const DevScalars* sc, const int* which_cell, const int* start, int* count,
                                int* tmp) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= sc->nlast) return;
+  if (i >= sc->nlast || halo_cut(sc)) return;
   int c = which_cell[i];
   int slot = atomicSub(&count[c], 1) - 1;
   tmp[start[c] + slot] = i;
@@ -372,6 +377,7 @@ __global__ void __launch_bounds__(SORT_NT) k_cell_sort(int ncells_p1, int natms,
                                                        const double* x, const double* y, const double* z,
                                                        double4_32a* xs, float4* xsf, TilePlan tp, CellGeom cg,
                                                        int* tile_rows, int* tile_info, int cap, DevScalars* sc) {
+  if (halo_cut(sc)) return;
   const int ncb = (ncells_p1 + SORT_NT / 32 - 1) / (SORT_NT / 32);
   if ((int)blockIdx.x >= ncb) {
     const int rb = blockIdx.x - ncb;
@@ -460,7 +466,7 @@ __global__ void __launch_bounds__(256) k_list_tiles(int natms, CellGeom cg, Tile
   __shared__ int s_first[TILE_MAX_ROWS], s_base[TILE_MAX_ROWS + 1];
   const int t = blockIdx.x;
   const int nst = tile_info[4 * t];
-  if (nst > cap) return;  // k_list_lanes then builds the list (uniform over the CTA)
+  if (nst > cap || halo_cut(sc)) return;  // k_list_lanes then builds the list (uniform over the CTA)
   const int nrows = tp.nrows;
   if (threadIdx.x < nrows) {
     s_first[threadIdx.x] = tile_rows[2 * (t * nrows + threadIdx.x)];
@@ -683,7 +689,7 @@ __global__ void __launch_bounds__(LANE_NT) k_list_lanes(int natms, CellGeom cg, 
   static_assert(STEP <= LANE_CAP / 2, "a step fits the column");
   __shared__ int2 s_buf[LANE_NT / 32][NA * LANE_LD];
   const int lane = threadIdx.x & 31, r = lane % G, w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  if (w * NA >= natms) return;
+  if (w * NA >= natms || halo_cut(sc)) return;
   int2* buf = s_buf[threadIdx.x >> 5];
   int2* const col = buf + (lane / G) * LANE_LD;
   const bool on = w * NA + lane / G < natms;
@@ -901,9 +907,9 @@ __device__ __forceinline__ int list_move_hits(int* li, int* ti, int n, Hit hit) 
 __global__ void __launch_bounds__(256) k_list_reorder(int natms, int* list, int ld, int* spos, int ldt,
                                                       const int* __restrict__ lfrzn, const int* __restrict__ ltg,
                                                       const int* __restrict__ list_excl, int ldx, int megfrz,
-                                                      int lbook) {
+                                                      int lbook, const DevScalars* sc) {
   const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (i >= natms) return;
+  if (i >= natms || halo_cut(sc)) return;
   int* li = list + (size_t)i * ld + 3;
   int* ti = spos + (size_t)i * ldt;
   const int n0 = li[0];
@@ -1251,18 +1257,18 @@ int list_build() {
     if (g.lbook || g.megfrz > 1) {  // (lists of tiles left out hold valid older entries, or none)
       k_list_reorder<<<nblocks((long long)n * 32, 256), 256, 0, st>>>(n, g.list, g.ld, g.spos, g.ldt, g.lfrzn, g.ltg,
                                                                       g.list_excl, g.p.max_exclude + 1, g.megfrz,
-                                                                      g.lbook ? 1 : 0);
+                                                                      g.lbook ? 1 : 0, g.sc);
       GB_LAUNCHED();
     }
     prof_end(P_LIST);
     gb_sync_scalars();  // (resolves the timings)
+    if (g.hsc->status & ST_HALO_OVERFLOW) return GB_ERR_HALO;  // (list_relocate_and_halo without its wait)
     if (!tiles || g.hsc->tile_over == 0) break;
     g.n_tile_over = g.hsc->tile_over;  // denser tiles than planned: this list and the later ones from the other kernel
     tiles = false;
     GB_CUDA(cudaMemsetAsync(&g.sc->ibig, 0, sizeof(int), st));
     GB_CUDA(cudaMemsetAsync(&g.sc->halo_fwd, 0, 2 * sizeof(int), st));  // halo_fwd, halo_bwd
   }
-  if (g.hsc->status & ST_HALO_OVERFLOW) return GB_ERR_HALO;  // (list_relocate_and_halo without its wait)
   if (g.hsc->status & ST_LIST_OVERFLOW) return GB_ERR_LIST_OVERFLOW;
   // every pair across the periodic boundary is listed from both of its atoms, once in a
   // forward pass and once in the backward halo pass; the sorted-position pair kernels

@@ -64,6 +64,24 @@ def test_tiles_above_their_capacity(gpu_lib, oracle_lib, monkeypatch):
     monkeypatch.delenv("GB_TILE_CAP")
 
 
+def test_halo_overflow_in_a_run_keeps_the_last_list(gpu_lib):
+    """A cluster of ions flying out of the middle of its box: in the second step its images
+    exceed mxatms, which ends the run with 56 before the list is built again."""
+    s = systems.nacl_melt(8)
+    s.cell = np.array([60.0, 0, 0, 0, 60.0, 0, 0, 0, 60.0])
+    s.kmax = (64, 64, 64)
+    s.vx[:] = 3000.0
+    s.vy[:] = s.vz[:] = 0.0
+    found = []  # the candidates that the builds since gb_init decided in FP64
+    for steps in (1, 4):
+        gpu_lib.init(s, max_list=512, mxatms=s.natms + 100)
+        gpu_lib.start()
+        st = gpu_lib.fn["md_run"](steps, (systems.GbStepStats * steps)())
+        assert st == (0 if steps == 1 else 56)
+        found.append(gpu_lib.pair_counts()[2])
+    assert found[0] > 0 and found[1] == found[0]
+
+
 def test_phase_timings_of_a_rebuild(gpu_lib):
     """Every phase's event pair is complete when the build's wait resolves the timings."""
     gpu_lib.init(systems.nacl_melt(16))
