@@ -941,6 +941,10 @@ ClKind* d_kinds = nullptr;
 float2* d_clt = nullptr;     // polynomials and scalars, when there are more clusters than resident lanes
 bool cl_small = false;
 int coop_blocks_small = 0, cs_threads = 32;
+const void* cl_kernel = nullptr;  // k_constrain_cl instantiation for the largest cluster
+
+// The form by FP64 instructions keeps k_constrain_cl: it is there to check the others.
+bool use_small() { return cl_small && !g.fp64_native; }
 
 // connected constraint clusters; false when one exceeds CL_MAXA atoms or CL_MAXC constraints
 bool build_clusters(const std::vector<int>& ci, const std::vector<int>& cj, std::vector<ClusterTab>& out) {
@@ -1136,12 +1140,17 @@ void integ_setup_constraints(const int32_t* listcon, const double* prmcon) {
       GB_CUDA(cudaFuncSetAttribute(k_constrain_small<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
       if (coop_blocks_small * (cs_threads / 32) < nwarp)
         GB_CUDA(cudaMalloc(&d_clt, sizeof(float2) * (CS_POLY + 2) * CS_MAXC * tabs.size()));
-    } else {
-      GB_CUDA(cudaMalloc(&d_clring, sizeof(double) * CL_RING * CL_SLOT * tabs.size()));
-      GB_CUDA(cudaMalloc(&d_clgsum, sizeof(double) * CL_MAXC * tabs.size()));
-      GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, k_constrain_cl<CL_MAXA, CL_MAXC>, CL_THREADS, 0));
-      coop_blocks_cl = std::max(1, std::min(bps * g.nsm, nblocks(n_clusters, CL_THREADS)));
     }
+    // and k_constrain_cl, for the other clusters and the FP64 form by instructions
+    GB_CUDA(cudaMalloc(&d_clring, sizeof(double) * CL_RING * CL_SLOT * tabs.size()));
+    GB_CUDA(cudaMalloc(&d_clgsum, sizeof(double) * CL_MAXC * tabs.size()));
+    // rigid 3-site molecules get register arrays sized 3 x 3 (more resident warps)
+    bool three = true;
+    for (const ClusterTab& T : tabs)
+      if ((T.meta & 15) > 3 || ((T.meta >> 4) & 15) > 3) three = false;
+    cl_kernel = three ? (const void*)k_constrain_cl<3, 3> : (const void*)k_constrain_cl<CL_MAXA, CL_MAXC>;
+    GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, cl_kernel, CL_THREADS, 0));
+    coop_blocks_cl = std::max(1, std::min(bps * g.nsm, nblocks(n_clusters, CL_THREADS)));
   }
 }
 
@@ -1220,20 +1229,21 @@ void integ_shake(int* iters, double* vircon, double* strcon) {
   if (iters) *iters = 0;
   if (g.ntcons <= 0) return;
   cudaStream_t st = g.stream;
+  const bool small = use_small();
   const int n = g.natms;
   const double tstep = g.p.tstep, hstep = 0.5 * tstep, rstep = 1.0 / tstep;
-  if (!cl_small) {
+  if (!small) {
     k_copy3<<<nblocks(n, 256), 256, 0, st>>>(n, g.x, g.y, g.z, g.ox, g.oy, g.oz);
     GB_LAUNCHED();
   }
   GB_CUDA(cudaMemsetAsync(d_flags, 0, sizeof(int) * (g.p.shake_maxit + CL_CHUNK + 2), st));
   ConArgs A;
   con_args(A, ST_STOP1);
-  const int nbs = cl_small ? coop_blocks_small : n_clusters ? coop_blocks_cl : coop_blocks_shake;
+  const int nbs = small ? coop_blocks_small : n_clusters ? coop_blocks_cl : coop_blocks_shake;
   A.blk = gb_blkacc(nbs * 6);
-  if (cl_small) A.gs = gb_grid_sum(nbs, cs_threads, 6, &g.sc->acc[A_STRCON]);
+  if (small) A.gs = gb_grid_sum(nbs, cs_threads, 6, &g.sc->acc[A_STRCON]);
   prof_begin(P_SHAKE);
-  if (cl_small) {
+  if (small) {
     launch_small<false>(A, rstep);
   } else if (n_clusters) {
     const ClusterTab* tabs = d_cltab;
@@ -1241,7 +1251,7 @@ void integ_shake(int* iters, double* vircon, double* strcon) {
     double *ring = d_clring, *gsum = d_clgsum;
     GB_CUDA(cudaMemsetAsync(d_clgsum, 0, sizeof(double) * CL_MAXC * n_clusters, st));
     void* args[] = {&A, &tabs, &ncl, &ring, &gsum, &rattle};
-    GB_CUDA(cudaLaunchCooperativeKernel((void*)k_constrain_cl<CL_MAXA, CL_MAXC>, nbs, CL_THREADS, args, 0, st));
+    GB_CUDA(cudaLaunchCooperativeKernel(cl_kernel, nbs, CL_THREADS, args, 0, st));
   } else {
     void* args[] = {&A};
     GB_CUDA(cudaLaunchCooperativeKernel((void*)k_shake, nbs, 256, args, 0, st));
@@ -1249,7 +1259,7 @@ void integ_shake(int* iters, double* vircon, double* strcon) {
   GB_LAUNCHED();
   prof_end(P_SHAKE);
   if (!A.gs.count) gb_reduce_blocks(A.blk, nbs, 6, &g.sc->acc[A_STRCON]);
-  if (!cl_small) {
+  if (!small) {
     k_shake_post<<<nblocks(n, 256), 256, 0, st>>>(n, g.acon_start, g.lfrzn, rstep, hstep, g.weight, g.x, g.y, g.z,
                                                    g.ox, g.oy, g.oz, g.vx, g.vy, g.vz, g.fx, g.fy, g.fz,
                                                    stop_if(ST_STOP1));
@@ -1269,20 +1279,21 @@ void integ_shake(int* iters, double* vircon, double* strcon) {
 void integ_rattle_launch(bool tags) {
   if (g.ntcons <= 0) return;
   cudaStream_t st = g.stream;
+  const bool small = use_small();
   GB_CUDA(cudaMemsetAsync(d_flags, 0, sizeof(int) * (g.p.shake_maxit + CL_CHUNK + 2), st));
   ConArgs A;
   con_args(A, ST_STOP2);
-  if (tags && !cl_small) integ_con_tags();
+  if (tags && !small) integ_con_tags();
   A.tags = tags;
   prof_begin(P_RATTLE);
-  if (cl_small) {
+  if (small) {
     launch_small<true>(A, 0.0);
   } else if (n_clusters) {
     const ClusterTab* tabs = d_cltab;
     int ncl = n_clusters, rattle = 1;
     double *ring = d_clring, *gsum = d_clgsum;
     void* args[] = {&A, &tabs, &ncl, &ring, &gsum, &rattle};
-    GB_CUDA(cudaLaunchCooperativeKernel((void*)k_constrain_cl<CL_MAXA, CL_MAXC>, coop_blocks_cl, CL_THREADS, args, 0, st));
+    GB_CUDA(cudaLaunchCooperativeKernel(cl_kernel, coop_blocks_cl, CL_THREADS, args, 0, st));
   } else {
     void* args[] = {&A};
     GB_CUDA(cudaLaunchCooperativeKernel((void*)k_rattle, coop_blocks_rattle, 256, args, 0, st));

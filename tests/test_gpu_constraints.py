@@ -1,5 +1,7 @@
 """SHAKE/RATTLE on clusters of every kind that the scalar-form kernel takes (one, two and
 three constraints, frozen atoms), on clusters beyond it, and on more clusters than threads."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -64,3 +66,29 @@ def test_more_clusters_than_threads(gpu_lib, monkeypatch):
     assert (sg[0].shake_iters, sg[0].rattle_iters) == (sc[0].shake_iters, sc[0].rattle_iters)
     for k in ("x", "y", "z", "vx", "vy", "vz"):
         assert np.abs(a[k] - b[k]).max() <= REL * np.abs(a[k]).max(), k
+
+
+def test_native_form_by_fp64_instructions(gpu_lib, oracle_lib, monkeypatch):
+    """The form that checks the others runs the FP64 cluster kernel: its SHAKE takes the launches of
+    the per-sweep FP64 kernels (the scalar-form kernel is a single one), also when it is chosen after gb_init."""
+    s = systems.spce_water(8)
+    n = {}
+    launches = gpu_lib._opt("kernel_launches", ctypes.c_int64, [])
+    prec = gpu_lib._opt("set_precision", ctypes.c_int, [ctypes.c_int])
+    for name, glob, at_init, then in (("fp64", "0", 0, 0), ("native", "0", 2, 2), ("later", "0", 0, 2),
+                                      ("global", "1", 2, 2)):
+        monkeypatch.setenv("GB_SHAKE_GLOBAL", glob)
+        gpu_lib.init(s, precision=at_init)
+        assert prec(then) == 0
+        gpu_lib.start()
+        k = launches()
+        gpu_lib.constraints_tags()
+        gpu_lib.apply_shake()
+        n[name] = launches() - k
+        if name in ("native", "later"):
+            oracle_lib.init(s)
+            oracle_lib.start()
+            (x,), (y,) = gpu_lib.md_vv(1), oracle_lib.md_vv(1)
+            assert (x.shake_iters, x.rattle_iters) == (y.shake_iters, y.rattle_iters)
+    monkeypatch.delenv("GB_SHAKE_GLOBAL")
+    assert n["native"] == n["later"] == n["global"] > n["fp64"]
