@@ -571,15 +571,17 @@ __global__ void __launch_bounds__(128) k_constrain_cl(ConArgs A, const ClusterTa
 // scalar by shuffles: a sweep is a chain of dependent operations, which one lane per
 // cluster ran at two warps a scheduler (0.133 and 0.090 ms).  q_c is evaluated as c0 +
 // sum_i t_i (l_i + sum_j q_ij t_j); the inner sums run over an added constant
-// (off_add_prod), and the scalars of a chunk's sweeps are kept in shared memory, so that
-// none is repeated.  It takes 0.090 ms (SHAKE) and 0.053 ms (RATTLE, which forms the bond
+// (off_add_prod; it grows with the cluster's bonds where they start far from their lengths:
+// sums that reach it lose their last bits, and SHAKE of molecules three times too large did
+// not converge), and the scalars of a chunk's sweeps are kept in shared memory, so that none is
+// repeated.  It takes 0.090 ms (SHAKE) and 0.053 ms (RATTLE, which forms the bond
 // vectors too) for 32,768 waters, 0.047 and 0.027 ms for 2,197: the operations of a sweep in
 // order, the FP64 set-up and epilogue, and five grid barriers.
 // Sweeps run in chunks of CS_CHUNK between grid barriers (20 steps of 2,197 molecules:
 // 8.6 ms with chunks of 8, 8.3 with 16 and with 31, which doubles the shared memory).
 constexpr int CS_CHUNK = 16, CS_MAXC = 3, CS_PERWARP = 10;
 constexpr int CS_THREADS = 704;  // one block per SM: 22 warps of at most 88 registers
-constexpr int CS_POLY = 14;      // float2 of the polynomials of a lane
+constexpr int CS_POLY = 15;      // float2 of the polynomials of a lane
 
 struct ClKind {        // clusters with equal masses, lengths and topology share one
   int na, nc;
@@ -587,7 +589,7 @@ struct ClKind {        // clusters with equal masses, lengths and topology share
   float2 K[CS_MAXC][CS_MAXC];           // double-float
   float2 tol_s[CS_MAXC], tol_r;         // bounds on |q| (2 tol d0) and |g| (2 tol / tstep)
   float2 two_m[CS_MAXC];                // gamma sum = two_m * t (SHAKE), double-float
-  float off;                            // 8 max(d0^2) rounded up to a power of two: exceeds |l| and its sums
+  float off;                            // 8 max(d0^2) rounded up to a power of two
   double W[CL_MAXA][CS_MAXC];
   double d0sq[CS_MAXC];
   double wh[CL_MAXA];                   // weight / hstep, 0: frozen
@@ -617,7 +619,8 @@ __device__ __forceinline__ df df_shfl(df a, int lane) {
 // The polynomials of a lane's constraint; index r is the constraint of the cluster r places
 // after its own, cyclically; q in the order 00, 01, 02, 11, 12, 22.
 struct ClPoly {
-  df c0, l[CS_MAXC];  // l over the constant off (SHAKE)
+  float off;          // a power of two, at least 8/3 of the |l| (SHAKE)
+  df c0, l[CS_MAXC];  // l over the constant off
   df q[6];
   df p0, p[CS_MAXC];
 };
@@ -672,23 +675,30 @@ __device__ __forceinline__ void cs_setup(const ConArgs& A, const ClusterTab& T, 
   B[5] = df_shfl(B[0], n2);
   if (!on) K[0] = K[1] = K[2] = df_make(0.f, 0.f);
 #pragma unroll
-  for (int k = 0; k < CS_MAXC; ++k) {
-    P.p[k] = df_mul(K[k], B[k]);
-    if (RATTLE) continue;
-    const df w = df_mul(K[k], df_dot(u, b[k]));
-    const df s = two_sum(D.off, 2.f * w.hi);
-    P.l[k] = df_make(s.hi, s.lo + 2.f * w.lo);
-  }
+  for (int k = 0; k < CS_MAXC; ++k) P.p[k] = df_mul(K[k], B[k]);
   if (!RATTLE) {
+    float m = 0.f;  // the largest |l|
+#pragma unroll
+    for (int k = 0; k < CS_MAXC; ++k) {
+      P.l[k] = df_mul(K[k], df_dot(u, b[k]));
+      m = fmaxf(m, 2.f * fabsf(P.l[k].hi));
+    }
+    P.off = D.off;
+    if (m > 0.375f * P.off) P.off = __uint_as_float(min((__float_as_uint(m) >> 23) + 4u, 254u) << 23);
+#pragma unroll
+    for (int k = 0; k < CS_MAXC; ++k) {
+      const df s = two_sum(P.off, 2.f * P.l[k].hi);
+      P.l[k] = df_make(s.hi, s.lo + 2.f * P.l[k].lo);
+    }
     P.p0 = on ? df_dot(u, b[0]) : df_make(1.f, 0.f);
-    int m = 0;
+    int i = 0;
 #pragma unroll
     for (int k = 0; k < CS_MAXC; ++k)
 #pragma unroll
-      for (int n = k; n < CS_MAXC; ++n, ++m) {
-        const df e = df_mul(df_mul(K[k], K[n]), B[m]);
+      for (int n = k; n < CS_MAXC; ++n, ++i) {
+        const df e = df_mul(df_mul(K[k], K[n]), B[i]);
         const float f = n == k ? 1.f : 2.f;
-        P.q[m] = df_make(f * e.hi, f * e.lo);
+        P.q[i] = df_make(f * e.hi, f * e.lo);
       }
   }
 }
@@ -696,7 +706,7 @@ __device__ __forceinline__ void cs_setup(const ConArgs& A, const ClusterTab& T, 
 // one sweep from the scalars t (own first): true when the constraint fails its test; the new
 // scalars in t
 template <bool RATTLE>
-__device__ __forceinline__ bool cs_sweep(const ClPoly& P, float off, float2 tol, int n1, int n2, df (&t)[CS_MAXC]) {
+__device__ __forceinline__ bool cs_sweep(const ClPoly& P, float2 tol, int n1, int n2, df (&t)[CS_MAXC]) {
   dacc a = {P.c0.hi, P.c0.lo};
   df step;
   bool fail;
@@ -718,7 +728,7 @@ __device__ __forceinline__ bool cs_sweep(const ClPoly& P, float off, float2 tol,
       dacc v = {P.l[i].hi, P.l[i].lo};
 #pragma unroll
       for (int j = i; j < CS_MAXC; ++j, ++m) off_add_prod(v, P.q[m], t[j]);
-      dacc_add_prod(a, df_make(__fsub_rn(v.s, off), v.c), t[i]);
+      dacc_add_prod(a, df_make(__fsub_rn(v.s, P.off), v.c), t[i]);
     }
     const df q = quick_two_sum(a.s, a.c);
     fail = !df_abs_less(q, tol);
@@ -749,6 +759,9 @@ __device__ __forceinline__ void cs_poly_io(float2* __restrict__ pbuf, size_t ld,
 #pragma unroll
   for (int k = 0; k < 6; ++k) io(7 + k, P.q[k]);
   io(13, P.p0);
+  df off = df_make(P.off, 0.f);
+  io(14, off);
+  P.off = off.hi;
 }
 
 // SHAKE with its epilogue (apply_shake: v += dr/dt, f += dr/dt m/(dt/2)) or RATTLE.  pbuf: when
@@ -797,12 +810,11 @@ __global__ void __launch_bounds__(CS_THREADS) k_constrain_small(ConArgs A, const
         t[2] = df_shfl(t[0], n2);
       }
       if (multi && in) pb[CS_POLY * ld] = make_float2(t[0].hi, t[0].lo);
-      const float off = D.off;
       const float2 tol = RATTLE ? D.tol_r : D.tol_s[c];
       unsigned b = 0;
       for (int s = 0; s < n; ++s) {
         cs_hist[s * blockDim.x + threadIdx.x] = make_float2(t[0].hi, t[0].lo);
-        if (cs_sweep<RATTLE>(P, off, tol, n1, n2, t)) b |= 1u << s;
+        if (cs_sweep<RATTLE>(P, tol, n1, n2, t)) b |= 1u << s;
       }
       if (on) bad |= b;
       if (multi && in) pb[(CS_POLY + 1) * ld] = make_float2(t[0].hi, t[0].lo);
@@ -840,7 +852,7 @@ __global__ void __launch_bounds__(CS_THREADS) k_constrain_small(ConArgs A, const
       t[1] = df_shfl(t[0], n1);
       t[2] = df_shfl(t[0], n2);
       const float2 tol = RATTLE ? D.tol_r : D.tol_s[c];
-      for (int s = 0; s < last; ++s) cs_sweep<RATTLE>(P, D.off, tol, n1, n2, t);
+      for (int s = 0; s < last; ++s) cs_sweep<RATTLE>(P, tol, n1, n2, t);
     } else if (done) {
       t[0] = df_of(cs_hist[last * blockDim.x + threadIdx.x]);
     }

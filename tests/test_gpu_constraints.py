@@ -92,3 +92,31 @@ def test_native_form_by_fp64_instructions(gpu_lib, oracle_lib, monkeypatch):
             assert (x.shake_iters, x.rattle_iters) == (y.shake_iters, y.rattle_iters)
     monkeypatch.delenv("GB_SHAKE_GLOBAL")
     assert n["native"] == n["later"] == n["global"] > n["fp64"]
+
+
+@pytest.mark.parametrize("factor", [1.2, 2.0, 3.0, 4.0, 6.0])
+def test_shake_of_stretched_molecules(gpu_lib, factor):
+    """Molecules whose bonds start far from their lengths: every constraint ends within its
+    tolerance, after the sweeps and with the stress of the FP64 cluster kernel."""
+    out = []
+    for precision in (0, 2):
+        s = systems.spce_water(6, box=19.7, rcut=7.0, kmax=32)
+        s.shake_tol = 1e-9
+        for v in (s.x, s.y, s.z):
+            o = np.repeat(v[0::3], 3)
+            v[:] = o + factor * (v - o)
+        gpu_lib.init(s, precision=precision)
+        gpu_lib.constraints_tags()
+        r = gpu_lib.apply_shake()
+        d = gpu_lib.download()
+        lc = s.listcon.reshape(-1, 3)
+        pos = np.stack([d[k] for k in "xyz"], 1)
+        b = pos[lc[:, 1] - 1] - pos[lc[:, 2] - 1]
+        d0 = s.prmcon[lc[:, 0] - 1]
+        # |b^2 - d0^2| / 2 < tol d0, and the rounding of coordinates below 32 A (2^-48 A each)
+        assert (np.abs((b ** 2).sum(1) - d0 ** 2) / (2.0 * d0)).max() < s.shake_tol + 1e-13 * factor
+        out.append((r["iters"], r["strcon"], pos))
+    (ia, sa, pa), (ib, sb, pb) = out
+    assert ia == ib
+    assert np.abs(sa - sb).max() <= 1e-9 * np.abs(sb).max()
+    assert np.abs(pa - pb).max() <= 1e-9
