@@ -588,10 +588,10 @@ struct ClKind {        // clusters with equal masses, lengths and topology share
   int li[CS_MAXC], lj[CS_MAXC];         // local ends of the constraints
   float2 K[CS_MAXC][CS_MAXC];           // double-float
   float2 tol_s[CS_MAXC], tol_r;         // bounds on |q| (2 tol d0) and |g| (2 tol / tstep)
-  float2 two_m[CS_MAXC];                // gamma sum = two_m * t (SHAKE), double-float
   float off;                            // 8 max(d0^2) rounded up to a power of two
   double W[CL_MAXA][CS_MAXC];
   double d0sq[CS_MAXC];
+  double two_m[CS_MAXC];                // gamma sum = two_m * t (SHAKE)
   double wh[CL_MAXA];                   // weight / hstep, 0: frozen
 };
 
@@ -836,9 +836,7 @@ __global__ void __launch_bounds__(CS_THREADS) k_constrain_small(ConArgs A, const
     (RATTLE ? A.sc->rattle_iters : A.sc->shake_iters) = nfinal > 0 ? nfinal : A.maxit;
     if (nfinal < 0) A.sc->status |= RATTLE ? ST_RATTLE_FAIL : ST_SHAKE_FAIL;
   }
-  df st[6];
-#pragma unroll
-  for (int k = 0; k < 6; ++k) st[k] = df_make(0.f, 0.f);
+  double st[6] = {0, 0, 0, 0, 0, 0};
   for (int cl0 = warp * CS_PERWARP; cl0 < ncl; cl0 += wstep) {
     const bool in = lane < 3 * CS_PERWARP && cl0 + sub < ncl;
     const int cl = in ? cl0 + sub : cl0;
@@ -867,17 +865,13 @@ __global__ void __launch_bounds__(CS_THREADS) k_constrain_small(ConArgs A, const
         r = r * fma(-0.5 * b2 * r, r, 1.5);
         tt *= r;  // unit bond vectors
       } else {
-        const df g = df_mul(df_of(D.two_m[c]), t[0]);
-        const df bd[3] = {dbl_split(b[0]), dbl_split(b[1]), dbl_split(b[2])};
+        const double g = D.two_m[c] * tt;
         int m = 0;
 #pragma unroll
         for (int p = 0; p < 3; ++p) {
-          const df gb = df_mul(g, bd[p]);
+          const double gb = -g * b[p];
 #pragma unroll
-          for (int q = p; q < 3; ++q, ++m) {
-            const df e = df_mul(gb, bd[q]);
-            st[m] = df_add(st[m], df_make(-e.hi, -e.lo));
-          }
+          for (int q = p; q < 3; ++q, ++m) st[m] = fma(gb, b[q], st[m]);
         }
       }
 #pragma unroll
@@ -912,10 +906,7 @@ __global__ void __launch_bounds__(CS_THREADS) k_constrain_small(ConArgs A, const
     }
   }
   if (!RATTLE) {
-    dfr sd[6];
-#pragma unroll
-    for (int k = 0; k < 6; ++k) sd[k] = to_dfr(st[k]);
-    block_reduce_store<6>(sd, A.blk);
+    block_reduce_store<6>(st, A.blk);
     grid_finish<6>(A.blk, A.gs);
   }
 }
@@ -1055,7 +1046,7 @@ bool build_kinds(const std::vector<ClusterTab>& tabs, const std::vector<double>&
       W[D.li[c]][c] -= iw[D.li[c]] / m;
       W[D.lj[c]][c] += iw[D.lj[c]] / m;
       D.d0sq[c] = len * len;
-      D.two_m[c] = split(2.0 / (m * dt * dt));
+      D.two_m[c] = 2.0 / (m * dt * dt);
       D.off = std::max(D.off, std::ldexp(1.f, std::ilogb(len * len) + 4));
       D.tol_s[c] = split(2.0 * (tol * len));
     }
