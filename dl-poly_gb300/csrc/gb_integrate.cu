@@ -580,7 +580,11 @@ __global__ void __launch_bounds__(128) k_constrain_cl(ConArgs A, const ClusterTa
 // Sweeps run in chunks of CS_CHUNK between grid barriers (20 steps of 2,197 molecules:
 // 8.6 ms with chunks of 8, 8.3 with 16 and with 31, which doubles the shared memory).
 constexpr int CS_CHUNK = 16, CS_MAXC = 3, CS_PERWARP = 10;
-constexpr int CS_THREADS = 704;  // one block per SM: 22 warps of at most 88 registers
+// One block per SM, of as many warps as the clusters need, up to the most whose registers (80 a
+// thread in SHAKE) it holds with the same number for each scheduler: 24, or 240 clusters a SM.  More
+// clusters than that keep their polynomials in memory between chunks and repeat the last
+// one (152 SMs, SHAKE and RATTLE: 35,937 clusters 0.094 and 0.061 ms, 39,304 0.172 and 0.101).
+constexpr int CS_THREADS = 768;
 constexpr int CS_POLY = 15;      // float2 of the polynomials of a lane
 
 struct ClKind {        // clusters with equal masses, lengths and topology share one
