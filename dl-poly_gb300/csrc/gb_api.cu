@@ -734,11 +734,7 @@ int gb_init(const gb_params* prm, int natms, const int32_t* ltype, const double*
     pair_setup();
     g.scaling = kR4pie0 / prm->epsq;
     double sq2 = 0.0;
-    g.qmax = 0.0;
-    for (int i = 0; i < natms; ++i) {
-      sq2 += chge[i] * chge[i];
-      g.qmax = std::max(g.qmax, std::fabs(chge[i]));
-    }
+    for (int i = 0; i < natms; ++i) sq2 += chge[i] * chge[i];
     g.self_interaction = -sq2 * (g.scaling * prm->alpha * (1.0 / 1.7724538509055161040) / 1.0);  // spme.F90:159-231
     g.ntcons = ntcons;
     if (ntcons > 0) integ_setup_constraints(listcon, prmcon);

@@ -234,7 +234,6 @@ struct Dev {
   std::vector<int> h_vdw_kind;
   std::vector<double> h_vdw_eps, h_vdw_sig;
   double elrc = 0, vlrc = 0, self_interaction = 0, scaling = 0;
-  double qmax = 0;               // largest |charge|
 
   // SPME grids live in gb_spme.cu (SpmeGrid); shared scratch here
   double* blkacc = nullptr;    // per-block partial accumulators

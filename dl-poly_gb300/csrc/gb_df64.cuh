@@ -192,14 +192,12 @@ __device__ __forceinline__ df fix_diff_full(long long a, long long b, float sh, 
 // sum and every product: |a.s| >= |x y|, so that t - a.s is exact and the second FMA gives
 // the rounding error of the first (Dekker's fast two-sum with the product unrounded).  Six
 // FP32 operations instead of dacc_add_prod's twelve; the sum's error is relative to C
-// (about 2^-48 C per term).  Start with (C, 0) and take the sum with off_value.
+// (about 2^-48 C per term).  Start with (C, 0).
 __device__ __forceinline__ void off_add_prod(dacc& a, df x, df y) {
   const float t = __fmaf_rn(x.hi, y.hi, a.s);
   const float r = __fmaf_rn(x.hi, y.hi, -__fsub_rn(t, a.s));
   a.c = __fmaf_rn(x.hi, y.lo, __fmaf_rn(x.lo, y.hi, __fadd_rn(a.c, r)));
   a.s = t;
 }
-
-__device__ __forceinline__ df off_value(const dacc& a, float c) { return two_sum(__fsub_rn(a.s, c), a.c); }
 
 #endif

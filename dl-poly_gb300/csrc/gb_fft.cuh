@@ -39,7 +39,7 @@ struct SpmeGeom {
 template <typename T, typename T2>
 struct FftKernels {
   void (*x_fwd)(const T*, T2*, FftPlan, const T2*, const T2*, int, int);
-  void (*x_inv)(const T2*, T*, FftPlan, const T2*, const T2*, int, int, unsigned*);
+  void (*x_inv)(const T2*, T*, FftPlan, const T2*, const T2*, int, int);
   void (*y_fwd)(T2*, int, int, FftPlan, const T2*);
   void (*y_inv)(T2*, int, int, FftPlan, const T2*);
   void (*z_conv)(T2*, int, int, int, FftPlan, const T2*, const T*, const T*, SpmeGeom, double*, GridSum);
@@ -328,7 +328,7 @@ __global__ void k_fft_x_fwd(const T* __restrict__ Q, T2* __restrict__ G, FftPlan
 
 template <typename T, typename T2, int NC>
 __global__ void k_fft_x_inv(const T2* __restrict__ G, T* __restrict__ Q, FftPlan pl, const T2* __restrict__ tw,
-                            const T2* __restrict__ twN, int nrows, int lines, unsigned* vmax) {
+                            const T2* __restrict__ twN, int nrows, int lines) {
   extern __shared__ unsigned char smem_raw[];
   const int M = NC ? NC : pl.N, Kx = M + 1, LD = fft_turns<T2>() ? fft_ld<T2>(M) : M;
   T2* a = reinterpret_cast<T2*>(smem_raw);
@@ -350,17 +350,8 @@ __global__ void k_fft_x_inv(const T2* __restrict__ G, T* __restrict__ Q, FftPlan
   }
   T2* r = fft_run<T, T2, -1, NC, XLINES>(a, b, pl, nl, tw);
   T2* Qc = reinterpret_cast<T2*>(Q);
-  unsigned m = 0;  // the bits of the largest |potential| of the grid, for the double-float gather
-  for (int e = threadIdx.x; e < nl * M; e += blockDim.x) {
-    const T2 v = r[fft_turns<T2>() ? e + (e / M) * (LD - M) : e];
-    Qc[row0 * M + e] = v;
-    if constexpr (std::is_same<T, dfr>::value)
-      m = max(m, max(__float_as_uint(v.x.hi) & 0x7fffffffu, __float_as_uint(v.y.hi) & 0x7fffffffu));
-  }
-  if constexpr (std::is_same<T, dfr>::value) {
-    m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0 && m > *reinterpret_cast<volatile unsigned*>(vmax)) atomicMax(vmax, m);
-  }
+  for (int e = threadIdx.x; e < nl * M; e += blockDim.x)
+    Qc[row0 * M + e] = r[fft_turns<T2>() ? e + (e / M) * (LD - M) : e];
 }
 
 // Y pass (stride Kx): tile of TX columns x N lines, in place

@@ -723,14 +723,8 @@ template <int P>
 __global__ void __launch_bounds__(256, 6) k_spme_gather_wdf(int natms, int ab, SpmeGeom sg, const int* __restrict__ gidx,
                                                          const dfr* __restrict__ gsp,
                                                          const float2* __restrict__ gq, const dfr* __restrict__ phi,
-                                                         float2 rk0, float2 rk1, float2 rk2, float qmax,
-                                                         const unsigned* __restrict__ vmax,
+                                                         float2 rk0, float2 rk1, float2 rk2,
                                                          float2* __restrict__ fout, double* blk, GridSum gs) {
-  // C of off_add_prod: a power of two, at least twice the largest |charge x potential|, which
-  // bounds every sum over a stencil (the spline values of a dimension are positive and add
-  // up to 1, the derivatives' magnitudes to about 1)
-  const float C = __uint_as_float(
-      min((__float_as_uint(__fmul_rn(__uint_as_float(*vmax), qmax)) >> 23) + 2u, 254u) << 23);
   constexpr int NS = 6 * P;  // spline components per atom: [value, derivative][x, y, z][point]
   static_assert(GATHER_AB == 8, "8 atoms per batch");
   __shared__ __align__(16) dfr sp[8][NS][GATHER_AB];  // per warp: component, atom
@@ -776,22 +770,21 @@ __global__ void __launch_bounds__(256, 6) k_spme_gather_wdf(int natms, int ab, S
         const dfr* c0 = phi + (y0 * K0 + xx);
         const dfr* c1 = phi + (y1 * K0 + xx);
         dacc a0, b0, a1, b1;
-        a0.s = b0.s = a1.s = b1.s = C;
-        a0.c = b0.c = a1.c = b1.c = 0.f;
+        a0.s = a0.c = b0.s = b0.c = a1.s = a1.c = b1.s = b1.c = 0.f;
 #pragma unroll
         for (int l = 0; l < P; ++l) {
           const df mz = spv(0, 2, l), dmz = spv(1, 2, l);
           const df p0 = ld_df(c0 + zo[l]), p1 = ld_df(c1 + zo[l]);
-          off_add_prod(a0, mz, p0);
-          off_add_prod(b0, dmz, p0);
-          off_add_prod(a1, mz, p1);
-          off_add_prod(b1, dmz, p1);
+          dacc_add_prod(a0, mz, p0);
+          dacc_add_prod(b0, dmz, p0);
+          dacc_add_prod(a1, mz, p1);
+          dacc_add_prod(b1, dmz, p1);
         }
         // y: My and dMy against the two columns' sums
         const df my0 = spv(0, 1, k), dmy0 = spv(1, 1, k);
         const df my1 = spv(0, 1, k + 4), dmy1 = spv(1, 1, k + 4);
-        const df ca0 = off_value(a0, C), cc0 = off_value(b0, C);
-        const df ca1 = off_value(a1, C), cc1 = off_value(b1, C);
+        const df ca0 = df_make(a0.s, a0.c), cc0 = df_make(b0.s, b0.c);
+        const df ca1 = df_make(a1.s, a1.c), cc1 = df_make(b1.s, b1.c);
         dacc A = dacc_prod(my0, ca0), B = dacc_prod(dmy0, ca0), C = dacc_prod(my0, cc0);
         dacc_add_prod(A, my1, ca1);
         dacc_add_prod(B, dmy1, ca1);
@@ -813,15 +806,14 @@ __global__ void __launch_bounds__(256, 6) k_spme_gather_wdf(int natms, int ab, S
           int yy = gy + k; if (yy >= K1) yy -= K1;
           const dfr* col = phi + (yy * K0 + xx);
           dacc za, zc;
-          za.s = zc.s = C;
-          za.c = zc.c = 0.f;
+          za.s = za.c = zc.s = zc.c = 0.f;
 #pragma unroll
           for (int l = 0; l < P; ++l) {
             const df ph = ld_df(col + zo[l]);
-            off_add_prod(za, spv(0, 2, l), ph);
-            off_add_prod(zc, spv(1, 2, l), ph);
+            dacc_add_prod(za, spv(0, 2, l), ph);
+            dacc_add_prod(zc, spv(1, 2, l), ph);
           }
-          const df ca = off_value(za, C), cc = off_value(zc, C);
+          const df ca = df_make(za.s, za.c), cc = df_make(zc.s, zc.c);
           const df mx = spv(0, 0, j), dmx = spv(1, 0, j);
           const df my = spv(0, 1, k), dmy = spv(1, 1, k);
           const df w0 = df_mul(mx, my);
@@ -966,7 +958,6 @@ struct SpmeGrid {
   double2* twh = nullptr;        // its twiddles e^{+2 pi i t/(K1/2)}
   float2* twhf = nullptr;
   int Kx = 0;                    // K1/2 + 1 complex columns of the half spectrum
-  float qmax = 0.f;              // at least the largest |charge|
   double* fspme = nullptr;     // 3*natms reciprocal forces (before scale, net removal)
   void* spread_ext = nullptr;  // per-brick spread tiles (nbricks x (B+p-1)^3)
   int* gidx = nullptr;         // warp gather: first grid index per dimension (truncation convention)
@@ -1099,11 +1090,10 @@ void grid_setup(SpmeGrid& S, const int* Kin, int p, bool fp64) {
   const size_t NG = (size_t)S.K[0] * S.K[1] * S.K[2];
   if (NG > (size_t)INT_MAX) throw (int)GB_ERR_ARG;  // the gathers index grid points with int offsets
   const size_t n = (size_t)g.natms;
-  S.qmax = std::nextafter((float)g.qmax, 3.0e38f);
   GB_CUDA(cudaMalloc(&S.spl, sizeof(double) * n * 3 * p));
   GB_CUDA(cudaMalloc(&S.nidx, sizeof(int) * 3 * n));
   GB_CUDA(cudaMalloc(&S.brick_of, sizeof(int) * n));
-  // after the counts: one unused, then the largest |potential|, the overflow entries, the pool
+  // after the counts: two unused, then the overflow entries, the pool
   GB_CUDA(cudaMalloc(&S.brick_count, sizeof(int) * (S.nbricks + 4)));
   // slots for three times the mean and some; at most 2,048 (their sorted copy is in shared memory)
   S.cap = std::min(2048, (int)std::min<size_t>(n, 3 * (n / S.nbricks) + 32));
@@ -1385,10 +1375,8 @@ void grid_run(SpmeGrid& S, bool coarse, float* rec, double* eng_rc, double* vir_
   GB_LAUNCHED();
   prof_end(pid(P_FFT_Y));
   prof_begin(pid(P_FFT_XI));
-  // (the largest |potential| goes to the zeroed entry after the brick counts)
-  unsigned* vmax = reinterpret_cast<unsigned*>(S.brick_count + S.nbricks + 1);
   fk.x_inv<<<nblocks(rows, XLINES), thx, fft_smem(M, XLINES, sizeof(T2)), st>>>(G, Q, S.planh, twh, tw1, rows,
-                                                                              XLINES, vmax);
+                                                                              XLINES);
   GB_LAUNCHED();
   prof_end(pid(P_FFT_XI));
   // gather
@@ -1414,7 +1402,7 @@ void grid_run(SpmeGrid& S, bool coarse, float* rec, double* eng_rc, double* vir_
     for (int a = 0; a < 3; ++a) df_split(rk[a], &rkd[a].x, &rkd[a].y);
     kern<<<nbg, 256, 0, st>>>(n, ab, S.sg, S.gidx, reinterpret_cast<const dfr*>(S.gsp),
                               reinterpret_cast<const float2*>(S.gw + 6 * (size_t)n), reinterpret_cast<const dfr*>(Q),
-                              rkd[0], rkd[1], rkd[2], S.qmax, vmax, reinterpret_cast<float2*>(S.fspme), blkg, gsg);
+                              rkd[0], rkd[1], rkd[2], reinterpret_cast<float2*>(S.fspme), blkg, gsg);
   } else if (warp_gather) {
     auto kern = p == 8 ? k_spme_gather_f32<8> : k_spme_gather_f32<6>;
     kern<<<nbg, 256, 0, st>>>(n, ab, reinterpret_cast<const float*>(g.xf), S.sg, S.gidx, S.gw,

@@ -616,3 +616,21 @@ def test_spme_side_stream_matches_one_stream(gpu_lib, monkeypatch, name, precisi
                   "engke"):
             assert getattr(x, f) == getattr(y, f), f
         assert list(x.stress) == list(y.stress)
+
+
+def test_spme_of_weak_charges_among_strong_ones(gpu_lib, oracle_lib):
+    """Reciprocal forces of atoms with 1e-4 of the others' charge, relative to their own size: the
+    gather's sums are rounded against the atom's own terms, not against the largest of the grid."""
+    s = systems.nacl_melt(16)
+    weak = np.arange(s.natms) % 8 < 2  # neighbours in the lattice: both signs
+    s.chge = np.where(weak, 1e-4 * s.chge, s.chge)
+    _pair(gpu_lib, oracle_lib, s)
+    gpu_lib.ewald_spme_forces()
+    oracle_lib.ewald_spme_forces()
+    a, b = gpu_lib.download(), oracle_lib.download()
+    # the mean net force, removed from every atom, belongs to the strong ones
+    d = {k: a[k][weak] - b[k][weak] for k in ("fx", "fy", "fz")}
+    for k in d:
+        own = np.sqrt((b[k][weak] ** 2).mean())
+        print(k, np.abs(d[k] - d[k].mean()).max() / own, np.abs(d[k]).max() / own)
+        assert np.abs(d[k] - d[k].mean()).max() <= 1e-11 * own, k
