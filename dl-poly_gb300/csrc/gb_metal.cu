@@ -365,11 +365,10 @@ __global__ void __launch_bounds__(256, 3) k_metal_forces(int natms, const DevSca
 // 0.89 ms (1.04 with 102 registers, two CTAs per SM; a fourth CTA spills and gains
 // nothing); latency of the partners and tables, at a third of the issue slots.
 //   positions   fixed point (PosRec): the separation is an exact integer difference
-//   r           to the last of 48 bits, and its fraction of a table interval from the r of
-//               the table's point; an atom's force is summed in FP64 (errors of forces
-//               against 64 bits 1.2e-13, the FP64 kernels 0.8e-13: both from r, on which
-//               the difference of a pair's terms depends forty times over; energies and
-//               stress are nearer than the FP64 kernels')
+//   r           to 1.4e-15 (rms), and its fraction of a table interval from the r of the
+//               table's point; an atom's force is summed in FP64 (rms errors against 64
+//               bits, 8,788 and 256,000 atoms: forces 5.0e-14 and 5.4e-14, of the FP64 kernels
+//               6.7e-14 and 7.4e-14; stress 1.6e-13 and 1.3e-13, theirs 1.6e-12 and 1.4e-12)
 // A pair near a cutoff, at an end of its table, next to the middle of two points, with a
 // negative density or outside the FP32 range takes the FP64 formulas of the kernels above (metal_density_slow,
 // metal_force_slow).  Densities and forces are summed in FP64 per sorted position and
@@ -409,37 +408,49 @@ __device__ __forceinline__ df met_norm2(df x, df y, df z) {
   return quick_two_sum(s2.hi, __fadd_rn(__fadd_rn(__fadd_rn(cx, cy), __fadd_rn(cz, s1.lo)), s2.lo));
 }
 
-// r and 1/r^2 (3e-14) of a double-float r^2 in the normal range.  The force of a metal pair is a
-// difference of terms that changes forty times as fast as r, so r gets the last bits: an
-// FP32 root s and the remainder (r^2 - s^2) / 2s with 1/s refined from the root's seed.
-__device__ __forceinline__ df met_dist(df r2, df* inv) {
+// r and 1/r^2 (relative error below 1e-14, rms 1.7e-15) of a double-float r^2 in the normal
+// range.  The force of a metal pair is a difference of terms that changes forty times as fast as
+// r, so r gets three words: the FP32 root to half an ulp (1/r refined from its seed), the
+// remainder (r^2 - s^2) / 2s and what FP32 leaves of that quotient.
+struct Root {
+  float s, q, x;
+};
+__device__ __forceinline__ Root met_dist(df r2, df* inv) {
   const float rs = rsqrtf(r2.hi);
-  const float s = __fmul_rn(r2.hi, rs);
-  const df ss = two_prod(s, s);
-  const float e = __fadd_rn(__fsub_rn(__fsub_rn(r2.hi, ss.hi), ss.lo), r2.lo);
+  const float q0 = __fmul_rn(rs, rs);
+  const float g0 = __fmaf_rn(-r2.hi, q0, 1.f);
+  const float h = __fmul_rn(0.5f, __fmaf_rn(rs, __fmul_rn(0.5f, g0), rs));  // 1 / 2r
+  const float s0 = __fmul_rn(r2.hi, __fadd_rn(h, h));
+  Root r;
+  r.s = __fmaf_rn(h, __fmaf_rn(-s0, s0, r2.hi), s0);
+  const df ss = two_prod(r.s, r.s);
+  const df e = two_sum(__fsub_rn(r2.hi, ss.hi), __fsub_rn(r2.lo, ss.lo));
+  r.q = __fmul_rn(h, e.hi);
+  // (s + q + x)^2 = r^2: x = (e - 2 s q - q^2) / 2s
+  r.x = __fmul_rn(h, __fmaf_rn(-r.q, r.q, __fadd_rn(__fmaf_rn(-r.q, __fadd_rn(r.s, r.s), e.hi), e.lo)));
   if (inv) {
-    const float q = __fmul_rn(rs, rs);
-    const float g = __fmaf_rn(-r2.lo, q, __fmaf_rn(-r2.hi, q, 1.f));  // 1 - r2 q, about 2^-21
+    const float q = __fmaf_rn(q0, g0, q0);
+    const float g = __fmaf_rn(-r2.lo, q, __fmaf_rn(-r2.hi, q, 1.f));  // 1 - r2 q
     *inv = quick_two_sum(q, __fmul_rn(q, __fmaf_rn(g, g, g)));
   }
-  const float y = __fmaf_rn(rs, __fmaf_rn(-s, rs, 1.f), rs);
-  return quick_two_sum(s, __fmul_rn(__fmul_rn(0.5f, y), e));
+  return r;
 }
 
-// table point l and fraction p in [-0.5, 0.5] of a double-float r; false at a table's ends and
+// table point l and fraction p in [-0.5, 0.5] of r; false at a table's ends and
 // next to the middle of two points (|p| = 0.5 to FP32, one lookup in 10^7), where the
 // interpolant jumps by an eighth of the third difference and FP64 decides which point is nearer.
 // p = (r - r_l) / dr from the point's own r: the product r / dr would be rounded at 2^-48 of
 // a coordinate of some thousand.
-__device__ __forceinline__ bool met_coord(const MetTab& t, const CoefF* __restrict__ c, df r, int* l, df* p) {
-  float k = rintf(__fmaf_rn(r.hi, t.rdr_h, t.nr_h));
+__device__ __forceinline__ bool met_coord(const MetTab& t, const CoefF* __restrict__ c, Root r, int* l, df* p) {
+  float k = rintf(__fmaf_rn(r.s, t.rdr_h, t.nr_h));
   if (!(k > 5.f && k < (float)(t.n - 1))) return false;
   int i = (int)k;
   df d;
   for (;;) {
     const float2 rk = *reinterpret_cast<const float2*>(&c[i].rh);
-    const df s = two_sum(r.hi, -rk.x);
-    const df q = quick_two_sum(s.hi, __fadd_rn(s.lo, __fsub_rn(r.lo, rk.y)));
+    const df b = two_sum(r.q, -rk.y);
+    const df s = two_sum(__fsub_rn(r.s, rk.x), b.hi);  // (neighbours: the difference is exact)
+    const df q = quick_two_sum(s.hi, __fadd_rn(s.lo, __fadd_rn(b.lo, r.x)));
     d = df_mul(q, df_make(t.rdr_h, t.rdr_l));
     // (the FP32 nearest integer may have been the other neighbour of a midpoint)
     if (d.hi > 0.5f && i + 1 == (int)k + 1) ++i;
@@ -594,7 +605,7 @@ __global__ void __launch_bounds__(MET_NT) k_metal_density_sorted(MetSorted S, Me
       bool slow = in_j < 0 || in_i < 0 || !met_plain(r2.hi);
       df to_i = df_make(0.f, 0.f), to_j = to_i;
       if (!slow) {
-        const df r = met_dist(r2, nullptr);
+        const Root r = met_dist(r2, nullptr);
         int l = 0;
         df f;
         if (in_j) {
@@ -691,7 +702,7 @@ __global__ void __launch_bounds__(MET_NT, 3) k_metal_forces_sorted(MetSorted S, 
       df gam = df_make(0.f, 0.f), num = gam, eng = gam;
       if (!slow) {
         df inv, f;
-        const df r = met_dist(r2, &inv);
+        const Root r = met_dist(r2, &inv);
         int l = 0, gl = -1;
         if (in_p) {
           slow = !met_coord(tp, S.fv + tp.off, r, &l, &f);

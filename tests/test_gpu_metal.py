@@ -88,3 +88,38 @@ def test_eam_pairs_next_to_a_midpoint(gpu_lib, oracle_lib, side, off):
         (fa, ra), (fb, rb) = out
         assert np.abs(fa - fb).max() <= 1e-10 * np.abs(fb).max()
         np.testing.assert_allclose(ra, rb, rtol=1e-10)
+
+
+def test_eam_distance_to_the_last_bits(gpu_lib):
+    """Isolated pairs under V = (r - 2.5)^2 / 2, whose force r - 2.5 shows the error of r itself:
+    1e-14 of the root and 0.4e-14 of r^2 (48 bits), relative to r, and as much of the force."""
+    n, step = 12, 16.0
+    rng = np.random.default_rng(11)
+    g = np.arange(n) * step - 0.5 * n * step + 0.5 * step
+    at = np.stack(np.meshgrid(g, g, g, indexing="ij"), -1).reshape(-1, 3)
+    d = rng.standard_normal(at.shape)
+    d *= (rng.uniform(2.2, 2.8, len(at)) / np.linalg.norm(d, axis=1))[:, None]
+    d = np.round(d * 2.0 ** 30) / 2.0 ** 30  # (coordinates and separations without rounding)
+    s = two_atoms(2.0, box=n * step)
+    pos = np.empty((2 * len(at), 3))
+    pos[0::2], pos[1::2] = at, at + d
+    m = len(pos)
+    s.ltype, s.chge, s.weight = np.ones(m, np.int32), np.zeros(m), np.full(m, 60.0)
+    s.lfrzn = np.zeros(m, np.int32)
+    s.x, s.y, s.z = (pos[:, k].copy() for k in range(3))
+    s.vx, s.vy, s.vz = (np.zeros(m) for _ in range(3))
+    r = np.linspace(1.0, 6.0, 401)
+    rho = np.linspace(0.0, 10.0, 401)
+    s.eam = [{"kind": "pair", "types": (1, 1), "start": 1.0, "finish": 6.0, "values": 0.5 * (r - 2.5) ** 2},
+             {"kind": "dens", "types": (1, 1), "start": 1.0, "finish": 6.0, "values": 1.0 + 0.0 * r},
+             {"kind": "embe", "types": (1, 1), "start": 0.0, "finish": 10.0, "values": 0.0 * rho}]
+    gpu_lib.init(s)
+    gpu_lib.start()
+    f = gpu_lib.download()
+    ld = d.astype(np.longdouble)
+    dist = np.sqrt((ld ** 2).sum(1))
+    along = sum(f[k][0::2] * ld[:, c] for c, k in enumerate(("fx", "fy", "fz"))) / dist
+    err = np.abs(along - (dist - np.longdouble(2.5)))
+    bound = 1.4e-14 * dist + 1.4e-14 * np.abs(dist - 2.5) + 2e-15  # (2e-15: the table's differences)
+    print(float((err / dist).max()), float(np.sqrt(((err / dist) ** 2).mean())))
+    assert (err <= bound).all()
