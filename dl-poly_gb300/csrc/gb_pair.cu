@@ -838,18 +838,19 @@ __device__ __forceinline__ df prod_pair(df a, df b) {
   return df_make(p.hi, __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.lo, b.hi, p.lo)));
 }
 
-// r (an FP32 root and its remainder to second order) and 1/r^2 (an FP32 reciprocal to the last
-// bit and its remainder) of a double-float r^2, both with relative errors below 1e-14
+// r (an FP32 root and its remainder) and 1/r^2 (an FP32 reciprocal to the last bit and its
+// remainder) of a double-float r^2.  Relative errors, rms and largest, of the operations with seeds
+// up to one ulp off: r 5.0e-15 and 3.4e-14, 1/r^2 2.4e-15 and 1.4e-14.
 __device__ __forceinline__ df dist_inv2(df r2, df* inv) {
   const float rs = rsqrtf(r2.hi);
   const float s = __fmul_rn(r2.hi, rs);
   const df ss = two_prod(s, s);
-  const float e = __fadd_rn(__fsub_rn(__fsub_rn(r2.hi, ss.hi), ss.lo), r2.lo);
+  const float e = __fadd_rn(__fsub_rn(r2.hi, ss.hi), __fsub_rn(r2.lo, ss.lo));
   const float q0 = __fmul_rn(rs, rs);
   const float g0 = __fmaf_rn(-r2.hi, q0, 1.f);  // 1 - r2 q0
   const float q = __fmaf_rn(q0, g0, q0);
   *inv = df_make(q, __fmul_rn(q, __fmaf_rn(-r2.lo, q, __fmaf_rn(-r2.hi, q, 1.f))));
-  const float rc = __fmaf_rn(rs, __fmul_rn(0.5f, g0), rs);  // 1/r to the last bit
+  const float rc = __fmaf_rn(rs, __fmul_rn(0.75f, g0), rs);  // 2 / (r + s)
   return quick_two_sum(s, __fmul_rn(__fmul_rn(0.5f, rc), e));
 }
 
