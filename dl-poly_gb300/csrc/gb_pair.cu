@@ -1173,8 +1173,7 @@ __global__ void __launch_bounds__(NT, 1024 / NT) k_pair_sorted(PairSortedArgs A,
 // image at its own position, in FP64 from the exact fixed-point forces), then each
 // slot's force onto its atom (a halo image's onto its source): integer sums.
 // The same launch sums the local atoms' energies and virials (eat), 4 values before the 6 of
-// the stress; the block sums are double-float, so that only the stress products and
-// running sums use the FP64 unit.
+// the stress, the block sums in FP64.
 __global__ void k_slot_stress_fold(int natms, const DevScalars* sc, const int* __restrict__ at_list,
                                    const int* __restrict__ src, const double* __restrict__ x,
                                    const double* __restrict__ y, const double* __restrict__ z,
@@ -1207,11 +1206,11 @@ __global__ void k_slot_stress_fold(int natms, const DevScalars* sc, const int* _
     atomicAdd(&fixp[3 * tgt + 1], (unsigned long long)f1);
     atomicAdd(&fixp[3 * tgt + 2], (unsigned long long)f2);
   }
-  dfr out[NACC_DF + 6];
+  double out[NACC_DF + 6];
 #pragma unroll
-  for (int c = 0; c < NACC_DF; ++c) out[c] = to_dfr(two_sum(e[c].s, e[c].c));
+  for (int c = 0; c < NACC_DF; ++c) out[c] = dacc_value(e[c]);
 #pragma unroll
-  for (int k = 0; k < 6; ++k) out[NACC_DF + k] = dfr(st[k]);
+  for (int k = 0; k < 6; ++k) out[NACC_DF + k] = st[k];
   block_reduce_store<NACC_DF + 6>(out, blk);
   grid_finish<NACC_DF + 6>(blk, gs);
 }

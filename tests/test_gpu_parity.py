@@ -634,3 +634,27 @@ def test_spme_of_weak_charges_among_strong_ones(gpu_lib, oracle_lib):
         own = np.sqrt((b[k][weak] ** 2).mean())
         print(k, np.abs(d[k] - d[k].mean()).max() / own, np.abs(d[k]).max() / own)
         assert np.abs(d[k] - d[k].mean()).max() <= 1e-11 * own, k
+
+
+@pytest.mark.parametrize("precision", [0, 1], ids=["fp64", "mixed"])
+def test_pair_stress_summed_in_fp64(gpu_lib, precision):
+    """The stress of a pair far from the origin is a difference of x (x) F terms ten times its
+    size: it equals the sum over the downloaded positions and forces to their FP64 roundings."""
+    s = systems.lj_pair(eps=100.0, sigma=2.0, r=2.3)
+    s.x = np.array([17.31, 18.77])
+    s.y = np.array([-16.93, -15.61])
+    s.z = np.array([15.47, 16.59])
+    gpu_lib.init(s, precision=precision)
+    gpu_lib.relocate()
+    gpu_lib.link_cell_pairs(want_list=False)
+    _, stress = gpu_lib.two_body_forces()
+    assert gpu_lib.pair_counts()[5] == 1
+    d = gpu_lib.download()
+    x = np.array([d[k] for k in "xyz"], np.longdouble)
+    f = np.array([d[k] for k in ("fx", "fy", "fz")], np.longdouble)
+    terms = x[:, None, :] * f[None, :, :]
+    want, size = terms.sum(-1), np.abs(terms).sum(-1)
+    got = stress.reshape(3, 3)
+    sign = np.sign(float(want[0, 0])) * np.sign(got[0, 0])
+    upper = np.triu(np.ones((3, 3), bool))  # the stress is symmetric, x (x) F only to rounding
+    assert (np.abs(sign * got - want)[upper] <= (4 * 2.0 ** -53 * size)[upper]).all()
