@@ -141,11 +141,11 @@ __device__ __forceinline__ long long fix40_df(df a) {
 
 // the fixed point of the product a * b without renormalising it, where a carries the scale
 // 2^40 already: the exact product's high part and the sum of its rounding error and cross
-// terms, each truncated toward zero
+// terms, each rounded to nearest (toward zero, the sum over the pairs of a system is biased)
 __device__ __forceinline__ long long fix_prod(df a, df b) {
   const float p = __fmul_rn(a.hi, b.hi);
   const float t = __fmaf_rn(a.hi, b.lo, __fmaf_rn(a.lo, b.hi, __fmaf_rn(a.hi, b.hi, -p)));
-  return __float2ll_rz(p) + __float2ll_rz(t);
+  return __float2ll_rn(p) + __float2ll_rn(t);
 }
 
 // (a - b) / scale of two fixed-point coordinates for |a - b| < 2^52: an exact integer

@@ -658,3 +658,24 @@ def test_pair_stress_summed_in_fp64(gpu_lib, precision):
     sign = np.sign(float(want[0, 0])) * np.sign(got[0, 0])
     upper = np.triu(np.ones((3, 3), bool))  # the stress is symmetric, x (x) F only to rounding
     assert (np.abs(sign * got - want)[upper] <= (4 * 2.0 ** -53 * size)[upper]).all()
+
+
+def test_pair_forces_rounded_to_the_nearest_unit(gpu_lib, oracle_lib):
+    """A small pair force (relative errors far below a unit) is within half a unit, 2^-41, of the
+    oracle's: rounded toward zero, the sums over many pairs are biased."""
+    off = []
+    for r in np.linspace(2.05, 4.0, 40):
+        s = systems.lj_pair(eps=0.01, sigma=2.0, r=2.0)
+        d = np.array([0.6, 0.48, 0.64]) * r
+        for k, v in zip("xyz", d):
+            setattr(s, k, np.array([-0.5 * v, 0.5 * v]))
+        f = []
+        for lib in (gpu_lib, oracle_lib):
+            lib.init(s)
+            lib.relocate()
+            lib.link_cell_pairs(want_list=False)
+            lib.two_body_forces()
+            o = lib.download()
+            f.append(np.array([o[k][0] for k in ("fx", "fy", "fz")]))
+        off.append(np.abs(f[0] - f[1]) - 1e-13 * np.abs(f[1]).max())
+    assert np.max(off) <= 2.0 ** -41
