@@ -733,8 +733,14 @@ int gb_init(const gb_params* prm, int natms, const int32_t* ltype, const double*
     build_tables(vdw_prm);
     pair_setup();
     g.scaling = kR4pie0 / prm->epsq;
-    double sq2 = 0.0;
-    for (int i = 0; i < natms; ++i) sq2 += chge[i] * chge[i];
+    double sq2 = 0.0, qmax = 0.0;
+    for (int i = 0; i < natms; ++i) {
+      sq2 += chge[i] * chge[i];
+      qmax = std::max(qmax, std::fabs(chge[i]));
+    }
+    // an atom's exclusion forces within a quarter of the sums' range, 2^63 units of 2^-40
+    g.excl_fixed = 0.43 * std::fabs(g.scaling) * prm->alpha * prm->alpha * qmax * qmax *
+                       std::max(prm->max_exclude, 1) < 2097152.0;
     g.self_interaction = -sq2 * (g.scaling * prm->alpha * (1.0 / 1.7724538509055161040) / 1.0);  // spme.F90:159-231
     g.ntcons = ntcons;
     if (ntcons > 0) integ_setup_constraints(listcon, prmcon);

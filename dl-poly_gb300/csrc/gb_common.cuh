@@ -234,6 +234,7 @@ struct Dev {
   std::vector<int> h_vdw_kind;
   std::vector<double> h_vdw_eps, h_vdw_sig;
   double elrc = 0, vlrc = 0, self_interaction = 0, scaling = 0;
+  bool excl_fixed = true;      // FP64 form: exclusion forces into the fixed-point sums (k_excl_fp64)
 
   // SPME grids live in gb_spme.cu (SpmeGrid); shared scratch here
   double* blkacc = nullptr;    // per-block partial accumulators

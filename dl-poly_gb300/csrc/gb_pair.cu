@@ -239,9 +239,10 @@ __global__ void __launch_bounds__(256, 3) k_pair_fp64(int natms, const DevScalar
 // atoms as one sequence, a lane each (a water's atoms have two, one and none, so that a thread
 // per atom left half of its FP64 issue slots idle: 0.058 ms for 98,304 atoms of water, now 0.034).
 // Forces go to the pairs' int64 fixed-point sums (fixp; in the FP64 form they join the others'
-// with k_fix_add_fp64), whose sum does not depend on the order; the FP64 form by instructions
-// (fixp = 0) adds them in FP64.  The force of an excluded pair is bounded (it vanishes with
-// r), below 2e4 q^2 internal units.  In the mixed form too this kernel stays in FP64: the
+// with k_fix_add_fp64), whose sum does not depend on the order; the FP64 form by instructions,
+// and the FP64 form where they might leave the sums' range (excl_fixed), add them in FP64
+// (fixp = 0).  The force of an excluded pair vanishes with r and is at most 0.43 alpha^2 q^2 /
+// (4 pi eps), 6e4 alpha^2 q^2 internal units (at 1/r = 1.03 alpha).  In the mixed form too this kernel stays in FP64: the
 // intramolecular exclusion terms cancel against the reciprocal energy (tens of millions of
 // internal units for water).
 __global__ void k_excl_fp64(int natms, const int* list, int ld, const double* x, const double* y, const double* z,
@@ -1362,15 +1363,17 @@ void pair_forces_sorted(PairGeom& pg, int nb2) {
     k_fix_add_fp64<<<nblocks(g.natms, 256), 256, 0, st>>>(g.natms, g.fixp, g.fx, g.fy, g.fz);
     GB_LAUNCHED();
   };
-  if (!g.lbook) add();
+  const bool excl_fixed = mixed || g.excl_fixed;
+  if (!g.lbook || !excl_fixed) add();
   prof_end(P_PAIR);
   if (g.lbook) {
     prof_begin(P_EXCL);
     const GridSum gse = gb_grid_sum(nb2, 128, 8, &g.sc->acc[A_EXCL]);
     k_excl_fp64<<<nb2, 128, 0, st>>>(g.natms, g.list, g.ld, g.x, g.y, g.z, g.chge, g.ltg, g.src, g.p.alpha,
-                                     g.scaling, g.p.rcut, g.fx, g.fy, g.fz, blk2, (unsigned long long*)g.fixp, gse);
+                                     g.scaling, g.p.rcut, g.fx, g.fy, g.fz, blk2,
+                                     excl_fixed ? (unsigned long long*)g.fixp : nullptr, gse);
     GB_LAUNCHED();
-    add();
+    if (excl_fixed) add();
     prof_end(P_EXCL);
     gb_grid_sum_done(gse, blk2, nb2, 8);
   }
@@ -1462,18 +1465,23 @@ void pair_forces(double* eng6, double* stress9) {
     prof_end(P_PAIR);
     gb_reduce_blocks(blk, nb, NACC_DF, &g.sc->acc[A_PAIR]);
     gb_reduce_blocks(blks, nbs, 6, &g.sc->acc[A_PAIR + NACC_DF]);
+    auto add = [&]() {
+      k_fix_add_fp64<<<nblocks(g.natms, 256), 256, 0, st>>>(g.natms, g.fixp, g.fx, g.fy, g.fz);
+      GB_LAUNCHED();
+    };
+    if (!g.lbook || !g.excl_fixed) add();
     if (g.lbook) {
       double* blk2 = blk + (size_t)nb * NACC;
       prof_begin(P_EXCL);
       const GridSum gse = gb_grid_sum(nb2, 128, 8, &g.sc->acc[A_EXCL]);
       k_excl_fp64<<<nb2, 128, 0, st>>>(g.natms, g.list, g.ld, g.x, g.y, g.z, g.chge, g.ltg, g.src, g.p.alpha,
-                                       g.scaling, g.p.rcut, g.fx, g.fy, g.fz, blk2, (unsigned long long*)g.fixp, gse);
+                                       g.scaling, g.p.rcut, g.fx, g.fy, g.fz, blk2,
+                                       g.excl_fixed ? (unsigned long long*)g.fixp : nullptr, gse);
       GB_LAUNCHED();
+      if (g.excl_fixed) add();
       prof_end(P_EXCL);
       gb_grid_sum_done(gse, blk2, nb2, 8);
     }
-    k_fix_add_fp64<<<nblocks(g.natms, 256), 256, 0, st>>>(g.natms, g.fixp, g.fx, g.fy, g.fz);
-    GB_LAUNCHED();
   } else if (g.precision == GB_FP64) {
     static int occ64 = 0;
     if (!occ64) GB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ64, k_pair_fp64, T, 0));

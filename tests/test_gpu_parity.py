@@ -679,3 +679,27 @@ def test_pair_forces_rounded_to_the_nearest_unit(gpu_lib, oracle_lib):
             f.append(np.array([o[k][0] for k in ("fx", "fy", "fz")]))
         off.append(np.abs(f[0] - f[1]) - 1e-13 * np.abs(f[1]).max())
     assert np.max(off) <= 2.0 ** -41
+
+
+@pytest.mark.parametrize("sorted_list", ["1", "0"])
+@pytest.mark.parametrize("charge", [2.0, 25.0])
+def test_exclusion_forces_beyond_the_fixed_point_range(gpu_lib, oracle_lib, monkeypatch, sorted_list, charge):
+    """The exclusion force of a molecule of +-25 e at alpha = 0.9 (3e7 internal units) exceeds what the
+    fixed-point sums hold (8.4e6): it is added in FP64."""
+    s = systems.lj_pair(eps=1.0, sigma=2.0, r=1.1)
+    s.chge = np.array([charge, -charge])
+    s.alpha = 0.9
+    s.kmax = (64, 64, 64)
+    s.max_exclude = 1
+    s.list_excl = np.array([[1, 2], [1, 1]], np.int32)
+    monkeypatch.setenv("GB_PAIR_SORTED", sorted_list)
+    _pair(gpu_lib, oracle_lib, s)
+    gpu_lib.link_cell_pairs(want_list=False)
+    oracle_lib.link_cell_pairs(want_list=False)
+    er, ee = oracle_lib.real_space_forces()[0], gpu_lib.real_space_forces()[0]
+    monkeypatch.delenv("GB_PAIR_SORTED")
+    a, b = gpu_lib.download(), oracle_lib.download()
+    f = np.abs(b["fx"]).max()
+    assert (f > 2.0 ** 23) == (charge > 20.0)
+    assert force_dev(a, b) < FP64_TOL
+    assert ee["engcpe_ex"] == pytest.approx(er["engcpe_ex"], rel=FP64_TOL)
