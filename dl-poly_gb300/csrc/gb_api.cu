@@ -348,16 +348,12 @@ int compute_forces(double* eng8, double* stress9, bool do_spme, bool do_real, bo
   // side stream once the pair kernel is launched, and run beside it
   const bool mts_side = mts && !full && g.use_overlap && do_real && !g.has_metal;
   if (mts && !mts_side) mts_coarse();
-  // SPME on the side stream while the pair kernel runs.  The plain FP64 form keeps one
-  // stream (its kernels are bound by the FP64 unit both sides share), and so does the
-  // double-float form in a large ionic system: each side fills the device with the same
-  // FP32 work, and the pair kernel's resident CTAs start late on the SMs that SPME holds.
-  // (NaCl, one stream / two, us per step: 32,768 ions 446 / 437, 85,184 893 / 893, 110,592
-  // 1140 / 1169, 262,144 2202 / 2289.  With exclusions, whose kernel SPME hides, two are
-  // better still: water, 98,304 atoms, 1466 / 1431; the mixed form at 262,144: 1190 / 1185.)
-  const bool crowded = g.precision == GB_FP64 && !g.lbook && g.natms > 90000;
+  // SPME on the side stream while the pair kernel runs (the plain FP64 form keeps one
+  // stream: its kernels are bound by the FP64 unit both sides share).  One stream / two, NaCl in
+  // the double-float form, us per step: 32,768 ions 436 / 433, 85,184 863 / 856, 110,592 1108 /
+  // 1097, 262,144 2130 / 2122; cutoff 9 A and a finer grid, 110,592 1216 / 1208.
   const bool overlap = g.use_overlap && full && !mts && do_real && !g.has_metal &&
-                       !(g.precision == GB_FP64 && g.fp64_native) && !crowded;
+                       !(g.precision == GB_FP64 && g.fp64_native);
   if (overlap) {
     const bool deferred = g.defer_scalars;
     g.defer_scalars = true;  // both sides leave their sums on the device; read once below
