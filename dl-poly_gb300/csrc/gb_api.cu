@@ -592,6 +592,8 @@ GridSum gb_grid_sum(int nb, int nt, int nv, double* out_dev) {
   return {nb <= 20 * std::max(rows, 1) ? (g.side ? &g.sc->count_s : &g.sc->count) : nullptr, out_dev};
 }
 
+unsigned long long* stamp_at(int k) { return g.time_regions ? &g.sc->t_ns[k] : nullptr; }
+
 // (a mask of 0, and no load, for bits that this system's kernels never set)
 StopIf stop_if(int mask) {
   const int can = (g.ntcons > 0 ? ST_RATTLE_FAIL : 0) | (g.has_metal ? ST_STOP2 : 0);
@@ -1101,8 +1103,8 @@ static void md_step_stats(const DevScalars* h, int32_t rebuilt, gb_step_stats& S
 // decision and the halo refresh or the list rebuild that it calls for, the forces (SPME
 // forked to the side stream) and stage 2; the second is captured again when a rebuild
 // changes the kernels that walk the list.  Langevin's stage 1 is launched (its noise is keyed
-// on the step).  The per-region timings of gb_last_timings are not taken on this path (the
-// total is).
+// on the step).  In plain NVE the total is the only timing; the other systems' kernels at the
+// ends of the regions store the device's clock beside the sums.
 static int md_run_deferred(int nsteps, gb_step_stats* stats) {
   if (g.ring_cap < nsteps) {
     if (g.ring) cudaFreeHost(g.ring);
@@ -1117,6 +1119,7 @@ static int md_run_deferred(int nsteps, gb_step_stats* stats) {
   GB_CUDA(cudaMemsetAsync(&g.sc->status, 0, sizeof(int), g.stream));
   g.defer_scalars = true;
   const bool plain = g.ntcons == 0 && g.ens == GB_NVE;
+  g.time_regions = !plain || g.has_metal;
   auto stage1 = [&]() {
     if (plain) {
       integ_stage1_check();
@@ -1174,6 +1177,8 @@ static int md_run_deferred(int nsteps, gb_step_stats* stats) {
     if (g.hsc->status & ST_RNG) break;  // Langevin's noise (stage 1) ends the call after the step
   }
   g.defer_scalars = false;
+  const bool regions = g.time_regions;
+  g.time_regions = false;
   GB_CUDA(cudaEventRecord(g.ev[6], g.stream));
   GB_CUDA(cudaEventSynchronize(g.ev[6]));
   if (code == GB_OK && last >= 0) {
@@ -1182,9 +1187,19 @@ static int md_run_deferred(int nsteps, gb_step_stats* stats) {
   }
   float span = 0.f;
   cudaEventElapsedTime(&span, g.ev[5], g.ev[6]);
-  for (int k = 0; k < 5; ++k) g.last_ms[k] = 0.0;
-  g.last_ms[4] = span;
-  g.last_ms[5] = span;
+  if (code == GB_OK) {
+    double list = 0.0, forces = 0.0;
+    for (int s = 0; regions && s < nsteps; ++s) {
+      const unsigned long long* t = g.ring[s].t_ns;
+      list += 1e-6 * (double)(t[1] - t[0]);
+      forces += 1e-6 * (double)(t[2] - t[1]);
+    }
+    g.last_ms[0] = list;
+    g.last_ms[1] = forces;
+    g.last_ms[2] = 0.0;
+    g.last_ms[3] = regions ? span - list - forces : 0.0;
+    g.last_ms[4] = g.last_ms[5] = span;
+  }
   if (stats)
     for (int s = 0; s < done; ++s) md_step_stats(&g.ring[s], rebuilt[s], stats[s]);
   if (last >= 0) {  // the sums of the last evaluation (none of a failed one)
@@ -1202,7 +1217,7 @@ int gb_md_run(int nsteps, gb_step_stats* stats) {
       try {
         return md_run_deferred(nsteps, stats);
       } catch (int e) {
-        g.defer_scalars = false;
+        g.defer_scalars = g.time_regions = false;
         throw;
       }
     }

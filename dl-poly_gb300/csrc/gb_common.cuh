@@ -57,6 +57,7 @@ struct DevScalars {
   int halo_fwd;     // list entries with a halo image found in the forward half shell (evaluated)
   int halo_bwd;     // list entries with a halo image found in the backward halo pass (skipped)
   unsigned count_s; // the same on the side stream
+  unsigned long long t_ns[3];  // MD loop: times of the end of stage 1, the start of the forces and of stage 2
   unsigned long long npairs_list;  // half-list entries walked by the pair kernel
   unsigned long long npairs_rc;    // unique pairs inside the cutoff
   double acc[96];   // energy / virial / stress accumulators
@@ -190,6 +191,7 @@ struct Dev {
   // to a pinned ring and read after the last step, so the host waits only for the
   // Verlet-list decision of each step
   bool defer_scalars = false;
+  bool time_regions = false;   // that loop takes gb_last_timings' regions
   bool use_deferred = true;    // GB_MD_DEFER=0 keeps the per-step read-back
   // that loop as CUDA graphs (GB_GRAPHS=0: every kernel launched by the host): stage 1 with
   // the Verlet-list check, and the forces with stage 2, captured once per call; the launch
@@ -488,6 +490,16 @@ int list_relocate_and_halo(bool wait = true);
 int list_refresh_halo();          // refresh halo positions (gb_list.cu)
 int list_build();                 // binning + pairs (gb_list.cu)
 void list_setup();                // link-cell geometry (gb_list.cu)
+// Nanoseconds of the device's clock into *at by one thread (null: nothing); the MD loop times its
+// regions so, at no launch (events at their ends took 10 to 16 us a step).
+__device__ __forceinline__ void stamp_time(unsigned long long* at) {
+  if (at && blockIdx.x == 0 && threadIdx.x == 0) {
+    unsigned long long t;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+    *at = t;
+  }
+}
+unsigned long long* stamp_at(int k);  // where the MD loop wants the k-th time, or null
 void list_pos_records(bool sorted);  // FP32 hi/lo positions by atom index and (sorted) per sorted position; clears the force sums
 void scan_exclusive(const int* in, int* out, int n);
 void pair_forces(double* eng6, double* stress9);  // gb_pair.cu (adds into forces)

@@ -69,8 +69,9 @@ __global__ void k_vv1(int n, const double* __restrict__ hdw, double tstep, const
 
 __global__ void k_vv2(int n, const double* __restrict__ hdw, const double* __restrict__ fx,
                       const double* __restrict__ fy, const double* __restrict__ fz, double* vx, double* vy,
-                      double* vz, StopIf stop) {
+                      double* vz, StopIf stop, unsigned long long* t_ns) {
   int i = blockIdx.x * blockDim.x + threadIdx.x;
+  stamp_time(t_ns);
   if (i >= n || stop.set()) return;
   const double tmp = hdw[i];
   if (tmp > 0.0) {
@@ -91,8 +92,9 @@ __global__ void __launch_bounds__(KIN_NT) k_kinstress(int n, const double* __res
                                                       const double* __restrict__ fx, const double* __restrict__ fy,
                                                       const double* __restrict__ fz, double* __restrict__ vx,
                                                       double* __restrict__ vy, double* __restrict__ vz, double* part,
-                                                      GridSum gs, StopIf stop) {
+                                                      GridSum gs, StopIf stop, unsigned long long* t_ns) {
   double a[6] = {0, 0, 0, 0, 0, 0};
+  stamp_time(t_ns);
   if (stop.set()) hdw = nullptr;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
     const double m = w[i];
@@ -122,8 +124,9 @@ __global__ void k_maxdisp(int n, const double* __restrict__ hdw, double tstep, c
                           double* __restrict__ vy, double* __restrict__ vz, double* __restrict__ x,
                           double* __restrict__ y, double* __restrict__ z, const double* __restrict__ xb,
                           const double* __restrict__ yb, const double* __restrict__ zb, double c0, double a0,
-                          unsigned long long* out, StopIf stop) {
+                          unsigned long long* out, StopIf stop, unsigned long long* t_ns) {
   double r2 = 0.0;
+  stamp_time(t_ns);
   if (stop.set()) hdw = nullptr;
   const long long quarter = __double_as_longlong(0.25 * c0);
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
@@ -1171,7 +1174,7 @@ void integ_forces_to_fp64() {
 static void launch_maxdisp(bool stage1) {
   k_maxdisp<<<std::min(nblocks(g.natms, 128), 4 * g.nsm), 128, 0, g.stream>>>(
       g.natms, stage1 ? g.hdw : nullptr, g.p.tstep, g.fx, g.fy, g.fz, g.vx, g.vy, g.vz, g.x, g.y, g.z, g.xbg, g.ybg,
-      g.zbg, g.cell[0], 1.0 / g.cell[0], (unsigned long long*)&g.sc->maxdisp, stop_if(ST_STOP1));
+      g.zbg, g.cell[0], 1.0 / g.cell[0], (unsigned long long*)&g.sc->maxdisp, stop_if(ST_STOP1), stamp_at(0));
   GB_LAUNCHED();
 }
 
@@ -1315,7 +1318,7 @@ static void launch_kinstress(bool kick) {
   const GridSum gs = gb_grid_sum(nb, KIN_NT, 6, &g.sc->acc[A_STRKIN]);
   double* part = gb_blkacc(nb * 6);
   k_kinstress<<<nb, KIN_NT, 0, g.stream>>>(g.natms, g.weight, g.lfrzn, kick ? g.hdw : nullptr, g.fx, g.fy, g.fz, g.vx,
-                                           g.vy, g.vz, part, gs, stop_if(ST_STOP2));
+                                           g.vy, g.vz, part, gs, stop_if(ST_STOP2), kick ? stamp_at(2) : nullptr);
   GB_LAUNCHED();
   gb_grid_sum_done(gs, part, nb, 6);
 }
@@ -1339,7 +1342,8 @@ void integ_vv(int stage, double* strkin, double* engke, int* iters, double* virc
     const bool fused = g.ntcons <= 0 && g.ens == GB_NVE;  // the kick and the kinetic stress in one pass
     prof_begin(P_VV);
     if (!fused) {
-      k_vv2<<<nblocks(n, 256), 256, 0, st>>>(n, g.hdw, g.fx, g.fy, g.fz, g.vx, g.vy, g.vz, stop_if(ST_STOP2));
+      k_vv2<<<nblocks(n, 256), 256, 0, st>>>(n, g.hdw, g.fx, g.fy, g.fz, g.vx, g.vy, g.vz, stop_if(ST_STOP2),
+                                             stamp_at(2));
       GB_LAUNCHED();
     }
     if (fused) launch_kinstress(true);

@@ -959,8 +959,9 @@ struct ForceZero {
 __global__ void k_pos_records(const DevScalars* sc, const int* __restrict__ sorted_pos, const double* __restrict__ x,
                               const double* __restrict__ y, const double* __restrict__ z, const double* __restrict__ q,
                               const int* __restrict__ ltype, double pos_scale, float4* xf, float4* xlo, float2* qdf,
-                              float4* xhs, PosRec* rec, uint2* xlh, ForceZero Z) {
+                              float4* xhs, PosRec* rec, uint2* xlh, ForceZero Z, unsigned long long* t_ns) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  stamp_time(t_ns);
   if (i < Z.natms) {
     if (Z.fx) { Z.fx[i] = 0.0; Z.fy[i] = 0.0; Z.fz[i] = 0.0; }
     if (Z.fixp) { Z.fixp[3 * i] = 0; Z.fixp[3 * i + 1] = 0; Z.fixp[3 * i + 2] = 0; }
@@ -1284,7 +1285,7 @@ void list_pos_records(bool sorted) {
                        sorted ? g.fixs : nullptr};
   k_pos_records<<<nblocks(g.mxatms, 256), 256, 0, g.stream>>>(
       g.sc, g.sorted_pos, g.x, g.y, g.z, g.chge, g.ltype, g.pos_scale, g.xf, g.xlo, f64 ? g.qdf : nullptr,
-      sorted ? g.xhs : nullptr, g.rec, f64 ? nullptr : g.xlh, Z);
+      sorted ? g.xhs : nullptr, g.rec, f64 ? nullptr : g.xlh, Z, stamp_at(1));
   GB_LAUNCHED();
 }
 

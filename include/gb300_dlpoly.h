@@ -308,9 +308,12 @@ int gb_set_precision(int precision);
 
 /* Device time (ms) of the last gb_md_run per region, CUDA events on the
  * library stream: [0] list+halo, [1] real-space, [2] SPME, [3] integrate,
- * [4] total.  Without learned MTS the total alone is taken ([0] to [3] are 0;
- * GB_MD_DEFER=0 in the environment at gb_init takes them all, with a wait per
- * step).  n = number of slots to copy. */
+ * [4] total.  In NVE without constraints, metals or learned MTS the total
+ * alone is taken ([0] to [3] are 0; GB_MD_DEFER=0 in the environment at
+ * gb_init takes them all, with a wait per step).  [1] holds SPME too (it runs
+ * beside the pair kernel; [2] is 0), and without learned MTS [3] is the rest of
+ * the total and the regions are read from the device's clock by the kernels at
+ * their ends.  n = number of slots to copy. */
 int gb_last_timings(double* ms, int n);
 
 /* Number of kernels the library launched since gb_init (its own count). */

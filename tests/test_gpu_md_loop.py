@@ -1,5 +1,7 @@
 """The MD loop that reads a step's sums after its last step, launched or replayed as CUDA graphs,
 against the loop that reads them at every step: constraints, thermostats and metals."""
+import ctypes
+
 import numpy as np
 import pytest
 
@@ -139,3 +141,29 @@ def test_failed_step_leaves_its_own_state(gpu_lib, monkeypatch, name, steps, gra
     assert [k == -1.0 for k in ka] == [k == -1.0 for k in kb] == [k >= good for k in range(n)]
     for k in ga:
         assert np.abs(ga[k] - gb[k]).max() <= 1e-12 * np.abs(ga[k]).max(), k
+
+
+@pytest.mark.parametrize("graphs", ["0", "1"])
+@pytest.mark.parametrize("name", ["water", "water_mixed_nose_hoover", "nacl_langevin", "eam", "nacl"])
+def test_region_timings_of_a_run(gpu_lib, monkeypatch, name, graphs):
+    """gb_last_timings: the regions of every run but plain NVE, which has the total alone."""
+    make, precision, ens, _ = RUNS.get(name, (lambda: systems.nacl_melt(16), 0, "nve", 0.0))
+    monkeypatch.setenv("GB_GRAPHS", graphs)
+    gpu_lib.init(make(), precision=precision)
+    monkeypatch.delenv("GB_GRAPHS")
+    if ens != "nve":
+        gpu_lib.set_ensemble(ens, temp=300.0, tau_t=0.05, chi=5.0)
+    gpu_lib.start()
+    read = gpu_lib._opt("last_timings", ctypes.c_int, [ctypes.POINTER(ctypes.c_double), ctypes.c_int])
+    for steps in (6, 3, 1):
+        gpu_lib.md_vv(steps)
+        t = (ctypes.c_double * 6)()
+        assert read(t, 6) == 0
+        listed, forces, spme, integ, total, span = t
+        assert 0.0 < total <= 1.02 * span and spme == 0.0
+        if name == "nacl":
+            assert listed == forces == integ == 0.0
+        else:
+            assert min(listed, forces, integ) > 0.0
+            assert listed + forces + integ == pytest.approx(total, rel=1e-6)
+            assert total >= 0.5 * span
