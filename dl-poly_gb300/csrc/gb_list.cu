@@ -58,6 +58,10 @@ __device__ __forceinline__ long long ordered(double v) {
   return b ^ ((b >> 63) & 0x7fffffffffffffffll);
 }
 
+__device__ __forceinline__ bool is_nan(double v) {
+  return (__double_as_longlong(v) & 0x7fffffffffffffffll) > 0x7ff0000000000000ll;
+}
+
 // relocate_particles (pbcshift, numerics.F90:1886-1930), set_halo_particles (halo.F90:153-356)
 // and vnl_set_check (neighbours.F90:305-343) in two launches.  The reference's images come
 // from six ordered exports (-x, +x, -y, +y, -z, +z), each a stable compaction of the atoms
@@ -116,10 +120,13 @@ __global__ void __launch_bounds__(HALO_NT) k_halo_count(HaloArgs A) {
                    z = wrap1(A.z[i], A.a[2], A.c[2], A.half_minus);
       A.x[i] = x; A.y[i] = y; A.z[i] = z;
       A.xb[i] = x; A.yb[i] = y; A.zb[i] = z;
-      const long long xx = ordered(red_coord(A.hg.rc, 0, x)), yy = ordered(red_coord(A.hg.rc, 1, y)),
-                      zz = ordered(red_coord(A.hg.rc, 2, z));
-      v = (xx <= lo_b[0] ? 1 : 0) | (xx >= hi_b[0] ? 2 : 0) | (yy <= lo_b[1] ? 4 : 0) | (yy >= hi_b[1] ? 8 : 0) |
-          (zz <= lo_b[2] ? 16 : 0) | (zz >= hi_b[2] ? 32 : 0);
+      const double red[3] = {red_coord(A.hg.rc, 0, x), red_coord(A.hg.rc, 1, y), red_coord(A.hg.rc, 2, z)};
+#pragma unroll
+      for (int d = 0; d < 3; ++d) {
+        const long long o = ordered(red[d]);
+        const int w = (o <= lo_b[d] ? 1 : 0) | (o >= hi_b[d] ? 2 : 0);
+        if (!is_nan(red[d])) v |= w << (2 * d);  // (a NaN compares false: not exported)
+      }
       A.code[i] = v;
       A.src[i] = i;
       A.shcode[i] = 13;
