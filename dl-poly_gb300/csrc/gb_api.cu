@@ -1098,13 +1098,14 @@ static void md_step_stats(const DevScalars* h, int32_t rebuilt, gb_step_stats& S
 // has left the state alone (StopIf), and the step counter goes back to the failing step.  Each
 // step's energy, virial and stress sums are
 // copied to a pinned ring with the step's other work and turned into gb_step_stats after
-// the last step.  With 3 or more steps the steps run as two CUDA graphs: stage 1 with the
+// the last step (of RING_STEPS at most, 4 MB: a longer run is taken in parts).  With 3 or more steps the steps run as two CUDA graphs: stage 1 with the
 // displacement check (its sums copied to the pinned scalars), then, after the host's
 // decision and the halo refresh or the list rebuild that it calls for, the forces (SPME
 // forked to the side stream) and stage 2; the second is captured again when a rebuild
 // changes the kernels that walk the list.  Langevin's stage 1 is launched (its noise is keyed
 // on the step).  In plain NVE the total is the only timing; the other systems' kernels at the
 // ends of the regions store the device's clock beside the sums.
+constexpr int RING_STEPS = 4096;
 static int md_run_deferred(int nsteps, gb_step_stats* stats) {
   if (g.ring_cap < nsteps) {
     if (g.ring) cudaFreeHost(g.ring);
@@ -1215,7 +1216,14 @@ int gb_md_run(int nsteps, gb_step_stats* stats) {
     if (nsteps < 0) return (int)GB_ERR_ARG;
     if (nsteps > 0 && g.use_deferred && !mts_active()) {
       try {
-        return md_run_deferred(nsteps, stats);
+        double ms[6] = {0, 0, 0, 0, 0, 0};
+        for (int s = 0; s < nsteps; s += RING_STEPS) {
+          const int code = md_run_deferred(std::min(RING_STEPS, nsteps - s), stats ? stats + s : nullptr);
+          if (code != GB_OK) return code;
+          for (int k = 0; k < 6; ++k) ms[k] += g.last_ms[k];
+        }
+        for (int k = 0; k < 6; ++k) g.last_ms[k] = ms[k];
+        return (int)GB_OK;
       } catch (int e) {
         g.defer_scalars = g.time_regions = false;
         throw;

@@ -167,3 +167,23 @@ def test_region_timings_of_a_run(gpu_lib, monkeypatch, name, graphs):
             assert min(listed, forces, integ) > 0.0
             assert listed + forces + integ == pytest.approx(total, rel=1e-6)
             assert total >= 0.5 * span
+
+
+def test_runs_longer_than_the_ring(gpu_lib, monkeypatch):
+    """4,100 steps in one call, of which the loop keeps 4,096 at a time: statistics and state of
+    every step as the loop that reads them at each step has them."""
+    out = []
+    for defer in ("0", "1"):
+        monkeypatch.setenv("GB_MD_DEFER", defer)
+        s = systems.lj_pair(eps=100.0, sigma=2.0, r=2.4)
+        gpu_lib.init(s)
+        gpu_lib.start()
+        out.append((gpu_lib.md_vv(4100), gpu_lib.download()))
+    monkeypatch.delenv("GB_MD_DEFER")
+    (sa, a), (sb, b) = out
+    for f in ("engke", "engvdw", "list_rebuilt"):
+        u, v = (np.array([getattr(x, f) for x in st]) for st in (sa, sb))
+        assert np.abs(u - v).max() <= 1e-12 * max(np.abs(u).max(), 1.0), f
+    assert sa[-1].engke != sa[0].engke
+    for k in a:
+        assert np.abs(a[k] - b[k]).max() <= 1e-12 * max(np.abs(a[k]).max(), 1.0), k
