@@ -760,7 +760,7 @@ int gb_init(const gb_params* prm, int natms, const int32_t* ltype, const double*
       g.use_mapped = !(m && m[0] == '0');
       const char* o = getenv("GB_OVERLAP");  // 0: SPME and the pair kernel on one stream
       g.use_overlap = !(o && o[0] == '0');
-      const char* gr = getenv("GB_GRAPHS");  // 0: the NVE loop's kernels launched one by one
+      const char* gr = getenv("GB_GRAPHS");  // 0: the MD loop's kernels launched one by one
       g.use_graphs = !(gr && gr[0] == '0');
       const char* t = getenv("GB_PAIR_NT");  // 256 / 1024: CTA size of the sorted pair kernels (else by form)
       g.pair_nt = t ? ((atoi(t) == 256) ? 256 : 1024) : 0;
@@ -1451,7 +1451,7 @@ const char* gb_strerror(int status) {
     case GB_ERR_RNG: return "a Gaussian deviate's rejection loop hit its iteration cap";
     case GB_ERR_DEVICE_WAIT: return "a tensor-core completion wait hit its iteration limit";
     case GB_ERR_MULTI_RANK: return "more than one MPI rank (comm%mxnode > 1): the device path runs one rank on one GPU";
-    case GB_ERR_TOO_LARGE: return "size exceeds the fixed scratch limit of gb_kinstress_noalloc (1,048,576 atoms)";
+    case GB_ERR_TOO_LARGE: return "more atoms than gb_kinstress_noalloc takes (1,048,576)";
     default: return "unknown status";
   }
 }

@@ -11,9 +11,11 @@
 // SHAKE and RATTLE are Jacobi iterations with one global convergence test per
 // sweep, exactly as the reference: a cooperative-grid kernel runs the sweeps
 // with grid-wide barriers, at most shake_maxit of them, and returns the
-// iteration count and a status bit instead of spinning.  Per-atom corrections
-// are summed in constraint order from a per-atom constraint table, and applied
-// listot(i) times, so positions round as the reference's do.
+// iteration count and a status bit instead of spinning.  k_shake and k_rattle sum
+// an atom's corrections in constraint order from a per-atom constraint table and apply
+// them listot(i) times, so positions round as the reference's do; k_constrain_cl adds a cluster's
+// in registers, and k_constrain_small (clusters of at most 3 constraints, but not in the FP64
+// form by instructions) sweeps one double-float scalar per constraint and moves the atoms once.
 #include <cooperative_groups.h>
 
 #include <algorithm>

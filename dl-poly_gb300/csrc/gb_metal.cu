@@ -361,8 +361,8 @@ __global__ void __launch_bounds__(256, 3) k_metal_forces(int natms, const DevSca
 // (1/64 of the FP32 rate): 95 FP64 instructions per 32 list entries, executed for whole
 // warps although a fifth of the entries lie beyond the cutoff.  Here an FP32 test of the
 // high parts queues the entries that may be inside, and 32 queued pairs at a time are
-// evaluated with every lane busy.  256,000 atoms: density 1.97 -> 0.45 ms, forces 4.35 ->
-// 0.89 ms (1.04 with 102 registers, two CTAs per SM; a fourth CTA spills and gains
+// evaluated with every lane busy.  256,000 atoms: density 1.97 -> 0.47 ms, forces 4.35 ->
+// 0.97 ms (1.04 with 102 registers, two CTAs per SM; a fourth CTA spills and gains
 // nothing); latency of the partners and tables, at a third of the issue slots.
 //   positions   fixed point (PosRec): the separation is an exact integer difference
 //   r           to 1.4e-15 (rms), and its fraction of a table interval from the r of the
